@@ -1,0 +1,538 @@
+"""What a user of this framework runs, as cases that can be timed and compared.
+
+The paths are those of the serving engines: decode passes and prompt passes of the dense NVFP4 decoder, decode of the bf16
+decoder, decode and prompt passes of the delta-rule hybrid, decode with latent attention, and the mixture-of-experts block at
+decode and at prompt sizes.  Shapes are those of `bench.py`; the depth is cut to 8 or 16 layers (all layers of a family are
+alike), weights are N(0, 0.02) in checkpoint layout, prompts are uniform random ids.  As in a deep model, a layer adds little
+to the residual stream: matrices that write to it are scaled by 1 / sqrt(2 * 64), and embeddings have unit size.
+
+Expert blocks are cases of their own: behind several layers, a router's choice hangs on the last bits of its input.
+"""
+from __future__ import annotations
+
+import math
+
+import torch
+
+from dgpp_b200.engine.llm_engine import LLMEngine
+from dgpp_b200.models.dense import DenseConfig, DenseLayer, DenseModel
+from dgpp_b200.models.gdn import GdnWeights
+from dgpp_b200.models.hybrid import HybridConfig, HybridLayer, HybridModel, HybridRunner
+from dgpp_b200.models.mla_moe import MlaLayer, MlaMoeConfig, MlaMoeModel, MlaMoeRunner, yarn_inv_freq
+from dgpp_b200.models.moe import MoEBlock, MoEConfig, MoEWeights
+from dgpp_b200.ops.reference import rope_inv_freq
+from dgpp_b200.quant.formats import QuantLinear
+
+STD = 0.02
+BRANCH = 1.0 / math.sqrt(2 * 64)   # of the matrices whose products are added to the residual stream
+EPS = 1e-6
+CHUNK = 2048                 # prompt tokens per pass, as `bench.py` has it
+ROOM = 4096                  # decode steps before a recurrent request starts over at its first position
+
+# one decoder shape per family (bench.py: the default run, its like-for-like extra, --config 4 and --config 2)
+DENSE = dict(layers=16, hidden=5120, q_heads=40, kv_heads=8, head_dim=128, ffn=17408, vocab=151936)
+BF16 = dict(layers=16, hidden=4096, q_heads=32, kv_heads=8, head_dim=128, ffn=17408, vocab=151936)
+HYBRID = dict(layers=16, hidden=2048, full_every=4, q_heads=16, kv_heads=2, head_dim=256, gdn_k_heads=16, gdn_v_heads=16,
+              gdn_dk=128, gdn_dv=128, ffn=5632, vocab=151936)      # as wide as 10 routed + 1 shared experts of 512
+LATENT = dict(layers=8, hidden=4096, heads=32, q_lora=1024, kv_lora=512, nope=128, rope=64, v_dim=128, ffn=12288,
+              dense_layers=8, vocab=129280)
+EXPERTS = {
+    "512": dict(hidden=2048, experts=512, top_k=10, moe_ffn=512, shared_ffn=512, router="softmax"),
+    "256": dict(hidden=4096, experts=256, top_k=8, moe_ffn=1536, shared_ffn=1536, n_group=8, topk_group=4, router="sigmoid",
+                routed_scaling=2.5),
+}
+
+
+def listed():
+    return [
+        # one user waiting for the next token: the smallest pass, bound by the weight stream and the launches' chain
+        {"name": "dense decode 1", "path": "dense decode", "requests": 1, "context": 2048},
+        # the headline of bench.py
+        {"name": "dense decode 8", "path": "dense decode", "requests": 8, "context": 2048},
+        # a busy server: many short conversations, an odd batch width
+        {"name": "dense decode 37", "path": "dense decode", "requests": 37, "context": 900},
+        # a question on top of a long shared prefix (prefix cache hit): few new tokens, ragged
+        {"name": "dense prompt 173", "path": "dense prompt", "tokens": 173, "prefix": 3000},
+        # cold prompts of the headline's lengths
+        {"name": "dense prompt 2048", "path": "dense prompt", "tokens": 2048, "prefix": 0},
+        {"name": "dense prompt 8192", "path": "dense prompt", "tokens": 8192, "prefix": 0},
+        # unquantised weights, one short conversation: the like-for-like extra of bench.py
+        {"name": "bf16 decode 1", "path": "bf16 decode", "requests": 1, "context": 64},
+        # the recurrent hybrid serving a few users, and taking in a prompt of no round length
+        {"name": "hybrid decode 8", "path": "hybrid decode", "requests": 8, "context": 2048},
+        {"name": "hybrid prompt 3001", "path": "hybrid prompt", "tokens": 3001, "prefix": 0},
+        # latent attention at the context of a longer document
+        {"name": "latent decode 8", "path": "latent decode", "requests": 8, "context": 4096},
+        # one layer's experts: a decode batch over many small experts, a prompt chunk over fewer large ones
+        {"name": "experts 8 rows", "path": "experts", "rows": 8, "shape": "512"},
+        {"name": "experts 2048 rows", "path": "experts", "rows": 2048, "shape": "256"},
+    ]
+
+
+def _log(rng, lo, hi):
+    return max(lo, min(hi, int(round(math.exp(rng.uniform(math.log(lo), math.log(hi)))))))
+
+
+def draw(rng):
+    path = rng.choice(["dense decode", "dense decode", "dense prompt", "dense prompt", "bf16 decode", "hybrid decode",
+                       "hybrid prompt", "latent decode", "experts", "experts"])
+    if path == "dense decode":
+        c = _log(rng, 1, 64)
+        return {"path": path, "requests": c, "context": _log(rng, 64, min(8192, 32768 // c))}
+    if path == "bf16 decode":
+        return {"path": path, "requests": _log(rng, 1, 8), "context": _log(rng, 32, 2048)}
+    if path == "dense prompt":
+        t = _log(rng, 16, 8000)
+        return {"path": path, "tokens": t, "prefix": rng.choice([0, rng.randrange(1, 8192 - t + 1)])}
+    if path == "hybrid decode":
+        c = _log(rng, 1, 32)
+        return {"path": path, "requests": c, "context": _log(rng, 64, min(4096, 16384 // c))}
+    if path == "hybrid prompt":
+        return {"path": path, "tokens": _log(rng, 32, 6000), "prefix": rng.choice([0, 1024])}
+    if path == "latent decode":
+        c = _log(rng, 1, 16)
+        return {"path": path, "requests": c, "context": _log(rng, 128, min(8192, 32768 // c))}
+    return {"path": path, "rows": _log(rng, 1, 4096), "shape": rng.choice(["512", "256"])}
+
+
+# ------------------------------------------------------------------------------------------------ weights and prompts
+def _nvfp4(w):
+    """fp32 [n, k] -> (packed e2m1 codes, e4m3 scales per 16, tensor scale), the checkpoint layout."""
+    n, k = w.shape
+    alpha = 5.5 * float(STD) / (6.0 * 448.0)
+    blk = w.view(n, k // 16, 16)
+    sf = (blk.abs().amax(-1) / (6.0 * alpha)).clamp(max=448.0).to(torch.float8_e4m3fn)
+    v = blk / (sf.float().clamp_min(2.0 ** -9) * alpha).unsqueeze(-1)
+    edges = torch.tensor([0.25, 0.75, 1.25, 1.75, 2.5, 3.5, 5.0], device=w.device)
+    code = torch.bucketize(v.abs(), edges, out_int32=True).to(torch.uint8)
+    code |= (v < 0).to(torch.uint8) << 3
+    code = code.view(n, k // 2, 2)
+    return code[..., 0] | (code[..., 1] << 4), sf.view(torch.uint8), alpha
+
+
+class _Source:
+    """The weights of one model, in the order in which they are asked for."""
+
+    def __init__(self, seed, fmt="nvfp4"):
+        self.gen = torch.Generator(device="cuda")
+        self.gen.manual_seed(seed)
+        self.fmt = fmt
+
+    def normal(self, *shape, std=STD):
+        return torch.randn(*shape, device="cuda", generator=self.gen) * std
+
+    def uniform(self, *shape):
+        return torch.rand(*shape, device="cuda", generator=self.gen)
+
+    def bf16(self, *shape, std=STD):
+        return self.normal(*shape, std=std).to(torch.bfloat16)
+
+    def matrix(self, n, k, fmt=None, gain=1.0):
+        w = self.normal(n, k)
+        if (fmt or self.fmt) == "bf16":
+            return QuantLinear("bf16", n, k, (w * gain).to(torch.bfloat16))
+        q, sf, alpha = _nvfp4(w)
+        return QuantLinear("nvfp4", n, k, q, sf, alpha * gain)
+
+
+def _prompts(case, seed, vocab):
+    """Token ids per request: the context of each (shorter from one request to the next, as users differ), and two more."""
+    gen = torch.Generator().manual_seed(seed + 77)
+    if "tokens" in case:
+        lens = [case["prefix"] + case["tokens"]]
+    else:
+        lens = [max(1, case["context"] - (i * case["context"]) // (2 * case["requests"])) + 2 for i in range(case["requests"])]
+    return [torch.randint(0, vocab, (n,), generator=gen).tolist() for n in lens]
+
+
+def _ones(n):
+    return torch.ones(n, dtype=torch.bfloat16, device="cuda")
+
+
+def _dense_model(seed, shape, fmt):
+    c = DenseConfig(weight_fmt=fmt, **shape)
+    s = _Source(seed, fmt)
+    d = c.head_dim
+    embed = s.bf16(c.vocab, c.hidden, std=1.0)
+    layers = [DenseLayer(_ones(c.hidden), _ones(c.hidden), s.matrix((c.q_heads + 2 * c.kv_heads) * d, c.hidden),
+                         s.matrix(c.hidden, c.q_heads * d, gain=BRANCH), s.matrix(2 * c.ffn, c.hidden),
+                         s.matrix(c.hidden, c.ffn, gain=BRANCH))
+              for _ in range(c.layers)]
+    inv, _ = rope_inv_freq(d, c.rope_theta, "cuda")
+    return DenseModel(c, embed, layers, _ones(c.hidden), s.matrix(c.vocab, c.hidden, "bf16"), inv_freq=inv.contiguous())
+
+
+def _hybrid_model(seed):
+    c = HybridConfig(**HYBRID)
+    s = _Source(seed)
+    g, d = c.gdn_cfg(), c.head_dim
+    embed = s.bf16(c.vocab, c.hidden, std=1.0)
+    layers = []
+    for i in range(c.layers):
+        L = HybridLayer(_ones(c.hidden), _ones(c.hidden))
+        if c.is_full(i):
+            L.qkv, L.o = s.matrix((c.q_heads + 2 * c.kv_heads) * d, c.hidden), s.matrix(c.hidden, c.q_heads * d, gain=BRANCH)
+        else:
+            L.gdn = GdnWeights(g, s.matrix(g.proj_cols, c.hidden, gain=4.0), s.bf16(g.conv_channels, g.conv_width, std=0.5), None,
+                               torch.log(s.uniform(g.v_heads) * 4 + 0.5), s.normal(g.v_heads, std=0.5),
+                               (1 + s.normal(g.dv, std=0.1)).to(torch.bfloat16), s.matrix(c.hidden, g.v_heads * g.dv, gain=BRANCH))
+        L.gate_up, L.down = s.matrix(2 * c.ffn, c.hidden), s.matrix(c.hidden, c.ffn, gain=BRANCH)
+        layers.append(L)
+    inv, _ = rope_inv_freq(d, c.rope_theta, "cuda")
+    return HybridModel(c, embed, layers, _ones(c.hidden), s.matrix(c.vocab, c.hidden, "bf16"), inv)
+
+
+def _latent_model(seed):
+    c = MlaMoeConfig(**LATENT)
+    s = _Source(seed)
+    embed = s.bf16(c.vocab, c.hidden, std=1.0)
+    layers = []
+    for _ in range(c.layers):
+        layers.append(MlaLayer(_ones(c.hidden), _ones(c.hidden), s.matrix(c.q_lora, c.hidden), _ones(c.q_lora),
+                               s.matrix(c.heads * (c.nope + c.rope), c.q_lora), s.matrix(c.kv_lora + c.rope, c.hidden),
+                               _ones(c.kv_lora), s.bf16(c.heads, c.nope, c.kv_lora, std=2 * STD),
+                               s.bf16(c.heads, c.v_dim, c.kv_lora, std=2 * STD),
+                               s.matrix(c.hidden, c.heads * c.v_dim, gain=BRANCH), s.matrix(2 * c.ffn, c.hidden),
+                               s.matrix(c.hidden, c.ffn, gain=BRANCH)))
+    inv = yarn_inv_freq(c.rope, c.rope_theta, 1.0, c.yarn_orig_ctx, device="cuda")
+    return MlaMoeModel(c, embed, layers, _ones(c.hidden), s.matrix(c.vocab, c.hidden, "bf16"), inv)
+
+
+def _expert_weights(seed, shape):
+    """The router, its selection bias, and all experts' matrices (the shared one last) as two stacks."""
+    c = MoEConfig(**EXPERTS[shape])
+    s = _Source(seed)
+    gate, bias = s.bf16(c.experts, c.hidden, std=4 * STD), s.normal(c.experts, std=0.05)
+    n = c.experts + 1
+    return c, gate, bias, s.matrix(n * 2 * c.moe_ffn, c.hidden), s.matrix(n * c.hidden, c.moe_ffn)
+
+
+def _rows_in(seed, rows, hidden):
+    """Normed rows: unit mean square, as the block's norm leaves them."""
+    s = _Source(seed + 5)
+    x = s.normal(rows, hidden, std=1.0)
+    return (x * torch.rsqrt(x.square().mean(-1, keepdim=True) + EPS)).to(torch.bfloat16)
+
+
+def prepare(case, seed):
+    path = case["path"]
+    if path == "experts":
+        c, gate, bias, gu, down = _expert_weights(seed, case["shape"])
+        part = lambda w, n: [QuantLinear("nvfp4", n, w.k, w.payload[i:i + n], w.scale[i:i + n], w.alpha)
+                             for i in range(0, w.n, n)]
+        gus, downs = part(gu, 2 * c.moe_ffn), part(down, c.hidden)
+        w = MoEWeights(c, gate, bias, gus[:-1], downs[:-1], gus[-1], downs[-1], e_end=c.experts)
+        w.stack()
+        rows = case["rows"]
+        xn = _rows_in(seed, rows, c.hidden)
+        return {"path": path, "block": MoEBlock(w, min(rows, 16), "cuda"), "xn": xn, "out": torch.empty_like(xn)}
+    if path in ("dense decode", "dense prompt", "bf16 decode"):
+        model = _dense_model(seed, BF16 if path == "bf16 decode" else DENSE, "bf16" if path == "bf16 decode" else "nvfp4")
+        ids = _prompts(case, seed, model.cfg.vocab)
+        eng = LLMEngine(model, max_batch=len(ids), max_seq_len=max(len(p) for p in ids) + 16, prefill_chunk=CHUNK)
+        if path == "dense prompt":
+            p = case["prefix"]
+            if p:
+                eng.prefill(0, ids[0][:p])
+            return {"path": path, "eng": eng, "ids": ids[0][p:], "prefix": p, "last": (case["tokens"] - 1) % CHUNK + 1}
+        for s, p in enumerate(ids):
+            eng.prefill(s, p[:-1])
+        s = {"path": path, "eng": eng, "next": torch.tensor([p[-1] for p in ids], dtype=torch.int32, device="cuda"),
+             "slots": list(range(len(ids)))}
+        run(s)                                       # the pass is captured once and kept
+        return s
+    model = _latent_model(seed) if path == "latent decode" else _hybrid_model(seed)
+    ids = _prompts(case, seed, model.cfg.vocab)
+    make = MlaMoeRunner if path == "latent decode" else HybridRunner
+    runner = make(model, max_rows=CHUNK, slots=len(ids), max_seq_len=max(len(p) for p in ids) + ROOM + 64, device="cuda")
+    if path == "hybrid prompt":
+        p = case["prefix"]
+        return {"path": path, "runner": runner, "before": ids[0][:p], "ids": ids[0][p:], "last": (case["tokens"] - 1) % CHUNK + 1}
+    for s, p in enumerate(ids):
+        runner.prefill(s, p[:-2], chunk=CHUNK)
+    slots = list(range(len(ids)))
+    runner.decode(slots, [p[-2] for p in ids])       # the pass is captured once and kept
+    return {"path": path, "runner": runner, "slots": slots, "next": [p[-1] for p in ids], "at": list(runner.lengths)}
+
+
+def run(state):
+    path = state["path"]
+    if path == "experts":
+        if state["xn"].shape[0] <= state["block"].max_rows:
+            return state["block"].forward(state["xn"], state["out"])
+        return state["block"].forward_gathered(state["xn"])
+    if path in ("dense decode", "bf16 decode"):
+        eng, slots = state["eng"], state["slots"]
+        eng.start_decode(slots, state["next"])
+        eng.decode_step(len(slots))
+        return eng.runner.logits[:len(slots)]
+    if path == "dense prompt":
+        eng = state["eng"]
+        eng.prefill(0, state["ids"], start_pos=state["prefix"])
+        return {"logits": eng.runner.logits[:1], "hidden": eng.runner.xn[:state["last"]]}
+    runner = state["runner"]
+    if path == "hybrid prompt":
+        runner.reset(0)
+        if state["before"]:
+            runner.prefill(0, state["before"], chunk=CHUNK)
+        logits = runner.prefill(0, state["ids"], chunk=CHUNK)
+        return {"logits": logits, "hidden": runner.xn[:state["last"]], "memory": runner.ssm_pool}
+    if runner.lengths[0] >= state["at"][0] + ROOM:   # the requests start over
+        runner.lengths[:] = state["at"]
+    logits = runner.decode(state["slots"], state["next"])
+    if path == "latent decode":
+        return logits[:len(state["slots"])]
+    return {"logits": logits[:len(state["slots"])], "memory": runner.ssm_pool}
+
+
+# ------------------------------------------------------------------------------------------------ what a pass needs
+FP4 = 0.5 + 1.0 / 16                                  # bytes of one weight
+
+
+def _contexts(case):
+    return [len(p) for p in _prompts(case, 0, 2)]
+
+
+def work(case):
+    path = case["path"]
+    if path == "experts":
+        c, rows = MoEConfig(**EXPERTS[case["shape"]]), case["rows"]
+        used = c.experts * (1 - (1 - c.top_k / c.experts) ** rows) + 1
+        one = 3 * c.hidden * c.moe_ffn
+        return {"bytes": used * one * FP4 + c.experts * c.hidden * 2 + 4 * rows * c.hidden,
+                "flops": 2.0 * rows * ((c.top_k + 1) * one + c.experts * c.hidden)}
+    decode = path.endswith("decode")
+    if decode:
+        spans = _contexts(case)
+        rows = len(spans)
+    else:
+        rows = case["tokens"] + (case["prefix"] if path == "hybrid prompt" else 0)
+        first = 0 if path == "hybrid prompt" else case["prefix"]
+        spans = [first + rows]
+    out_rows = rows if decode else 1
+    if path == "latent decode":
+        c = LATENT
+        per = c["hidden"] * c["q_lora"] + c["q_lora"] * c["heads"] * (c["nope"] + c["rope"]) + c["hidden"] * (c["kv_lora"] + c["rope"])
+        per += c["hidden"] * c["heads"] * c["v_dim"] + 3 * c["hidden"] * c["ffn"]
+        up = c["heads"] * (c["nope"] + c["v_dim"]) * c["kv_lora"]
+        weights = c["layers"] * (per * FP4 + up * 2)
+        macs = c["layers"] * (per + up)
+        cached = c["layers"] * (c["kv_lora"] + c["rope"]) * 2
+        att = c["layers"] * c["heads"] * (2 * c["kv_lora"] + c["rope"])
+        state = 0.0
+    elif path.startswith("hybrid"):
+        c = HYBRID
+        full = c["layers"] // c["full_every"]
+        lin = c["layers"] - full
+        nv = c["gdn_v_heads"] * c["gdn_dv"]
+        chan = 2 * c["gdn_k_heads"] * c["gdn_dk"] + nv
+        per_full = c["hidden"] * c["head_dim"] * (2 * c["q_heads"] + 2 * c["kv_heads"])
+        per_lin = c["hidden"] * (chan + 2 * nv + 2 * c["gdn_v_heads"])
+        macs = full * per_full + lin * per_lin + c["layers"] * 3 * c["hidden"] * c["ffn"]
+        weights = macs * FP4
+        cached = full * 2 * c["kv_heads"] * (c["head_dim"] + 4)
+        att = full * 2 * c["q_heads"] * c["head_dim"]
+        state = lin * nv * c["gdn_dk"] * 4.0
+        macs += lin * 3 * nv * c["gdn_dk"]
+    else:
+        c = BF16 if path == "bf16 decode" else DENSE
+        macs = c["layers"] * (c["hidden"] * c["head_dim"] * (2 * c["q_heads"] + 2 * c["kv_heads"]) + 3 * c["hidden"] * c["ffn"])
+        weights = macs * (2 if path == "bf16 decode" else FP4)
+        cached = c["layers"] * 2 * c["kv_heads"] * (c["head_dim"] + 4)
+        att = c["layers"] * 2 * c["q_heads"] * c["head_dim"]
+        state = 0.0
+    pairs = sum(spans) if decode else rows * (spans[0] - (rows - 1) / 2)      # (query, key) pairs of one head
+    bytes_ = weights + c["vocab"] * c["hidden"] * 2 + sum(spans) * cached + rows * c["hidden"] * 2 + out_rows * c["vocab"] * 4
+    bytes_ += (2 if decode else 1) * state * (out_rows if decode else 1) + (0 if decode else rows * c["hidden"] * 2)
+    return {"bytes": float(bytes_), "flops": 2.0 * (rows * macs + pairs * att + out_rows * c["vocab"] * c["hidden"])}
+
+
+def tolerance(case):
+    """Two correct passes at this precision differ as each differs from `exact`: bf16 streams over many layers and an FP8
+    cache (1.2e-2 to 2.2e-2 measured), or one block of bf16 products (4.4e-3 measured)."""
+    return {"rel": 0.015, "max": 0.3} if case["path"] == "experts" else {"rel": 0.03, "max": 0.5}
+
+
+# ------------------------------------------------------------------------------------------------ the same in 64 bits
+def _dequant(w):
+    if w.fmt == "bf16":
+        return w.payload.double()
+    level = torch.tensor([0, 0.5, 1, 1.5, 2, 3, 4, 6, 0, -0.5, -1, -1.5, -2, -3, -4, -6], dtype=torch.float64, device="cuda")
+    v = torch.stack((level[(w.payload & 15).int()], level[(w.payload >> 4).int()]), -1).view(w.n, w.k // 16, 16)
+    v *= (w.scale.view(torch.float8_e4m3fn).double() * w.alpha).view(w.n, w.k // 16, 1)
+    return v.view(w.n, w.k)
+
+
+def _times(x, w):
+    """x times the transposed matrix, a slice of its rows at a time."""
+    step = max(1, (1 << 28) // w.k)
+    cut = lambda t, i: t[i:i + step]
+    parts = []
+    for i in range(0, w.n, step):
+        n = min(step, w.n - i)
+        parts.append(x @ _dequant(QuantLinear(w.fmt, n, w.k, cut(w.payload, i), None if w.scale is None else cut(w.scale, i), w.alpha)).t())
+    return torch.cat(parts, -1)
+
+
+def _norm64(x):
+    return x * torch.rsqrt(x.square().mean(-1, keepdim=True) + EPS)
+
+
+def _rotate(x, pos, inv):
+    """x [T, ..., d]: the first half of the last axis against the second."""
+    a = pos.double().unsqueeze(-1) * inv.double()
+    a = a.view(a.shape[0], *([1] * (x.dim() - 2)), a.shape[1])
+    u, v = x.chunk(2, -1)
+    return torch.cat([u * a.cos() - v * a.sin(), v * a.cos() + u * a.sin()], -1)
+
+
+def _through_fp8(x):
+    s = x.abs().amax(-1, keepdim=True) / 448.0
+    s = torch.where(s > 0, s, torch.ones_like(s))
+    return (x / s).float().to(torch.float8_e4m3fn).double() * s
+
+
+def _attend(q, k, v, scale):
+    """Causal attention of one request, q [T, h, d], k and v [T, h or fewer, d], some query rows at a time."""
+    T, h, _ = q.shape
+    group = h // k.shape[1]
+    out = []
+    step = max(1, (1 << 27) // (h * T))
+    kt, vt = k.permute(1, 2, 0), v.transpose(0, 1)                           # [hk, d, T], [hk, T, dv]
+    pos = torch.arange(T, device=q.device)
+    for i in range(0, T, step):
+        qi = q[i:i + step]
+        n = qi.shape[0]
+        qg = qi.view(n, k.shape[1], group, -1).permute(1, 2, 0, 3).reshape(k.shape[1], group * n, -1)
+        s = torch.bmm(qg, kt).view(k.shape[1], group, n, T) * scale
+        s.masked_fill_(pos[None, None, None, :] > pos[i:i + n][None, None, :, None], float("-inf"))
+        p = torch.softmax(s, -1).view(k.shape[1], group * n, T)
+        o = torch.bmm(p, vt).view(k.shape[1], group, n, -1)
+        out.append(o.permute(2, 0, 1, 3).reshape(n, -1))
+    return torch.cat(out)
+
+
+def _grouped_attention(c, inv, L, xn, cuts):
+    d, hq, hk = c.head_dim, c.q_heads, c.kv_heads
+    qkv = _times(xn, L.qkv)
+    out = []
+    for a, b in cuts:
+        pos = torch.arange(b - a, device="cuda")
+        q, k, v = qkv[a:b].split([hq * d, hk * d, hk * d], -1)
+        q, k = _rotate(q.reshape(-1, hq, d), pos, inv), _rotate(k.reshape(-1, hk, d), pos, inv)
+        out.append(_attend(q, _through_fp8(k), _through_fp8(v.reshape(-1, hk, d)), d ** -0.5))
+    return _times(torch.cat(out), L.o)
+
+
+def _latent_attention(c, inv, L, xn, cuts):
+    q = _times(_norm64(_times(xn, L.q_a)), L.q_b).view(-1, c.heads, c.nope + c.rope)
+    kv = _times(xn, L.kv_a)
+    out = []
+    for a, b in cuts:
+        pos = torch.arange(b - a, device="cuda")
+        lat = _norm64(kv[a:b, :c.kv_lora])
+        kr = _rotate(kv[a:b, c.kv_lora:], pos, inv)
+        qn, qr = q[a:b, :, :c.nope], _rotate(q[a:b, :, c.nope:], pos, inv)
+        k = torch.cat([torch.einsum("hnd,td->thn", L.w_uk.double(), lat), kr.unsqueeze(1).expand(-1, c.heads, -1)], -1)
+        v = torch.einsum("hvd,td->thv", L.w_uv.double(), lat)
+        out.append(_attend(torch.cat([qn, qr], -1), k, v, (c.nope + c.rope) ** -0.5))
+    return _times(torch.cat(out), L.o)
+
+
+def _delta_rule(c, w, xn, cuts, memory):
+    proj = _times(xn, w.in_proj)
+    nq, nv, ch = c.k_heads * c.dk, c.v_heads * c.dv, c.conv_channels
+    out = []
+    silu = torch.nn.functional.silu
+    for slot, (a, b) in enumerate(cuts):
+        p = proj[a:b]
+        T = b - a
+        past = torch.cat([p.new_zeros(c.conv_width - 1, ch), p[:, :ch]])
+        mixed = silu(sum(past[i:i + T] * w.conv_w[:, i].double() for i in range(c.conv_width)))
+        q, k, v = mixed[:, :nq].view(T, -1, c.dk), mixed[:, nq:2 * nq].view(T, -1, c.dk), mixed[:, 2 * nq:].view(T, -1, c.dv)
+        rep = c.v_heads // c.k_heads
+        q = (q * torch.rsqrt(q.square().sum(-1, keepdim=True) + 1e-6) * c.dk ** -0.5).repeat_interleave(rep, 1)
+        k = (k * torch.rsqrt(k.square().sum(-1, keepdim=True) + 1e-6)).repeat_interleave(rep, 1)
+        al, be = p[:, ch + nv:ch + nv + c.v_heads], p[:, ch + nv + c.v_heads:]
+        decay = torch.exp(-w.A_log.double().exp() * torch.nn.functional.softplus(al + w.dt_bias.double()))
+        beta = torch.sigmoid(be)
+        S = memory[slot]                                                     # [heads, dk, dv]
+        o = torch.empty(T, c.v_heads, c.dv, dtype=torch.float64, device="cuda")
+        for t in range(T):
+            S.mul_(decay[t].view(-1, 1, 1))
+            u = beta[t].view(-1, 1, 1) * (v[t].unsqueeze(1) - torch.bmm(k[t].unsqueeze(1), S))
+            S.baddbmm_(k[t].unsqueeze(2), u)
+            torch.bmm(q[t].unsqueeze(1), S, out=o[t].unsqueeze(1))
+        z = p[:, ch:ch + nv].view(T, c.v_heads, c.dv)
+        out.append((_norm64(o) * w.norm_w.double() * silu(z)).view(T, nv))
+    return _times(torch.cat(out), w.out_proj)
+
+
+def _ffn64(xn, gate_up, down):
+    g, u = _times(xn, gate_up).chunk(2, -1)
+    return _times(torch.nn.functional.silu(g) * u, down)
+
+
+@torch.no_grad()
+def exact(case, seed):
+    path = case["path"]
+    if path == "experts":
+        c, gate, bias, gu, down = _expert_weights(seed, case["shape"])
+        x = _rows_in(seed, case["rows"], c.hidden).double()
+        logits = x @ gate.double().t()
+        scores = torch.softmax(logits, -1) if c.router == "softmax" else torch.sigmoid(logits)
+        pick = scores + bias.double()
+        if c.n_group > 1:
+            g = pick.view(len(x), c.n_group, -1)
+            best = g.topk(2, -1).values.sum(-1).topk(c.topk_group, -1).indices
+            keep = torch.zeros(g.shape[:2], dtype=torch.bool, device="cuda").scatter_(1, best, True)
+            pick = g.masked_fill(~keep.unsqueeze(-1), float("-inf")).view(len(x), -1)
+        ids = pick.topk(c.top_k, -1).indices
+        wts = scores.gather(1, ids)
+        wts = wts / (wts.sum(-1, keepdim=True) + 1e-20) * c.routed_scaling
+        part = lambda w, n, e: QuantLinear("nvfp4", n, w.k, w.payload[e * n:(e + 1) * n], w.scale[e * n:(e + 1) * n], w.alpha)
+        out = _ffn64(x, part(gu, 2 * c.moe_ffn, c.experts), part(down, c.hidden, c.experts))
+        for e in ids.unique().tolist():
+            row, at = (ids == e).nonzero(as_tuple=True)
+            y = _ffn64(x[row], part(gu, 2 * c.moe_ffn, e), part(down, c.hidden, e))
+            out.index_add_(0, row, y * wts[row, at].unsqueeze(-1))
+        return out
+    if path.startswith("hybrid"):
+        model, mix = _hybrid_model(seed), None
+    elif path == "latent decode":
+        model, mix = _latent_model(seed), _latent_attention
+    else:
+        model = _dense_model(seed, BF16 if path == "bf16 decode" else DENSE, "bf16" if path == "bf16 decode" else "nvfp4")
+        mix = _grouped_attention
+    c = model.cfg
+    ids = _prompts(case, seed, c.vocab)
+    cuts, n = [], 0
+    for p in ids:
+        cuts.append((n, n + len(p)))
+        n += len(p)
+    x = model.embed[torch.tensor(sum(ids, []), device="cuda")].double()
+    memory = []
+    for L in model.layers:
+        xn = _norm64(x)
+        if mix is not None:
+            x = x + mix(c, model.inv_freq, L, xn, cuts)
+        elif L.gdn is None:
+            x = x + _grouped_attention(c, model.inv_freq, L, xn, cuts)
+        else:
+            g = c.gdn_cfg()
+            memory.append(torch.zeros(len(ids), g.v_heads, g.dk, g.dv, dtype=torch.float64, device="cuda"))
+            x = x + _delta_rule(g, L.gdn, xn, cuts, memory[-1])
+        step = 4096
+        x = torch.cat([x[i:i + step] + _ffn64(_norm64(x[i:i + step]), L.gate_up, L.down) for i in range(0, n, step)])
+    xn = _norm64(x)
+    last = xn[torch.tensor([b - 1 for _, b in cuts], device="cuda")]
+    logits = _times(last, model.head)
+    if path.endswith("prompt"):
+        out = {"logits": logits, "hidden": xn[n - ((case["tokens"] - 1) % CHUNK + 1):]}
+    elif path == "hybrid decode":
+        out = {"logits": logits}
+    else:
+        return logits
+    if path.startswith("hybrid"):
+        out["memory"] = torch.stack(memory)
+    return out
