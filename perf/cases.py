@@ -236,6 +236,7 @@ def prepare(case, seed):
                 eng.prefill(0, ids[0][:p])
             return {"path": path, "eng": eng, "ids": ids[0][p:], "prefix": p, "last": (case["tokens"] - 1) % CHUNK + 1}
         for s, p in enumerate(ids):
+            assert eng.kv.reserve(s, len(p))         # room for the token to come, as admission sees to
             eng.prefill(s, p[:-1])
         s = {"path": path, "eng": eng, "next": torch.tensor([p[-1] for p in ids], dtype=torch.int32, device="cuda"),
              "slots": list(range(len(ids)))}
