@@ -99,10 +99,13 @@ rmsnorm_kernel(const bf16* __restrict__ resid, const bf16* __restrict__ delta, c
 
 // gate_up: [rows, 2*inter] (gate then up); out: [rows, inter].  limit > 0 clamps gate above and up both sides.
 // alpha > 0 selects the scaled-sigmoid form  gate * sigmoid(alpha * gate) * (up + 1)  (alpha = 0: silu(gate) * up).
+// tiles (optional, one entry per bn rows): rows of tiles with a negative entry are skipped.
 __global__ void __launch_bounds__(kRowThreads)
-swiglu_kernel(const bf16* __restrict__ gate_up, bf16* __restrict__ out, int inter, float limit, float alpha) {
+swiglu_kernel(const bf16* __restrict__ gate_up, bf16* __restrict__ out, int inter, float limit, float alpha,
+              const int32_t* __restrict__ tiles, int bn) {
   pdl_wait();
-  const size_t row = blockIdx.y;
+  const size_t row = blockIdx.y + static_cast<size_t>(blockIdx.z) * gridDim.y;
+  if (tiles != nullptr && tiles[row / bn] < 0) return;
   const bf16* g = gate_up + row * 2 * inter;
   const bf16* u = g + inter;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -336,7 +339,20 @@ DGPP_API int dgpp_swiglu(const void* gate_up, void* out, int rows, int inter, fl
   if (rows == 0) return 0;
   dim3 grid(dgpp_ceil_div(inter / 8, kRowThreads), rows);
   swiglu_kernel<<<grid, kRowThreads, 0, st>>>(static_cast<const bf16*>(gate_up), static_cast<bf16*>(out), inter,
-                                             limit, alpha);
+                                             limit, alpha, nullptr, 1);
+  DGPP_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+// The same over `n_tiles` tiles of bn rows; tiles with a negative entry are skipped.
+DGPP_API int dgpp_swiglu_tiles(const void* gate_up, void* out, const void* tiles, int n_tiles, int bn, int inter, float limit,
+                               float alpha, cudaStream_t st) {
+  DGPP_REQUIRE(inter % 8 == 0, "swiglu: inter %d must be a multiple of 8", inter);
+  DGPP_REQUIRE(tiles != nullptr && bn >= 1 && n_tiles <= 65535, "swiglu: bad tile list");
+  if (n_tiles <= 0) return 0;
+  dim3 grid(dgpp_ceil_div(inter / 8, kRowThreads), bn, n_tiles);
+  swiglu_kernel<<<grid, kRowThreads, 0, st>>>(static_cast<const bf16*>(gate_up), static_cast<bf16*>(out), inter, limit, alpha,
+                                             static_cast<const int32_t*>(tiles), bn);
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -1,24 +1,33 @@
 // W4A16 prefill GEMM on CTA pairs: out[T, N] = alpha * x[T, K] . W[N, K]^T (+ residual), 4-bit weights (NVFP4 with
-// e4m3 scales per 16, or MXFP4 with e8m0 scales per 32) expanded to bf16 in shared memory, bf16 activations, fp32
-// accumulation in TMEM.  Same arithmetic as the single-CTA kernel of gemm_tc.cu (bit-identical results: same
-// converted operands, same K order), different tiling:
+// e4m3 scales per 16, or MXFP4 with e8m0 scales per 32) expanded to bf16 on the way into TENSOR MEMORY, bf16
+// activations, fp32 accumulation in TMEM.  Same arithmetic as the single-CTA kernel of gemm_tc.cu (bit-identical
+// results without split-K: same converted operands, same K order), different tiling:
 //
-//   two CTAs of a cluster (one TPC) own 256 weight rows x 256 tokens.  Each CTA streams and converts ITS 128 weight
-//   rows and loads ITS 128 tokens of the activation tile; one `tcgen05.mma.cta_group::2` per K = 16 step, issued by
-//   the first CTA, multiplies all 256 rows by all 256 tokens, each SM reading the other's half of the activation tile
-//   out of its shared memory.  Per K = 64 block an SM therefore moves 16 KB of activations from L2 instead of 32 KB,
-//   which is what bounds the single-CTA kernel at prefill sizes (a 128 x 256 tile reuses the bf16 activation tile too
-//   little).  No TMA multicast: every CTA issues plain loads into its own shared memory onto its own barriers.
+//   two CTAs of a cluster (one TPC) own 256 weight rows x bn tokens (bn <= 256).  Each CTA streams and converts ITS 128
+//   weight rows and loads ITS half of the tokens; one `tcgen05.mma.cta_group::2` per K = 16 step, issued by the first
+//   CTA, multiplies all 256 rows by all bn tokens.  The converted weights are the A operand and live in TMEM: a
+//   converter thread owns one weight row = one TMEM lane, so 64 weights leave its registers as one `tcgen05.st` and
+//   never cross shared memory.  (With A in shared memory a K = 64 step of 256 tokens takes 643 cycles, with A in TMEM 544; the
+//   arithmetic's own minimum is 512.)  No TMA multicast: every CTA issues plain loads into its own shared memory.
+//
+// TMEM (all 512 columns): the accumulator (256) and four A stages of 128 K (64 columns each).  Persistent: one pair per TPC
+// walks (tile, split) units, tokens fastest, so that the pairs running together share few weight tiles and all token
+// tiles of a chunk stay in L2.
+//
+// What bounds it: at wide tiles the tensor pipe (2048 x 34816 x 5120: 474 us = 1540 TFLOP/s, 0.91 of the measured cuBLAS burst rate;
+// the single-CTA kernel 1216 us), at narrow ones the MMA thread's chain and the conversion (8 x 34816 x 5120: 46 us, 510
+// cycles per K = 64 block; 73 us).  2048 x 5120 x 17408: 564 -> 266 us, 173 x 5120 x 5120: 71 -> 26 us.
 //
 // Handshakes (all waits bounded, expiry -> status code, everything unwinds, TMEM freed):
-//   local, per CTA:   raw_full / raw_empty (TMA -> converters), a_full (converters -> MMA side), b_full (TMA -> MMA
-//                     side);
-//   second -> first:  a relay thread of the second CTA waits for its own a_full / b_full of block i and arrives on
-//                     peer_ready[i % SA] of the first CTA (release / acquire at cluster scope);
-//   first -> both:    `tcgen05.commit` with a CTA mask arrives on a_empty / b_empty / acc_full at the same offset in
-//                     both CTAs when the MMAs that read those stages have completed.
-// Warp roles (320 threads): warp 0 TMA producer, warp 1 MMA issuer (first CTA) or relay (second CTA) + TMEM owner,
-// warps 2..9 converters, warps 2..5 epilogue.
+//   own CTA:          raw_full / raw_empty (TMA -> converters), acc_full (MMA -> epilogue);
+//   both -> first:    activation tiles of both CTAs complete on full of the first CTA (`cta_group::2` loads may signal the
+//                     pair's other barrier), converter warps of both arrive there too, epilogue warps on acc_empty;
+//   first -> both:    `tcgen05.commit` with a CTA mask arrives on done / acc_full of both CTAs when the MMAs of a block (of a
+//                     tile) have completed; the producers and the converters both wait for `done`.
+// (Arrivals on the other CTA's barriers release at CTA scope: what they order is tensor memory, by the tcgen05 fences; a
+// cluster-scope release took 1100 cycles per arrival, three times a block's MMAs.)
+// Warp roles (768 threads): warp 0 MMA issuer (first CTA) and TMEM owner, 1 TMA producer, 4..19 converters (four sets take turns
+// at the K = 64 blocks), 20..23 epilogue.
 // (reference counterpart: src/kernels/fp4w_gemm.cu, the W4A16 prefill GEMM.)
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -33,85 +42,115 @@
 namespace dgpp {
 
 constexpr int kPrBM = 128;          // weight rows per CTA
-constexpr int kPrTok = 128;         // tokens per CTA (half of the pair's 256-token tile)
-constexpr int kPrBN = 256;          // tokens per pair tile = MMA N
 constexpr int kPrBK = 64;
-constexpr int kPrThreads = 320;
-constexpr int kPrConvWarps = 8;
-constexpr int kPrSB = 8, kPrSA = 3, kPrSR = 2;
-constexpr int kPrStageB = kPrTok * 128;     // 16 KB
-constexpr int kPrStageA = kPrBM * 128;      // 16 KB of bf16 (64 K per row)
-constexpr int kPrStageRaw = kPrBM * 128;    // 16 KB of packed fp4 (256 K per row)
-constexpr int kPrStageSf = kPrBM * 16;      // 2 KB of e4m3 scales (NVFP4)
+constexpr int kPrMaxBN = 256;       // tokens per pair tile = MMA N, at most
+constexpr int kPrSets = 4;            // converter sets of four warps; set s takes block s of every 256 K
+constexpr int kPrMma = 0, kPrTma = 1, kPrConv = 4, kPrEpi = kPrConv + kPrSets * 4;   // first warp of each role
+constexpr int kPrEpiWarps = 8;        // two per lane quadrant, taking turns at 16 columns
+constexpr int kPrThreads = (kPrEpi + kPrEpiWarps) * 32;
+constexpr int kPrStages = 4, kPrSR = 4;   // stages of 128 K (activations and converted weights), raw stages of 256 K
+constexpr int kPrHalfB = kPrMaxBN / 2 * 128;    // 16 KB: half of the tile's tokens, 64 K each
+constexpr int kPrStageB = 2 * kPrHalfB;
+constexpr int kPrStageRaw = kPrBM * 128;        // 16 KB of packed fp4 (256 K per row)
+constexpr int kPrStageSf = kPrBM * 16;          // 2 KB of e4m3 scales (NVFP4)
+constexpr int kPrStaging = 16 * 64;             // one epilogue warp's 16 tokens x 32 columns of bf16
+constexpr uint32_t kPrColA = kPrMaxBN;      // first TMEM column of the A stages
+constexpr uint32_t kPrTmemCols = 512;
 
 struct PairParams {
   float alpha;
   bf16* out;
   const bf16* resid;
   const uint8_t* sf_plain;   // MXFP4: e8m0 scales [N, K / 32]
+  float* ws;                 // split-K partials [splits, T, N]
+  uint32_t* counters;        // two per tile, zero at rest
   DeviceStatus* status;
   int T, N, K, ldc;
+  int bn, m_tiles, units, splits, kb_per_split;
+  int vec;                   // rows of `out` (and `resid`) can be accessed as 16-byte vectors
+  // Grouped form (experts): the matrices are stacked along N ([experts * N, K], N a multiple of 256); token tile t holds rows
+  // t * bn .. of x and `out` and belongs to matrix groups[t] (negative: nothing to do).  The block scales come in the
+  // order of the block-scaled kernels (tile_scales: [128 rows][256 K][4 x 512 bytes]), with one factor per matrix.
+  const int32_t* groups;
+  const float* group_alpha;
+  const uint8_t* sf_tiled;
+  int n_tiles;
 };
 
 constexpr size_t pair_smem_bytes() {
-  return 1024 + static_cast<size_t>(kPrSB) * kPrStageB + static_cast<size_t>(kPrSA) * kPrStageA +
-         static_cast<size_t>(kPrSR) * (kPrStageRaw + kPrStageSf) + (2 * kPrSB + 3 * kPrSA + 2 * kPrSR + 1) * 8 + 64;
+  return 1024 + static_cast<size_t>(kPrStages) * kPrStageB + static_cast<size_t>(kPrSR) * (kPrStageRaw + kPrStageSf) +
+         kPrEpiWarps * kPrStaging + (2 * kPrStages + 2 * kPrSR + 2) * 8 + 64;
 }
 
-__device__ __forceinline__ bool wait_bar_cluster(uint64_t* bar, uint32_t parity) {
-  for (int i = 0; i < 4096; ++i)
-    if (mbar_try_wait_cluster(bar, parity)) return true;
-  const long long t0 = clock64();
-  for (;;) {
-    for (int i = 0; i < 2048; ++i)
-      if (mbar_try_wait_cluster(bar, parity)) return true;
-    if (clock64() - t0 > 4000000000ll) return false;
+// Arrive on a barrier of the pair's first CTA (`addr`: its shared::cluster address); CTA-scope release.
+__device__ __forceinline__ void mbar_arrive_pair(uint32_t addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+
+// One K = 64 block of a row: 32 packed bytes -> 32 words of two bf16 each, element 2j in the low half of word j, 2^-14 times
+// the weight (the epilogue's factor makes up for it).  A code's three magnitude bits, moved to bits 8..6 of a bf16, read as
+// value * 2^-126 (code 1, 0.5, as a subnormal); the bf16 scale carries 2^112.  With the code in the high nibble of a byte, one
+// byte permute of (w << 4, w) puts the codes of both halves in place and spreads their signs over the bytes above
+// (its sign-replicating selectors); a shift and a mask finish both.  The integer pipe, which has half the rate of the
+// multiplier's, gets two instructions for two weights; the f16 conversion of the same codes took five and made it
+// the kernel's bound (50 % busy at 840 cycles per block; 384 are the MMAs of a 192-token tile).
+__device__ __forceinline__ void expand_e2m1x64(const Pack16& w0, const Pack16& w1, const bf162 (&s)[4], uint32_t (&o)[32]) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const uint32_t w = q < 4 ? w0.w[q] : w1.w[q - 4], we = w << 4;
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+      uint32_t x;   // (prmt itself: __byte_perm drops the replicate bit of a selector)
+      asm("prmt.b32 %0, %1, %2, %3;" : "=r"(x) : "r"(we), "r"(w), "r"(j | (j + 8) << 4 | (j + 4) << 8 | (j + 12) << 12));
+      const uint32_t r = (x << 2) & 0x81C081C0u;
+      const bf162 v = __hmul2(*reinterpret_cast<const bf162*>(&r), s[q >> 1]);
+      o[q * 4 + j] = *reinterpret_cast<const uint32_t*>(&v);
+    }
   }
 }
 
-template <int WMODE>   // 1 = NVFP4, 3 = MXFP4
+template <int WMODE, bool GROUPED>   // 1 = NVFP4, 3 = MXFP4
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPrThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA,   // packed weights as bytes [N, K / 2], box 128 x 128
-                    const __grid_constant__ CUtensorMap tmB,   // activations bf16 [T, K], box 64 x 128
+                    const __grid_constant__ CUtensorMap tmB,   // activations bf16 [T, K], box 64 x bn / 2
                     const __grid_constant__ CUtensorMap tmSf,  // NVFP4 scales [N, K / 16], box 16 x 128
                     PairParams p) {
   extern __shared__ __align__(1024) unsigned char smem_dyn[];
+  // (the pad to 1024 is the same in both CTAs of a pair: their windows have one layout)
   unsigned char* sp = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
-  unsigned char* sB = sp;    sp += kPrSB * kPrStageB;
-  unsigned char* sA = sp;    sp += kPrSA * kPrStageA;
+  unsigned char* sB = sp;    sp += kPrStages * kPrStageB;
   unsigned char* sRaw = sp;  sp += kPrSR * kPrStageRaw;
   unsigned char* sSf = sp;   sp += kPrSR * kPrStageSf;
-  uint64_t* b_full = reinterpret_cast<uint64_t*>(sp);
-  uint64_t* b_empty = b_full + kPrSB;
-  uint64_t* a_full = b_empty + kPrSB;
-  uint64_t* a_empty = a_full + kPrSA;
-  uint64_t* peer_ready = a_empty + kPrSA;      // used in the first CTA only
-  uint64_t* raw_full = peer_ready + kPrSA;
+  unsigned char* sOut = sp;  sp += kPrEpiWarps * kPrStaging;
+  uint64_t* full = reinterpret_cast<uint64_t*>(sp);     // used in the first CTA: activation tiles and converter warps of both
+  uint64_t* done = full + kPrStages;                    // the MMAs of the stage have completed
+  uint64_t* raw_full = done + kPrStages;
   uint64_t* raw_empty = raw_full + kPrSR;
   uint64_t* acc_full = raw_empty + kPrSR;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+  uint64_t* acc_empty = acc_full + 1;                   // used in the first CTA: the epilogue warps of each CTA
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  int* last_flag = const_cast<int*>(abort_flag) + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_ctarank();
-  const int n0 = blockIdx.x * kPrBM;
-  const int m0 = blockIdx.y * kPrBN;
-  const int mh = m0 + static_cast<int>(rank) * kPrTok;
-  const int nkb = p.K / kPrBK;
+  const int rank = static_cast<int>(cluster_ctarank());
+  const int first_unit = static_cast<int>(blockIdx.x) >> 1, unit_step = static_cast<int>(gridDim.x) >> 1;
+  const int num_kb = p.K / kPrBK;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kPrSB; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
-    for (int i = 0; i < kPrSA; ++i) { mbar_init(&a_full[i], kPrConvWarps); mbar_init(&a_empty[i], 1); mbar_init(&peer_ready[i], 1); }
-    for (int i = 0; i < kPrSR; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], kPrConvWarps); }
+    for (int i = 0; i < kPrStages; ++i) { mbar_init(&full[i], 1 + 2 * 2 * 4); mbar_init(&done[i], 1); }
+    for (int i = 0; i < kPrSR; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], kPrSets * 4); }
     mbar_init(acc_full, 1);
+    mbar_init(acc_empty, 2 * kPrEpiWarps);
     *abort_flag = 0;
+    *last_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
-    if (WMODE == 1) tma_prefetch_desc(&tmSf);
+    if (WMODE == 1 && !GROUPED) tma_prefetch_desc(&tmSf);
   }
-  if (warp == 1) {
-    tmem_alloc_pair(tmem_slot, kPrBN);
+  if (warp == kPrMma) {
+    tmem_alloc_pair(tmem_slot, kPrTmemCols);
     tmem_relinquish_pair();
   }
   tc_fence_before();
@@ -121,159 +160,343 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA,   // packed weights
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();
 
-  if (warp == 0) {
+  // Unit u: k64 blocks [kb0, kb0 + nk), a multiple of four; first weight row (n0 in the tensor map, nc as a column of the output) and
+  // first token of the tile.  False: nothing to do.
+  auto unit_at = [&](int u, int& n0, int& nc, int& m0, int& split, int& kb0, int& nk, float& alpha) {
+    alpha = p.alpha;
+    if (GROUPED) {
+      const int tile = u / p.n_tiles, e = p.groups[tile];
+      nc = (u % p.n_tiles) * 2 * kPrBM + rank * kPrBM;
+      n0 = e * p.N + nc;
+      m0 = tile * p.bn;
+      split = 0; kb0 = 0; nk = num_kb;
+      if (e < 0) return false;
+      alpha *= p.group_alpha[e];
+      return true;
+    }
+    const int tile = u / p.splits;
+    split = u % p.splits;
+    n0 = nc = (tile / p.m_tiles) * 2 * kPrBM + rank * kPrBM;
+    m0 = (tile % p.m_tiles) * p.bn;
+    kb0 = split * p.kb_per_split;
+    nk = min(p.kb_per_split, num_kb - kb0);
+    return true;
+  };
+
+  if (warp == kPrTma) {
     // ------------------------------------------------------------------ TMA producer (own weights, own token half)
     if (elect_one()) {
-      for (int i = 0; i < nkb; ++i) {
-        if (i % 4 == 0) {
-          const int r = i / 4, sr = r % kPrSR;
-          if (!wait_bar(&raw_empty[sr], ((r / kPrSR) & 1) ^ 1)) { report(p.status, kTimeoutStageEmpty, 21); *abort_flag = 1; break; }
-          mbar_expect_tx(&raw_full[sr], kPrStageRaw + (WMODE == 1 ? kPrStageSf : 0));
-          tma_load_2d(sRaw + sr * kPrStageRaw, &tmA, i * 32, n0, &raw_full[sr]);
-          if (WMODE == 1) tma_load_2d(sSf + sr * kPrStageSf, &tmSf, i * 4, n0, &raw_full[sr]);
+      const uint32_t stage_b = static_cast<uint32_t>(p.bn / 2) * 128u;
+      int it = 0;
+      bool ok = true;
+      for (int u = first_unit; u < p.units && ok; u += unit_step) {
+        int n0, nc, m0, split, kb0, nk;
+        float alpha;
+        if (!unit_at(u, n0, nc, m0, split, kb0, nk, alpha)) continue;
+        const int mh = m0 + rank * (p.bn / 2);
+        for (int i = 0; i < nk; ++i, ++it) {
+          const int kb = kb0 + i;
+          if ((it & 3) == 0) {
+            const int r = it >> 2, sr = r % kPrSR;
+            if (!wait_bar(&raw_empty[sr], ((r / kPrSR) & 1) ^ 1)) { report(p.status, kTimeoutStageEmpty, 21); *abort_flag = 1; ok = false; break; }
+            mbar_expect_tx(&raw_full[sr], kPrStageRaw + (WMODE == 1 ? kPrStageSf : 0));
+            tma_load_2d(sRaw + sr * kPrStageRaw, &tmA, kb * 32, n0, &raw_full[sr]);
+            if (GROUPED)
+              bulk_load_1d(sSf + sr * kPrStageSf, p.sf_tiled + (static_cast<size_t>(n0 / kPrBM) * (p.K / 256) + (kb >> 2)) * kPrStageSf, kPrStageSf, &raw_full[sr]);
+            else if (WMODE == 1) tma_load_2d(sSf + sr * kPrStageSf, &tmSf, kb * 4, n0, &raw_full[sr]);
+          }
+          const int stg = it >> 1, sl = stg % kPrStages;
+          if ((it & 1) == 0) {
+            if (!wait_bar(&done[sl], ((stg / kPrStages) & 1) ^ 1)) { report(p.status, kTimeoutStageEmpty, 22); *abort_flag = 1; ok = false; break; }
+            if (rank == 0) mbar_expect_tx(&full[sl], 4 * stage_b);
+          }
+          tma_load_2d_pair(sB + sl * kPrStageB + (it & 1) * kPrHalfB, &tmB, kb * kPrBK, mh, mapa_shared(smem_u32(&full[sl]), 0u));
         }
-        const int sb = i % kPrSB;
-        if (!wait_bar(&b_empty[sb], ((i / kPrSB) & 1) ^ 1)) { report(p.status, kTimeoutStageEmpty, 22); *abort_flag = 1; break; }
-        mbar_expect_tx(&b_full[sb], kPrStageB);
-        tma_load_2d(sB + sb * kPrStageB, &tmB, i * kPrBK, mh, &b_full[sb]);
-        if (*abort_flag) break;
       }
     }
-  } else if (warp == 1) {
-    if (elect_one()) {
-      if (rank == 0) {
-        // ---------------------------------------------------------------- MMA issuer of the pair
-        constexpr uint32_t idesc = umma_idesc_f16(2 * kPrBM, kPrBN, 1u, 1u);
-        for (int i = 0; i < nkb; ++i) {
-          const int sb = i % kPrSB, sa = i % kPrSA;
-          if (!wait_bar(&b_full[sb], (i / kPrSB) & 1)) { report(p.status, kTimeoutTmaFull, 23); *abort_flag = 1; break; }
-          if (!wait_bar(&a_full[sa], (i / kPrSA) & 1)) { report(p.status, kTimeoutConvert, 24); *abort_flag = 1; break; }
-          if (!wait_bar_cluster(&peer_ready[sa], (i / kPrSA) & 1)) { report(p.status, kTimeoutPeerFlag, 25); *abort_flag = 1; break; }
+  } else if (warp == kPrMma) {
+    // ------------------------------------------------------------------ MMA issuer of the pair
+    // One thread, one wait per 128 K: this loop is the chain that the tensor pipe waits for.  A wait takes 200 cycles
+    // even when its barrier completed long ago, so separate waits for activations and weights per 64 K made a loop
+    // of 740 cycles, whatever the tile (MMAs of 64 K x 256 tokens: 544).
+    if (rank == 0 && elect_one()) {
+      const uint32_t idesc = umma_idesc_f16(2 * kPrBM, static_cast<uint32_t>(p.bn), 1u, 1u);
+      const uint32_t b_base = smem_u32(sB);
+      int sl = 0, tc = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int u = first_unit; u < p.units && ok; u += unit_step) {
+        int n0, nc, m0, split, kb0, nk;
+        float alpha;
+        if (!unit_at(u, n0, nc, m0, split, kb0, nk, alpha)) continue;
+        if (!wait_bar(acc_empty, (tc & 1) ^ 1)) { report(p.status, kTimeoutAccum, 23); *abort_flag = 1; break; }
+        for (int i = 0; i < nk; i += 2) {
+          if (!wait_bar(&full[sl], ph)) { report(p.status, kTimeoutConvert, 24); *abort_flag = 1; ok = false; break; }
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(sA + sa * kPrStageA), b_addr = smem_u32(sB + sb * kPrStageB);
+          const uint32_t b_addr = b_base + sl * kPrStageB, a_col = tmem_base + kPrColA + sl * 64;
 #pragma unroll
-          for (int kk = 0; kk < kPrBK / 16; ++kk)
-            umma_f16_pair(tmem_base, umma_desc_sw128(a_addr + kk * 32), umma_desc_sw128(b_addr + kk * 32), idesc,
-                          (i > 0 || kk > 0) ? 1u : 0u);
-          umma_commit_pair(&b_empty[sb], 3);
-          umma_commit_pair(&a_empty[sa], 3);
-          if (*abort_flag) break;
+          for (int kk = 0; kk < 8; ++kk)
+            umma_f16_pair_ts(tmem_base, a_col + kk * 8, umma_desc_sw128(b_addr + (kk >> 2) * kPrHalfB + (kk & 3) * 32), idesc,
+                             (i > 0 || kk > 0) ? 1u : 0u);
+          umma_commit_pair(&done[sl], 3);
+          if (++sl == kPrStages) { sl = 0; ph ^= 1; }
         }
         umma_commit_pair(acc_full, 3);
-      } else {
-        // ---------------------------------------------------------------- relay: this CTA's stages of block i are ready
-        for (int i = 0; i < nkb; ++i) {
-          const int sb = i % kPrSB, sa = i % kPrSA;
-          if (!wait_bar(&b_full[sb], (i / kPrSB) & 1)) { report(p.status, kTimeoutTmaFull, 26); *abort_flag = 1; break; }
-          if (!wait_bar(&a_full[sa], (i / kPrSA) & 1)) { report(p.status, kTimeoutConvert, 27); *abort_flag = 1; break; }
-          mbar_arrive_remote(mapa_shared(smem_u32(&peer_ready[sa]), 0u));
-          if (*abort_flag) break;
-        }
+        ++tc;
       }
     }
-  } else {
-    // ------------------------------------------------------------------ converters (warps 2..9): e2m1 -> bf16
-    const int ct = threadIdx.x - 64;       // 0..255
-    const int row = ct >> 1, half = ct & 1;
-    for (int i = 0; i < nkb; ++i) {
-      const int r = i / 4, sub = i % 4, sr = r % kPrSR, sa = i % kPrSA;
-      bool ok = true;
-      if (sub == 0) ok = wait_bar(&raw_full[sr], (r / kPrSR) & 1);
-      if (ok) ok = wait_bar(&a_empty[sa], ((i / kPrSA) & 1) ^ 1);
-      if (!ok) { report(p.status, kTimeoutTmaFull, 28); *abort_flag = 1; break; }
-      const unsigned char* raw = sRaw + sr * kPrStageRaw + row * 128;
-      unsigned char* dst = sA + sa * kPrStageA + row * 128;
-      // 32 weights = 16 packed bytes at logical 16-byte chunk (sub * 2 + half) of the swizzled 128-byte row
-      const int cl = sub * 2 + half;
-      Pack16 w;
-      w.u = *reinterpret_cast<const uint4*>(raw + ((cl ^ (row & 7)) << 4));
-      float s0f, s1f;
-      if (WMODE == 1) {
-        const unsigned char* sf = sSf + sr * kPrStageSf + row * 16 + sub * 4 + half * 2;
-        s0f = e4m3_to_f32(sf[0]);
-        s1f = e4m3_to_f32(sf[1]);
-      } else {
-        const int nrow = min(n0 + row, p.N - 1);
-        s0f = s1f = e8m0_to_f32(p.sf_plain[static_cast<size_t>(nrow) * (p.K / 32) + i * 2 + half]);
+  } else if (warp >= kPrConv && warp < kPrEpi) {
+    // ------------------------------------------------------------------ converters: e2m1 -> bf16 -> TMEM
+    const int set = (warp - kPrConv) >> 2, q = warp & 3, row = q * 32 + lane;
+    const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
+    const float k112 = 5.192296858534828e33f;
+    int it = set;              // this set's next k64 block, counted over all units
+    bool ok = true;
+    for (int u = first_unit; u < p.units && ok; u += unit_step) {
+      int n0, nc, m0, split, kb0, nk;
+      float alpha;
+      if (!unit_at(u, n0, nc, m0, split, kb0, nk, alpha)) continue;
+      // MXFP4: two scale bytes per block by plain loads, one block of this set ahead
+      const uint8_t* sf_row = nullptr;
+      uint32_t e8 = 0;
+      if (WMODE == 3) {
+        sf_row = p.sf_plain + static_cast<size_t>(min(n0 + row, p.N - 1)) * (p.K / 32) + kb0 * 2;
+        e8 = *reinterpret_cast<const uint16_t*>(sf_row + set * 2);
       }
-      // f16 bits >> 3 read as bf16 equal value * 2^-112; 2^112 is folded into the (exact) bf16 scale
-      const bf162 s0 = __float2bfloat162_rn(s0f * 5.192296858534828e33f);
-      const bf162 s1 = __float2bfloat162_rn(s1f * 5.192296858534828e33f);
-      Pack16 o[4];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        __half2 h = e2m1x2_to_h2(w.b[j]);
-        const uint32_t hb = *reinterpret_cast<uint32_t*>(&h);
-        uint32_t bb = ((hb & 0x7FFF7FFFu) >> 3) | (hb & 0x80008000u);
-        bf162 v = __hmul2(*reinterpret_cast<bf162*>(&bb), j < 8 ? s0 : s1);
-        o[j >> 2].w[j & 3] = *reinterpret_cast<uint32_t*>(&v);
-      }
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        *reinterpret_cast<uint4*>(dst + (((half * 4 + c) ^ (row & 7)) << 4)) = o[c].u;
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&a_full[sa]);
-        if (sub == 3 || i == nkb - 1) mbar_arrive(&raw_empty[sr]);
-      }
-      if (*abort_flag) break;
-    }
-  }
-
-  // ------------------------------------------------------------------ epilogue (warps 2..5): own 128 rows x 256 tokens
-  if (warp >= 2 && warp < 6) {
-    const int q = warp & 3;
-    const bool ok = nkb > 0 ? wait_bar_cluster(acc_full, 0) : true;
-    if (!ok) { report(p.status, kTimeoutAccum, 29); *abort_flag = 1; }
-    tc_fence_after();
-    const int n = n0 + q * 32 + lane;
-    const int cols = min(kPrBN, p.T - m0);
-    if (ok && !*abort_flag) {
-#pragma unroll 1
-      for (int c0 = 0; c0 < kPrBN; c0 += 16) {
-        if (c0 >= cols) break;
-        uint32_t r[16];
-        if (nkb > 0) {
-          tmem_ld_x16(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + c0, r);
-          tmem_ld_wait();
+      for (int i = set; i < nk; i += kPrSets, it += kPrSets) {
+        const int r = it >> 2, sr = r % kPrSR, stg = it >> 1, sl = stg % kPrStages;
+        bool okw = wait_bar(&raw_full[sr], (r / kPrSR) & 1);
+        const unsigned char* raw = sRaw + sr * kPrStageRaw + row * 128;
+        Pack16 w0, w1;
+        w0.u = *reinterpret_cast<const uint4*>(raw + (((set * 2) ^ (row & 7)) << 4));
+        w1.u = *reinterpret_cast<const uint4*>(raw + (((set * 2 + 1) ^ (row & 7)) << 4));
+        bf162 s[4];
+        if (WMODE == 1) {
+          const uint32_t four = *reinterpret_cast<const uint32_t*>(
+              sSf + sr * kPrStageSf + (GROUPED ? set * 512 + lane * 16 + q * 4 : row * 16 + set * 4));
+          const float2 lo = __half22float2(e4m3x2_to_h2(static_cast<uint16_t>(four & 0xFFFFu)));
+          const float2 hi = __half22float2(e4m3x2_to_h2(static_cast<uint16_t>(four >> 16)));
+          s[0] = __float2bfloat162_rn(lo.x * k112); s[1] = __float2bfloat162_rn(lo.y * k112);
+          s[2] = __float2bfloat162_rn(hi.x * k112); s[3] = __float2bfloat162_rn(hi.y * k112);
         } else {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) r[j] = 0;
+          s[0] = s[1] = __float2bfloat162_rn(e8m0_to_f32(static_cast<uint8_t>(e8 & 255u)) * k112);
+          s[2] = s[3] = __float2bfloat162_rn(e8m0_to_f32(static_cast<uint8_t>(e8 >> 8)) * k112);
+          if (i + kPrSets < nk) e8 = *reinterpret_cast<const uint16_t*>(sf_row + (i + kPrSets) * 2);
         }
-        if (n < p.N) {
+        uint32_t o[32];
+        expand_e2m1x64(w0, w1, s, o);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&raw_empty[sr]);   // this warp is done with the raw stage
+        if (okw) okw = wait_bar(&done[sl], ((stg / kPrStages) & 1) ^ 1);   // the stage's columns are free
+        if (!okw) { report(p.status, kTimeoutTmaFull, 26); *abort_flag = 1; }
+        ok = __all_sync(0xffffffffu, okw && !*abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        tmem_st_x32(tmem_base + kPrColA + sl * 64 + (it & 1) * 32 + lane_addr, o);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_pair(mapa_shared(smem_u32(&full[sl]), 0u));
+      }
+    }
+  } else if (warp >= kPrEpi) {
+    // ------------------------------------------------------------------ epilogue: own 128 rows x bn tokens
+    const int q = warp & 3;
+    const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
+    const int half = (warp - kPrEpi) >> 2;
+    bf16* stage = reinterpret_cast<bf16*>(sOut + (warp - kPrEpi) * kPrStaging);
+    int tc = 0;
+    for (int u = first_unit; u < p.units; u += unit_step) {
+      int n0, nc, m0, split, kb0, nk;
+      float alpha;
+      if (!unit_at(u, n0, nc, m0, split, kb0, nk, alpha)) continue;
+      const uint32_t d = tmem_base + lane_addr;
+      bool ok = wait_bar(acc_full, tc & 1);
+      if (!ok) { report(p.status, kTimeoutAccum, 27); *abort_flag = 1; }
+      ok = __all_sync(0xffffffffu, ok && !*abort_flag);
+      tc_fence_after();
+      const int nw = nc + q * 32, n = nw + lane;   // this warp's first column, this lane's
+      const int cols = min(p.bn, p.T - m0);
+      float* wsp = p.splits > 1 ? p.ws + (static_cast<size_t>(split) * p.T + m0) * p.N : nullptr;
+      if (ok) {
+#pragma unroll 1
+        for (int c0 = half * 16; c0 < cols; c0 += 32) {
+          uint32_t r[16];
+          tmem_ld_x16(d + c0, r);
+          const int live = min(16, cols - c0);
+          if (p.splits > 1) {
+            if (n < p.N) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int m = c0 + j;
-            if (m < cols) {
-              const size_t o = static_cast<size_t>(m0 + m) * p.ldc + n;
-              float y = __uint_as_float(r[j]) * p.alpha;
-              if (p.resid) y = bf16_to_f32(p.resid[o]) + bf16_to_f32(f32_to_bf16(y));
-              p.out[o] = f32_to_bf16(y);
+              for (int j = 0; j < 16; ++j)
+                if (j < live) wsp[static_cast<size_t>(c0 + j) * p.N + n] = __uint_as_float(r[j]);
+            }
+          } else if (p.vec) {
+            // turned around through the warp's staging tile: every lane then writes 8 columns of one token
+#pragma unroll
+            for (int j = 0; j < 16; ++j) stage[j * 32 + lane] = f32_to_bf16(__uint_as_float(r[j]) * alpha);
+            __syncwarp();
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int m = h * 8 + (lane >> 2), seg = lane & 3;
+              if (m < live && nw + seg * 8 < p.N) {
+                Pack16 v;
+                v.u = *reinterpret_cast<const uint4*>(stage + m * 32 + seg * 8);
+                const size_t at = static_cast<size_t>(m0 + c0 + m) * p.ldc + nw + seg * 8;
+                if (p.resid) {
+                  Pack16 x;
+                  x.u = *reinterpret_cast<const uint4*>(p.resid + at);
+#pragma unroll
+                  for (int j = 0; j < 8; ++j) v.h[j] = f32_to_bf16(bf16_to_f32(x.h[j]) + bf16_to_f32(v.h[j]));
+                }
+                *reinterpret_cast<uint4*>(p.out + at) = v.u;
+              }
+            }
+            __syncwarp();
+          } else if (n < p.N) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              if (j < live) {
+                const size_t at = static_cast<size_t>(m0 + c0 + j) * p.ldc + n;
+                float y = __uint_as_float(r[j]) * alpha;
+                if (p.resid) y = bf16_to_f32(p.resid[at]) + bf16_to_f32(f32_to_bf16(y));
+                p.out[at] = f32_to_bf16(y);
+              }
             }
           }
         }
       }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_pair(mapa_shared(smem_u32(acc_empty), 0u));
+      if (p.splits > 1) {
+        // publish the partials; the last CTA on this half tile adds them in ascending split order
+        uint32_t* counter = p.counters + (u / p.splits) * 2 + rank;
+        __threadfence();
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (warp == kPrEpi && lane == 0) {
+          const uint32_t prev = atomicAdd(counter, 1u);
+          *last_flag = (prev == static_cast<uint32_t>(p.splits - 1)) ? 1 : 0;
+        }
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (*last_flag) {
+          __threadfence();
+          if (p.vec) {
+            // a warp takes whole rows of the half tile, four columns per lane, four rows' partials in flight
+            const int n4 = nc + lane * 4, wrow = warp - kPrEpi;
+            if (n4 < p.N) {
+              for (int mb = wrow; mb < cols; mb += 4 * kPrEpiWarps) {
+                float4 acc[4];
+#pragma unroll
+                for (int mm = 0; mm < 4; ++mm) acc[mm] = make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int s0 = 0; s0 < p.splits; ++s0) {
+                  float4 t[4];
+#pragma unroll
+                  for (int mm = 0; mm < 4; ++mm)
+                    t[mm] = mb + mm * kPrEpiWarps < cols
+                                ? __ldcg(reinterpret_cast<const float4*>(p.ws + (static_cast<size_t>(s0) * p.T + m0 + mb + mm * kPrEpiWarps) * p.N + n4))
+                                : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                  for (int mm = 0; mm < 4; ++mm) { acc[mm].x += t[mm].x; acc[mm].y += t[mm].y; acc[mm].z += t[mm].z; acc[mm].w += t[mm].w; }
+                }
+#pragma unroll
+                for (int mm = 0; mm < 4; ++mm) {
+                  const int m = mb + mm * kPrEpiWarps;
+                  if (m >= cols) break;
+                  const size_t at = static_cast<size_t>(m0 + m) * p.ldc + n4;
+                  float y[4] = {acc[mm].x * alpha, acc[mm].y * alpha, acc[mm].z * alpha, acc[mm].w * alpha};
+                  union { uint2 u; bf16 h[4]; } v, x;
+                  if (p.resid) x.u = *reinterpret_cast<const uint2*>(p.resid + at);
+#pragma unroll
+                  for (int j = 0; j < 4; ++j) {
+                    v.h[j] = f32_to_bf16(y[j]);
+                    if (p.resid) v.h[j] = f32_to_bf16(bf16_to_f32(x.h[j]) + bf16_to_f32(v.h[j]));
+                  }
+                  *reinterpret_cast<uint2*>(p.out + at) = v.u;
+                }
+              }
+            }
+          } else if (n < p.N) {
+            for (int m = half; m < cols; m += 2) {
+              float acc = 0.f;
+              for (int s0 = 0; s0 < p.splits; ++s0) acc += __ldcg(p.ws + (static_cast<size_t>(s0) * p.T + m0 + m) * p.N + n);
+              const size_t at = static_cast<size_t>(m0 + m) * p.ldc + n;
+              float y = acc * alpha;
+              if (p.resid) y = bf16_to_f32(p.resid[at]) + bf16_to_f32(f32_to_bf16(y));
+              p.out[at] = f32_to_bf16(y);
+            }
+          }
+          if (warp == kPrEpi && lane == 0) *counter = 0;
+        }
+      }
+      if (!ok) break;
+      ++tc;
     }
   }
   tc_fence_before();
   __syncthreads();
-  cluster_barrier();      // neither CTA leaves (or frees TMEM) while the other may still read its shared memory
-  if (warp == 1) tmem_dealloc_pair(tmem_base, kPrBN);
+  cluster_barrier();      // neither CTA leaves (or frees TMEM) while the other may still read its memory or arrive there
+  if (warp == kPrMma) tmem_dealloc_pair(tmem_base, kPrTmemCols);
 }
 
-template <int WMODE>
-static int launch_pair(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tSf, const PairParams& p, cudaStream_t st) {
-  auto kern = gemm_tc_pair_kernel<WMODE>;
-  static bool attr = false;
-  constexpr size_t smem = pair_smem_bytes();
-  static_assert(smem <= 227 * 1024, "shared memory budget exceeded");
-  if (!attr) {
+// Pairs that fit the device at once (one per TPC; a GPC with an odd number of SMs in use gives one less).
+template <int WMODE, bool GROUPED>
+static int pair_slots(int* slots) {
+  static int cached = 0;
+  if (!cached) {
+    auto kern = gemm_tc_pair_kernel<WMODE, GROUPED>;
+    constexpr size_t smem = pair_smem_bytes();
+    static_assert(kPrSets == 4, "a set's blocks are the same quarter of every raw stage");
+    static_assert(smem <= 227 * 1024, "shared memory budget exceeded");
     DGPP_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    attr = true;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2, 1, 1);
+    cfg.blockDim = dim3(kPrThreads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    DGPP_CUDA_OK(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
+    DGPP_REQUIRE(n >= 1, "gemm_tc_pair: no CTA pair fits this device");
+    cached = n;
   }
-  dim3 grid(p.N / kPrBM, dgpp_ceil_div(p.T, kPrBN), 1);
-  kern<<<grid, kPrThreads, smem, st>>>(tA, tB, tSf, p);
+  *slots = cached;
+  return 0;
+}
+
+// Token tile and K splits of one product.  A K = 64 block of a bn-token tile was measured at 400 + 1.2 bn cycles (64 tokens: 507,
+// 128: 540, 192: 622, 256: 741), a tile's drain at 15 bn (the accumulator is not double-buffered: its other half holds
+// the converted weights); splits cost their partials' way to memory and back and 5500 cycles.  The product takes as many
+// units one after the other as one pair gets: wide tiles reuse a converted weight more often, narrower ones (or
+// splits, where there are fewer tiles than pairs) fill the last round.  Up to 64 rows the splits are those of 64 rows: a row's
+// bits do not depend on how many decode rows share its pass.
+static void pair_shape(int T, int N, int K, int slots, int max_splits, int* bn_out, int* splits_out) {
+  double best = 0;
+  *bn_out = kPrMaxBN;
+  *splits_out = 1;
+  const int rows = T;
+  if (T < 64) T = 64;
+  const int nt = dgpp_ceil_div(N, 2 * kPrBM), raws = K / 256;
+  for (int bn = kPrMaxBN; bn >= 16; bn -= 16) {
+    if (bn < kPrMaxBN && bn - 16 >= T) continue;          // a smaller tile holds all rows
+    const int tiles = nt * dgpp_ceil_div(T, bn);
+    for (int s = 1; s <= max_splits && s <= raws; ++s) {
+      const int per = dgpp_ceil_div(raws, s);
+      if (dgpp_ceil_div(raws, per) != s) continue;
+      const int rounds = dgpp_ceil_div(tiles * s, slots);
+      const double unit = per * 4 * (400 + 1.2 * bn) + 15.0 * bn + 500;
+      const double cost = rounds * unit + (s > 1 ? 5500 + 8.0 * T * N * s / 3200 : 0.0);
+      if (best == 0 || cost < best) { best = cost; *bn_out = bn; *splits_out = s; }
+    }
+  }
+  if (rows < 64) *bn_out = dgpp_ceil_div(rows, 16) * 16;
+}
+
+template <int WMODE, bool GROUPED>
+static int launch_pair(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tSf, const PairParams& p, int slots, cudaStream_t st) {
+  const int pairs = p.units < slots ? p.units : slots;
+  gemm_tc_pair_kernel<WMODE, GROUPED><<<2 * pairs, kPrThreads, pair_smem_bytes(), st>>>(tA, tB, tSf, p);
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -282,27 +505,90 @@ static int launch_pair(const CUtensorMap& tA, const CUtensorMap& tB, const CUten
 
 using namespace dgpp;
 
-// wmode: 1 nvfp4 (w_scale = e4m3 scales [N, K / 16]), 3 mxfp4 (w_scale = e8m0 scales [N, K / 32]).  N % 256 == 0,
-// K % 256 == 0.  out bf16 [T, ldc]; resid optional (out = bf16(resid + bf16(alpha * acc))).
+// wmode: 1 nvfp4 (w_scale = e4m3 scales [N, K / 16]), 3 mxfp4 (w_scale = e8m0 scales [N, K / 32]).  K % 256 == 0.
+// out bf16 [T, ldc]; resid optional (out = bf16(resid + bf16(alpha * acc))).  bn: token tile, a multiple of 16 up to
+// 256, or 0 = chosen here; splits: K splits, or 0 = chosen here among those that the workspace (ws_floats fp32 values,
+// n_counters counters that are zero at rest) holds.
 DGPP_API int dgpp_gemm_tc_pair(int wmode, const void* x, int64_t x_stride, const void* w, const void* w_scale, float alpha,
-                               void* out, const void* resid, int ldc, int T, int N, int K, cudaStream_t st) {
+                               void* out, const void* resid, int ldc, int T, int N, int K, int bn, int splits, void* ws,
+                               int64_t ws_floats, void* counters, int n_counters, cudaStream_t st) {
   DGPP_REQUIRE(wmode == 1 || wmode == 3, "gemm_tc_pair: 4-bit weights only (wmode %d)", wmode);
-  DGPP_REQUIRE(T >= 1 && N >= 256 && N % 256 == 0, "gemm_tc_pair: N %d must be a multiple of 256", N);
-  DGPP_REQUIRE(K % 256 == 0, "gemm_tc_pair: K %d must be a multiple of 256", K);
+  DGPP_REQUIRE(T >= 1 && N >= 1, "gemm_tc_pair: empty problem");
+  DGPP_REQUIRE(K % 256 == 0 && K > 0, "gemm_tc_pair: K %d must be a multiple of 256", K);
   DGPP_REQUIRE(out != nullptr && w_scale != nullptr, "gemm_tc_pair: output and scales required");
+  DGPP_REQUIRE(bn >= 0 && bn <= kPrMaxBN && bn % 16 == 0, "gemm_tc_pair: token tile %d (a multiple of 16 up to %d)", bn, kPrMaxBN);
+  DGPP_REQUIRE(splits >= 0 && (splits <= 1 || (ws && counters)), "gemm_tc_pair: split-K needs a workspace with counters");
+  DGPP_REQUIRE((reinterpret_cast<uintptr_t>(w_scale) & 15) == 0, "gemm_tc_pair: scales must be 16-byte aligned");
+  int slots = 0;
+  if (wmode == 1 ? pair_slots<1, false>(&slots) : pair_slots<3, false>(&slots)) return -1;
+  int most = 1;
+  if (ws && counters) {
+    const int64_t by_ws = ws_floats / (static_cast<int64_t>(T < 64 ? 64 : T) * N);
+    most = static_cast<int>(by_ws < 8 ? (by_ws < 1 ? 1 : by_ws) : 8);
+    if (2LL * dgpp_ceil_div(N, 2 * kPrBM) * dgpp_ceil_div(T, 16) > n_counters) most = 1;
+  }
+  int pick_bn, pick_splits;
+  pair_shape(T, N, K, slots, most, &pick_bn, &pick_splits);
+  if (bn == 0) bn = pick_bn;
+  if (splits == 0) splits = pick_splits;
+  DGPP_REQUIRE(splits <= most || splits == 1, "gemm_tc_pair: %d splits do not fit the workspace", splits);
   PairParams p;
-  p.alpha = alpha;
+  p.alpha = alpha * 16384.f;    // the converted weights carry 2^-14
   p.out = static_cast<bf16*>(out);
   p.resid = static_cast<const bf16*>(resid);
   p.sf_plain = wmode == 3 ? static_cast<const uint8_t*>(w_scale) : nullptr;
+  p.ws = static_cast<float*>(ws);
+  p.counters = static_cast<uint32_t*>(counters);
   p.status = device_status_ptr();
   p.T = T; p.N = N; p.K = K; p.ldc = ldc;
+  p.groups = nullptr; p.group_alpha = nullptr; p.sf_tiled = nullptr; p.n_tiles = 0;
+  p.bn = bn;
+  p.m_tiles = dgpp_ceil_div(T, bn);
+  const int raws = K / 256, per = dgpp_ceil_div(raws, splits);
+  p.kb_per_split = per * 4;
+  p.splits = dgpp_ceil_div(raws, per);
+  p.units = p.m_tiles * dgpp_ceil_div(N, 2 * kPrBM) * p.splits;
+  p.vec = N % 8 == 0 && ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && (reinterpret_cast<uintptr_t>(resid) & 15) == 0 &&
+          (reinterpret_cast<uintptr_t>(ws) & 15) == 0;
   CUtensorMap tA, tB, tSf;
   memset(&tSf, 0, sizeof(tSf));
-  if (make_tmap_2d(&tB, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, T, x_stride * 2, 64, kPrTok, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
+  if (make_tmap_2d(&tB, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, T, x_stride * 2, 64, bn / 2, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
   if (make_tmap_2d(&tA, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K / 2, N, K / 2, 128, kPrBM, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
   if (wmode == 1 &&
       make_tmap_2d(&tSf, w_scale, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K / 16, N, K / 16, 16, kPrBM, CU_TENSOR_MAP_SWIZZLE_NONE))
     return -1;
-  return wmode == 1 ? launch_pair<1>(tA, tB, tSf, p, st) : launch_pair<3>(tA, tB, tSf, p, st);
+  return wmode == 1 ? launch_pair<1, false>(tA, tB, tSf, p, slots, st) : launch_pair<3, false>(tA, tB, tSf, p, slots, st);
+}
+
+// Grouped linear over a stack of NVFP4 matrices w [experts * N, K / 2] with block scales in tile_scales order and one factor per matrix
+// (group_alpha [experts]): rows t * bn .. of out = those of x times matrix groups[t]; tiles with a negative entry are
+// left alone.  N and K multiples of 256, bn a multiple of 16 up to 256; x and out hold tiles * bn rows.
+DGPP_API int dgpp_gemm_tc_pair_grouped(const void* x, int64_t x_stride, const void* w, const void* sf_tiled, const void* group_alpha,
+                                       const void* groups, void* out, int ldc, int tiles, int N, int K, int experts, int bn,
+                                       cudaStream_t st) {
+  DGPP_REQUIRE(N > 0 && N % 256 == 0 && K > 0 && K % 256 == 0, "gemm_tc_pair_grouped: N %d and K %d must be multiples of 256", N, K);
+  DGPP_REQUIRE(bn >= 16 && bn <= kPrMaxBN && bn % 16 == 0, "gemm_tc_pair_grouped: token tile %d", bn);
+  DGPP_REQUIRE(tiles >= 1 && experts >= 1 && groups && group_alpha && sf_tiled && out, "gemm_tc_pair_grouped: bad group arguments");
+  DGPP_REQUIRE((reinterpret_cast<uintptr_t>(sf_tiled) & 15) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && ldc % 8 == 0,
+               "gemm_tc_pair_grouped: scales and output rows must be 16-byte aligned");
+  int slots = 0;
+  if (pair_slots<1, true>(&slots)) return -1;
+  PairParams p;
+  memset(&p, 0, sizeof(p));
+  p.alpha = 16384.f;             // the converted weights carry 2^-14
+  p.out = static_cast<bf16*>(out);
+  p.status = device_status_ptr();
+  p.T = tiles * bn; p.N = N; p.K = K; p.ldc = ldc;
+  p.bn = bn; p.m_tiles = tiles; p.splits = 1; p.kb_per_split = K / kPrBK;
+  p.n_tiles = N / (2 * kPrBM);
+  p.units = tiles * p.n_tiles;
+  p.vec = 1;
+  p.groups = static_cast<const int32_t*>(groups);
+  p.group_alpha = static_cast<const float*>(group_alpha);
+  p.sf_tiled = static_cast<const uint8_t*>(sf_tiled);
+  CUtensorMap tA, tB, tSf;
+  memset(&tSf, 0, sizeof(tSf));
+  if (make_tmap_2d(&tB, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, static_cast<uint64_t>(tiles) * bn, x_stride * 2, 64, bn / 2, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
+  if (make_tmap_2d(&tA, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K / 2, static_cast<uint64_t>(experts) * N, K / 2, 128, kPrBM, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
+  return launch_pair<1, true>(tA, tB, tSf, p, slots, st);
 }

@@ -70,6 +70,18 @@ def swiglu(gate_up: torch.Tensor, out: Optional[torch.Tensor] = None, limit: flo
     return out
 
 
+_lib.declare("dgpp_swiglu_tiles", [P, P, P, I, I, I, F, F, P])
+
+
+def swiglu_tiles(gate_up: torch.Tensor, out: torch.Tensor, tiles: torch.Tensor, bn: int, limit: float = 0.0,
+                 alpha: float = 0.0) -> torch.Tensor:
+    """`swiglu` over tiles of bn rows; rows of tiles with a negative entry in `tiles` are skipped."""
+    _chk(gate_up, torch.bfloat16, "gate_up")
+    call("dgpp_swiglu_tiles", ptr(gate_up), ptr(out), ptr(tiles), tiles.numel(), bn, out.shape[-1], float(limit), float(alpha),
+         stream_ptr())
+    return out
+
+
 def argmax(logits: torch.Tensor, id_base: int = 0, out_id: Optional[torch.Tensor] = None,
            out_val: Optional[torch.Tensor] = None):
     rows, vocab = logits.shape
@@ -132,25 +144,42 @@ def pick_splits(rows: int, n: int, k: int, bn: int, sms: int = 148) -> int:
     return max(1, min(want, kb // 8))
 
 
-# 4-bit weights at prefill sizes can run on CTA pairs (`gemm_tc_pair.cu`: 256 weight rows x 256 tokens per pair, each
-# SM loading half of the activation tile); results are bit-identical to the single-CTA kernel.  Off by default: it
-# measured slower (537 against 596-662 TFLOP/s at 2048 x 34816 x 5120).
-PAIR_GEMM = False
-PAIR_GEMM_MIN_ROWS = 512
+# 4-bit weights at prefill sizes run on CTA pairs (`gemm_tc_pair.cu`: 256 weight rows x up to 256 tokens per pair, converted
+# weights in tensor memory).  Without split-K the results are those of the single-CTA kernel bit for bit.
+PAIR_GEMM = True
+PAIR_GEMM_MIN_ROWS = 1
 
-_lib.declare("dgpp_gemm_tc_pair", [I, P, L, P, P, F, P, P, I, I, I, I, P])
+_lib.declare("dgpp_gemm_tc_pair", [I, P, L, P, P, F, P, P, I, I, I, I, I, I, P, L, P, I, P])
 
 
-def gemm_tc_pair(x: torch.Tensor, w: QuantLinear, out: Optional[torch.Tensor] = None,
-                 resid: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """The W4A16 linear on CTA pairs (NVFP4 / MXFP4 weights, N a multiple of 256)."""
+def gemm_tc_pair(x: torch.Tensor, w: QuantLinear, out: Optional[torch.Tensor] = None, resid: Optional[torch.Tensor] = None,
+                 bn: int = 0, splits: int = 1, ws: Optional[GemmWorkspace] = None) -> torch.Tensor:
+    """The W4A16 linear on CTA pairs (NVFP4 / MXFP4 weights).  bn: tokens per tile (a multiple of 16 up to 256; 0: chosen by the
+    library); splits: K splits (0: chosen by the library)."""
     _chk(x, torch.bfloat16, "x")
     rows, k = x.shape
-    assert k == w.k and w.fmt in ("nvfp4", "mxfp4") and w.n % 256 == 0 and k % 256 == 0
+    assert k == w.k and w.fmt in ("nvfp4", "mxfp4") and k % 256 == 0
     if out is None:
         out = torch.empty(rows, w.n, dtype=torch.bfloat16, device=x.device)
+    if splits != 1:
+        ws = ws or default_workspace(x.device)
+    wsp, cnt = (ws.partials, ws.counters) if splits != 1 else (None, None)
     call("dgpp_gemm_tc_pair", _FMT_GEMM[w.fmt], ptr(x), x.stride(0), ptr(w.payload), ptr(w.scale), float(w.alpha), ptr(out),
-         ptr(resid), out.stride(0), rows, w.n, k, stream_ptr())
+         ptr(resid), out.stride(0), rows, w.n, k, bn, splits, ptr(wsp), wsp.numel() if wsp is not None else 0, ptr(cnt),
+         cnt.numel() if cnt is not None else 0, stream_ptr())
+    return out
+
+
+_lib.declare("dgpp_gemm_tc_pair_grouped", [P, L, P, P, P, P, P, I, I, I, I, I, I, P])
+
+
+def gemm_tc_pair_grouped(x: torch.Tensor, wq, wsf_tiled, alphas, out: torch.Tensor, n: int, k: int, experts: int, tiles,
+                         bn: int) -> torch.Tensor:
+    """W4A16 over stacked expert matrices (NVFP4, scales in `tile_scales` order): rows t * bn .. of `out` are those of x times
+    matrix tiles[t]; tiles with a negative entry are left alone."""
+    _chk(x, torch.bfloat16, "x")
+    call("dgpp_gemm_tc_pair_grouped", ptr(x), x.stride(0), ptr(wq), ptr(wsf_tiled), ptr(alphas), ptr(tiles), ptr(out), n,
+         tiles.numel(), n, k, experts, bn, stream_ptr())
     return out
 
 
@@ -164,8 +193,8 @@ def gemm_tc(x: torch.Tensor, w: QuantLinear, out: Optional[torch.Tensor] = None,
     assert k == w.k, (k, w.k)
     assert w.fmt in _FMT_GEMM, w.fmt
     if (PAIR_GEMM and out32 is None and bn is None and splits in (None, 1) and rows >= PAIR_GEMM_MIN_ROWS
-            and w.fmt in ("nvfp4", "mxfp4") and w.n % 256 == 0 and k % 256 == 0):
-        return gemm_tc_pair(x, w, out=out, resid=resid)
+            and w.fmt in ("nvfp4", "mxfp4") and k % 256 == 0 and w.scale.data_ptr() % 16 == 0):
+        return gemm_tc_pair(x, w, out=out, resid=resid, splits=splits or 0, ws=ws)
     if out is None and out32 is None:
         out = torch.empty(rows, w.n, dtype=torch.bfloat16, device=x.device)
     ldc = (out if out is not None else out32).stride(0)
