@@ -268,13 +268,14 @@ class HybridRunner:
         for st in self.gdn_state.values():
             st.reset(slot)
 
-    def _ffn(self, i: int, L: HybridLayer, xn: torch.Tensor, out: torch.Tensor, xa=None) -> None:
+    def _ffn(self, i: int, L: HybridLayer, xn: torch.Tensor, out: torch.Tensor, xa=None, prompt: bool = False) -> None:
         if L.moe is not None and i in self.ep:
             (self.ep_small[i] if xn.shape[0] <= 16 else self.ep[i]).forward(xn, out=out)
             return
         if L.moe is not None:
             blk = self.moe.get(i)
-            wide = self.moe_wide.get(i)
+            # (prompt rows take the gathered path whether or not wide blocks exist: their bits must not depend on speculation)
+            wide = None if prompt else self.moe_wide.get(i)
             if blk is not None and xn.shape[0] <= blk.max_rows:
                 blk.forward(xn, out, xa=xa if (xa is not None and blk.bn == xa.bn and blk.terms == xa.terms) else None)
             elif wide is not None and xn.shape[0] <= wide.max_rows:
@@ -345,7 +346,7 @@ class HybridRunner:
                 xa = dq.norm(x, L.post_norm, c.eps, delta=delta, x_out=xn, tag="h")
             else:
                 ops.rmsnorm(x, L.post_norm, c.eps, delta=delta, out=xn)
-            self._ffn(i, L, xn, delta, xa=xa)
+            self._ffn(i, L, xn, delta, xa=xa, prompt=chunk_slot is not None)
         ops.rmsnorm(x, m.final_norm, c.eps, delta=delta, out=xn)
         sel = xn if all_logits else xn[rows - 1:rows]
         return ops.gemm_tc(sel, m.head, out32=self.logits[:sel.shape[0]])

@@ -278,6 +278,8 @@ class MoEBlock:
         (reference counterparts: src/kernels/glm_moe.cu:1382 segment count, :1553 tile list, :1121 grouped MMA.)"""
         c, w = self.c, self.w
         T = xn.shape[0]
+        if self.prefill_terms > 1 and c.hidden % 256 == 0 and c.moe_ffn % 256 == 0:
+            return self._gathered_bf16(xn)
         bn, R = 64, self.prefill_terms
         max_tiles = (T * c.top_k + bn - 1) // bn + self.local_experts
         ws = _prefill_workspace(xn.device, max_tiles, bn, c.hidden, c.moe_ffn, R)
@@ -301,6 +303,33 @@ class MoEBlock:
             sh = ops.linear(ops.swiglu(ops.linear(xn, w.shared_gu), limit=c.swiglu_limit, alpha=c.swiglu_alpha), w.shared_down)
         out = torch.empty(T, c.hidden, dtype=BF, device=xn.device)
         return ops.moe_combine_rows(y.view(rows, c.hidden), sh, pair_row, wts, out)
+
+    def _gathered_bf16(self, xn: torch.Tensor) -> torch.Tensor:
+        """`forward_gathered` with bf16 activations: the tiles' rows go through the W4A16 GEMM on CTA pairs as they are, so no
+        quantiser runs and a product is one bf16 MMA instead of one per residual term.  A tile costs a pair about
+        the same up to 128 rows, so tiles are as wide as most experts' rows need."""
+        c, w = self.c, self.w
+        T = xn.shape[0]
+        mean = T * c.top_k / c.experts
+        bn = next((b for b in (32, 64, 128) if mean * 1.25 <= b), 192)
+        max_tiles = (T * c.top_k + bn - 1) // bn + self.local_experts
+        ws = _prefill_workspace(xn.device, max_tiles, bn, c.hidden, c.moe_ffn, 0)
+        ids, wts = ops.moe_route(xn, w.gate, w.bias, c.top_k, c.n_group, c.topk_group, c.router == "softmax",
+                                 c.norm_topk_prob, c.routed_scaling)
+        tiles = ws["tile_expert"][:max_tiles]
+        pair_row, _, _ = ops.moe_segment_sort(ids, bn, max_tiles, self.e0, self.e1, ws["pair_row"][:T * c.top_k], tiles,
+                                              ws["n_tiles"])
+        rows = max_tiles * bn
+        xs, h, act, y = ws["xs"][:rows], ws["h"].view(-1, 2 * c.moe_ffn)[:rows], ws["act"][:rows], ws["y"].view(-1, c.hidden)[:rows]
+        ops.moe_gather_rows(xn, pair_row, xs, c.top_k)
+        ops.gemm_tc_pair_grouped(xs, w.gu_q, w.gu_sf, w.gu_alpha, h, 2 * c.moe_ffn, c.hidden, self.stack_experts, tiles, bn)
+        ops.swiglu_tiles(h, act, tiles, bn, c.swiglu_limit, c.swiglu_alpha)
+        ops.gemm_tc_pair_grouped(act, w.down_q, w.down_sf, w.down_alpha, y, c.hidden, c.moe_ffn, self.stack_experts, tiles, bn)
+        sh = None
+        if w.shared_gu is not None:
+            sh = ops.linear(ops.swiglu(ops.linear(xn, w.shared_gu), limit=c.swiglu_limit, alpha=c.swiglu_alpha), w.shared_down)
+        out = torch.empty(T, c.hidden, dtype=BF, device=xn.device)
+        return ops.moe_combine_rows(y, sh, pair_row, wts, out)
 
     def forward_looped(self, xn: torch.Tensor) -> torch.Tensor:
         """Oracle of forward_gathered: one exact W4A16 GEMM pair per active expert over its gathered rows (host loop)."""
@@ -337,8 +366,10 @@ def _prefill_workspace(device, max_tiles: int, bn: int, hidden: int, ffn: int, t
                   n_tiles=torch.zeros(1, **i32),
                   xs=torch.zeros(rows, hidden, dtype=BF, device=device),
                   h=torch.zeros(max_tiles, bn, 2 * ffn, dtype=BF, device=device),
-                  y=torch.zeros(max_tiles, bn, hidden, dtype=BF, device=device),
-                  qa_x=ops.QuantAct(rows, hidden, terms, bn, device),
-                  qa_mid=ops.QuantAct(rows, ffn, terms, bn, device))
+                  y=torch.zeros(max_tiles, bn, hidden, dtype=BF, device=device))
+        if terms:
+            ws.update(qa_x=ops.QuantAct(rows, hidden, terms, bn, device), qa_mid=ops.QuantAct(rows, ffn, terms, bn, device))
+        else:      # bf16 activations
+            ws["act"] = torch.zeros(rows, ffn, dtype=BF, device=device)
         _PREFILL_WS[key] = ws
     return ws

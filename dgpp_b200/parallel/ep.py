@@ -103,8 +103,14 @@ class EpMoE:
         self.xs = shared("xs", lambda: torch.zeros(rows, c.hidden, dtype=BF, device=device))
         self.h = shared("h", lambda: torch.zeros(self.max_tiles, self.bn, 2 * c.moe_ffn, dtype=BF, device=device))
         self.y = shared("y", lambda: torch.zeros(self.max_tiles, self.bn, c.hidden, dtype=BF, device=device))
-        self.qa_x = shared("qa_x", lambda: ops.QuantAct(rows, c.hidden, act_terms, self.bn, device))
-        self.qa_mid = shared("qa_mid", lambda: ops.QuantAct(rows, c.moe_ffn, act_terms, self.bn, device))
+        # bf16 activations through the W4A16 GEMM on CTA pairs, as MoEBlock.forward_gathered does (the same bits per row);
+        # a single term asks for 4-bit activations
+        self.bf16 = act_terms > 1 and c.hidden % 256 == 0 and c.moe_ffn % 256 == 0
+        if self.bf16:
+            self.act = shared("act", lambda: torch.zeros(rows, c.moe_ffn, dtype=BF, device=device))
+        else:
+            self.qa_x = shared("qa_x", lambda: ops.QuantAct(rows, c.hidden, act_terms, self.bn, device))
+            self.qa_mid = shared("qa_mid", lambda: ops.QuantAct(rows, c.moe_ffn, act_terms, self.bn, device))
 
     def forward(self, xn: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """xn: this rank's rows [T, H] bf16 (1 <= T <= max_rows; every rank calls with its own T).  Returns [T, H]."""
@@ -123,13 +129,20 @@ class EpMoE:
                              self.n_tiles)
         call("dgpp_ep_gather", self.comm, ptr(self.recv_src), ptr(self.pair_row), ptr(self.xs), k, H, E, mp, st)
         rows = self.max_tiles * self.bn
-        xa = ops.act_quant_nvfp4(self.xs, self.terms, out=self.qa_x, group_list=self.tiles, group_rows=self.bn)
-        ops.gemm_fp4_grouped(xa, w.gu_q, w.gu_sf, w.gu_alpha, self.h, self.bn, 2 * c.moe_ffn, H, self.local, self.tiles,
-                             group_b=True)
-        xm = ops.act_quant_nvfp4(self.h.view(rows, 2 * c.moe_ffn), self.terms, out=self.qa_mid, mode="swiglu",
-                                 limit=c.swiglu_limit, alpha=c.swiglu_alpha, group_list=self.tiles, group_rows=self.bn)
-        ops.gemm_fp4_grouped(xm, w.down_q, w.down_sf, w.down_alpha, self.y, self.bn, H, c.moe_ffn, self.local, self.tiles,
-                             group_b=True)
+        if self.bf16:
+            h, y = self.h.view(rows, 2 * c.moe_ffn), self.y.view(rows, H)
+            stacked = w.gu_q.shape[0] // (2 * c.moe_ffn)
+            ops.gemm_tc_pair_grouped(self.xs, w.gu_q, w.gu_sf, w.gu_alpha, h, 2 * c.moe_ffn, H, stacked, self.tiles, self.bn)
+            ops.swiglu_tiles(h, self.act, self.tiles, self.bn, c.swiglu_limit, c.swiglu_alpha)
+            ops.gemm_tc_pair_grouped(self.act, w.down_q, w.down_sf, w.down_alpha, y, H, c.moe_ffn, stacked, self.tiles, self.bn)
+        else:
+            xa = ops.act_quant_nvfp4(self.xs, self.terms, out=self.qa_x, group_list=self.tiles, group_rows=self.bn)
+            ops.gemm_fp4_grouped(xa, w.gu_q, w.gu_sf, w.gu_alpha, self.h, self.bn, 2 * c.moe_ffn, H, self.local, self.tiles,
+                                 group_b=True)
+            xm = ops.act_quant_nvfp4(self.h.view(rows, 2 * c.moe_ffn), self.terms, out=self.qa_mid, mode="swiglu",
+                                     limit=c.swiglu_limit, alpha=c.swiglu_alpha, group_list=self.tiles, group_rows=self.bn)
+            ops.gemm_fp4_grouped(xm, w.down_q, w.down_sf, w.down_alpha, self.y, self.bn, H, c.moe_ffn, self.local, self.tiles,
+                                 group_b=True)
         call("dgpp_ep_return", self.comm, ptr(self.recv_src), ptr(self.pair_row), ptr(self.y), k, H, E, mp, st)
         sh = None
         if w.shared_gu is not None:

@@ -257,3 +257,65 @@ def test_pair_gemm_is_bit_identical_to_the_single_cta_kernel(fmt, rows, n, k):
     assert torch.equal(got, want) and torch.equal(got_r, want_r)
     ref = (x.float() @ w.dequant().float().t())
     assert (got.float() - ref).abs().max().item() <= 2e-2 * ref.abs().max().item() + 1e-2
+
+
+@pytest.mark.parametrize("rows,n,k,bn,splits", [(1, 256, 256, 0, 1), (15, 8224, 512, 16, 1), (17, 520, 1024, 32, 1), (257, 768, 768, 256, 1),
+                                                (300, 384, 512, 240, 1), (8, 512, 2048, 0, 3), (173, 1000, 2048, 96, 4),
+                                                (64, 260, 1024, 0, 2)])
+def test_pair_gemm_tiles_and_splits(rows, n, k, bn, splits):
+    """Token tiles of any multiple of 16, ragged N (full and partial row vectors), one round and several: the single-CTA kernel's
+    bits without splits.  With splits only the fp32 sums are grouped differently (1e-5 of the sum of |terms|, k <= 2048 adds
+    in 2^-24), then one bf16 rounding of each (2^-8)."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from dgpp_b200.ops import core as ops
+    from dgpp_b200.quant.formats import random_quant_linear
+
+    dev = torch.device("cuda:0")
+    torch.manual_seed(rows * n)
+    w = random_quant_linear(n, k, "nvfp4", dev)
+    x = torch.randn(rows, k, device=dev).to(torch.bfloat16)
+    resid = torch.randn(rows, n, device=dev).to(torch.bfloat16)
+    old = ops.PAIR_GEMM
+    try:
+        ops.PAIR_GEMM = False
+        want, want_r = ops.gemm_tc(x, w, splits=1), ops.gemm_tc(x, w, resid=resid, splits=1)
+    finally:
+        ops.PAIR_GEMM = old
+    for _ in range(2):                                   # the second call finds the counters as the first left them
+        got, got_r = ops.gemm_tc_pair(x, w, bn=bn, splits=splits), ops.gemm_tc_pair(x, w, resid=resid, bn=bn, splits=splits)
+        torch.cuda.synchronize()
+        ops.check_status()
+        if splits == 1:
+            assert torch.equal(got, want) and torch.equal(got_r, want_r)
+        else:
+            terms = x.float().abs() @ w.dequant().abs().t()
+            assert ((got.float() - want.float()).abs() <= 2 ** -7 * want.float().abs() + 1e-5 * terms).all()
+            assert ((got_r.float() - want_r.float()).abs() <= 2 ** -7 * (want.float().abs() + want_r.float().abs()) + 1e-5 * terms).all()
+
+
+@pytest.mark.parametrize("bn", [32, 128, 192])
+def test_pair_gemm_grouped_equals_the_plain_form_per_matrix(bn):
+    """Stacked matrices, tiles in any order with skipped ones between: every tile's rows are those of the plain product with its
+    matrix, skipped tiles keep what was there."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from dgpp_b200.ops import core as ops
+    from dgpp_b200.quant.formats import random_quant_linear
+
+    dev = torch.device("cuda:0")
+    torch.manual_seed(bn)
+    n, k, experts = 512, 768, 5
+    ws = [random_quant_linear(n, k, "nvfp4", dev) for _ in range(experts)]
+    q, sf = torch.cat([w.payload for w in ws]), torch.cat([w.tiled_scales().reshape(-1) for w in ws])
+    alphas = torch.tensor([w.alpha for w in ws], device=dev)
+    groups = [3, 0, 0, -1, 4, 1, -1]
+    x = torch.randn(len(groups) * bn, k, device=dev).to(torch.bfloat16)
+    out = torch.full((len(groups) * bn, n), 7.0, device=dev, dtype=torch.bfloat16)
+    ops.gemm_tc_pair_grouped(x, q, sf, alphas, out, n, k, experts, torch.tensor(groups, dtype=torch.int32, device=dev), bn)
+    torch.cuda.synchronize()
+    ops.check_status()
+    for t, e in enumerate(groups):
+        rows = slice(t * bn, (t + 1) * bn)
+        want = ops.gemm_tc_pair(x[rows], ws[e]) if e >= 0 else torch.full_like(out[rows], 7.0)
+        assert torch.equal(out[rows], want), (t, e)
