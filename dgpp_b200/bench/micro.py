@@ -130,7 +130,6 @@ def bench_gemm_tc(args, dev):
     ops.check_status()
     report(args, "gemm_tc", ms, bytes_=ws[0].nbytes + rows * k * 2 + rows * n * 2, flops=2.0 * rows * n * k, rows=rows, n=n, k=k,
            fmt=args.fmt, cta_pairs=bool(ops.PAIR_GEMM and rows >= ops.PAIR_GEMM_MIN_ROWS and args.fmt in ("nvfp4", "mxfp4")))
-                                        and n % 256 == 0))
 
 
 def bench_gemm_fp8(args, dev):
