@@ -75,11 +75,17 @@ struct Fp4Params {
   unsigned long long* trace;  // debug: CTA (0,0,0) stores %globaltimer at 7 points of its life (see dgpp_gemm_fp4_set_trace)
   int preload;             // dense mode: issue the weight half of the first ring stages before waiting on the preceding grid
   // Split-K inside a thread-block cluster (decode projections with few output tiles): the gridDim.z CTAs of one output
-  // tile form a cluster (1, 1, splits); each runs its share of the K stages, then the partial accumulators of ranks
-  // 1.. travel through distributed shared memory into rank 0's (by then idle) operand ring and rank 0 adds them in
-  // ascending rank order.  No workspace, no global counters; two cluster barriers.
+  // tile form a cluster (1, 1, splits); each runs its share of the K stages and leaves its partial sums in its (by then
+  // idle) operand ring; every rank then adds its share of the tokens over all rings, in ascending rank order, through
+  // distributed shared memory.  No workspace, no global counters; two cluster barriers.
   int cluster_split;
 };
+
+__device__ __forceinline__ float ld_shared_cluster_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
 
 // One bf16 of the finished output tile -> slot `rank` of every rank (destinations staggered by rank).
 __device__ __forceinline__ void push_value(const Fp4Params& p, int parity, size_t idx, bf16 v) {
@@ -286,80 +292,70 @@ gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmA,   // packed weights as 
   }
   if (p.cluster_split) {
     // Every thread of every CTA of the cluster passes the same two barriers, whatever happened before (a CTA that
-    // gave up on a wait still arrives), so the cluster cannot block on a peer.
+    // gave up on a wait still arrives), so the cluster cannot block on a peer.  Each CTA leaves its partial sums in its own
+    // (by then idle) operand ring and folds every splits-th token of all of them, in ascending rank order (with the all-reduce push
+    // rank 0 folds them all: one CTA raises the tile's flag).
     const int q = warp & 3;
     const int cols = min(bn_tok, p.T - m0);
-    float* red = reinterpret_cast<float*>(sA);          // rank 0: [splits - 1][bn_tok][128] partials of the peers
-    cluster_barrier();                                   // every CTA's mainloop is over: rank 0's operand ring is idle
-    if (warp >= 2 && split > 0 && acc_ok && !*abort_flag) {
-      for (int c0 = 0; c0 < bn_tok; c0 += 16) {
-        if (c0 >= cols) break;
+    float* red = reinterpret_cast<float*>(sA);          // [bn_tok][128]
+    float scale[4];                                      // of this CTA's first tokens, requested before the barrier
+    if (warp >= 2) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int m = split + i * splits;
+        scale[i] = (p.push || m >= cols) ? 0.f : gvec[m0 + m];
+      }
+      for (int c0 = 0; c0 < cols; c0 += 16) {
         float v[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) v[j] = 0.f;
-        if (nst > 0) {
+        if (nst > 0 && acc_ok) {
           for (int r = 0; r < p.R; ++r) {
             uint32_t rr[16];
             tmem_ld_x16(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + r * bn_tok + c0, rr);
-            tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(rr[j]);
           }
         }
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int m = c0 + j;
-          if (m < cols)
-            st_shared_cluster_f32(mapa_shared(smem_u32(red + (static_cast<size_t>(split - 1) * bn_tok + m) * kF4BM + q * 32 + lane), 0u),
-                                  v[j]);
-        }
+        for (int j = 0; j < 16; ++j)
+          if (c0 + j < cols) red[(c0 + j) * kF4BM + q * 32 + lane] = v[j];
       }
     }
-    cluster_barrier();                                   // the partials have landed in rank 0
-    if (warp >= 2 && split == 0) {
+    cluster_barrier();                                   // every rank's partial sums are in place
+    if (warp >= 2 && (split == 0 || !p.push)) {
       const int n = n0 + q * 32 + lane;
       const uint32_t push_epoch = p.push ? *p.comm.epoch + 1 : 0u;
       const int push_parity = push_epoch & 1;
-      if (acc_ok && !*abort_flag) {
-        for (int c0 = 0; c0 < bn_tok; c0 += 16) {
-          if (c0 >= cols) break;
-          float v[16];
+      if (acc_ok && !*abort_flag && n < p.N) {
+        const int step = p.push ? 1 : splits;
+        for (int m = p.push ? 0 : split, i = 0; m < cols; m += step, ++i) {
+          const uint32_t at = smem_u32(red + m * kF4BM + q * 32 + lane);
+          float t[8];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = 0.f;
-          if (nst > 0) {
-            for (int r = 0; r < p.R; ++r) {
-              uint32_t rr[16];
-              tmem_ld_x16(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + r * bn_tok + c0, rr);
-              tmem_ld_wait();
+          for (int r = 0; r < 8; ++r)
+            if (r < splits) t[r] = ld_shared_cluster_f32(mapa_shared(at, static_cast<uint32_t>(r)));
+          float acc = t[0];
 #pragma unroll
-              for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(rr[j]);
-            }
+          for (int r = 1; r < 8; ++r)
+            if (r < splits) acc += t[r];
+          const size_t o = static_cast<size_t>(m0 + m) * p.ldc + n;
+          const float g = (p.push || i > 3) ? gvec[m0 + m] : (i == 0 ? scale[0] : (i == 1 ? scale[1] : (i == 2 ? scale[2] : scale[3])));
+          float y = acc * alpha * g;
+          if (p.push) {
+            push_value(p, push_parity, static_cast<size_t>(m0 + m) * p.N + n, f32_to_bf16(y));
+            continue;
           }
-          if (n < p.N) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const int m = c0 + j;
-              if (m < cols) {
-                float acc = v[j];
-                for (int s2 = 1; s2 < splits; ++s2) acc += red[(static_cast<size_t>(s2 - 1) * bn_tok + m) * kF4BM + q * 32 + lane];
-                const size_t o = static_cast<size_t>(m0 + m) * p.ldc + n;
-                float y = acc * alpha * gvec[m0 + m];
-                if (p.push) {
-                  push_value(p, push_parity, static_cast<size_t>(m0 + m) * p.N + n, f32_to_bf16(y));
-                  continue;
-                }
-                if (p.out32) p.out32[o] = y;
-                if (p.out) {
-                  if (p.resid) y = bf16_to_f32(p.resid[o]) + bf16_to_f32(f32_to_bf16(y));
-                  p.out[o] = f32_to_bf16(y);
-                }
-              }
-            }
+          if (p.out32) p.out32[o] = y;
+          if (p.out) {
+            if (p.resid) y = bf16_to_f32(p.resid[o]) + bf16_to_f32(f32_to_bf16(y));
+            p.out[o] = f32_to_bf16(y);
           }
         }
       }
       if (p.push) push_flags(p, push_parity, push_epoch, warp, lane);
     }
+    cluster_barrier();                                   // nobody leaves while its partial sums may still be read
   } else if (warp >= 2) {
     const int q = warp & 3;
     const bool ok = acc_ok;
@@ -666,8 +662,7 @@ static int launch_fp4(const CUtensorMap& tA, const CUtensorMap& tB, const Fp4Par
   dim3 grid(p.grid_x > 0 ? p.grid_x : dgpp_ceil_div(p.N, kF4BM), dgpp_ceil_div(p.T, bn_tok), splits);
   if (p.cluster_split) {
     DGPP_REQUIRE(splits >= 2 && splits <= 8, "gemm_fp4: cluster split-K takes 2..8 splits, got %d", splits);
-    DGPP_REQUIRE(static_cast<size_t>(splits - 1) * bn_tok * kF4BM * 4 <= static_cast<size_t>(C::S) * kF4StageA,
-                 "gemm_fp4: %d splits x %d tokens do not fit the operand ring for the cluster fold", splits, bn_tok);
+    static_assert(static_cast<size_t>(BN) * kF4BM * 4 <= C::S * C::stage_bytes(), "a CTA's partial sums fit its operand ring");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(kF4Threads, 1, 1);

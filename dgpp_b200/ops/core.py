@@ -371,10 +371,10 @@ def gemm_fp4(xa: QuantAct, w: QuantLinear, out: Optional[torch.Tensor] = None,
         out = torch.empty(rows, w.n, dtype=torch.bfloat16, device=dev)
     ldc = w.n if push_comm and out is None and out32 is None else (out if out is not None else out32).stride(0)
     if cluster is None:
-        cluster = CLUSTER_SPLITK
+        cluster = CLUSTER_SPLITK or (FP4_SPLIT_POLICY == "auto" and not push_comm and splits is None)
     if splits is None:
         splits = pick_cluster_splits(rows, w.n, w.k, bn) if cluster else pick_splits_fp4(rows, w.n, w.k, bn)
-    cluster = cluster and 2 <= splits <= 8 and (splits - 1) * bn * 512 <= 65536
+    cluster = cluster and 2 <= splits <= 8
     wsp = cnt = None
     if splits > 1 and not cluster:
         ws = ws or default_workspace(dev)
@@ -409,27 +409,23 @@ def configure(fp4_splits: Optional[str] = None, cluster_splitk: Optional[bool] =
 
 
 def pick_cluster_splits(rows: int, n: int, k: int, bn: int) -> int:
-    """Cluster split-K for projections with few output tiles (decode qkv / o / down): a CTA that walks 20+ K stages
-    alone is bound by the latency of its own scale-copy -> MMA -> commit chain, not by bandwidth; splitting K over the
-    CTAs of a cluster shortens the chain and puts two CTAs on every SM.  At least 4 stages per CTA, cluster sizes 2 / 4 /
-    8, and two to three resident CTAs per SM in total."""
-    tiles = math.ceil(n / 128) * math.ceil(rows / bn)
-    stages = k // 256
-    if rows > 64 or tiles > 74 or stages < 8:
-        return 1
-    want = min(8, max(1, 444 // tiles), stages // 4)
-    s = 1
-    while s * 2 <= want and (s * 2 - 1) * bn * 512 <= 65536:      # cluster sizes 2 / 4 / 8
-        s *= 2
-    return s
+    """Cluster split-K for projections with few output tiles: a CTA that walks many K stages alone is bound by the latency of its
+    own scale-copy -> MMA -> commit chain (600 cycles per stage), not by bandwidth.  As many CTAs as run at once (264 of the 296
+    that two per SM would be: clusters do not fill a GPC evenly), two stages each at least.  Measured at 8 rows, us unsplit /
+    split through the workspace / so: 5120 x 5120 12.4 / 12.0 / 8.5, 5120 x 17408 28 / 16.8 / 13.2, 2048 x 5632 12.5 / 10.3 / 6.5,
+    11264 x 2048 9.0 / 10.8 / 8.4, 24576 x 4096 14.9 / 21.4 / 18.9.  The same at every row count, so that a row's bits do
+    not depend on how many share its pass."""
+    tiles, stages = math.ceil(n / 128) * math.ceil(rows / bn), k // 256
+    return max(1, min(8, 264 // tiles, stages // 2)) if tiles <= 99 else 1
 
 
 # Split-K policy of the block-scaled GEMM in the weight-streaming regime.  "resident": split until one resident wave
 # (two CTAs per SM) covers the problem, so that with the pre-wait weight preload most of a CTA's K range is already
 # in its ring when the activations arrive; "legacy": split only long-K, few-tile problems.
-# Measured on the 27B-class decode step: C8 7.14 ms legacy / 7.34 ms resident, C1 165.7 / 169.8 tok/s -- the fold's
-# fences and counter round trip cost more than the shorter K range saves once 8 rows share the weights, so "auto"
-# takes resident for a single row and legacy otherwise.
+# Measured on the 27B-class decode step: C8 7.14 ms legacy / 7.34 ms resident, C1 165.7 / 169.8 tok/s -- the workspace fold's
+# fences and counter round trip cost more than the shorter K range saves once 8 rows share the weights.  "auto" folds through
+# distributed shared memory instead (`pick_cluster_splits`), except with the all-reduce push, which takes resident for a
+# single row and legacy otherwise.
 FP4_SPLIT_POLICY = "auto"
 
 
