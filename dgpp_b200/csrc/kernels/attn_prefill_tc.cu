@@ -4,15 +4,21 @@
 // from the cache pages by TMA exactly as stored (e4m3 bytes); nothing converts them:
 //
 //   MMA1   S[q, t]  = (Q1 + Q2)[q, d] . K[t, d]^T          Q split into two e4m3 terms (A operand, K-major)
-//   softmax (thread = query row): s = S * q_scale[q] * k_scale[t] * sm_scale, causal mask, running max / sum,
+//   softmax (two threads per query row, 64 tokens each): s = S * q_scale[q] * k_scale[t] * sm_scale, causal mask, running max / sum,
 //           P[q, t] = p * v_scale[t] * c_tile split into two e4m3 terms, written as the next A operand
 //   MMA2   O_tile[q, d] = (P1 + P2)[q, t] . V[t, d]        V is the B operand read MN-major (d contiguous)
-//   accumulate (thread = query row, 128 fp32 registers): o = o * corr + O_tile / c_tile
+//   accumulate (two threads per query row, 64 fp32 registers each): o = o * corr + O_tile / c_tile
 //
 // S is double buffered in TMEM so MMA1 of tile i + 1 overlaps the softmax of tile i; the PV product of tile i
 // runs while the softmax threads exponentiate tile i + 1.  Both splits keep ~2^-8 relative operand error
 // (e4m3 value + e4m3 residual), K and V are exact.
-// Warps: 0 = TMA producer (pages + their scales), 1 = MMA issuer / TMEM owner, 2..5 = softmax (one row each).
+// Warps: 0 = TMA producer (pages + their scales), 1 = MMA issuer / TMEM owner, 2..9 = softmax: warps w and w + 4 share a TMEM lane
+// quadrant, the first has a row's tokens (and output columns) 0..63, the second 64..127; the halves of a row exchange
+// their maxima at the barrier that the tile's V scales need anyway, and their sums once at the end.
+// What bounds it: the softmax threads (some 25 instructions per score and 60 waits for TMEM loads per tile); one warp per
+// scheduler could not hide its own latencies.  Row tiles are dealt longest first.
+// One thread per row / two: a whole pass of 16 layers, 40 query and 8 KV heads at 8192 rows 119.0 / 110.9 ms, 2048 rows 22.98 / 21.85, 173 rows
+// 5.25 / 4.95 (the linears of the pass are in both figures).
 // (reference counterparts: src/kernels/full_attn.cu:442,679,983 tile / TMA / fp8-compute prefill kernels.)
 #include <cuda.h>
 #include <math.h>
@@ -25,7 +31,8 @@
 
 namespace dgpp {
 
-constexpr int kApThreads = 192;
+constexpr int kApThreads = 320;
+constexpr int kApHalf = 64;       // tokens and output columns of one softmax thread
 constexpr int kApTile = 128;
 constexpr int kApStages = 3;
 
@@ -45,12 +52,12 @@ __device__ __forceinline__ uint32_t sw128_off(uint32_t row, uint32_t byte_in_row
   return row * 128u + ((((byte_in_row >> 4) ^ (row & 7u)) << 4) | (byte_in_row & 15u));
 }
 
-// Row maximum of raw score * k_scale over one 128-token tile (thread = query row, scores read from TMEM).
+// Row maximum of raw score * k_scale over the 64 tokens from `cb` of a tile (scores read from TMEM).
 template <bool kMask>
-__device__ __forceinline__ float tile_row_max(uint32_t taddr, const float* ks, int t0, int my_pos, int my_first) {
+__device__ __forceinline__ float tile_row_max(uint32_t taddr, const float* ks, int cb, int t0, int my_pos, int my_first) {
   float mt = -INFINITY;
 #pragma unroll 2
-  for (int c0 = 0; c0 < kApTile; c0 += 16) {
+  for (int c0 = cb; c0 < cb + kApHalf; c0 += 16) {
     uint32_t raw[16];
     tmem_ld_x16(taddr + c0, raw);
     tmem_ld_wait();
@@ -73,14 +80,14 @@ __device__ __forceinline__ float tile_row_max(uint32_t taddr, const float* ks, i
   return mt;
 }
 
-// Probabilities of one tile: p = 2^(raw * k_scale * sm - m); P = p * v_scale * c_tile as two e4m3 terms written
+// Probabilities of 64 tokens: p = 2^(raw * k_scale * sm - m); P = p * v_scale * c_tile as two e4m3 terms written
 // to row r of the swizzled A operand (term 2 one tile further).  Returns the row sum of p.
 template <bool kMask>
 __device__ __forceinline__ float tile_probs(uint32_t taddr, const float* ks, const float* vs, unsigned char* sP, int r,
-                                            float sm, float neg_m, float c_tile, int t0, int my_pos, int my_first) {
+                                            float sm, float neg_m, float c_tile, int cb, int t0, int my_pos, int my_first) {
   float lsum = 0.f;
 #pragma unroll 2
-  for (int c0 = 0; c0 < kApTile; c0 += 16) {
+  for (int c0 = cb; c0 < cb + kApHalf; c0 += 16) {
     uint32_t raw[16];
     tmem_ld_x16(taddr + c0, raw);
     tmem_ld_wait();
@@ -125,7 +132,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
   unsigned char* sV = sp;  sp += kApStages * kTileBytes;
   float* sKs = reinterpret_cast<float*>(sp);  sp += kApStages * kApTile * sizeof(float);
   float* sVs = reinterpret_cast<float*>(sp);  sp += kApStages * kApTile * sizeof(float);
-  float* red = reinterpret_cast<float*>(sp);  sp += 2 * 8 * sizeof(float);
+  float* red = reinterpret_cast<float*>(sp);  sp += 2 * 16 * sizeof(float);           // [parity][4 maxima of V scales, 8 verdicts]
+  float* mx = reinterpret_cast<float*>(sp);   sp += 2 * 2 * kApTile * sizeof(float);  // [parity][half][row] maxima (last: row sums)
   uint64_t* kv_full = reinterpret_cast<uint64_t*>(sp);
   uint64_t* kv_empty = kv_full + kApStages;
   uint64_t* s_full = kv_empty + kApStages;   // [2]
@@ -135,8 +143,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int head = blockIdx.y, kvh = head / (p.hq / p.hkv);
-  const int row0 = blockIdx.x * kApTile;                      // first chunk row of this CTA
+  const int head = blockIdx.x, kvh = head / (p.hq / p.hkv);
+  const int row0 = static_cast<int>(gridDim.y - 1 - blockIdx.y) * kApTile;   // first chunk row of this CTA, the longest spans first
   const int rows = min(kApTile, p.T - row0);
   const int last_pos = p.pos0 + row0 + rows - 1;
   const int first_pos = p.pos0 + row0;
@@ -147,7 +155,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
   if (threadIdx.x == 0) {
     for (int i = 0; i < kApStages; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1); }
     mbar_init(&s_full[0], 1); mbar_init(&s_full[1], 1);
-    mbar_init(p_full, 4);
+    mbar_init(p_full, 8);
     mbar_init(o_full, 1);
     *abort_flag = 0;
     fence_mbar_init();
@@ -159,35 +167,39 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     tmem_relinquish();
   }
   pdl_wait();
-  // ---- quantise this CTA's query rows into two e4m3 terms (thread = row)
+  // ---- quantise this CTA's query rows into two e4m3 terms (two threads per row, 64 columns each)
   float q_scale = 1.f;
   if (warp >= 2) {
-    const int r = (warp & 3) * 32 + lane;   // the TMEM lane quadrant this warp may read: warp % 4
-    float v[D];
+    const int r = (warp & 3) * 32 + lane, half = (warp - 2) >> 2;   // the TMEM lane quadrant this warp may read: warp % 4
+    float v[kApHalf];
     float amax = 0.f;
     if (r < rows) {
       const uint4* src = reinterpret_cast<const uint4*>(p.q + static_cast<size_t>(row0 + r) * p.q_stride + head * D);
 #pragma unroll
-      for (int c = 0; c < D / 8; ++c) {
-        Pack16 x;
-        x.u = src[c];
+      for (int c = 0; c < kApHalf / 8; ++c) {
+        Pack16 x, y;
+        x.u = src[half * (kApHalf / 8) + c];
+        y.u = src[(half ^ 1) * (kApHalf / 8) + c];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) { v[c * 8 + j] = bf16_to_f32(x.h[j]); amax = fmaxf(amax, fabsf(v[c * 8 + j])); }
+        for (int j = 0; j < 8; ++j) {
+          v[c * 8 + j] = bf16_to_f32(x.h[j]);
+          amax = fmaxf(amax, fmaxf(fabsf(v[c * 8 + j]), fabsf(bf16_to_f32(y.h[j]))));
+        }
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < D; ++j) v[j] = 0.f;
+      for (int j = 0; j < kApHalf; ++j) v[j] = 0.f;
     }
     q_scale = amax > 0.f ? amax / 448.f : 1.f;
     const float inv = 1.f / q_scale;
 #pragma unroll
-    for (int c = 0; c < D / 16; ++c) {
+    for (int c = 0; c < kApHalf / 16; ++c) {
       Pack16 a, b;
 #pragma unroll
       for (int j = 0; j < 8; ++j)
         f32x2_to_e4m3x2_two_term(v[c * 16 + 2 * j] * inv, v[c * 16 + 2 * j + 1] * inv, a.s[j], b.s[j]);
-      *reinterpret_cast<uint4*>(sQ + sw128_off(r, c * 16)) = a.u;
-      *reinterpret_cast<uint4*>(sQ + kTileBytes + sw128_off(r, c * 16)) = b.u;
+      *reinterpret_cast<uint4*>(sQ + sw128_off(r, half * kApHalf + c * 16)) = a.u;
+      *reinterpret_cast<uint4*>(sQ + kTileBytes + sw128_off(r, half * kApHalf + c * 16)) = b.u;
     }
     fence_proxy_async_smem();
   }
@@ -268,57 +280,60 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
       }
     }
   } else {
-    // ------------------------------------------------------------------ softmax + accumulation (thread = query row)
-    const int quad = warp & 3;
+    // ------------------------------------------------------------------ softmax + accumulation (two threads per query row)
+    const int quad = warp & 3, half = (warp - 2) >> 2, cb = half * kApHalf;
     const int r = quad * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
     const int my_pos = p.pos0 + row0 + r;
     const int my_first = (p.window > 0 && my_pos + 1 > p.window) ? my_pos + 1 - p.window : 0;
     const float sm = p.scale * 1.4426950408889634f * q_scale;
     float m_run = -INFINITY, l_run = 0.f, inv_c_prev = 0.f;
-    float o[D];
+    float o[kApHalf];
 #pragma unroll
-    for (int j = 0; j < D; ++j) o[j] = 0.f;
+    for (int j = 0; j < kApHalf; ++j) o[j] = 0.f;
     bool ok = true;
     for (int i = 0; i < ntiles; ++i) {
       const int s = i % kApStages, b = i & 1;
-      bool okw = ok && wait_bar(&s_full[b], (i >> 1) & 1);
+      const bool okw = ok && wait_bar(&s_full[b], (i >> 1) & 1);
       if (!okw && ok) { report(p.status, kTimeoutAccum, 35); *abort_flag = 1; }
       tc_fence_after();
       const float* ks = sKs + s * kApTile;
       const float* vs = sVs + s * kApTile;
       const int t0 = base + i * kApTile;
-      // tile-wide max of the V scales (fixes the range of the e4m3 P operand)
-      {
-        float vm = (t0 + r <= last_pos) ? vs[r] : 0.f;
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, off));
-        if (lane == 0) { red[(i & 1) * 8 + quad] = vm; red[(i & 1) * 8 + 4 + quad] = (okw && !*abort_flag) ? 0.f : 1.f; }
-      }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      const float* rr = red + (i & 1) * 8;
-      if (rr[4] + rr[5] + rr[6] + rr[7] != 0.f) { ok = false; break; }
-      const float vmax = fmaxf(fmaxf(rr[0], rr[1]), fmaxf(rr[2], rr[3]));
-      const float c_tile = vmax > 0.f ? 256.f / vmax : 0.f;
-      // pass 1: row maximum of the scaled, masked scores (the scores are re-read from TMEM in pass 2 instead of
-      // being kept in 128 registers next to the 128 output accumulators)
+      // pass 1: maximum of this thread's scaled, masked scores (the scores are re-read from TMEM in pass 2 instead of being
+      // kept in registers next to the output accumulators)
       // warp-uniform choice: tcgen05.ld is .sync.aligned, every lane of the warp must take the same path
       const bool full = __all_sync(0xffffffffu, (t0 + kApTile - 1 <= my_pos) && (t0 >= my_first)) != 0;
-      const float mt = full ? tile_row_max<false>(tmem_s + b * 128 + lane_addr, ks, t0, my_pos, my_first)
-                            : tile_row_max<true>(tmem_s + b * 128 + lane_addr, ks, t0, my_pos, my_first);
+      mx[b * 2 * kApTile + half * kApTile + r] =
+          full ? tile_row_max<false>(tmem_s + b * 128 + lane_addr, ks, cb, t0, my_pos, my_first)
+               : tile_row_max<true>(tmem_s + b * 128 + lane_addr, ks, cb, t0, my_pos, my_first);
+      // tile-wide max of the V scales (fixes the range of the e4m3 P operand)
+      {
+        float vm = (half == 0 && t0 + r <= last_pos) ? vs[r] : 0.f;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, off));
+        if (lane == 0) {
+          if (half == 0) red[b * 16 + quad] = vm;
+          red[b * 16 + 4 + half * 4 + quad] = (okw && !*abort_flag) ? 0.f : 1.f;
+        }
+      }
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      const float* rr = red + b * 16;
+      if (rr[4] + rr[5] + rr[6] + rr[7] + rr[8] + rr[9] + rr[10] + rr[11] != 0.f) { ok = false; break; }
+      const float vmax = fmaxf(fmaxf(rr[0], rr[1]), fmaxf(rr[2], rr[3]));
+      const float c_tile = vmax > 0.f ? 256.f / vmax : 0.f;
+      const float mt = fmaxf(mx[b * 2 * kApTile + r], mx[b * 2 * kApTile + kApTile + r]);
       const float mn = fmaxf(m_run, mt * sm);   // sm > 0: scaling commutes with the maximum
       const float corr = (m_run == -INFINITY) ? 0.f : fast_exp2(m_run - mn);
       m_run = mn;
-      float lsum = 0.f;
       // the previous tile's PV product must be folded in before P is overwritten
       if (i > 0) {
         if (__all_sync(0xffffffffu, wait_bar(o_full, (i - 1) & 1))) {
           tc_fence_after();
 #pragma unroll
-          for (int c0 = 0; c0 < D; c0 += 16) {
+          for (int c0 = 0; c0 < kApHalf; c0 += 16) {
             uint32_t raw[16];
-            tmem_ld_x16(tmem_o + lane_addr + c0, raw);
-            tmem_ld_wait();
+            tmem_ld_x16(tmem_o + lane_addr + cb + c0, raw);
 #pragma unroll
             for (int j = 0; j < 16; ++j) o[c0 + j] += __uint_as_float(raw[j]) * inv_c_prev;
           }
@@ -328,11 +343,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
         }
       }
 #pragma unroll
-      for (int j = 0; j < D; ++j) o[j] *= corr;
+      for (int j = 0; j < kApHalf; ++j) o[j] *= corr;
       // pass 2: probabilities -> two e4m3 terms of P (row r of the A operand)
       const float neg_m = (mn == -INFINITY) ? 0.f : -mn;
-      lsum = full ? tile_probs<false>(tmem_s + b * 128 + lane_addr, ks, vs, sP, r, sm, neg_m, c_tile, t0, my_pos, my_first)
-                  : tile_probs<true>(tmem_s + b * 128 + lane_addr, ks, vs, sP, r, sm, neg_m, c_tile, t0, my_pos, my_first);
+      const float lsum = full ? tile_probs<false>(tmem_s + b * 128 + lane_addr, ks, vs, sP, r, sm, neg_m, c_tile, cb, t0, my_pos, my_first)
+                              : tile_probs<true>(tmem_s + b * 128 + lane_addr, ks, vs, sP, r, sm, neg_m, c_tile, cb, t0, my_pos, my_first);
       l_run = l_run * corr + lsum;
       inv_c_prev = c_tile > 0.f ? 1.f / c_tile : 0.f;
       fence_proxy_async_smem();
@@ -344,10 +359,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
       if (__all_sync(0xffffffffu, wait_bar(o_full, (ntiles - 1) & 1))) {
         tc_fence_after();
 #pragma unroll
-        for (int c0 = 0; c0 < D; c0 += 16) {
+        for (int c0 = 0; c0 < kApHalf; c0 += 16) {
           uint32_t raw[16];
-          tmem_ld_x16(tmem_o + lane_addr + c0, raw);
-          tmem_ld_wait();
+          tmem_ld_x16(tmem_o + lane_addr + cb + c0, raw);
 #pragma unroll
           for (int j = 0; j < 16; ++j) o[c0 + j] += __uint_as_float(raw[j]) * inv_c_prev;
         }
@@ -356,11 +370,16 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
         *abort_flag = 1;
       }
     }
+    // a row's probability mass: the two threads' sums, in the same order for both (the maxima of both parities are behind a barrier)
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    mx[half * kApTile + r] = l_run;
+    asm volatile("bar.sync 1, 256;" ::: "memory");
     if (r < rows) {
-      const float inv_l = l_run > 0.f ? 1.f / l_run : 0.f;
-      uint4* dst = reinterpret_cast<uint4*>(p.out + (static_cast<size_t>(row0 + r) * p.hq + head) * D);
+      const float l = mx[r] + mx[kApTile + r];
+      const float inv_l = l > 0.f ? 1.f / l : 0.f;
+      uint4* dst = reinterpret_cast<uint4*>(p.out + (static_cast<size_t>(row0 + r) * p.hq + head) * D + cb);
 #pragma unroll
-      for (int c = 0; c < D / 8; ++c) {
+      for (int c = 0; c < kApHalf / 8; ++c) {
         Pack16 x;
 #pragma unroll
         for (int j = 0; j < 8; ++j) x.h[j] = f32_to_bf16(o[c * 8 + j] * inv_l);
@@ -403,7 +422,7 @@ DGPP_API int dgpp_attn_prefill_tc(const void* q, int64_t q_stride, const void* k
     return -1;
   if (make_tmap_2d(&tV, v_cache, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, 128, total_rows, 128, 128, page, CU_TENSOR_MAP_SWIZZLE_128B))
     return -1;
-  constexpr size_t smem = 1024 + (4 + 2 * kApStages) * kApTile * 128 + 2 * kApStages * kApTile * 4 + 64 +
+  constexpr size_t smem = 1024 + (4 + 2 * kApStages) * kApTile * 128 + 2 * kApStages * kApTile * 4 + 2 * 16 * 4 + 4 * kApTile * 4 +
                           (2 * kApStages + 4) * 8 + 64;
   static bool attr = false;
   if (!attr) {
@@ -411,7 +430,7 @@ DGPP_API int dgpp_attn_prefill_tc(const void* q, int64_t q_stride, const void* k
                                       static_cast<int>(smem)));
     attr = true;
   }
-  dim3 grid(dgpp_ceil_div(T, kApTile), hq);
+  dim3 grid(hq, dgpp_ceil_div(T, kApTile));
   attn_prefill_tc_kernel<<<grid, kApThreads, smem, st>>>(tK, tV, p);
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
