@@ -303,7 +303,11 @@ class DenseRunner:
         pending = False
         sp_in = False
         splits = self.decode_splits if (decode and rows <= 256) else 1
-        fp4 = self.decode_fp4 and decode and rows <= self.fp4_rows and all(
+        # above 32 rows the terms of a row fill a 192-column tile and the W4A16 GEMM on CTA pairs is the faster one, without
+        # quantisers (37 rows, 16 layers of 5120 / 17408: 3005 -> 2796 us a pass); the all-reduce push keeps its epilogues, and with
+        # the split choice pinned (speculation) a row keeps its bits at every width
+        cap = self.fp4_rows if (ops.PIN_SPLIT_ROWS or self.fuse_ar) else min(32, self.fp4_rows)
+        fp4 = self.decode_fp4 and decode and rows <= cap and all(
             w.k % 256 == 0 for w in (m.layers[0].qkv, m.layers[0].o, m.layers[0].down))
         lora = self.lora
         fused = fp4 and decode and self.embed_spans is None and self._fused_ok(rows)
