@@ -70,27 +70,28 @@ __global__ void __launch_bounds__(256) mla_q_absorb_kernel(const bf16* __restric
   extern __shared__ float sm_q[];
   float* qs = sm_q;                              // [8][nope]
   float* part = sm_q + kGlueRows * nope;         // [8 warps][8 rows][64]
-  pdl_wait();
   const int h = blockIdx.x, r0 = blockIdx.y * kGlueRows, tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
   const int nr = min(kGlueRows, rows - r0);
   const int dq = nope + dr;
+  const int d0 = blockIdx.z * 64 + lane * 2;
+  const bool live = d0 < dc;
+  const int per = (nope + 7) / 8;
+  const int n0 = warp * per, n1 = live ? min(nope, n0 + per) : n0;
+  const bf16* wp = w_uk + static_cast<size_t>(h) * nope * dc + (live ? d0 : 0);
+  uint32_t early[16];      // the first sixteen weights: they do not depend on the preceding grid
+#pragma unroll
+  for (int j = 0; j < 16; ++j) early[j] = n0 + j < n1 ? *reinterpret_cast<const uint32_t*>(wp + static_cast<size_t>(n0 + j) * dc) : 0u;
+  pdl_wait();
   for (int i = tid; i < kGlueRows * nope; i += 256) {
     const int r = i / nope, n = i % nope;
     qs[i] = r < nr ? bf16_to_f32(q[(static_cast<size_t>(r0 + r) * heads + h) * dq + n]) : 0.f;
   }
   __syncthreads();
-  const int d0 = blockIdx.z * 64 + lane * 2;
-  const bool live = d0 < dc;
-  const int per = (nope + 7) / 8;
-  const int n0 = warp * per, n1 = min(nope, n0 + per);
   float acc[kGlueRows][2];
 #pragma unroll
   for (int r = 0; r < kGlueRows; ++r) { acc[r][0] = 0.f; acc[r][1] = 0.f; }
-  const bf16* wp = w_uk + static_cast<size_t>(h) * nope * dc + (live ? d0 : 0);
-#pragma unroll 16
-  for (int n = n0; n < (live ? n1 : n0); ++n) {
-    const uint32_t w2 = *reinterpret_cast<const uint32_t*>(wp + static_cast<size_t>(n) * dc);
+  auto add = [&](int n, uint32_t w2) {
     const float w0 = __uint_as_float(w2 << 16), w1 = __uint_as_float(w2 & 0xffff0000u);
 #pragma unroll
     for (int r = 0; r < kGlueRows; ++r) {
@@ -98,7 +99,12 @@ __global__ void __launch_bounds__(256) mla_q_absorb_kernel(const bf16* __restric
       acc[r][0] = fmaf(qv, w0, acc[r][0]);
       acc[r][1] = fmaf(qv, w1, acc[r][1]);
     }
-  }
+  };
+#pragma unroll
+  for (int j = 0; j < 16; ++j)
+    if (n0 + j < n1) add(n0 + j, early[j]);
+#pragma unroll 16
+  for (int n = n0 + 16; n < n1; ++n) add(n, *reinterpret_cast<const uint32_t*>(wp + static_cast<size_t>(n) * dc));
 #pragma unroll
   for (int r = 0; r < kGlueRows; ++r) {
     part[(warp * kGlueRows + r) * 64 + lane * 2] = acc[r][0];
@@ -136,30 +142,43 @@ __global__ void __launch_bounds__(256) mla_q_absorb_kernel(const bf16* __restric
 __global__ void __launch_bounds__(256) mla_v_up_kernel(const bf16* __restrict__ lat, const bf16* __restrict__ w_uv,
                                                        bf16* __restrict__ out, int rows, int heads, int vdim, int dc) {
   extern __shared__ float ls[];                // [8][chunks][9]: one latent row = dc / 8 chunks of 8 values, padded
-  pdl_wait();
   const int h = blockIdx.x, r0 = blockIdx.y * kGlueRows, tid = threadIdx.x;
   const int nr = min(kGlueRows, rows - r0);
   const int chunks = dc / 8;
-  for (int i = tid; i < kGlueRows * dc; i += 256) {
-    const int r = i / dc, d = i % dc;
-    ls[(r * chunks + d / 8) * 9 + d % 8] = r < nr ? bf16_to_f32(lat[(static_cast<size_t>(r0 + r) * heads + h) * dc + d]) : 0.f;
-  }
-  __syncthreads();
   const int warp = tid >> 5, lane = tid & 31;
   const int g = lane & 15;
   const int v = blockIdx.z * 16 + warp * 2 + (lane >> 4);
   const bool live = v < vdim;
   const bf16* wp = w_uv + (static_cast<size_t>(h) * vdim + (live ? v : 0)) * dc;
-  float acc[kGlueRows];
-#pragma unroll
-  for (int r = 0; r < kGlueRows; ++r) acc[r] = 0.f;
-  for (int c0 = 0; c0 < chunks; c0 += 64) {          // up to four chunks per thread and round
-    Pack16 w[4];
+  Pack16 w[4];
+  auto load_w = [&](int c0) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int c = c0 + g + 16 * k;
       w[k].u = (c < chunks) ? *reinterpret_cast<const uint4*>(wp + c * 8) : make_uint4(0u, 0u, 0u, 0u);
     }
+  };
+  const bool wide = (reinterpret_cast<uintptr_t>(lat) & 15) == 0;
+  load_w(0);               // weights do not depend on the preceding grid
+  pdl_wait();
+  for (int i = tid; i < kGlueRows * chunks; i += 256) {
+    const int r = i / chunks, c = i % chunks;
+    const bf16* src = lat + (static_cast<size_t>(r0 + r) * heads + h) * dc + c * 8;
+    Pack16 x;
+    x.u = make_uint4(0u, 0u, 0u, 0u);
+    if (r < nr && wide) x.u = *reinterpret_cast<const uint4*>(src);
+    else if (r < nr)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x.h[j] = src[j];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ls[i * 9 + j] = bf16_to_f32(x.h[j]);
+  }
+  __syncthreads();
+  float acc[kGlueRows];
+#pragma unroll
+  for (int r = 0; r < kGlueRows; ++r) acc[r] = 0.f;
+  for (int c0 = 0; c0 < chunks; c0 += 64) {          // up to four chunks per thread and round
+    if (c0 > 0) load_w(c0);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int c = c0 + g + 16 * k;

@@ -88,6 +88,24 @@ def test_mla_decode_tensor_cores(dev, heads, page, splits, ctxs):
         assert (out[r].float() - want).abs().max().item() < 1.5e-2, ("sparse", r, n)
 
 
+@pytest.mark.parametrize("heads,splits", [(5, 2), (32, 18), (32, 64), (33, 65), (3, 130)])
+def test_mla_decode_split_counts(dev, heads, splits):
+    """The combine of 2 .. 130 splits (one or several rounds of 64), most of them empty, against one split of the same kernel.  Both round
+    their probabilities to bf16, relative to another maximum, and their outputs: 2^-8 of the largest latent (under 4) covers the
+    two together, a lost or doubled split would be far off."""
+    from dgpp_b200.ops import core as ops
+
+    dc, dr, ctxs = 512, 64, [1, 513, 4096, 129]
+    cache, table = _pool(dev, len(ctxs), ctxs, 64, dc + dr, seed=5)
+    q = (torch.randn(len(ctxs), heads, dc + dr, device=dev) * 0.3).to(BF)
+    row_req = torch.arange(len(ctxs), dtype=torch.int32, device=dev)
+    pos = torch.tensor([c - 1 for c in ctxs], dtype=torch.int32, device=dev)
+    out, one = (ops.mla_decode(q, cache, table, row_req, pos, 0.07, dc, dr, splits=n, tensor_cores=True) for n in (splits, 1))
+    torch.cuda.synchronize()
+    ops.check_status()
+    assert (out.float() - one.float()).abs().max().item() <= 2.0 ** -8 * 4
+
+
 def test_indexer_scores_and_topk(dev):
     from dgpp_b200.models.mla import gather_rows, index_scores_reference, topk_reference
     from dgpp_b200.ops import core as ops
