@@ -253,6 +253,8 @@ class HybridRunner:
             return 1
         if self.spec_rows:
             rows = 1      # verify rows must fold their KV range exactly like a plain decode row does
+        if self.c.head_dim == 256:      # one CTA per SM: no second wave
+            return max(1, min(self.max_splits, 148 // (self.c.kv_heads * rows)))
         return max(1, min(self.max_splits, -(-160 // (self.c.kv_heads * rows))))
 
     def _state_tensors(self):

@@ -105,7 +105,7 @@ class RowRunner:
             ops.attn_prefill_tc(qkv, qkv.stride(0), cache, self.kv.block_table[chunk_slot], pos0, hq, hkv, d,
                                 self.att_scale, out=out, rows=rows)
         elif self.tc_attn and rows <= 32:
-            splits = max(1, min(32, -(-160 // (hkv * rows))))
+            splits = max(1, min(32, 148 // (hkv * rows) if d == 256 else -(-160 // (hkv * rows))))   # (256: one CTA per SM)
             ops.attn_decode_tc(qkv, qkv.stride(0), cache, self.kv.block_table, row_req, positions, hq, hkv, d,
                                self.att_scale, splits=splits, scratch=self.att_scratch, out=out)
         else:
