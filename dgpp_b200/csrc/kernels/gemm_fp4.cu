@@ -81,12 +81,6 @@ struct Fp4Params {
   int cluster_split;
 };
 
-__device__ __forceinline__ float ld_shared_cluster_f32(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-  return v;
-}
-
 // One bf16 of the finished output tile -> slot `rank` of every rank (destinations staggered by rank).
 __device__ __forceinline__ void push_value(const Fp4Params& p, int parity, size_t idx, bf16 v) {
   for (int r = 0; r < p.comm.world; ++r) {

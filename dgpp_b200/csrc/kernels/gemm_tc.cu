@@ -82,6 +82,7 @@ struct GemmParams {
   // bf16 weights, one output (bf16 or fp32), 16-byte aligned rows, no split: the finished tile is turned around in shared memory
   // (all eight spare warps read the accumulator) and leaves as 16-byte vectors along N
   int staged;
+  int cluster;   // bf16 weights and a small token tile: the K splits of a tile are a cluster
 };
 
 template <int BN>
@@ -108,7 +109,7 @@ __device__ __forceinline__ uint32_t bf12_escape(const uint32_t* __restrict__ esc
 // Converted operands are bf16 (kind::f16 requires A and B
 // to have the same 16-bit type; mixing an f16 A with a bf16 B is an illegal instruction on sm_100a).
 template <int BN, int WMODE, int SB, int SA, int SR>
-__global__ void __launch_bounds__(kGemmThreads, (WMODE != 0 && BN <= 32) ? 2 : 1)
+__global__ void __launch_bounds__(kGemmThreads, BN <= 32 ? 2 : 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA,   // bf16 weights, or packed raw weights (uint8)
                const __grid_constant__ CUtensorMap tmB,   // activations bf16 [T, K]
                const __grid_constant__ CUtensorMap tmSf,  // NVFP4 scales (uint8) [N, K/16]
@@ -438,8 +439,52 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA,   // bf16 weights, or pa
       }
     }
   }
+  if (!kQuant && p.cluster) {
+    // Split K inside a cluster (1, 1, splits): every CTA leaves its partial sums in its own idle ring, every rank adds each splits-th
+    // token of all of them, in ascending rank order.  Every thread passes both barriers, whatever happened before.
+    const int q = warp & 3, cols = min(BN, p.T - m0);
+    float* red = reinterpret_cast<float*>(sB);            // [BN][kBM]
+    if (warp >= 2 && warp < 6) {
+      const bool ok = nkb > 0 && wait_bar(acc_full, 0) && !*abort_flag;
+      if (!ok && nkb > 0) { report(p.status, kTimeoutAccum, 8); *abort_flag = 1; }
+      tc_fence_after();
+      for (int c0 = 0; c0 < cols; c0 += 16) {
+        uint32_t r[16];
+        if (ok) {
+          tmem_ld_x16(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + c0, r);
+          tmem_ld_wait();
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (c0 + j < cols) red[(c0 + j) * kBM + q * 32 + lane] = ok ? __uint_as_float(r[j]) : 0.f;
+      }
+    }
+    cluster_barrier();
+    const int n = n0 + q * 32 + lane;
+    if (warp >= 2 && n < p.N && !*abort_flag) {
+      for (int m = split + (warp >= 6 ? splits : 0); m < cols; m += 2 * splits) {
+        const uint32_t at = smem_u32(red + m * kBM + q * 32 + lane);
+        float t[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+          if (r < splits) t[r] = ld_shared_cluster_f32(mapa_shared(at, static_cast<uint32_t>(r)));
+        float acc = 0.f;
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+          if (r < splits) acc += t[r];
+        const size_t o = static_cast<size_t>(m0 + m) * p.ldc + n;
+        float y = acc * p.alpha;
+        if (p.out32) p.out32[o] = y;
+        if (p.out) {
+          if (p.resid) y = bf16_to_f32(p.resid[o]) + bf16_to_f32(f32_to_bf16(y));
+          p.out[o] = f32_to_bf16(y);
+        }
+      }
+    }
+    cluster_barrier();                                    // nobody leaves while its partial sums may still be read
+  }
   // ------------------------------------------------------------------ epilogue (warps 2..5)
-  if ((kQuant || !p.staged) && warp >= 2 && warp < 6) {
+  if ((kQuant || !(p.staged || p.cluster)) && warp >= 2 && warp < 6) {
     const int q = warp & 3;  // TMEM lane quadrant this warp may read
     const bool ok = nkb > 0 ? wait_bar(acc_full, 0) : true;
     if (!ok) { report(p.status, kTimeoutAccum, 6); *abort_flag = 1; }
@@ -572,7 +617,8 @@ template <int BN, int WMODE>
 struct GemmCfg {
   static constexpr bool kQuant = WMODE != 0;
   // ring depths: deep raw prefetch for small BN (weight streaming), wide B ring for large BN
-  static constexpr int kBf16Depth = (200 * 1024) / (BN * 128 + kBM * 128);
+  // (bf16 weights and a small token tile: two CTAs per SM too, 6 or 5 stages each: a pass of 16 bf16 layers 2241 -> 2206 us)
+  static constexpr int kBf16Depth = ((BN <= 32 ? 112 : 200) * 1024) / (BN * 128 + kBM * 128);
   // Quantised weights with a small token tile run two CTAs per SM (<= 113 KB each): the second CTA hides
   // the converter <-> tensor-core handshakes of the first while both keep HBM requests in flight.
   // (BF12 carries an 8 KB exponent plane per raw stage; its B ring is shallower to stay under two CTAs per SM)
@@ -607,6 +653,23 @@ static int launch_gemm(const CUtensorMap& tA, const CUtensorMap& tB, const CUten
     attr = true;
   }
   dim3 grid(dgpp_ceil_div(p.N, kBM), dgpp_ceil_div(p.T, BN), splits);
+  if (p.cluster) {
+    static_assert(WMODE != 0 || BN > 32 || C::SB * BN * 128 >= BN * kBM * 4, "a CTA's partial sums fit its activation ring");
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kGemmThreads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = static_cast<unsigned>(splits);
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    DGPP_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tA, tB, tSf, p));
+    return 0;
+  }
   kern<<<grid, kGemmThreads, smem, st>>>(tA, tB, tSf, p);
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
@@ -692,6 +755,10 @@ static int gemm_tc_impl(int wmode, int a_f16, int bn, const void* x, int64_t x_s
   splits = dgpp_ceil_div(num_kb, per);
   const uintptr_t dst = reinterpret_cast<uintptr_t>(out ? out : out32);
   p.staged = wmode == 0 && splits == 1 && !comm_push && !resid && (out == nullptr) != (out32 == nullptr) && N % 8 == 0 && ldc % 8 == 0 && dst % 16 == 0;
+
+  // Decode rows of bf16 weights: partial sums stay in shared memory.  1 row, us through the workspace with its fences and counters / so:
+  // 6144 x 4096 14.0 / 12.2, 4096 x 4096 12.1 / 9.9, 4096 x 17408 29.0 / 26.6 (7.7, 5.1 and 21.8 at the copy rate).
+  p.cluster = wmode == 0 && bn <= 32 && splits >= 2 && splits <= 8 && !comm_push && !comm_ag && !groups;
 
   CUtensorMap tA, tB, tSf;
   memset(&tSf, 0, sizeof(tSf));

@@ -395,3 +395,23 @@ def test_prefix_cache_hit_reproduces_the_uncached_tokens(dev, plen):
     m = s.meters()
     assert m["prefix_hit_tokens"] >= 2 * (plen // 64) * 64
     assert outs[1] == outs[0] and outs[2] == outs[0], outs
+
+
+@pytest.mark.parametrize("rows,bn,n,k,splits", [(1, 16, 128, 64 * 17, 8), (13, 16, 200, 64 * 17, 5), (16, 16, 72, 1048, 3), (17, 32, 328, 64 * 8, 7),
+                                                (32, 32, 256, 64 * 2, 2), (40, 16, 136, 64 * 9, 4)])
+def test_gemm_tc_bf16_splits_in_a_cluster(dev, rows, bn, n, k, splits):
+    """Small integers, whose sums are exact in fp32 in any order: every split count and destination gives the exact product."""
+    from dgpp_b200.ops import core as ops
+    from dgpp_b200.quant.formats import QuantLinear
+
+    torch.manual_seed(rows)
+    x, w = (torch.randint(-4, 5, (m, k), device=dev).to(torch.bfloat16) for m in (rows, n))
+    q = QuantLinear("bf16", n, k, w, alpha=0.5)
+    want = 0.5 * (x.double() @ w.double().t())
+    y32 = ops.gemm_tc(x, q, out32=torch.full((rows, n), float("nan"), device=dev), bn=bn, splits=splits)
+    res = torch.randint(-8, 9, (rows, n), device=dev).to(torch.bfloat16)
+    y = ops.gemm_tc(x, q, resid=res, bn=bn, splits=splits)
+    torch.cuda.synchronize()
+    ops.check_status()
+    assert torch.equal(y32.double(), want)
+    assert torch.equal(y, (res.float() + want.float().to(torch.bfloat16).float()).to(torch.bfloat16))
