@@ -90,6 +90,7 @@ __global__ void __launch_bounds__(kRouterThreads) moe_router_select_kernel(Route
   __shared__ float grp[64];
   __shared__ float wred[kRouterThreads / 32];
   __shared__ int pick_id[kMoeMaxTopK];
+  __shared__ int keep[64];
   pdl_wait();
   const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   for (int e = tid; e < a.E; e += kRouterThreads) score[e] = a.logits_out[t * a.logits_stride + e] + (a.logit_bias ? a.logit_bias[e] : 0.f);
@@ -140,64 +141,63 @@ __global__ void __launch_bounds__(kRouterThreads) moe_router_select_kernel(Route
       grp[tid] = b1 + (per > 1 ? b2 : 0.f);
     }
     __syncthreads();
-    if (tid == 0) {
-      // keep the topk_group best groups (ties to the lower group id); the others can no longer be selected
-      bool keep[64];
-      for (int g = 0; g < a.n_group; ++g) keep[g] = false;
-      for (int r = 0; r < a.topk_group; ++r) {
-        int best = -1;
-        for (int g = 0; g < a.n_group; ++g)
-          if (!keep[g] && (best < 0 || grp[g] > grp[best])) best = g;
-        if (best >= 0) keep[best] = true;
-      }
-      for (int g = 0; g < a.n_group; ++g)
-        if (!keep[g])
-          for (int e = g * per; e < (g + 1) * per; ++e) sel[e] = -INFINITY;
+    // keep the topk_group best groups (ties to the lower group id); the others can no longer be selected
+    if (tid < a.n_group) {
+      int better = 0;
+      for (int g = 0; g < a.n_group; ++g) better += (grp[g] > grp[tid] || (grp[g] == grp[tid] && g < tid)) ? 1 : 0;
+      keep[tid] = better < a.topk_group;
     }
     __syncthreads();
+    for (int e = tid; e < a.E; e += kRouterThreads)
+      if (!keep[e / per]) sel[e] = -INFINITY;
+    __syncthreads();
   }
-  // k rounds of arg-max by warp 0 (ties to the lower expert id)
+  // k rounds of arg-max by warp 0 (ties to the lower expert id); a lane keeps its experts' values in registers, lane r the r-th pick
   if (wid == 0) {
+    constexpr int kPer = kMoeMaxExperts / 32;
+    float v[kPer];
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) v[q] = q * 32 + lane < a.E ? sel[q * 32 + lane] : -INFINITY;
+    int mine = 0;
     for (int r = 0; r < a.k; ++r) {
       float bv = -INFINITY;
       int bi = 0x7fffffff;
-      for (int e = lane; e < a.E; e += 32) {
-        const float v = sel[e];
-        if (v > bv || (v == bv && e < bi)) { bv = v; bi = e; }
-      }
+#pragma unroll
+      for (int q = 0; q < kPer; ++q)
+        if (v[q] > bv || (v[q] == bv && bi == 0x7fffffff)) { bv = v[q]; bi = q * 32 + lane; }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
         const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
         if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
       }
-      if (lane == 0) {
-        pick_id[r] = bi < a.E ? bi : 0;
-        if (bi < a.E) sel[bi] = -INFINITY;
-      }
-      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < kPer; ++q)
+        if (bi == q * 32 + lane) v[q] = -INFINITY;
+      if (lane == r) mine = bi < a.E ? bi : 0;
     }
-    if (lane == 0) {
-      // ascending ids (insertion sort, k <= 16), weights from the uncorrected scores
-      for (int i = 1; i < a.k; ++i) {
-        const int v = pick_id[i];
-        int j = i - 1;
-        while (j >= 0 && pick_id[j] > v) { pick_id[j + 1] = pick_id[j]; --j; }
-        pick_id[j + 1] = v;
-      }
-      if (a.softmax == 2) {
-        float m = -INFINITY;
-        for (int i = 0; i < a.k; ++i) m = fmaxf(m, score[pick_id[i]]);
-        for (int i = 0; i < a.k; ++i) score[pick_id[i]] = expf(score[pick_id[i]] - m);
-      }
-      float sum = 0.f;
-      for (int i = 0; i < a.k; ++i) sum += score[pick_id[i]];
-      for (int i = 0; i < a.k; ++i) {
-        float w = score[pick_id[i]];
-        if (a.norm_topk || a.softmax == 2) w = w / (sum + 1e-20f);
-        a.ids[t * a.k + i] = pick_id[i];
-        a.weights[t * a.k + i] = w * a.scaling;
-      }
+    // ascending ids, weights from the uncorrected scores, summed in that order
+    int at = 0;
+    for (int r = 0; r < a.k; ++r) {
+      const int other = __shfl_sync(0xffffffffu, mine, r);
+      at += (other < mine || (other == mine && r < lane)) ? 1 : 0;
+    }
+    if (lane < a.k) pick_id[at] = mine;
+    __syncwarp();
+    const int id = pick_id[min(lane, a.k - 1)];
+    float w = score[id];
+    if (a.softmax == 2) {
+      float m = w;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+      w = expf(w - m);
+    }
+    float sum = 0.f;
+    for (int i = 0; i < a.k; ++i) sum += __shfl_sync(0xffffffffu, w, i);
+    if (lane < a.k) {
+      if (a.norm_topk || a.softmax == 2) w = w / (sum + 1e-20f);
+      a.ids[t * a.k + lane] = id;
+      a.weights[t * a.k + lane] = w * a.scaling;
     }
   }
 }

@@ -38,6 +38,23 @@ def test_router_matches_reference(dev, experts, k, n_group, topk_group, router):
     assert (ids[:, 1:] > ids[:, :-1]).all()                     # ascending, no duplicates
 
 
+@pytest.mark.parametrize("experts,k,n_group,topk_group,router", [(512, 16, 1, 1, "softmax"), (8, 8, 1, 1, "sigmoid"), (40, 1, 1, 1, "softmax"),
+                                                                 (256, 16, 64, 5, "sigmoid"), (256, 8, 8, 8, "sigmoid")])
+def test_router_ties_go_to_the_lower_ids(dev, experts, k, n_group, topk_group, router):
+    """Zero rows: every expert and every group ties, so groups 0.. and experts 0.. are picked, each with weight 1 / k (exact in fp32 up to
+    the k additions and one division: 2 k 2^-24)."""
+    from dgpp_b200.models.moe import MoEConfig, MoEWeights
+    from dgpp_b200.ops import core as ops
+
+    w = MoEWeights.random_init(MoEConfig(hidden=256, experts=experts, top_k=k, moe_ffn=256, n_group=n_group, topk_group=topk_group,
+                                         router=router), dev, seed=2, fmt="bf16")
+    x = torch.zeros(3, 256, device=dev, dtype=BF)
+    ids, wts = ops.moe_route(x, w.gate, None, k, n_group, topk_group, router == "softmax", True, 1.0)
+    torch.cuda.synchronize()
+    assert ids.tolist() == [list(range(k))] * 3
+    assert (wts - 1.0 / k).abs().max().item() <= 2 * k * 2.0 ** -24
+
+
 @pytest.mark.parametrize("rows,shared", [(1, 0), (8, 512), (16, 0)])
 def test_moe_block_matches_reference(dev, rows, shared):
     from dgpp_b200.models.moe import MoEBlock, MoEConfig, MoEWeights, moe_reference
