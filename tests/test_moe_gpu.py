@@ -55,6 +55,21 @@ def test_router_ties_go_to_the_lower_ids(dev, experts, k, n_group, topk_group, r
     assert (wts - 1.0 / k).abs().max().item() <= 2 * k * 2.0 ** -24
 
 
+@pytest.mark.parametrize("rows,experts,hidden", [(150, 512, 2048), (1187, 37, 264), (2368, 4, 512)])
+def test_router_logits_do_not_depend_on_the_batch(dev, rows, experts, hidden):
+    """Prompt sizes (tiles of experts and tokens, both with a remainder) against the same rows eight at a time: the same bits."""
+    from dgpp_b200.ops import core as ops
+
+    torch.manual_seed(rows)
+    x, gate = torch.randn(rows, hidden, device=dev).to(BF), torch.randn(experts, hidden, device=dev).to(BF)
+    all_, few = (torch.full((rows, experts), float("nan"), device=dev) for _ in range(2))
+    ops.moe_route(x, gate, None, 2, logits_out=all_)
+    for r in range(0, rows, 8):
+        ops.moe_route(x[r:r + 8], gate, None, 2, logits_out=few[r:r + 8])
+    torch.cuda.synchronize()
+    assert torch.equal(all_, few)
+
+
 @pytest.mark.parametrize("rows,shared", [(1, 0), (8, 512), (16, 0)])
 def test_moe_block_matches_reference(dev, rows, shared):
     from dgpp_b200.models.moe import MoEBlock, MoEConfig, MoEWeights, moe_reference
