@@ -232,6 +232,8 @@ class MoEBlock:
         self.qa_in = shared("qa_in", lambda: ops.QuantAct(self.bn, c.hidden, act_terms, self.bn, device))
         self.qa_mid = shared("qa_mid", lambda: ops.QuantAct(nslots * self.bn, c.moe_ffn, act_terms, self.bn, device))
         self.nslots = nslots
+        self.logits = torch.empty(max_rows, c.experts, dtype=torch.float32, device=device)
+        self._views: dict = {}
         self.shared = None
         if w.shared_gu is not None and self.sh_slot < 0:
             self.shared = shared("shared", lambda: torch.zeros(max_rows, c.hidden, dtype=BF, device=device))
@@ -249,14 +251,18 @@ class MoEBlock:
         assert rows <= self.max_rows
         if xa is None:
             xa = ops.act_quant_nvfp4(xn, self.terms, out=self.qa_in)
+        views = self._views.get(rows)
+        if views is None:      # (slices cost the host more than the launches between them)
+            views = self._views[rows] = (self.ids[:rows], self.wts[:rows], self.h.view(self.nslots * self.bn, 2 * c.moe_ffn),
+                                         self.logits[:rows])
+        ids, wts, h, logits = views
         ops.moe_route(xn, w.gate, w.bias, c.top_k, c.n_group, c.topk_group, c.router == "softmax", c.norm_topk_prob,
-                      c.routed_scaling, ids=self.ids[:rows], weights=self.wts[:rows])
-        ops.moe_active(self.ids[:rows], rows, c.experts, self.slots, self.group_list, self.slot_of, self.n_active,
-                       self.e0, self.e1)
+                      c.routed_scaling, ids=ids, weights=wts, logits_out=logits)
+        ops.moe_active(ids, rows, c.experts, self.slots, self.group_list, self.slot_of, self.n_active, self.e0, self.e1)
         ops.gemm_fp4_grouped(xa, w.gu_q, w.gu_sf, w.gu_alpha, self.h, rows, 2 * c.moe_ffn, c.hidden, self.stack_experts,
                              self.group_list, group_b=False)
-        xm = ops.act_quant_nvfp4(self.h.view(self.nslots * self.bn, 2 * c.moe_ffn), self.terms, out=self.qa_mid,
-                                 mode="swiglu", limit=c.swiglu_limit, alpha=c.swiglu_alpha, group_list=self.group_list, group_rows=rows)
+        xm = ops.act_quant_nvfp4(h, self.terms, out=self.qa_mid, mode="swiglu", limit=c.swiglu_limit, alpha=c.swiglu_alpha,
+                                 group_list=self.group_list, group_rows=rows)
         ops.gemm_fp4_grouped(xm, w.down_q, w.down_sf, w.down_alpha, self.y, rows, c.hidden, c.moe_ffn, self.stack_experts,
                              self.group_list, group_b=True)
         sh = self.y[self.sh_slot] if self.sh_slot >= 0 else None          # [bn, H]: the shared expert's rows
@@ -266,9 +272,9 @@ class MoEBlock:
             ops.gemm_fp4(xs, w.shared_down_k, out=self.shared[:rows])
             sh = self.shared
         if push_comm:
-            ops.moe_combine_push(self.y, sh, self.ids[:rows], self.wts[:rows], self.slot_of, push_comm, rows)
+            ops.moe_combine_push(self.y, sh, ids, wts, self.slot_of, push_comm, rows)
             return None
-        return ops.moe_combine(self.y, sh, self.ids[:rows], self.wts[:rows], self.slot_of, out, rows)
+        return ops.moe_combine(self.y, sh, ids, wts, self.slot_of, out, rows)
 
     def forward_gathered(self, xn: torch.Tensor) -> torch.Tensor:
         """Prefill-sized batches, all on the device: router, counting sort of the (token, k) pairs by expert into tiles

@@ -101,9 +101,14 @@ def declare(name: str, argtypes) -> None:
     _SIGNATURES[name] = list(argtypes)
 
 
+_FNS: dict = {}
+
+
 def _fn(name: str):
-    lib = load()
-    fn = getattr(lib, name)
+    fn = _FNS.get(name)
+    if fn is not None:
+        return fn
+    fn = _FNS[name] = getattr(load(), name)
     if not getattr(fn, "_dgpp_typed", False):
         fn.argtypes = _SIGNATURES[name]
         fn.restype = I
@@ -119,8 +124,15 @@ def ptr(t) -> int | None:
     return t.data_ptr()
 
 
+# handle of a device's current stream without a Stream object around it (3 us of every launch)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device_index = getattr(torch._C, "_cuda_getDevice", None)
+
+
 def stream_ptr(stream=None) -> int:
     if stream is None:
+        if _raw_stream is not None and _device_index is not None and torch.cuda.is_initialized():
+            return _raw_stream(_device_index())
         stream = torch.cuda.current_stream()
     return stream.cuda_stream
 
