@@ -10,7 +10,7 @@
 //     S_C = gamma_C S_0 + (diag(gamma_C / gamma) K)^T U
 // Kernel 1 (gdn_chunk_prep_kernel) is parallel over (chunk, head): it builds L and P from K K^T and Q K^T, inverts
 // I + L by forward substitution in shared memory and leaves W, U0, P and G in scratch.  Kernel 2
-// (gdn_chunk_state_kernel) walks the chunks of a head in order, one CTA per (head, 32 state columns), with the state
+// (gdn_chunk_state_kernel) walks the chunks of a head in order, one CTA per (head, 16 state columns), with the state
 // slice resident in shared memory: three small GEMMs per chunk instead of 64 dependent token steps.
 // All arithmetic is fp32 on the CUDA cores with fixed summation orders (deterministic); against the token-sequential
 // kernel the results differ by fp32 re-association only.
@@ -24,8 +24,12 @@
 namespace dgpp {
 
 constexpr int kGcC = 64;          // tokens per chunk
-constexpr int kGcCols = 32;       // state columns per CTA of the sequential kernel
 constexpr int kGcThreads = 256;
+// State columns and threads per CTA of the sequential kernel.  It is bound by its shared-memory reads (600 16-byte loads per warp and
+// chunk, four cycles each), so what counts is how many SMs share them: 16 heads of 128 columns are 128 CTAs at 16 columns (32
+// columns and 256 threads: 64 CTAs; 2048 and 953 tokens together 497 us, 370 so), and two of them fit an SM when there are more heads.
+constexpr int kGcCols = 16;
+constexpr int kGsThreads = kGcCols * 8;
 
 struct GdnChunkArgs {
   const float* qn;        // [T, hk, dk] unit-norm queries (scaled by dk^-1/2)
@@ -205,10 +209,10 @@ __global__ void __launch_bounds__(kGcThreads) gdn_chunk_prep_kernel(GdnChunkArgs
 }
 
 // ------------------------------------------------------------------------------------------------ kernel 2
-// grid (dv / 32, hv), 256 threads; the CTA owns state columns [32 * blockIdx.x, +32) of head blockIdx.y for the whole
-// run.  Shared memory: S [DK][32], two operand buffers A[2][C][DK + 4] (W, Q, K of a chunk pass through them in turn:
-// while one is multiplied the next is copied in with cp.async), Ps [C][C + 4], U [C][32], g[2][C].
-// Output tiles are [C, 32]: thread (ty = tid / 8 -> rows 2 ty, 2 ty + 1; tx = tid % 8 -> columns 4 tx .. 4 tx + 3).
+// grid (dv / 16, hv), 128 threads; the CTA owns state columns [16 * blockIdx.x, +16) of head blockIdx.y for the whole
+// run.  Shared memory: S [DK][16], two operand buffers A[2][C][DK + 4] (W, Q, K of a chunk pass through them in turn:
+// while one is multiplied the next is copied in with cp.async), Ps [C][C + 4], U [C][16], g[2][C].
+// Output tiles are [C, 16]: thread (ty = tid / 4 -> rows 2 ty, 2 ty + 1; tx = tid % 4 -> columns 4 tx .. 4 tx + 3).
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
   const uint32_t d = smem_u32(dst);
   const int n = valid ? 16 : 0;           // 0 source bytes: the 16 destination bytes are zero-filled
@@ -218,24 +222,24 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 template <int DK>
-__global__ void __launch_bounds__(kGcThreads) gdn_chunk_state_kernel(GdnChunkArgs a) {
+__global__ void __launch_bounds__(kGsThreads) gdn_chunk_state_kernel(GdnChunkArgs a) {
   constexpr int LD = DK + 4, LP = kGcC + 4;
   extern __shared__ __align__(16) float gsm[];
-  float* Ss = gsm;                          // [DK][32]
+  float* Ss = gsm;                          // [DK][16]
   float* Ab = Ss + DK * kGcCols;            // [2][C][LD]
   float* Ps = Ab + 2 * kGcC * LD;           // [C][LP]
-  float* Us = Ps + kGcC * LP;               // [C][32]
+  float* Us = Ps + kGcC * LP;               // [C][16]
   float* gb = Us + kGcC * kGcCols;          // [2][C]
   pdl_wait();
   const int tid = threadIdx.x, h = blockIdx.y, j0 = blockIdx.x * kGcCols;
   const int hk_idx = h / (a.hv / a.hk);
-  const int ty = tid / 8, tx = tid % 8;
+  const int ty = tid / 4, tx = tid % 4;
   float* sp = a.state + (static_cast<size_t>(h) * DK) * a.dv + j0;
-  for (int i = tid; i < DK * kGcCols; i += kGcThreads) Ss[i] = sp[static_cast<size_t>(i / kGcCols) * a.dv + i % kGcCols];
+  for (int i = tid; i < DK * kGcCols; i += kGsThreads) Ss[i] = sp[static_cast<size_t>(i / kGcCols) * a.dv + i % kGcCols];
   // asynchronous copy of C rows of DK floats (rows >= n are zero-filled) into operand buffer `buf`
   auto load_rows = [&](int buf, const float* src, int64_t row_stride, int n) {
     float* dst = Ab + buf * kGcC * LD;
-    for (int i = tid; i < kGcC * (DK / 4); i += kGcThreads) {
+    for (int i = tid; i < kGcC * (DK / 4); i += kGsThreads) {
       const int r = i / (DK / 4), q4 = i % (DK / 4);
       cp_async16(dst + r * LD + q4 * 4, src + static_cast<size_t>(r < n ? r : 0) * row_stride + q4 * 4, r < n);
     }
@@ -249,7 +253,7 @@ __global__ void __launch_bounds__(kGcThreads) gdn_chunk_state_kernel(GdnChunkArg
   auto load_qp = [&](int buf, int c, int t0, int n) {
     const size_t ch = static_cast<size_t>(c) * a.hv + h;
     load_rows(buf, a.qn + (static_cast<size_t>(t0) * a.hk + hk_idx) * DK, static_cast<int64_t>(a.hk) * DK, n);
-    for (int i = tid; i < kGcC * (kGcC / 4); i += kGcThreads) {
+    for (int i = tid; i < kGcC * (kGcC / 4); i += kGsThreads) {
       const int r = i / (kGcC / 4), q4 = i % (kGcC / 4);
       cp_async16(Ps + r * LP + q4 * 4, a.P + ch * kGcC * kGcC + r * kGcC + q4 * 4, true);
     }
@@ -378,7 +382,7 @@ __global__ void __launch_bounds__(kGcThreads) gdn_chunk_state_kernel(GdnChunkArg
     buf ^= 1;                                          // the next chunk's W is (being) copied into Ab[buf]
   }
   __syncthreads();
-  for (int i = tid; i < DK * kGcCols; i += kGcThreads) sp[static_cast<size_t>(i / kGcCols) * a.dv + i % kGcCols] = Ss[i];
+  for (int i = tid; i < DK * kGcCols; i += kGsThreads) sp[static_cast<size_t>(i / kGcCols) * a.dv + i % kGcCols] = Ss[i];
 }
 
 }  // namespace dgpp
@@ -392,7 +396,7 @@ DGPP_API int dgpp_gdn_chunk_scan(const void* qn, const void* kn, const void* dec
                                  int64_t v_stride, void* state, void* out, void* scratch, int64_t scratch_floats, int T,
                                  int hk, int hv, int dk, int dv, cudaStream_t st) {
   DGPP_REQUIRE(dk == 64 || dk == 128, "gdn_chunk: key dim %d (64 or 128)", dk);
-  DGPP_REQUIRE(dv % kGcCols == 0 && hk > 0 && hv % hk == 0, "gdn_chunk: bad head geometry hk %d hv %d dv %d", hk, hv, dv);
+  DGPP_REQUIRE(dv % 32 == 0 && hk > 0 && hv % hk == 0, "gdn_chunk: bad head geometry hk %d hv %d dv %d", hk, hv, dv);
   if (T == 0) return 0;
   const int chunks = dgpp_ceil_div(T, kGcC);
   const int64_t per = static_cast<int64_t>(chunks) * hv * kGcC;
@@ -423,10 +427,10 @@ DGPP_API int dgpp_gdn_chunk_scan(const void* qn, const void* kn, const void* dec
   dim3 g1(chunks, hv), g2(dv / kGcCols, hv);
   if (dk == 64) {
     gdn_chunk_prep_kernel<64><<<g1, kGcThreads, smem1, st>>>(a);
-    gdn_chunk_state_kernel<64><<<g2, kGcThreads, smem2, st>>>(a);
+    gdn_chunk_state_kernel<64><<<g2, kGsThreads, smem2, st>>>(a);
   } else {
     gdn_chunk_prep_kernel<128><<<g1, kGcThreads, smem1, st>>>(a);
-    gdn_chunk_state_kernel<128><<<g2, kGcThreads, smem2, st>>>(a);
+    gdn_chunk_state_kernel<128><<<g2, kGsThreads, smem2, st>>>(a);
   }
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
