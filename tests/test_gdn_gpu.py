@@ -84,3 +84,22 @@ def test_kda_per_channel_decay_recurrence(dev, dk, hk, hv):
     assert (snap[1] - s_ref).abs().max().item() <= 1e-3 * s_ref.abs().max().item() + 1e-4
     assert (out2[:2].float() - w1.float()).abs().max().item() <= 2e-2 * w1.float().abs().max().item() + 1e-3
     assert torch.equal(state2[2], snap[3]) and torch.equal(state2[0], snap[7])
+
+
+@pytest.mark.parametrize("T,C,bias,gap", [(1, 512, True, 0), (2, 514, False, 2), (16, 2, True, 6), (17, 1026, True, 0), (47, 640, False, 4),
+                                          (33, 511, True, 1)])
+def test_conv_of_a_run_equals_the_one_token_form(dev, T, C, bias, gap):
+    """Consecutive tokens of one request as sixteen-token runs per thread (an odd width or stride keeps the general form) against the general
+    kernel: the same bits, the same carried tail."""
+    from dgpp_b200.ops import core as ops
+
+    torch.manual_seed(T)
+    x = torch.randn(T, C + gap, device=dev).to(BF)[:, gap // 2:gap // 2 + C]
+    w, b = torch.randn(C, 4, device=dev).to(BF), torch.randn(C, device=dev).to(BF) if bias else None
+    tail = torch.randn(3, 3, C, device=dev)
+    slots = torch.full((T,), 1, dtype=torch.int32, device=dev)
+    for row_slot, slot in ((None, 1), (slots, 0)):
+        s1, s2 = tail.clone(), tail.clone()
+        y = ops.gdn_conv(x, w, b, s1, torch.empty(T, C, dtype=BF, device=dev), row_slot=row_slot, slot=slot)
+        want = ops.gdn_conv(x, w, b, s2, torch.empty(T, C, dtype=BF, device=dev), row_slot=slots, seg=T)
+        assert torch.equal(y, want) and torch.equal(s1, s2)
