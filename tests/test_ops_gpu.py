@@ -415,3 +415,19 @@ def test_gemm_tc_bf16_splits_in_a_cluster(dev, rows, bn, n, k, splits):
     ops.check_status()
     assert torch.equal(y32.double(), want)
     assert torch.equal(y, (res.float() + want.float().to(torch.bfloat16).float()).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("inter,rows,bn", [(8, 9, 3), (256, 33, 11), (520, 14, 7), (2056, 5, 1), (4096, 6, 2)])
+def test_swiglu_of_several_rows_per_block(dev, inter, rows, bn):
+    """Blocks of 8, 3, 2 and 1 rows with remainders; the rows of a skipped tile are left alone."""
+    from dgpp_b200.ops import core as ops, reference as ref
+
+    torch.manual_seed(inter)
+    gu = torch.randn(rows, 2 * inter, device=dev).to(torch.bfloat16)
+    _close(ops.swiglu(gu), ref.swiglu(gu), 2 ** -7, 1e-3)
+    tiles = torch.arange(rows // bn, dtype=torch.int32, device=dev)
+    tiles[1] = -1
+    out = ops.swiglu_tiles(gu, torch.full((rows, inter), 7.0, device=dev, dtype=torch.bfloat16), tiles, bn)
+    keep = torch.ones(rows, dtype=torch.bool, device=dev)
+    keep[bn:2 * bn] = False
+    assert torch.equal(out[keep], ops.swiglu(gu)[keep]) and (out[~keep] == 7.0).all()
