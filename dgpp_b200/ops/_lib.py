@@ -108,11 +108,10 @@ def _fn(name: str):
     fn = _FNS.get(name)
     if fn is not None:
         return fn
-    fn = _FNS[name] = getattr(load(), name)
-    if not getattr(fn, "_dgpp_typed", False):
-        fn.argtypes = _SIGNATURES[name]
-        fn.restype = I
-        fn._dgpp_typed = True
+    fn = getattr(load(), name)
+    fn.argtypes = _SIGNATURES[name]
+    fn.restype = I
+    _FNS[name] = fn      # typed before another thread can find it: without its argument types ctypes passes pointers as 32-bit ints
     return fn
 
 

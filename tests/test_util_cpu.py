@@ -135,3 +135,23 @@ def test_process_memory_file_residency_and_prefill_progress(tmp_path):
     assert p.most_stalled(100)[0] == "b"
     p.end("b")
     assert p.most_stalled(100)[0] == "a" and len(p.snapshot(100)) == 1
+
+
+def test_a_kernel_entry_is_typed_before_other_threads_can_find_it(monkeypatch):
+    """The table of resolved entries is read without a lock, so an entry must have its argument types when it gets there: ctypes
+    passes the pointers of an untyped function as 32-bit integers."""
+    from dgpp_b200.ops import _lib
+
+    class Entry:
+        def __setattr__(self, key, value):
+            assert "dgpp_status_read" not in _lib._FNS, f"visible before its {key} was set"
+            object.__setattr__(self, key, value)
+
+    class Lib:
+        dgpp_status_read = Entry()
+
+    monkeypatch.setattr(_lib, "_FNS", {})
+    monkeypatch.setattr(_lib, "load", Lib)
+    fn = _lib._fn("dgpp_status_read")
+    assert fn.argtypes == _lib._SIGNATURES["dgpp_status_read"] and fn.restype is _lib.I
+    assert _lib._fn("dgpp_status_read") is fn
