@@ -131,6 +131,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA,   // packed weights
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* last_flag = const_cast<int*>(abort_flag) + 1;
+  volatile int* epi_failed = last_flag + 1;             // an epilogue warp gave up (split K: read between two barriers of the unit)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = static_cast<int>(cluster_ctarank());
@@ -144,6 +145,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA,   // packed weights
     mbar_init(acc_empty, 2 * kPrEpiWarps);
     *abort_flag = 0;
     *last_flag = 0;
+    *epi_failed = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
@@ -304,11 +306,23 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA,   // packed weights
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     const int half = (warp - kPrEpi) >> 2;
     bf16* stage = reinterpret_cast<bf16*>(sOut + (warp - kPrEpi) * kPrStaging);
+    // Counts this CTA in at its half tile; true, and the counter back at zero, for the last of the splits.
+    auto count_in = [&](int u) {
+      uint32_t* counter = p.counters + (u / p.splits) * 2 + rank;
+      const bool last = atomicAdd(counter, 1u) == static_cast<uint32_t>(p.splits - 1);
+      if (last) *counter = 0;
+      return last;
+    };
     int tc = 0;
+    bool dead = false;      // split K: a warp gave up; the remaining units only count themselves in (the counters end at zero)
     for (int u = first_unit; u < p.units; u += unit_step) {
       int n0, nc, m0, split, kb0, nk;
       float alpha;
       if (!unit_at(u, n0, nc, m0, split, kb0, nk, alpha)) continue;
+      if (dead) {
+        if (warp == kPrEpi && lane == 0) count_in(u);
+        continue;
+      }
       const uint32_t d = tmem_base + lane_addr;
       bool ok = wait_bar(acc_full, tc & 1);
       if (!ok) { report(p.status, kTimeoutAccum, 27); *abort_flag = 1; }
@@ -368,15 +382,16 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA,   // packed weights
       __syncwarp();
       if (lane == 0) mbar_arrive_pair(mapa_shared(smem_u32(acc_empty), 0u));
       if (p.splits > 1) {
-        // publish the partials; the last CTA on this half tile adds them in ascending split order
-        uint32_t* counter = p.counters + (u / p.splits) * 2 + rank;
+        // publish the partials; the last CTA on this half tile adds them in ascending split order.  The eight warps leave the
+        // barriers of a unit together: what one of them gave up on is known to all behind the first (nobody writes it
+        // again before the second), and all go on without waiting.
         __threadfence();
+        if (!ok && lane == 0) *epi_failed = 1;
         asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (warp == kPrEpi && lane == 0) {
-          const uint32_t prev = atomicAdd(counter, 1u);
-          *last_flag = (prev == static_cast<uint32_t>(p.splits - 1)) ? 1 : 0;
-        }
+        dead = *epi_failed != 0;
+        if (warp == kPrEpi && lane == 0) *last_flag = count_in(u) ? 1 : 0;
         asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (dead) continue;
         if (*last_flag) {
           __threadfence();
           if (p.vec) {
@@ -424,10 +439,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA,   // packed weights
               p.out[at] = f32_to_bf16(y);
             }
           }
-          if (warp == kPrEpi && lane == 0) *counter = 0;
         }
       }
-      if (!ok) break;
+      if (!ok) break;      // (unsplit: the warps share no barrier)
       ++tc;
     }
   }

@@ -3,6 +3,7 @@ from __future__ import annotations
 
 import math
 import os
+import weakref
 from typing import Optional
 
 import torch
@@ -115,8 +116,10 @@ class GemmWorkspace:
     def __init__(self, device, max_partial_floats: int = 1 << 24, max_tiles: int = 1 << 16):
         self.partials = torch.empty(max_partial_floats, dtype=torch.float32, device=device)
         self.counters = torch.zeros(max_tiles, dtype=torch.int32, device=device)
+        _WORKSPACES.add(self)
 
 
+_WORKSPACES = weakref.WeakSet()
 _WS: dict = {}
 
 
@@ -579,7 +582,14 @@ def msa_index_select(iqk, index_cache, block_table, row_req, positions, ih: int,
 
 
 def check_status() -> None:
-    _lib.check_status()
+    """Synchronise and raise if any kernel gave up on a wait.  The arrival counters of the split-K workspaces are then set back: a count
+    that a broken launch left behind would make later products fold before their partials are there."""
+    try:
+        _lib.check_status()
+    except RuntimeError:
+        for ws in list(_WORKSPACES):
+            ws.counters.zero_()
+        raise
 
 
 _lib.declare("dgpp_segment_copy", [P, I, L, P])

@@ -319,3 +319,24 @@ def test_pair_gemm_grouped_equals_the_plain_form_per_matrix(bn):
         rows = slice(t * bn, (t + 1) * bn)
         want = ops.gemm_tc_pair(x[rows], ws[e]) if e >= 0 else torch.full_like(out[rows], 7.0)
         assert torch.equal(out[rows], want), (t, e)
+
+
+@pytest.mark.parametrize("rows,n,k,splits", [(8, 40960, 512, 2), (128, 10240, 2048, 8)])
+def test_pair_gemm_split_counters_are_at_rest_after_several_units_per_pair(rows, n, k, splits):
+    """More (tile, split) units than pairs, so that every pair counts itself in at several tiles: all counters end at zero, and a second
+    product through the same workspace gives the same bits."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from dgpp_b200.ops import core as ops
+    from dgpp_b200.quant.formats import random_quant_linear
+
+    dev = torch.device("cuda:0")
+    torch.manual_seed(n)
+    w = random_quant_linear(n, k, "nvfp4", dev)
+    x = torch.randn(rows, k, device=dev).to(torch.bfloat16)
+    ws = ops.GemmWorkspace(dev)
+    one = ops.gemm_tc_pair(x, w, splits=splits, ws=ws)
+    torch.cuda.synchronize()
+    ops.check_status()
+    assert not ws.counters.any()
+    assert torch.equal(ops.gemm_tc_pair(x, w, splits=splits, ws=ws), one)

@@ -155,3 +155,27 @@ def test_a_kernel_entry_is_typed_before_other_threads_can_find_it(monkeypatch):
     fn = _lib._fn("dgpp_status_read")
     assert fn.argtypes == _lib._SIGNATURES["dgpp_status_read"] and fn.restype is _lib.I
     assert _lib._fn("dgpp_status_read") is fn
+
+
+def test_a_reported_error_sets_the_split_counters_back(monkeypatch):
+    """A launch that gave up may leave arrival counts behind; once its error has been raised and cleared the workspaces are at rest."""
+    from dgpp_b200.ops import _lib, core as ops
+
+    code = [3]
+
+    def call(name, *args):
+        if name == "dgpp_status_read":
+            import ctypes as C
+            C.cast(args[0], C.POINTER(C.c_int))[0] = code[0]
+        elif name == "dgpp_status_clear":
+            code[0] = 0
+
+    monkeypatch.setattr(_lib, "call", call)
+    ws = ops.GemmWorkspace("cpu", max_partial_floats=16, max_tiles=8)
+    ws.counters[2] = 1
+    with pytest.raises(RuntimeError, match="code=3"):
+        ops.check_status()
+    assert not ws.counters.any()
+    ws.counters[2] = 1
+    ops.check_status()                      # no error: a product may be counting
+    assert ws.counters[2] == 1
