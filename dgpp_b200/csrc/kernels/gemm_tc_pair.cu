@@ -483,19 +483,19 @@ static int pair_slots(int* slots) {
 // 128: 540, 192: 622, 256: 741), a tile's drain at 15 bn (the accumulator is not double-buffered: its other half holds
 // the converted weights); splits cost their partials' way to memory and back and 5500 cycles.  The product takes as many
 // units one after the other as one pair gets: wide tiles reuse a converted weight more often, narrower ones (or
-// splits, where there are fewer tiles than pairs) fill the last round.  Up to 64 rows the splits are those of 64 rows: a row's
-// bits do not depend on how many decode rows share its pass.
-static void pair_shape(int T, int N, int K, int slots, int max_splits, int* bn_out, int* splits_out) {
+// splits, where there are fewer tiles than pairs) fill the last round.  Up to 128 rows the splits are those of 64 rows, above there
+// are none: on either side of that line a row's bits do not depend on how many others share its pass, and prompt products
+// touch no workspace, so that products on several streams share nothing.
+constexpr int kPrSplitRows = 128;
+
+// Cheapest tile and split count for T rows, splits between `fewest` and `most`.
+static void pair_search(int T, int N, int K, int slots, int fewest, int most, int* bn_out, int* splits_out) {
   double best = 0;
-  *bn_out = kPrMaxBN;
-  *splits_out = 1;
-  const int rows = T;
-  if (T < 64) T = 64;
   const int nt = dgpp_ceil_div(N, 2 * kPrBM), raws = K / 256;
   for (int bn = kPrMaxBN; bn >= 16; bn -= 16) {
     if (bn < kPrMaxBN && bn - 16 >= T) continue;          // a smaller tile holds all rows
     const int tiles = nt * dgpp_ceil_div(T, bn);
-    for (int s = 1; s <= max_splits && s <= raws; ++s) {
+    for (int s = fewest; s <= most && s <= raws; ++s) {
       const int per = dgpp_ceil_div(raws, s);
       if (dgpp_ceil_div(raws, per) != s) continue;
       const int rounds = dgpp_ceil_div(tiles * s, slots);
@@ -504,7 +504,14 @@ static void pair_shape(int T, int N, int K, int slots, int max_splits, int* bn_o
       if (best == 0 || cost < best) { best = cost; *bn_out = bn; *splits_out = s; }
     }
   }
-  if (rows < 64) *bn_out = dgpp_ceil_div(rows, 16) * 16;
+}
+
+static void pair_shape(int T, int N, int K, int slots, int max_splits, int* bn_out, int* splits_out) {
+  *bn_out = kPrMaxBN;
+  *splits_out = 1;
+  if (T <= kPrSplitRows) pair_search(64, N, K, slots, 1, max_splits, bn_out, splits_out);
+  if (T < 64) *bn_out = dgpp_ceil_div(T, 16) * 16;
+  if (T > 64) pair_search(T, N, K, slots, *splits_out, *splits_out, bn_out, splits_out);
 }
 
 template <int WMODE, bool GROUPED>
@@ -521,8 +528,8 @@ using namespace dgpp;
 
 // wmode: 1 nvfp4 (w_scale = e4m3 scales [N, K / 16]), 3 mxfp4 (w_scale = e8m0 scales [N, K / 32]).  K % 256 == 0.
 // out bf16 [T, ldc]; resid optional (out = bf16(resid + bf16(alpha * acc))).  bn: token tile, a multiple of 16 up to
-// 256, or 0 = chosen here; splits: K splits, or 0 = chosen here among those that the workspace (ws_floats fp32 values,
-// n_counters counters that are zero at rest) holds.
+// 256, or 0 = chosen here; splits: K splits, or 0 = chosen here (none above 128 rows) among those that the workspace (ws_floats fp32
+// values, n_counters counters that are zero at rest) holds for 128 rows.
 DGPP_API int dgpp_gemm_tc_pair(int wmode, const void* x, int64_t x_stride, const void* w, const void* w_scale, float alpha,
                                void* out, const void* resid, int ldc, int T, int N, int K, int bn, int splits, void* ws,
                                int64_t ws_floats, void* counters, int n_counters, cudaStream_t st) {
@@ -537,15 +544,18 @@ DGPP_API int dgpp_gemm_tc_pair(int wmode, const void* x, int64_t x_stride, const
   if (wmode == 1 ? pair_slots<1, false>(&slots) : pair_slots<3, false>(&slots)) return -1;
   int most = 1;
   if (ws && counters) {
-    const int64_t by_ws = ws_floats / (static_cast<int64_t>(T < 64 ? 64 : T) * N);
+    const int room = T < kPrSplitRows ? kPrSplitRows : T;      // (rows: the same limit for every T that has splits)
+    const int64_t by_ws = ws_floats / (static_cast<int64_t>(room) * N);
     most = static_cast<int>(by_ws < 8 ? (by_ws < 1 ? 1 : by_ws) : 8);
-    if (2LL * dgpp_ceil_div(N, 2 * kPrBM) * dgpp_ceil_div(T, 16) > n_counters) most = 1;
+    if (2LL * dgpp_ceil_div(N, 2 * kPrBM) * dgpp_ceil_div(room, 16) > n_counters) most = 1;
   }
   int pick_bn, pick_splits;
   pair_shape(T, N, K, slots, most, &pick_bn, &pick_splits);
   if (bn == 0) bn = pick_bn;
   if (splits == 0) splits = pick_splits;
-  DGPP_REQUIRE(splits <= most || splits == 1, "gemm_tc_pair: %d splits do not fit the workspace", splits);
+  DGPP_REQUIRE(splits == 1 || (splits <= 8 && static_cast<int64_t>(splits) * T * N <= ws_floats &&
+                               2LL * dgpp_ceil_div(N, 2 * kPrBM) * dgpp_ceil_div(T, bn) <= n_counters),
+               "gemm_tc_pair: %d splits do not fit the workspace", splits);
   PairParams p;
   p.alpha = alpha * 16384.f;    // the converted weights carry 2^-14
   p.out = static_cast<bf16*>(out);

@@ -151,6 +151,8 @@ def pick_splits(rows: int, n: int, k: int, bn: int, sms: int = 148) -> int:
 # weights in tensor memory).  Without split-K the results are those of the single-CTA kernel bit for bit.
 PAIR_GEMM = True
 PAIR_GEMM_MIN_ROWS = 1
+# Passes of up to this many rows split K, all alike; above it the products share no workspace and are the same at every row count.
+PAIR_SPLIT_ROWS = 128
 
 _lib.declare("dgpp_gemm_tc_pair", [I, P, L, P, P, F, P, P, I, I, I, I, I, I, P, L, P, I, P])
 
@@ -158,12 +160,14 @@ _lib.declare("dgpp_gemm_tc_pair", [I, P, L, P, P, F, P, P, I, I, I, I, I, I, P, 
 def gemm_tc_pair(x: torch.Tensor, w: QuantLinear, out: Optional[torch.Tensor] = None, resid: Optional[torch.Tensor] = None,
                  bn: int = 0, splits: int = 1, ws: Optional[GemmWorkspace] = None) -> torch.Tensor:
     """The W4A16 linear on CTA pairs (NVFP4 / MXFP4 weights).  bn: tokens per tile (a multiple of 16 up to 256; 0: chosen by the
-    library); splits: K splits (0: chosen by the library)."""
+    library); splits: K splits (0: chosen by the library; none above PAIR_SPLIT_ROWS rows)."""
     _chk(x, torch.bfloat16, "x")
     rows, k = x.shape
     assert k == w.k and w.fmt in ("nvfp4", "mxfp4") and k % 256 == 0
     if out is None:
         out = torch.empty(rows, w.n, dtype=torch.bfloat16, device=x.device)
+    if splits == 0 and rows > PAIR_SPLIT_ROWS:
+        splits = 1
     if splits != 1:
         ws = ws or default_workspace(x.device)
     wsp, cnt = (ws.partials, ws.counters) if splits != 1 else (None, None)

@@ -340,3 +340,32 @@ def test_pair_gemm_split_counters_are_at_rest_after_several_units_per_pair(rows,
     ops.check_status()
     assert not ws.counters.any()
     assert torch.equal(ops.gemm_tc_pair(x, w, splits=splits, ws=ws), one)
+
+
+@pytest.mark.parametrize("n,k", [(5120, 17408), (2048, 5632), (520, 2048)])
+def test_pair_gemm_rows_do_not_depend_on_the_batch(n, k):
+    """Up to 128 rows all passes split K alike, above none does (the single-CTA kernel's unsplit bits): on either side of that line a
+    row has the same bits whatever the number of rows."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from dgpp_b200.ops import core as ops
+    from dgpp_b200.quant.formats import random_quant_linear
+
+    dev = torch.device("cuda:0")
+    torch.manual_seed(n)
+    w = random_quant_linear(n, k, "nvfp4", dev)
+    x = torch.randn(2048, k, device=dev).to(torch.bfloat16)
+    some = ops.gemm_tc(x[:128], w)
+    for rows in (1, 8, 63, 64, 65, 100):
+        assert torch.equal(ops.gemm_tc(x[:rows], w), some[:rows]), rows
+    many = ops.gemm_tc(x, w)
+    for rows in (129, 173, 256, 300, 512, 953, 1024):
+        assert torch.equal(ops.gemm_tc(x[:rows], w), many[:rows]), rows
+    old = ops.PAIR_GEMM
+    try:
+        ops.PAIR_GEMM = False
+        assert torch.equal(ops.gemm_tc(x[:173], w, splits=1), many[:173])
+    finally:
+        ops.PAIR_GEMM = old
+    torch.cuda.synchronize()
+    ops.check_status()

@@ -179,3 +179,26 @@ def test_a_reported_error_sets_the_split_counters_back(monkeypatch):
     ws.counters[2] = 1
     ops.check_status()                      # no error: a product may be counting
     assert ws.counters[2] == 1
+
+
+@pytest.mark.parametrize("rows,shared", [(1, True), (128, True), (129, False), (173, False), (1000, False), (2048, False)])
+def test_prompt_products_of_4_bit_weights_share_no_workspace(monkeypatch, rows, shared):
+    """Above 128 rows a 4-bit linear neither splits K nor hands the library the device's shared partials and counters, so that callers on
+    several streams do not meet there."""
+    import torch
+
+    from dgpp_b200.ops import core as ops
+    from dgpp_b200.quant.formats import QuantLinear
+
+    seen = []
+    monkeypatch.setattr(ops, "_chk", lambda *a: None)
+    monkeypatch.setattr(ops, "stream_ptr", lambda *a: 0)
+    monkeypatch.setattr(ops, "call", lambda name, *a: seen.append((name, a)))
+    ws = ops.GemmWorkspace("cpu", max_partial_floats=16, max_tiles=8)
+    monkeypatch.setattr(ops, "default_workspace", lambda dev: ws)
+    w = QuantLinear("nvfp4", 5120, 256, torch.zeros(5120, 128, dtype=torch.uint8), scale=torch.zeros(5120, 16, dtype=torch.uint8))
+    ops.linear(torch.zeros(rows, 256, dtype=torch.bfloat16), w)
+    (name, a), = seen
+    assert name == "dgpp_gemm_tc_pair"
+    splits, partials, counters = a[13], a[14], a[16]
+    assert (splits, partials, counters) == ((0, ws.partials.data_ptr(), ws.counters.data_ptr()) if shared else (1, None, None))
