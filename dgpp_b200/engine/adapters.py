@@ -292,7 +292,8 @@ class KernelEngine(EmbedSplice, SlotSampling, rt.SchedulerEngine):
         """spec_drafts > 0: greedy speculative decoding with context-lookup drafts.  Every decode pass carries, per
         request, its pending token plus up to `spec_drafts` proposed continuations as extra rows of the same batch;
         the rows' own greedy picks verify the drafts (longest matching prefix + one bonus token), so the output is
-        token for token what plain greedy decoding gives.  Rejected positions are simply overwritten later: the
+        token for token what plain greedy decoding gives (of an engine with `pin_split_rows`, where plain passes have more
+        than 32 rows).  Rejected positions are simply overwritten later: the
         dense family has no state besides the KV cache.  (reference counterparts: src/engine/speculative.hpp
         GreedySpeculator / judge_verify, src/engine/lookup_draft.hpp, verify rows batched into the decode pass.)"""
         super().__init__()
@@ -302,6 +303,10 @@ class KernelEngine(EmbedSplice, SlotSampling, rt.SchedulerEngine):
         self.drafts = [rt.LookupDraft(2, 4) for _ in range(engine.max_batch)] if self.spec_k else None
         self.schedule = [rt.VerifySchedule(0, self.spec_k, min(self.spec_k, 3)) for _ in range(engine.max_batch)] \
             if self.spec_k else None
+        if self.spec_k:
+            # one arithmetic at every width of a pass: a row with drafts beside it computes what it would alone
+            engine.runner.verifies_drafts = True
+            engine.graphs.clear()
         self.spec_graphs = {}
         self.spec_proposed = self.spec_accepted = 0
         self.pending = [None] * engine.max_batch

@@ -105,6 +105,7 @@ class DenseRunner:
         self.fused_decode = fused_decode
         self._fused_plans, self._fused_bufs = {}, None
         self.fp4_rows = min(64, decode_rows or max_rows)
+        self.verifies_drafts = False      # decode passes carry draft rows, which are to be what plain rows would be (set by the engine)
         if self.decode_fp4:
             bn = min(64, ops.pick_bn(self.fp4_rows))
             for k in {H, self.hq * d, I}:
@@ -213,6 +214,13 @@ class DenseRunner:
                                    self.hkv, self.d, self.scale, splits=1, out=attn, window=L.window)
             plan[li + 1].launch()
 
+    def fp4_width(self) -> int:
+        """Widest decode pass whose linears take the block-scaled FP4 kernels.  Above 32 rows the terms of a row fill a 192-column tile
+        and the W4A16 GEMM on CTA pairs is the faster one, without quantisers (37 rows, 16 layers of 5120 / 17408: 3005 -> 2796
+        us a pass); the all-reduce push keeps its epilogues, and where draft rows are verified (or the split choice is pinned) a
+        row keeps its bits at every width."""
+        return self.fp4_rows if (self.verifies_drafts or ops.PIN_SPLIT_ROWS or self.fuse_ar) else min(32, self.fp4_rows)
+
     def linear(self, x, w, out, fp4: bool):
         if fp4 and w.fmt == "nvfp4" and w.k % 256 == 0:
             xa = ops.act_quant_nvfp4(x, self.act_terms, out=self.qa[w.k])
@@ -303,11 +311,7 @@ class DenseRunner:
         pending = False
         sp_in = False
         splits = self.decode_splits if (decode and rows <= 256) else 1
-        # above 32 rows the terms of a row fill a 192-column tile and the W4A16 GEMM on CTA pairs is the faster one, without
-        # quantisers (37 rows, 16 layers of 5120 / 17408: 3005 -> 2796 us a pass); the all-reduce push keeps its epilogues, and with
-        # the split choice pinned (speculation) a row keeps its bits at every width
-        cap = self.fp4_rows if (ops.PIN_SPLIT_ROWS or self.fuse_ar) else min(32, self.fp4_rows)
-        fp4 = self.decode_fp4 and decode and rows <= cap and all(
+        fp4 = self.decode_fp4 and decode and rows <= self.fp4_width() and all(
             w.k % 256 == 0 for w in (m.layers[0].qkv, m.layers[0].o, m.layers[0].down))
         lora = self.lora
         fused = fp4 and decode and self.embed_spans is None and self._fused_ok(rows)

@@ -369,6 +369,54 @@ def test_speculative_lookup_decode_equals_plain_greedy(dev):
     assert m1["decode_passes"] <= m0["decode_passes"]
 
 
+def test_speculative_passes_of_more_than_32_rows_keep_the_bits_of_a_row(dev):
+    """A verify pass of 40 rows and a plain pass of eight of them: the same logits, bit for bit; and with the split choice pinned a plain
+    engine of 36 requests gives the tokens of one whose passes carry draft rows too.  (Prompts fill a chunk: no pass mixes prompt and decode rows.)"""
+    from dgpp_b200.engine.adapters import KernelEngine
+    from dgpp_b200.engine.llm_engine import LLMEngine
+    from dgpp_b200.engine.options import EngineOptions
+    from dgpp_b200.models.dense import DenseConfig, DenseModel
+    from dgpp_b200.ops import core as ops
+    from dgpp_b200.runtime import rt
+
+    cfg = DenseConfig.tiny(hidden=512, q_heads=4, kv_heads=2, head_dim=128, ffn=1024, vocab=2048, layers=2)
+    model = DenseModel.random_init(cfg, device=dev, seed=0, std=0.05)
+    g = torch.Generator().manual_seed(12)
+    prompts = [torch.randint(0, cfg.vocab, (8,), generator=g).tolist() * 8 for _ in range(36)]
+
+    def engine(spec, **options):
+        return KernelEngine(LLMEngine(model, max_batch=64, max_seq_len=128, prefill_chunk=64, options=EngineOptions(**options)), spec_drafts=spec)
+
+    eng = engine(3)
+    r = eng.e.runner
+    for s in range(40):
+        assert eng.e.kv.reserve(s, 1)
+    tok = torch.randint(0, cfg.vocab, (40,), generator=g).to(dev, torch.int32)
+    pos, req = torch.zeros(40, dtype=torch.int32, device=dev), torch.arange(40, dtype=torch.int32, device=dev)
+    wide = r.forward(40, tok, pos, req, decode=True)[:8].clone()
+    assert torch.equal(r.forward(8, tok[:8], pos[:8], req[:8], decode=True), wide)
+
+    def run(eng):
+        s = rt.Scheduler(eng, rt.SchedulerConfig())
+        for i, p in enumerate(prompts):
+            s.submit(str(i), p, 30)
+        s.run(100000)
+        out = {}
+        for kind, rid, a, b in s.events():
+            if kind == "token":
+                out.setdefault(rid, []).append(a)
+        ops.check_status()
+        return out
+
+    eng = engine(3)
+    spec = run(eng)
+    assert max(eng.spec_graphs) > 36 and len(spec) == 36
+    try:
+        assert run(engine(0, pin_split_rows=True)) == spec
+    finally:
+        EngineOptions().apply_process_wide()
+
+
 @pytest.mark.parametrize("plen", [300, 77])
 def test_prefix_cache_hit_reproduces_the_uncached_tokens(dev, plen):
     """The same prompt twice through scheduler + kernel engine: the second run attaches the cached KV blocks, prefills
