@@ -295,7 +295,7 @@ class MoEBlock:
         pair_row, _, _ = ops.moe_segment_sort(ids, bn, max_tiles, self.e0, self.e1, ws["pair_row"][:T * c.top_k], tiles,
                                               ws["n_tiles"])
         rows = max_tiles * bn
-        xs, h, y = ws["xs"][:rows], ws["h"][:max_tiles], ws["y"][:max_tiles]
+        xs, h, y = ws["xs"][:rows], ws["h"][:rows].view(max_tiles, bn, -1), ws["y"][:rows].view(max_tiles, bn, -1)
         ops.moe_gather_rows(xn, pair_row, xs, c.top_k)
         xa = ops.act_quant_nvfp4(xs, R, out=ws["qa_x"], group_list=tiles, group_rows=bn)
         ops.gemm_fp4_grouped(xa, w.gu_q, w.gu_sf, w.gu_alpha, h, bn, 2 * c.moe_ffn, c.hidden, self.local_experts, tiles,
@@ -326,7 +326,7 @@ class MoEBlock:
         pair_row, _, _ = ops.moe_segment_sort(ids, bn, max_tiles, self.e0, self.e1, ws["pair_row"][:T * c.top_k], tiles,
                                               ws["n_tiles"])
         rows = max_tiles * bn
-        xs, h, act, y = ws["xs"][:rows], ws["h"].view(-1, 2 * c.moe_ffn)[:rows], ws["act"][:rows], ws["y"].view(-1, c.hidden)[:rows]
+        xs, h, act, y = ws["xs"][:rows], ws["h"][:rows], ws["act"][:rows], ws["y"][:rows]
         ops.moe_gather_rows(xn, pair_row, xs, c.top_k)
         ops.gemm_tc_pair_grouped(xs, w.gu_q, w.gu_sf, w.gu_alpha, h, 2 * c.moe_ffn, c.hidden, self.stack_experts, tiles, bn)
         ops.swiglu_tiles(h, act, tiles, bn, c.swiglu_limit, c.swiglu_alpha)
@@ -361,18 +361,23 @@ _PREFILL_WS: dict = {}
 
 
 def _prefill_workspace(device, max_tiles: int, bn: int, hidden: int, ffn: int, terms: int) -> dict:
-    """Tile buffers of MoEBlock.forward_gathered, kept per (device, geometry) and grown to the largest tile count."""
-    key = (str(device), bn, hidden, ffn, terms)
+    """Buffers of MoEBlock.forward_gathered, one set per (device, geometry, activation form) grown to the largest need.  All tile widths
+    share it: rows are flat, every pass fills what it reads."""
+    key = (str(device), hidden, ffn, terms)
+    rows = max_tiles * bn
     ws = _PREFILL_WS.get(key)
-    if ws is None or ws["max_tiles"] < max_tiles:
-        rows = max_tiles * bn
+    if ws is None or ws["max_tiles"] < max_tiles or ws["rows"] < rows:
+        if ws is not None:
+            max_tiles, rows = max(max_tiles, ws["max_tiles"]), max(rows, ws["rows"])
+            _PREFILL_WS.pop(key)      # (given back before the larger set is taken)
+            ws = None
         i32 = dict(dtype=torch.int32, device=device)
-        ws = dict(max_tiles=max_tiles,
+        ws = dict(max_tiles=max_tiles, rows=rows,
                   pair_row=torch.empty(rows, **i32), tile_expert=torch.full((max_tiles,), -1, **i32),
                   n_tiles=torch.zeros(1, **i32),
                   xs=torch.zeros(rows, hidden, dtype=BF, device=device),
-                  h=torch.zeros(max_tiles, bn, 2 * ffn, dtype=BF, device=device),
-                  y=torch.zeros(max_tiles, bn, hidden, dtype=BF, device=device))
+                  h=torch.zeros(rows, 2 * ffn, dtype=BF, device=device),
+                  y=torch.zeros(rows, hidden, dtype=BF, device=device))
         if terms:
             ws.update(qa_x=ops.QuantAct(rows, hidden, terms, bn, device), qa_mid=ops.QuantAct(rows, ffn, terms, bn, device))
         else:      # bf16 activations

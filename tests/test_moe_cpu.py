@@ -55,3 +55,17 @@ def test_mxfp4_is_reexpressed_exactly_in_the_block_scaled_layout():
     assert r.payload.data_ptr() == q.payload.data_ptr()
     w[9] *= 1e9                                   # more than 18 octaves between block scales: refused, not rounded
     assert mxfp4_as_nvfp4(quantize(w, "mxfp4")) is None
+
+
+def test_prompt_buffers_are_one_set_for_all_tile_widths(monkeypatch):
+    """Passes of any length and tile width share the buffers of the largest one."""
+    from dgpp_b200.models import moe
+
+    monkeypatch.setattr(moe, "_PREFILL_WS", {})
+    big = moe._prefill_workspace("cpu", 12, 128, 256, 256, 0)
+    for tiles, bn in ((12, 32), (10, 64), (12, 128), (8, 192)):
+        assert moe._prefill_workspace("cpu", tiles, bn, 256, 256, 0) is big
+    more = moe._prefill_workspace("cpu", 40, 32, 256, 256, 0)          # more tiles of fewer rows
+    assert len(moe._PREFILL_WS) == 1 and more["tile_expert"].numel() == 40 and more["xs"].shape[0] == more["pair_row"].numel() == 12 * 128
+    wide = moe._prefill_workspace("cpu", 10, 192, 256, 256, 0)
+    assert len(moe._PREFILL_WS) == 1 and wide["tile_expert"].numel() == 40 and all(wide[b].shape[0] == 1920 for b in ("xs", "h", "act", "y"))
