@@ -398,8 +398,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA,   // bf16 weights, or pa
   if constexpr (!kQuant) {
     if (p.staged && warp >= 2) {
       const int q = warp & 3, half = (warp - 2) >> 2;
-      const bool ok = wait_bar(acc_full, 0) && !*abort_flag;
+      bool ok = wait_bar(acc_full, 0) && !*abort_flag;
       if (!ok) { report(p.status, kTimeoutAccum, 7); *abort_flag = 1; }
+      ok = __all_sync(0xffffffffu, ok);                  // the TMEM loads below stay warp-uniform
       tc_fence_after();
       const int cols = min(BN, p.T - m0), at = q * 32 + lane;
       // the operand rings are idle once the accumulator is complete (sB and sA are one block of shared memory)
@@ -445,8 +446,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA,   // bf16 weights, or pa
     const int q = warp & 3, cols = min(BN, p.T - m0);
     float* red = reinterpret_cast<float*>(sB);            // [BN][kBM]
     if (warp >= 2 && warp < 6) {
-      const bool ok = nkb > 0 && wait_bar(acc_full, 0) && !*abort_flag;
+      bool ok = nkb > 0 && wait_bar(acc_full, 0) && !*abort_flag;
       if (!ok && nkb > 0) { report(p.status, kTimeoutAccum, 8); *abort_flag = 1; }
+      ok = __all_sync(0xffffffffu, ok);                  // the TMEM loads below stay warp-uniform
       tc_fence_after();
       for (int c0 = 0; c0 < cols; c0 += 16) {
         uint32_t r[16];
@@ -486,8 +488,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA,   // bf16 weights, or pa
   // ------------------------------------------------------------------ epilogue (warps 2..5)
   if ((kQuant || !(p.staged || p.cluster)) && warp >= 2 && warp < 6) {
     const int q = warp & 3;  // TMEM lane quadrant this warp may read
-    const bool ok = nkb > 0 ? wait_bar(acc_full, 0) : true;
+    bool ok = nkb > 0 ? wait_bar(acc_full, 0) : true;
     if (!ok) { report(p.status, kTimeoutAccum, 6); *abort_flag = 1; }
+    ok = __all_sync(0xffffffffu, ok && !*abort_flag);     // the TMEM loads below stay warp-uniform
     tc_fence_after();
     const int n = n0 + q * 32 + lane;
     const int cols = min(BN, p.T - m0);
@@ -499,7 +502,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA,   // bf16 weights, or pa
       push_owner = min(static_cast<int>(blockIdx.y) / p.tiles_per_rank, p.comm.world - 1);
       push_dst = reinterpret_cast<bf16*>(payload(p.comm, push_owner, push_epoch & 1, p.comm.rank));
     }
-    if (ok && !*abort_flag) {
+    if (ok) {
       float* wsp = splits > 1 ? p.ws + (static_cast<size_t>(split) * p.T + m0) * p.N : nullptr;
 #pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += 16) {
