@@ -162,7 +162,7 @@ def main() -> int:
     ap.add_argument("--mtp", type=int, default=0, choices=(0, 1, 2, 3),
                     help="--config 4: speculative decoding with this many MTP drafts per step (0 = off)")
     ap.add_argument("--moe-prefill-terms", type=int, default=1, choices=(1, 2, 3),
-                    help="--config 2/3/4: residual NVFP4 terms of the activations in the expert GEMMs at prefill sizes")
+                    help="--config 2/3/4: activations of the expert GEMMs at prefill sizes: 1 = one NVFP4 term, 2 and 3 = bf16")
     ap.add_argument("--layers", type=int, default=64, help="debug only: a run with fewer layers is not a valid number")
     ap.add_argument("--reducer", default="peer", choices=["peer", "nccl"])
     ap.add_argument("--prefill-lens", default="2048,8192,32768", help="cold-prefill lengths timed as extras ('' = none)")

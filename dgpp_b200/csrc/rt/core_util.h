@@ -245,7 +245,7 @@ struct ClusterConfig {
   bool engine_fp4_preload = true;           // weight half of the first ring stages issued before the grid dependency
   bool engine_layer_kernel = false;         // decode through the persistent decode-layer kernel
   bool engine_seq_parallel = true;          // tensor-parallel prefill keeps the residual stream sharded by token tile
-  int engine_moe_prefill_terms = 3;         // residual NVFP4 terms of the activations in expert GEMMs at prefill sizes (1..3)
+  int engine_moe_prefill_terms = 3;         // activations of the expert GEMMs at prefill sizes: 1 = one NVFP4 term, 2 and 3 = bf16
   int engine_mtp_depth = 0;                 // speculative decoding: MTP drafts per step (0 = off, up to 3)
   bool engine_pin_split_rows = false;       // split-K choices ignore one row vs several (plain == speculative bits)
   std::string log_level = "info";

@@ -21,7 +21,7 @@ class EngineOptions:
     fp4_preload: bool = True          # weight half of the first ring stages issued before the grid dependency
     layer_kernel: bool = False        # decode through the persistent decode-layer kernel
     seq_parallel: bool = True         # tensor-parallel prefill: residual stream sharded by token tile between the blocks
-    moe_prefill_terms: int = 3        # residual NVFP4 terms of the activations in the expert GEMMs at prefill sizes
+    moe_prefill_terms: int = 3        # activations of the expert GEMMs at prefill sizes: 1 = one NVFP4 term, 2 and 3 = bf16
     mtp_depth: int = 0                # speculative decoding with the MTP head: drafts per step (0 = off)
     pin_split_rows: bool = False      # split-K choices ignore one row vs several (plain and speculative rows: same bits)
 

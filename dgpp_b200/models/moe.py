@@ -186,9 +186,9 @@ def moe_reference(x: torch.Tensor, w: MoEWeights, ids=None, wts=None) -> torch.T
 class MoEBlock:
     """Device buffers + launch sequence of one MoE block for up to `max_rows` decode rows."""
 
-    # residual NVFP4 terms of the activations at prefill sizes (tiles of 64 rows).  3 = the decode path's arithmetic
-    # (near-bf16 activations); 1 = plain W4A4 (4-bit activations, a third of the tensor-core and quantiser work).
-    # Class-wide so one deployment key sets it for every block.
+    # Activations of the expert products at prefill sizes: 1 = one NVFP4 term (plain W4A4, tiles of 64 rows through the block-scaled
+    # GEMM); 2 and 3, once residual NVFP4 terms, = bf16 as they are (tiles of 32 to 192 rows through the W4A16 GEMM on CTA
+    # pairs, nearer to the exact product than three terms).  Class-wide so one deployment key sets it for every block.
     PREFILL_TERMS = 3
 
     def __init__(self, w: MoEWeights, max_rows: int, device, act_terms: int = 3, prefill_terms: Optional[int] = None,
@@ -277,16 +277,16 @@ class MoEBlock:
         return ops.moe_combine(self.y, sh, ids, wts, self.slot_of, out, rows)
 
     def forward_gathered(self, xn: torch.Tensor) -> torch.Tensor:
-        """Prefill-sized batches, all on the device: router, counting sort of the (token, k) pairs by expert into tiles
-        of 64 rows, row gather, then the decode path's kernels with every tile as one slot -- residual-term quantiser,
-        grouped block-scaled gate/up GEMM, SwiGLU quantiser, grouped down GEMM -- and the ordered combine.  The tile
-        buffers are shared by all blocks of a device (one MoE block runs at a time).
+        """Prefill-sized batches, all on the device: router, counting sort of the (token, k) pairs by expert into tiles, row
+        gather, gate / up product, SwiGLU and down product over the tiles, and the ordered combine.  Here the form with
+        4-bit activations: tiles of 64 rows through the decode path's kernels, every tile one slot (quantiser, grouped block-scaled GEMM).
+        The tile buffers are shared by all blocks of a device (one MoE block runs at a time).
         (reference counterparts: src/kernels/glm_moe.cu:1382 segment count, :1553 tile list, :1121 grouped MMA.)"""
         c, w = self.c, self.w
         T = xn.shape[0]
-        if self.prefill_terms > 1 and c.hidden % 256 == 0 and c.moe_ffn % 256 == 0:
+        if self.prefill_terms > 1:
             return self._gathered_bf16(xn)
-        bn, R = 64, self.prefill_terms
+        bn, R = 64, 1
         max_tiles = (T * c.top_k + bn - 1) // bn + self.local_experts
         ws = _prefill_workspace(xn.device, max_tiles, bn, c.hidden, c.moe_ffn, R)
         ids, wts = ops.moe_route(xn, w.gate, w.bias, c.top_k, c.n_group, c.topk_group, c.router == "softmax",

@@ -1,7 +1,7 @@
 """Expert parallelism with token-sharded all-to-all dispatch / combine over NVLink peer memory.
 
 Every rank routes ITS rows, stores each (token, k) pair's row into the receive area of the rank that owns the expert,
-runs the grouped block-scaled expert GEMMs over what it received (sorted into 64-row tiles per local expert), stores the
+runs the grouped expert GEMMs over what it received (sorted into 64-row tiles per local expert), stores the
 result rows back into the sources' return areas, and folds its own rows' results in ascending k order.  All transfers
 are plain peer stores from our kernels (`csrc/kernels/ep_moe.cu`) with bounded flag waits; NCCL only carries the IPC
 handles at construction.  The result is bit-identical to the single-rank prefill path of `MoEBlock` whatever the number
@@ -64,11 +64,12 @@ class EpMoE:
     shared expert, a copy of it (the shared expert runs on the rank's own rows)."""
 
     def __init__(self, w: MoEWeights, max_rows: int, device, group=None, act_terms: int = 3, comm=None, pool=None):
-        """comm: a communicator from `open_comm` shared by the blocks of one model (their exchanges are sequential; the
-        slot size must fit max_rows * top_k pairs); pool: a dict through which those blocks share their tile buffers."""
+        """act_terms: 1 for 4-bit activations, more for bf16 ones (as `MoEBlock.PREFILL_TERMS`); comm: a communicator from
+        `open_comm` shared by the blocks of one model (their exchanges are sequential; the slot size must fit
+        max_rows * top_k pairs); pool: a dict through which those blocks share their tile buffers."""
         c = w.cfg
         assert w.gu_q is not None, "call MoEWeights.stack() on the device first"
-        self.w, self.c, self.dev, self.terms = w, c, device, act_terms
+        self.w, self.c, self.dev = w, c, device
         self.max_rows, self.max_pairs = max_rows, max_rows * c.top_k
         lib = _lib.load()
         lib.dgpp_ep_slot_bytes.restype = L
@@ -105,12 +106,12 @@ class EpMoE:
         self.y = shared("y", lambda: torch.zeros(self.max_tiles, self.bn, c.hidden, dtype=BF, device=device))
         # bf16 activations through the W4A16 GEMM on CTA pairs, as MoEBlock.forward_gathered does (the same bits per row);
         # a single term asks for 4-bit activations
-        self.bf16 = act_terms > 1 and c.hidden % 256 == 0 and c.moe_ffn % 256 == 0
+        self.bf16 = act_terms > 1
         if self.bf16:
             self.act = shared("act", lambda: torch.zeros(rows, c.moe_ffn, dtype=BF, device=device))
         else:
-            self.qa_x = shared("qa_x", lambda: ops.QuantAct(rows, c.hidden, act_terms, self.bn, device))
-            self.qa_mid = shared("qa_mid", lambda: ops.QuantAct(rows, c.moe_ffn, act_terms, self.bn, device))
+            self.qa_x = shared("qa_x", lambda: ops.QuantAct(rows, c.hidden, 1, self.bn, device))
+            self.qa_mid = shared("qa_mid", lambda: ops.QuantAct(rows, c.moe_ffn, 1, self.bn, device))
 
     def forward(self, xn: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """xn: this rank's rows [T, H] bf16 (1 <= T <= max_rows; every rank calls with its own T).  Returns [T, H]."""
@@ -136,10 +137,10 @@ class EpMoE:
             ops.swiglu_tiles(h, self.act, self.tiles, self.bn, c.swiglu_limit, c.swiglu_alpha)
             ops.gemm_tc_pair_grouped(self.act, w.down_q, w.down_sf, w.down_alpha, y, H, c.moe_ffn, stacked, self.tiles, self.bn)
         else:
-            xa = ops.act_quant_nvfp4(self.xs, self.terms, out=self.qa_x, group_list=self.tiles, group_rows=self.bn)
+            xa = ops.act_quant_nvfp4(self.xs, 1, out=self.qa_x, group_list=self.tiles, group_rows=self.bn)
             ops.gemm_fp4_grouped(xa, w.gu_q, w.gu_sf, w.gu_alpha, self.h, self.bn, 2 * c.moe_ffn, H, self.local, self.tiles,
                                  group_b=True)
-            xm = ops.act_quant_nvfp4(self.h.view(rows, 2 * c.moe_ffn), self.terms, out=self.qa_mid, mode="swiglu",
+            xm = ops.act_quant_nvfp4(self.h.view(rows, 2 * c.moe_ffn), 1, out=self.qa_mid, mode="swiglu",
                                      limit=c.swiglu_limit, alpha=c.swiglu_alpha, group_list=self.tiles, group_rows=self.bn)
             ops.gemm_fp4_grouped(xm, w.down_q, w.down_sf, w.down_alpha, self.y, self.bn, H, c.moe_ffn, self.local, self.tiles,
                                  group_b=True)
