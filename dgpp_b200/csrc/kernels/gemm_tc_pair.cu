@@ -5,7 +5,8 @@
 //
 //   two CTAs of a cluster (one TPC) own 256 weight rows x bn tokens (bn <= 256).  Each CTA streams and converts ITS 128
 //   weight rows and loads ITS half of the tokens; one `tcgen05.mma.cta_group::2` per K = 16 step, issued by the first
-//   CTA, multiplies all 256 rows by all bn tokens.  The converted weights are the A operand and live in TMEM: a
+//   CTA, multiplies all 256 rows by all bn tokens (a pair's MMA takes multiples of 32 columns: a tile of another width
+//   carries some of the next rows along and drops them).  The converted weights are the A operand and live in TMEM: a
 //   converter thread owns one weight row = one TMEM lane, so 64 weights leave its registers as one `tcgen05.st` and
 //   never cross shared memory.  (With A in shared memory a K = 64 step of 256 tokens takes 643 cycles, with A in TMEM 544; the
 //   arithmetic's own minimum is 512.)  No TMA multicast: every CTA issues plain loads into its own shared memory.
@@ -67,6 +68,7 @@ struct PairParams {
   DeviceStatus* status;
   int T, N, K, ldc;
   int bn, m_tiles, units, splits, kb_per_split;
+  int width;                 // columns of a tile's MMAs: bn, rounded up to a multiple of 32
   int vec;                   // rows of `out` (and `resid`) can be accessed as 16-byte vectors
   // Grouped form (experts): the matrices are stacked along N ([experts * N, K], N a multiple of 256); token tile t holds rows
   // t * bn .. of x and `out` and belongs to matrix groups[t] (negative: nothing to do).  The block scales come in the
@@ -112,7 +114,7 @@ __device__ __forceinline__ void expand_e2m1x64(const Pack16& w0, const Pack16& w
 template <int WMODE, bool GROUPED>   // 1 = NVFP4, 3 = MXFP4
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPrThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA,   // packed weights as bytes [N, K / 2], box 128 x 128
-                    const __grid_constant__ CUtensorMap tmB,   // activations bf16 [T, K], box 64 x bn / 2
+                    const __grid_constant__ CUtensorMap tmB,   // activations bf16 [T, K], box 64 x width / 2
                     const __grid_constant__ CUtensorMap tmSf,  // NVFP4 scales [N, K / 16], box 16 x 128
                     PairParams p) {
   extern __shared__ __align__(1024) unsigned char smem_dyn[];
@@ -188,14 +190,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA,   // packed weights
   if (warp == kPrTma) {
     // ------------------------------------------------------------------ TMA producer (own weights, own token half)
     if (elect_one()) {
-      const uint32_t stage_b = static_cast<uint32_t>(p.bn / 2) * 128u;
+      const uint32_t stage_b = static_cast<uint32_t>(p.width / 2) * 128u;
       int it = 0;
       bool ok = true;
       for (int u = first_unit; u < p.units && ok; u += unit_step) {
         int n0, nc, m0, split, kb0, nk;
         float alpha;
         if (!unit_at(u, n0, nc, m0, split, kb0, nk, alpha)) continue;
-        const int mh = m0 + rank * (p.bn / 2);
+        const int mh = m0 + rank * (p.width / 2);
         for (int i = 0; i < nk; ++i, ++it) {
           const int kb = kb0 + i;
           if ((it & 3) == 0) {
@@ -222,7 +224,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA,   // packed weights
     // even when its barrier completed long ago, so separate waits for activations and weights per 64 K made a loop
     // of 740 cycles, whatever the tile (MMAs of 64 K x 256 tokens: 544).
     if (rank == 0 && elect_one()) {
-      const uint32_t idesc = umma_idesc_f16(2 * kPrBM, static_cast<uint32_t>(p.bn), 1u, 1u);
+      const uint32_t idesc = umma_idesc_f16(2 * kPrBM, static_cast<uint32_t>(p.width), 1u, 1u);
       const uint32_t b_base = smem_u32(sB);
       int sl = 0, tc = 0;
       uint32_t ph = 0;
@@ -492,8 +494,8 @@ constexpr int kPrSplitRows = 128;
 static void pair_search(int T, int N, int K, int slots, int fewest, int most, int* bn_out, int* splits_out) {
   double best = 0;
   const int nt = dgpp_ceil_div(N, 2 * kPrBM), raws = K / 256;
-  for (int bn = kPrMaxBN; bn >= 16; bn -= 16) {
-    if (bn < kPrMaxBN && bn - 16 >= T) continue;          // a smaller tile holds all rows
+  for (int bn = kPrMaxBN; bn >= 32; bn -= 32) {
+    if (bn < kPrMaxBN && bn - 32 >= T) continue;          // a smaller tile holds all rows
     const int tiles = nt * dgpp_ceil_div(T, bn);
     for (int s = fewest; s <= most && s <= raws; ++s) {
       const int per = dgpp_ceil_div(raws, s);
@@ -510,7 +512,7 @@ static void pair_shape(int T, int N, int K, int slots, int max_splits, int* bn_o
   *bn_out = kPrMaxBN;
   *splits_out = 1;
   if (T <= kPrSplitRows) pair_search(64, N, K, slots, 1, max_splits, bn_out, splits_out);
-  if (T < 64) *bn_out = dgpp_ceil_div(T, 16) * 16;
+  if (T < 64) *bn_out = dgpp_ceil_div(T, 32) * 32;
   if (T > 64) pair_search(T, N, K, slots, *splits_out, *splits_out, bn_out, splits_out);
 }
 
@@ -567,6 +569,7 @@ DGPP_API int dgpp_gemm_tc_pair(int wmode, const void* x, int64_t x_stride, const
   p.T = T; p.N = N; p.K = K; p.ldc = ldc;
   p.groups = nullptr; p.group_alpha = nullptr; p.sf_tiled = nullptr; p.n_tiles = 0;
   p.bn = bn;
+  p.width = dgpp_ceil_div(bn, 32) * 32;
   p.m_tiles = dgpp_ceil_div(T, bn);
   const int raws = K / 256, per = dgpp_ceil_div(raws, splits);
   p.kb_per_split = per * 4;
@@ -576,7 +579,7 @@ DGPP_API int dgpp_gemm_tc_pair(int wmode, const void* x, int64_t x_stride, const
           (reinterpret_cast<uintptr_t>(ws) & 15) == 0;
   CUtensorMap tA, tB, tSf;
   memset(&tSf, 0, sizeof(tSf));
-  if (make_tmap_2d(&tB, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, T, x_stride * 2, 64, bn / 2, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
+  if (make_tmap_2d(&tB, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, T, x_stride * 2, 64, p.width / 2, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
   if (make_tmap_2d(&tA, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K / 2, N, K / 2, 128, kPrBM, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
   if (wmode == 1 &&
       make_tmap_2d(&tSf, w_scale, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K / 16, N, K / 16, 16, kPrBM, CU_TENSOR_MAP_SWIZZLE_NONE))
@@ -603,7 +606,7 @@ DGPP_API int dgpp_gemm_tc_pair_grouped(const void* x, int64_t x_stride, const vo
   p.out = static_cast<bf16*>(out);
   p.status = device_status_ptr();
   p.T = tiles * bn; p.N = N; p.K = K; p.ldc = ldc;
-  p.bn = bn; p.m_tiles = tiles; p.splits = 1; p.kb_per_split = K / kPrBK;
+  p.bn = bn; p.width = dgpp_ceil_div(bn, 32) * 32; p.m_tiles = tiles; p.splits = 1; p.kb_per_split = K / kPrBK;
   p.n_tiles = N / (2 * kPrBM);
   p.units = tiles * p.n_tiles;
   p.vec = 1;
@@ -612,7 +615,7 @@ DGPP_API int dgpp_gemm_tc_pair_grouped(const void* x, int64_t x_stride, const vo
   p.sf_tiled = static_cast<const uint8_t*>(sf_tiled);
   CUtensorMap tA, tB, tSf;
   memset(&tSf, 0, sizeof(tSf));
-  if (make_tmap_2d(&tB, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, static_cast<uint64_t>(tiles) * bn, x_stride * 2, 64, bn / 2, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
+  if (make_tmap_2d(&tB, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, static_cast<uint64_t>(tiles) * bn, x_stride * 2, 64, p.width / 2, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
   if (make_tmap_2d(&tA, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K / 2, static_cast<uint64_t>(experts) * N, K / 2, 128, kPrBM, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
   return launch_pair<1, true>(tA, tB, tSf, p, slots, st);
 }
