@@ -181,15 +181,16 @@ class LLMEngine:
     def launches_per_step(self, b: Optional[int] = None) -> int:
         """Kernel launches of this package inside one decode step: the kernel-node count of the captured graph of
         batch width `b` (any captured width when b is None); without a captured graph, the launch sequence counted
-        from the runner's layer walk."""
+        from the runner's layer walk (for `max_batch` rows when b is None)."""
         if self.graphs:
             g = self.graphs.get(b) if b is not None else None
             g = g or next(iter(self.graphs.values()))
             return int(g.kernel_nodes)
         c = self.model.cfg
         r = self.runner
-        if r.decode_fp4:
-            per_layer = 10 + (1 if r.decode_splits > 1 else 0)          # 4 quantisers, 4 GEMMs, rope / append, attention
+        if r.decode_fp4 and (b or self.max_batch) <= r.fp4_width():
+            # 4 quantisers (one folds the split attention where it can), 4 GEMMs, rope / append, attention
+            per_layer = 10 + (1 if r.decode_splits > 1 and not (r.fuse_combine and r.attn_tc) else 0)
             if r.reducer is not None and not r.fuse_ar:
                 per_layer += 2 * r.reducer.launches_per_all_reduce
         else:

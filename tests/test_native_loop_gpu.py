@@ -146,3 +146,19 @@ def test_mixed_pass_runs_decoders_with_the_readers_chunk(dev):
     lg1, lg2 = k1.e.runner.logits[:1].float(), k2.e.runner.logits[:1].float()
     assert torch.nn.functional.cosine_similarity(lg1[0], lg2[0], dim=0).item() >= 0.995
     assert first1 == first2 or lg2[0].topk(2).values.diff().abs().item() < 0.05 * lg2[0].abs().max().item()
+
+
+@pytest.mark.parametrize("b", [8, 40])
+def test_counted_launches_of_a_step_are_the_captured_ones(dev, b):
+    """The launch count without a captured graph, in the block-scaled form and (above 32 rows) in the W4A16 form, against the kernel
+    nodes of the graph."""
+    from dgpp_b200.engine.llm_engine import LLMEngine
+    from dgpp_b200.models.dense import DenseConfig, DenseModel
+
+    cfg = DenseConfig.tiny(hidden=512, q_heads=4, kv_heads=2, head_dim=128, ffn=1024, vocab=2048, layers=3)
+    model = DenseModel.random_init(cfg, device=dev, seed=3, std=0.05)
+    eng = LLMEngine(model, max_batch=b, max_seq_len=64, prefill_chunk=64)
+    counted = eng.launches_per_step(b)
+    eng.generate([[1, 2, 3]] * b, max_tokens=3)
+    assert eng.launches_per_step(b) == eng.graphs[b].kernel_nodes
+    assert counted == eng.graphs[b].kernel_nodes
