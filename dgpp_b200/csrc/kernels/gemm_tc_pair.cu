@@ -481,13 +481,15 @@ static int pair_slots(int* slots) {
   return 0;
 }
 
-// Token tile and K splits of one product.  A K = 64 block of a bn-token tile was measured at 400 + 1.2 bn cycles (64 tokens: 507,
-// 128: 540, 192: 622, 256: 741), a tile's drain at 15 bn (the accumulator is not double-buffered: its other half holds
-// the converted weights); splits cost their partials' way to memory and back and 5500 cycles.  The product takes as many
-// units one after the other as one pair gets: wide tiles reuse a converted weight more often, narrower ones (or
-// splits, where there are fewer tiles than pairs) fill the last round.  Up to 128 rows the splits are those of 64 rows, above there
-// are none: on either side of that line a row's bits do not depend on how many others share its pass, and prompt products
-// touch no workspace, so that products on several streams share nothing.
+// Token tile and K splits of one product.  Measured costs: a K = 64 block 527 cycles up to 192 tokens (526 at 32, 528 at 128: the
+// chain of waits and the conversion, not the MMAs), 627 at 224 and 689 at 256; a tile's start and drain 24 bn + 2000 (the
+// accumulator is not double-buffered: its other half holds the converted weights); the fold of s splits 3000 and s round trips
+// to L2 for every 32 tokens.  The product takes as many units one after the other as one pair gets: wide tiles reuse a converted
+// weight more often, narrower ones (or splits, where there are fewer tiles than pairs) fill the last round.  Up to 128 rows the
+// splits are those of 64 rows, above there are none: on either side of that line a row's bits do not depend on how many others
+// share its pass, and prompt products touch no workspace, so that products on several streams share nothing.  Against the best of
+// all tiles and splits, us: 8 x 4096 x 1536 10.6 / 10.3, 37 x 5120 x 17408 35.9 / 35.9, 64 x 2048 x 5632 14.9 / 14.9, 173 x 5120 x 17408
+// 78.7 / 78.6, 953 x 2048 x 5632 29.6 / 29.5.
 constexpr int kPrSplitRows = 128;
 
 // Cheapest tile and split count for T rows, splits between `fewest` and `most`.
@@ -501,8 +503,8 @@ static void pair_search(int T, int N, int K, int slots, int fewest, int most, in
       const int per = dgpp_ceil_div(raws, s);
       if (dgpp_ceil_div(raws, per) != s) continue;
       const int rounds = dgpp_ceil_div(tiles * s, slots);
-      const double unit = per * 4 * (400 + 1.2 * bn) + 15.0 * bn + 500;
-      const double cost = rounds * unit + (s > 1 ? 5500 + 8.0 * T * N * s / 3200 : 0.0);
+      const double unit = per * 4 * (527 + (bn > 192 ? 2.5 * (bn - 192) : 0.0)) + 24.0 * bn + 2000;
+      const double cost = rounds * unit + (s > 1 ? 3000 + 600.0 * s * dgpp_ceil_div(bn, 32) : 0.0);
       if (best == 0 || cost < best) { best = cost; *bn_out = bn; *splits_out = s; }
     }
   }
