@@ -225,8 +225,11 @@ __global__ void __launch_bounds__(256) gdn_conv_kernel(ConvArgs a) {
 // The output pass over the consecutive rows of one request, four taps, even channel counts and 4-byte aligned rows.  Memory bound: a
 // thread has two neighbouring channels of sixteen tokens, whose inputs it requests at once and keeps as a sliding window, so an input is
 // read 1.2 times and not four times, and the taps once.  Same taps in the same order as above: the same bits.
-// grid (C / 512, T / 16).  2048 and 953 tokens x 6144 together: one channel of one token per thread 128 us, 34 so.
+// grid (C / 512, T / 16).  2048 and 953 tokens x 6144 together: one channel of one token per thread 128 us, 34 so.  A thread's sixteen
+// tokens take their time even when few threads run: from half a million inputs on (us in the general form / so: 16 x 6144
+// 5.1 / 7.7, 64 x 6144 7.4 / 7.9, 1024 x 512 7.9 / 7.9, 128 x 6144 9.7 / 7.9, 300 x 6144 16.6 / 9.2).
 constexpr int kConvRun = 16;
+constexpr int64_t kConvRunInputs = 1 << 19;
 
 __global__ void __launch_bounds__(256) gdn_conv_run_kernel(ConvArgs a) {
   pdl_wait();
@@ -468,7 +471,7 @@ static int gdn_conv_launch(const void* x, int64_t x_stride, const void* w, const
     return 0;
   }
   const bool pairs = C % 2 == 0 && x_stride % 2 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 3) == 0;
-  if (sequential && seg == 0 && W == 4 && pairs)
+  if (sequential && seg == 0 && W == 4 && pairs && static_cast<int64_t>(T) * C >= kConvRunInputs)
     gdn_conv_run_kernel<<<dim3(dgpp_ceil_div(C, 512), dgpp_ceil_div(T, kConvRun)), 256, 0, st>>>(a);
   else
     gdn_conv_kernel<<<dim3(dgpp_ceil_div(C, 256), T), 256, 0, st>>>(a);

@@ -87,10 +87,11 @@ def test_kda_per_channel_decay_recurrence(dev, dk, hk, hv):
 
 
 @pytest.mark.parametrize("T,C,bias,gap", [(1, 512, True, 0), (2, 514, False, 2), (16, 2, True, 6), (17, 1026, True, 0), (47, 640, False, 4),
-                                          (33, 511, True, 1)])
+                                          (33, 511, True, 1), (1024, 512, True, 0), (1025, 514, False, 6), (87, 6144, True, 2),
+                                          (1100, 511, False, 1)])
 def test_conv_of_a_run_equals_the_one_token_form(dev, T, C, bias, gap):
-    """Consecutive tokens of one request as sixteen-token runs per thread (an odd width or stride keeps the general form) against the general
-    kernel: the same bits, the same carried tail."""
+    """Consecutive tokens of one request as sixteen-token runs per thread (from half a million inputs on; an odd width or stride keeps the
+    general form) against the general kernel: the same bits, the same carried tail."""
     from dgpp_b200.ops import core as ops
 
     torch.manual_seed(T)
