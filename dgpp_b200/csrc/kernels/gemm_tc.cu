@@ -616,12 +616,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA,   // bf16 weights, or pa
 }
 
 // ---------------------------------------------------------------------------------- host side
-template <int BN, int WMODE>
+template <int BN, int WMODE, bool DEEP>
 struct GemmCfg {
   static constexpr bool kQuant = WMODE != 0;
   // ring depths: deep raw prefetch for small BN (weight streaming), wide B ring for large BN
-  // (bf16 weights and a small token tile: two CTAs per SM too, 6 or 5 stages each: a pass of 16 bf16 layers 2241 -> 2206 us)
-  static constexpr int kBf16Depth = ((BN <= 32 ? 112 : 200) * 1024) / (BN * 128 + kBM * 128);
+  // (bf16 weights and a small token tile: two CTAs per SM too, 6 or 5 stages each: a pass of 16 bf16 layers 2241 -> 2206 us;
+  // DEEP: eight stages, one CTA per SM)
+  static constexpr int kBf16Depth = ((BN <= 32 && !DEEP ? 112 : 200) * 1024) / (BN * 128 + kBM * 128);
   // Quantised weights with a small token tile run two CTAs per SM (<= 113 KB each): the second CTA hides
   // the converter <-> tensor-core handshakes of the first while both keep HBM requests in flight.
   // (BF12 carries an 8 KB exponent plane per raw stage; its B ring is shallower to stay under two CTAs per SM)
@@ -642,10 +643,10 @@ struct GemmCfg {
   }
 };
 
-template <int BN, int WMODE>
+template <int BN, int WMODE, bool DEEP = false>
 static int launch_gemm(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tSf, const GemmParams& p,
                        int splits, cudaStream_t st) {
-  using C = GemmCfg<BN, WMODE>;
+  using C = GemmCfg<BN, WMODE, DEEP>;
   auto kern = gemm_tc_kernel<BN, WMODE, C::SB, C::SA, C::SR>;
   static bool attr = false;
   constexpr size_t smem = C::smem();
@@ -792,8 +793,12 @@ static int gemm_tc_impl(int wmode, int a_f16, int bn, const void* x, int64_t x_s
                      CU_TENSOR_MAP_SWIZZLE_NONE))
       return -1;
   }
+  // One CTA per SM at most: the deep ring (us, eight stages / as many as two CTAs per SM leave: 1 x 11264 x 2048 15.0 / 15.7,
+  // 32 x 11264 x 2048 15.0 / 16.4, 32 x 12288 x 4096 25.6 / 27.0).
+  const bool deep = wmode == 0 && !p.cluster && static_cast<int64_t>(dgpp_ceil_div(N, kBM)) * dgpp_ceil_div(T, bn) * splits <= 148;
 #define DGPP_GEMM_BN(BNV)                                                       \
   if (bn == BNV) {                                                              \
+    if (deep && BNV <= 32) return launch_gemm<BNV, 0, BNV <= 32>(tA, tB, tSf, p, splits, st); \
     if (wmode == 0) return launch_gemm<BNV, 0>(tA, tB, tSf, p, splits, st);      \
     if (wmode == 1) return launch_gemm<BNV, 1>(tA, tB, tSf, p, splits, st);      \
     if (wmode == 2) return launch_gemm<BNV, 2>(tA, tB, tSf, p, splits, st);      \

@@ -137,14 +137,15 @@ def pick_bn(rows: int) -> int:
     return 256
 
 
-def pick_splits(rows: int, n: int, k: int, bn: int, sms: int = 148) -> int:
-    """Split K until the grid covers the SMs (weight-streaming regime only)."""
+def pick_splits(rows: int, n: int, k: int, bn: int, sms: int = 148, most: int = 148) -> int:
+    """Split K until the grid covers the SMs (weight-streaming regime only).  most: 8 for bf16 weights, whose decode rows fold up to eight
+    splits inside a cluster (us, 2048 x 5632: nine through the workspace 15.0 at 8 rows and 28.2 at 32, eight so 10.1 and 11.2)."""
     tiles = math.ceil(n / 128) * math.ceil(rows / bn)
     if tiles >= sms or rows > 128:
         return 1
     kb = k // 64
     want = max(1, sms // tiles)
-    return max(1, min(want, kb // 8))
+    return max(1, min(want, kb // 8, most))
 
 
 # 4-bit weights at prefill sizes run on CTA pairs (`gemm_tc_pair.cu`: 256 weight rows x up to 256 tokens per pair, converted
@@ -208,7 +209,7 @@ def gemm_tc(x: torch.Tensor, w: QuantLinear, out: Optional[torch.Tensor] = None,
     if bn is None:
         bn = pick_bn(rows)
     if splits is None:
-        splits = pick_splits(rows, w.n, k, bn)
+        splits = pick_splits(rows, w.n, k, bn, most=8 if w.fmt == "bf16" else 148)
     if a_f16 is None:
         a_f16 = A_F16_DEFAULT if w.fmt == "nvfp4" else 0
     wsp = cnt = None

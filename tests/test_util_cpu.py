@@ -202,3 +202,14 @@ def test_prompt_products_of_4_bit_weights_share_no_workspace(monkeypatch, rows, 
     assert name == "dgpp_gemm_tc_pair"
     splits, partials, counters = a[13], a[14], a[16]
     assert (splits, partials, counters) == ((0, ws.partials.data_ptr(), ws.counters.data_ptr()) if shared else (1, None, None))
+
+
+def test_split_counts_of_decode_products():
+    """bf16 rows split at most eightfold (what a cluster folds), at every width up to 128 rows alike."""
+    from dgpp_b200.ops import core as ops
+
+    for n, k in ((2048, 5632), (1024, 8192), (4096, 4096), (520, 2048)):
+        counts = {ops.pick_splits(rows, n, k, ops.pick_bn(rows), most=8) for rows in (1, 16, 17, 33, 64, 128)}
+        assert len(counts) == 1 and 1 <= min(counts) <= 8
+        assert ops.pick_splits(129, n, k, 256, most=8) == 1
+    assert ops.pick_splits(8, 2048, 5632, 16) == 9 and ops.pick_splits(8, 2048, 5632, 16, most=8) == 8
