@@ -381,7 +381,7 @@ def gemm_fp4(xa: QuantAct, w: QuantLinear, out: Optional[torch.Tensor] = None,
     if cluster is None:
         cluster = CLUSTER_SPLITK or (FP4_SPLIT_POLICY == "auto" and not push_comm and splits is None)
     if splits is None:
-        splits = pick_cluster_splits(rows, w.n, w.k, bn) if cluster else pick_splits_fp4(rows, w.n, w.k, bn)
+        splits = pick_cluster_splits(rows, w.n, w.k, bn, xa.terms) if cluster else pick_splits_fp4(rows, w.n, w.k, bn)
     cluster = cluster and 2 <= splits <= 8
     wsp = cnt = None
     if splits > 1 and not cluster:
@@ -416,15 +416,18 @@ def configure(fp4_splits: Optional[str] = None, cluster_splitk: Optional[bool] =
         call("dgpp_gemm_fp4_set_preload", int(bool(fp4_preload)))
 
 
-def pick_cluster_splits(rows: int, n: int, k: int, bn: int) -> int:
+def pick_cluster_splits(rows: int, n: int, k: int, bn: int, terms: int = 1) -> int:
     """Cluster split-K for projections with few output tiles: a CTA that walks many K stages alone is bound by the latency of its
-    own scale-copy -> MMA -> commit chain (600 cycles per stage), not by bandwidth.  As many CTAs as run at once (264 of the 296
-    that two per SM would be: clusters do not fill a GPC evenly), two stages each at least.  Measured at 8 rows, us unsplit /
-    split through the workspace / so: 5120 x 5120 12.4 / 12.0 / 8.5, 5120 x 17408 28 / 16.8 / 13.2, 2048 x 5632 12.5 / 10.3 / 6.5,
-    11264 x 2048 9.0 / 10.8 / 8.4, 24576 x 4096 14.9 / 21.4 / 18.9.  The same at every row count, so that a row's bits do
-    not depend on how many share its pass."""
+    own scale-copy -> MMA -> commit chain (600 cycles per stage), not by bandwidth.  As many CTAs as run at once, two stages each at
+    least: 264 of the 296 that two per SM would be (clusters do not fill a GPC evenly), 120 of 148 where a tile's columns
+    (terms x tokens) leave room for one.  Measured at 8 rows of 16, us unsplit / split through the workspace / so: 5120 x 5120 12.4 /
+    12.0 / 8.5, 5120 x 17408 28 / 16.8 / 13.2, 2048 x 5632 12.5 / 10.3 / 6.5, 11264 x 2048 9.0 / 10.8 / 8.4, 24576 x 4096 14.9 / 21.4 /
+    18.9; at 64 rows (192 columns), 264 CTAs / 120: 5120 x 5120 22.9 / 15.9, 5120 x 17408 31.1 / 25.4, 2048 x 5632 18.2 / 11.6,
+    11264 x 2048 25.7 / 18.6.  The same at every row count of one token tile, so that a row's bits do not depend on how many
+    share its pass."""
     tiles, stages = math.ceil(n / 128) * math.ceil(rows / bn), k // 256
-    return max(1, min(8, 264 // tiles, stages // 2)) if tiles <= 99 else 1
+    ctas = 264 if terms * bn <= 96 else 120
+    return max(1, min(8, ctas // tiles, stages // 2)) if tiles <= 99 else 1
 
 
 # Split-K policy of the block-scaled GEMM in the weight-streaming regime.  "resident": split until one resident wave

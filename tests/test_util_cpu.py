@@ -213,3 +213,14 @@ def test_split_counts_of_decode_products():
         assert len(counts) == 1 and 1 <= min(counts) <= 8
         assert ops.pick_splits(129, n, k, 256, most=8) == 1
     assert ops.pick_splits(8, 2048, 5632, 16) == 9 and ops.pick_splits(8, 2048, 5632, 16, most=8) == 8
+
+
+@pytest.mark.parametrize("terms,bn,ctas", [(3, 16, 264), (3, 32, 264), (1, 64, 264), (2, 64, 120), (3, 64, 120)])
+def test_cluster_splits_run_in_one_wave(terms, bn, ctas):
+    """As many CTAs as an SM's shared memory leaves room for (two of up to 96 columns, one of more), the same count at every row count."""
+    from dgpp_b200.ops import core as ops
+
+    for n, k in ((520, 2048), (2048, 5632), (11264, 2048), (5120, 5120), (7168, 5120), (5120, 17408), (34816, 5120)):
+        counts = {ops.pick_cluster_splits(rows, n, k, bn, terms) for rows in (1, 8, bn)}
+        s, tiles = counts.pop(), -(-n // 128)
+        assert not counts and (s == 1 or (s <= 8 and s * tiles <= ctas and k // 256 // s >= 2))
