@@ -215,11 +215,12 @@ class DenseRunner:
             plan[li + 1].launch()
 
     def fp4_width(self) -> int:
-        """Widest decode pass whose linears take the block-scaled FP4 kernels.  Above 32 rows the terms of a row fill a 192-column tile
-        and the W4A16 GEMM on CTA pairs is the faster one, without quantisers (37 rows, 16 layers of 5120 / 17408: 3005 -> 2796
-        us a pass); the all-reduce push keeps its epilogues, and where draft rows are verified (or the split choice is pinned) a
-        row keeps its bits at every width."""
-        return self.fp4_rows if (self.verifies_drafts or ops.PIN_SPLIT_ROWS or self.fuse_ar) else min(32, self.fp4_rows)
+        """Widest decode pass whose linears take the block-scaled FP4 kernels.  Above 32 rows three terms fill a 192-column tile and the
+        W4A16 GEMM on CTA pairs is the faster one, without quantisers (37 rows, 16 layers of 5120 / 17408: 3005 -> 2796 us a
+        pass); fewer terms were asked for by the caller and fit two CTAs per SM.  The all-reduce push keeps its epilogues, and
+        where draft rows are verified (or the split choice is pinned) a row keeps its bits at every width."""
+        wide = self.act_terms < 3 or self.verifies_drafts or ops.PIN_SPLIT_ROWS or self.fuse_ar
+        return self.fp4_rows if wide else min(32, self.fp4_rows)
 
     def linear(self, x, w, out, fp4: bool):
         if fp4 and w.fmt == "nvfp4" and w.k % 256 == 0:

@@ -224,3 +224,19 @@ def test_cluster_splits_run_in_one_wave(terms, bn, ctas):
         counts = {ops.pick_cluster_splits(rows, n, k, bn, terms) for rows in (1, 8, bn)}
         s, tiles = counts.pop(), -(-n // 128)
         assert not counts and (s == 1 or (s <= 8 and s * tiles <= ctas and k // 256 // s >= 2))
+
+
+def test_width_of_block_scaled_decode_passes(monkeypatch):
+    """Three terms leave the block-scaled kernels above 32 rows; fewer terms, draft rows, the all-reduce push and pinned splits stay."""
+    from types import SimpleNamespace
+
+    from dgpp_b200.engine.runner import DenseRunner
+    from dgpp_b200.ops import core as ops
+
+    def width(**kw):
+        return DenseRunner.fp4_width(SimpleNamespace(**{**dict(fp4_rows=64, act_terms=3, verifies_drafts=False, fuse_ar=False), **kw}))
+
+    assert width() == 32 and width(fp4_rows=8) == 8
+    assert width(act_terms=1) == width(act_terms=2) == width(verifies_drafts=True) == width(fuse_ar=True) == 64
+    monkeypatch.setattr(ops, "PIN_SPLIT_ROWS", True)
+    assert width() == 64
