@@ -303,19 +303,9 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-// D (256 rows: lanes 0..127 of each CTA's TMEM) (+)= A (each CTA's own 128 rows) * B (N columns, each CTA holding N / 2
-// of them at the same shared-memory offset).  Issued by one thread of the pair's first CTA only.
-__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                              uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The same product with A in tensor memory: each CTA's TMEM holds its own 128 rows (row = lane) at the same columns, two 16-bit
-// elements of consecutive K per 32-bit column, so a K = 16 step reads 8 columns.
+// D (256 rows: lanes 0..127 of each CTA's TMEM) (+)= A (each CTA's own 128 rows) * B (N columns, each CTA holding N / 2 of them at the
+// same shared-memory offset).  A is in tensor memory: row = lane, two 16-bit elements of consecutive K per 32-bit column, at the
+// same columns of both CTAs, so a K = 16 step reads 8 columns.  Issued by one thread of the pair's first CTA only.
 __device__ __forceinline__ void umma_f16_pair_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
                                                  uint32_t accumulate) {
   asm volatile(
@@ -345,23 +335,6 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-// Arrive on a barrier of another CTA of the cluster (address from mapa_shared), releasing this thread's prior writes.
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// try_wait that acquires at cluster scope (the arrival came from the other CTA of the pair).
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred P;\n\t"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, P;\n\t}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
 // ---- thread-block clusters: barrier over all threads of all CTAs, distributed shared memory stores
 __device__ __forceinline__ void cluster_barrier() {
   __syncwarp();   // the .aligned forms want the whole warp at the instruction (callers come out of elected-lane code)
