@@ -1,4 +1,4 @@
-// W4A16 prefill GEMM on CTA pairs: out[T, N] = alpha * x[T, K] . W[N, K]^T (+ residual), 4-bit weights (NVFP4 with
+// W4A16 GEMM on CTA pairs: out[T, N] = alpha * x[T, K] . W[N, K]^T (+ residual), 4-bit weights (NVFP4 with
 // e4m3 scales per 16, or MXFP4 with e8m0 scales per 32) expanded to bf16 on the way into TENSOR MEMORY, bf16
 // activations, fp32 accumulation in TMEM.  Same arithmetic as the single-CTA kernel of gemm_tc.cu (bit-identical
 // results without split-K: same converted operands, same K order), different tiling:
@@ -27,8 +27,8 @@
 //                     tile) have completed; the producers and the converters both wait for `done`.
 // (Arrivals on the other CTA's barriers release at CTA scope: what they order is tensor memory, by the tcgen05 fences; a
 // cluster-scope release took 1100 cycles per arrival, three times a block's MMAs.)
-// Warp roles (768 threads): warp 0 MMA issuer (first CTA) and TMEM owner, 1 TMA producer, 4..19 converters (four sets take turns
-// at the K = 64 blocks), 20..23 epilogue.
+// Warp roles (896 threads): warp 0 MMA issuer (first CTA) and TMEM owner, 1 TMA producer, 4..19 converters (four sets take turns
+// at the K = 64 blocks), 20..27 epilogue.
 // (reference counterpart: src/kernels/fp4w_gemm.cu, the W4A16 prefill GEMM.)
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>

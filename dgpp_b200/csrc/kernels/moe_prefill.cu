@@ -1,13 +1,14 @@
 // Mixture-of-experts at prefill sizes: counting sort of the (token, k-slot) pairs by expert, tile list, row gather and
-// ordered combine around the grouped block-scaled expert GEMM (gemm_fp4.cu, grouped mode with one token tile per slot).
+// ordered combine around the grouped expert GEMMs: on bf16 rows in tiles of 32 to 192 (gemm_tc_pair.cu), or with 4-bit activations
+// in tiles of 64 (gemm_fp4.cu, grouped mode with one token tile per slot).
 //
 //   moe_segment_sort_kernel   one CTA.  Histogram of the pairs per local expert, tiles per expert = ceil(n_e / bn),
 //                             exclusive scan -> first tile of every expert; then a STABLE rank of every pair inside its
 //                             expert (pairs keep their (token, k) order), so row = tile * bn + rank % bn is a pure function
 //                             of the routing result.  Outputs pair_row [T * k] (-1: expert lives on another rank),
 //                             tile_expert [max_tiles] (local expert of every tile, -1 beyond the last one), n_tiles.
-//   moe_gather_rows_kernel    xs[pair_row[p]] = x[p / k]   (bf16 rows; the quantiser and the grouped GEMM then see
-//                             every tile as one "slot" of bn token rows)
+//   moe_gather_rows_kernel    xs[pair_row[p]] = x[p / k]   (bf16 rows; the quantiser, where there is one, and the grouped GEMM then
+//                             see every tile as one "slot" of bn token rows)
 //   moe_combine_rows_kernel   out[t] = sum_j w[t, j] * y[pair_row[t, j]] (+ shared[t]) in ascending j, fp32, one rounding
 //
 // (reference counterparts: src/kernels/glm_moe.cu:1382 moe_segment_count_kernel, :1553 moe_tile_list_kernel, gather /

@@ -241,7 +241,7 @@ struct ClusterConfig {
   bool engine_fuse_combine = true;          // fold the split-KV partials inside the o projection's quantiser
   bool engine_l2_prefetch = false;          // GEMMs ask L2 for the next projection's weights
   std::string engine_fp4_splits = "auto";   // split-K policy of the block-scaled GEMM: auto | resident | legacy
-  bool engine_cluster_splitk = false;       // split-K through distributed shared memory instead of the workspace
+  bool engine_cluster_splitk = false;       // split-K through distributed shared memory under resident / legacy too (auto does so by itself)
   bool engine_fp4_preload = true;           // weight half of the first ring stages issued before the grid dependency
   bool engine_layer_kernel = false;         // decode through the persistent decode-layer kernel
   bool engine_seq_parallel = true;          // tensor-parallel prefill keeps the residual stream sharded by token tile

@@ -17,7 +17,7 @@ class EngineOptions:
     fuse_combine: bool = True         # fold the split-KV partials inside the o projection's quantiser
     l2_prefetch: bool = False         # GEMMs ask L2 for the next projection's weights (measured slower; off)
     fp4_splits: str = "auto"          # split-K policy of the block-scaled GEMM: auto | resident | legacy
-    cluster_splitk: bool = False      # split-K through distributed shared memory instead of the workspace
+    cluster_splitk: bool = False      # split-K through distributed shared memory under resident / legacy too (auto does so by itself)
     fp4_preload: bool = True          # weight half of the first ring stages issued before the grid dependency
     layer_kernel: bool = False        # decode through the persistent decode-layer kernel
     seq_parallel: bool = True         # tensor-parallel prefill: residual stream sharded by token tile between the blocks

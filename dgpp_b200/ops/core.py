@@ -365,9 +365,10 @@ def gemm_fp4(xa: QuantAct, w: QuantLinear, out: Optional[torch.Tensor] = None,
              splits: Optional[int] = None, ws: Optional[GemmWorkspace] = None, push_comm=None,
              prefetch: Optional[QuantLinear] = None, cluster: Optional[bool] = None) -> torch.Tensor:
     """Block-scaled NVFP4 tensor-core linear on pre-quantised activations (token tile = xa.bn).
-    splits > 1: split K.  cluster (default: on): the CTAs of one output tile form a thread-block cluster and fold
-    their partial accumulators through distributed shared memory (no workspace); off: partials go through a global
-    workspace and the last CTA of a tile folds them.
+    splits > 1: split K.  cluster: the CTAs of one output tile form a thread-block cluster and fold their partial accumulators through
+    distributed shared memory (no workspace; up to eight splits); otherwise partials go through a global workspace and the last
+    CTA of a tile folds them.  Default: the cluster where the count is chosen here under the "auto" policy and nothing is pushed, or
+    wherever the process asks for it (`configure`).
     prefetch: the projection that runs next; its packed weights are requested into L2 by this kernel's CTAs once
     their own loads are issued (fills the HBM-idle time of the small kernels in between; a hint, never needed).
     push_comm: native peer-communicator handle; the finished bf16 tiles are then stored into every rank's
@@ -404,8 +405,8 @@ CLUSTER_SPLITK = False
 
 def configure(fp4_splits: Optional[str] = None, cluster_splitk: Optional[bool] = None,
               fp4_preload: Optional[bool] = None) -> None:
-    """Process-wide GEMM policies: split-K policy ("auto" | "resident" | "legacy"), split-K through a thread-block
-    cluster, and the pre-wait weight preload."""
+    """Process-wide GEMM policies: split-K policy ("auto" | "resident" | "legacy"), split-K through a thread-block cluster also where
+    "auto" would not (the other policies, the push, explicit counts), and the pre-wait weight preload."""
     global CLUSTER_SPLITK, FP4_SPLIT_POLICY
     if fp4_splits is not None:
         assert fp4_splits in ("auto", "resident", "legacy")
