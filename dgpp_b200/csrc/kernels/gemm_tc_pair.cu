@@ -16,8 +16,8 @@
 // tiles of a chunk stay in L2.
 //
 // What bounds it: at wide tiles the tensor pipe (2048 x 34816 x 5120: 474 us = 1540 TFLOP/s, 0.91 of the measured cuBLAS burst rate;
-// the single-CTA kernel 1216 us), at narrow ones the MMA thread's chain and the conversion (8 x 34816 x 5120: 46 us, 510
-// cycles per K = 64 block; 73 us).  2048 x 5120 x 17408: 564 -> 266 us, 173 x 5120 x 5120: 71 -> 26 us.
+// the single-CTA kernel 1216 us), at narrow ones the MMA thread's chain and the conversion (8 x 34816 x 5120: 46 us, 480
+// cycles per K = 64 block; 73 us).  2048 x 5120 x 17408: 564 -> 266 us, 173 x 5120 x 5120: 71 -> 27 us.
 //
 // Handshakes (all waits bounded, expiry -> status code, everything unwinds, TMEM freed):
 //   own CTA:          raw_full / raw_empty (TMA -> converters), acc_full (MMA -> epilogue);
@@ -481,15 +481,16 @@ static int pair_slots(int* slots) {
   return 0;
 }
 
-// Token tile and K splits of one product.  Measured costs: a K = 64 block 527 cycles up to 192 tokens (526 at 32, 528 at 128: the
-// chain of waits and the conversion, not the MMAs), 627 at 224 and 689 at 256; a tile's start and drain 24 bn + 2000 (the
-// accumulator is not double-buffered: its other half holds the converted weights); the fold of s splits 3000 and s round trips
-// to L2 for every 32 tokens.  The product takes as many units one after the other as one pair gets: wide tiles reuse a converted
-// weight more often, narrower ones (or splits, where there are fewer tiles than pairs) fill the last round.  Up to 128 rows the
-// splits are those of 64 rows, above there are none: on either side of that line a row's bits do not depend on how many others
-// share its pass, and prompt products touch no workspace, so that products on several streams share nothing.  Against the best of
-// all tiles and splits, us: 8 x 4096 x 1536 10.6 / 10.3, 37 x 5120 x 17408 35.9 / 35.9, 64 x 2048 x 5632 14.9 / 14.9, 173 x 5120 x 17408
-// 78.7 / 78.6, 953 x 2048 x 5632 29.6 / 29.5.
+// Token tile and K splits of one product.  The product takes as many units one after the other as one pair gets: wide tiles reuse a
+// converted weight more often, narrower ones (or splits, where there are fewer tiles than pairs) fill the last round.  A K = 64
+// block counts as 400 + 1.2 bn cycles, a tile's drain as 15 bn + 500 (the accumulator is not double-buffered: its other half
+// holds the converted weights), s splits as 1000 and 400 s for every 32 tokens of a tile (their fold is s round trips to L2).
+// These are fitted to whole products, 21 shapes of 512 x 512 to 34816 x 5120 at 1 to 2048 rows with every tile and split count
+// (alone, a block takes 480 cycles up to 160 tokens, 530 at 192 and 655 at 256; with that the choice is the worse one): what they
+// choose is within 1.1 % of the best above 128 rows, and 1.2 % on average, 19 % at most (128 x 2560 x 8192) up to 128 rows.
+// Up to 128 rows the splits are those of 128 rows, above there are none: on either side of that line a row's bits do not depend
+// on how many others share its pass, and prompt products touch no workspace, so that products on several streams share
+// nothing.  (A long K over few tiles pays for that: 173 x 5120 x 17408 79 us, 47 in three splits.)
 constexpr int kPrSplitRows = 128;
 
 // Cheapest tile and split count for T rows, splits between `fewest` and `most`.
@@ -503,8 +504,8 @@ static void pair_search(int T, int N, int K, int slots, int fewest, int most, in
       const int per = dgpp_ceil_div(raws, s);
       if (dgpp_ceil_div(raws, per) != s) continue;
       const int rounds = dgpp_ceil_div(tiles * s, slots);
-      const double unit = per * 4 * (527 + (bn > 192 ? 2.5 * (bn - 192) : 0.0)) + 24.0 * bn + 2000;
-      const double cost = rounds * unit + (s > 1 ? 3000 + 600.0 * s * dgpp_ceil_div(bn, 32) : 0.0);
+      const double unit = per * 4 * (400 + 1.2 * bn) + 15.0 * bn + 500;
+      const double cost = rounds * unit + (s > 1 ? 1000 + 400.0 * s * dgpp_ceil_div(bn < T ? bn : T, 32) : 0.0);
       if (best == 0 || cost < best) { best = cost; *bn_out = bn; *splits_out = s; }
     }
   }
@@ -513,9 +514,8 @@ static void pair_search(int T, int N, int K, int slots, int fewest, int most, in
 static void pair_shape(int T, int N, int K, int slots, int max_splits, int* bn_out, int* splits_out) {
   *bn_out = kPrMaxBN;
   *splits_out = 1;
-  if (T <= kPrSplitRows) pair_search(64, N, K, slots, 1, max_splits, bn_out, splits_out);
-  if (T < 64) *bn_out = dgpp_ceil_div(T, 32) * 32;
-  if (T > 64) pair_search(T, N, K, slots, *splits_out, *splits_out, bn_out, splits_out);
+  if (T <= kPrSplitRows) pair_search(kPrSplitRows, N, K, slots, 1, max_splits, bn_out, splits_out);
+  pair_search(T, N, K, slots, *splits_out, *splits_out, bn_out, splits_out);
 }
 
 template <int WMODE, bool GROUPED>
