@@ -16,7 +16,7 @@
 // tiles of a chunk stay in L2.
 //
 // What bounds it: at wide tiles the tensor pipe (2048 x 34816 x 5120: 474 us = 1540 TFLOP/s, 0.91 of the measured cuBLAS burst rate;
-// the single-CTA kernel 1216 us), at narrow ones the MMA thread's chain and the conversion (8 x 34816 x 5120: 46 us, 480
+// the single-CTA kernel 1216 us), at narrow ones the MMA thread's chain and the conversion (8 x 34816 x 5120: 49 us, 480
 // cycles per K = 64 block; 73 us).  2048 x 5120 x 17408: 564 -> 266 us, 173 x 5120 x 5120: 71 -> 27 us.
 //
 // Handshakes (all waits bounded, expiry -> status code, everything unwinds, TMEM freed):
