@@ -358,21 +358,29 @@ class MoEBlock:
 
 
 _PREFILL_WS: dict = {}
+_PREFILL_WS_CAPTURED: list = []      # smaller sets that captured passes still work in
+
+
+def _capturing(device) -> bool:
+    return torch.device(device).type == "cuda" and torch.cuda.is_current_stream_capturing()
 
 
 def _prefill_workspace(device, max_tiles: int, bn: int, hidden: int, ffn: int, terms: int) -> dict:
     """Buffers of MoEBlock.forward_gathered, one set per (device, geometry, activation form) grown to the largest need.  All tile widths
-    share it: rows are flat, every pass fills what it reads."""
+    share it: rows are flat, every pass fills what it reads.  A set that a captured pass (decode rows beyond a block's width) works
+    in is kept when a larger one takes its place: the graph holds its addresses."""
     key = (str(device), hidden, ffn, terms)
     rows = max_tiles * bn
     ws = _PREFILL_WS.get(key)
     if ws is None or ws["max_tiles"] < max_tiles or ws["rows"] < rows:
         if ws is not None:
             max_tiles, rows = max(max_tiles, ws["max_tiles"]), max(rows, ws["rows"])
+            if ws["captured"]:
+                _PREFILL_WS_CAPTURED.append(ws)
             _PREFILL_WS.pop(key)      # (given back before the larger set is taken)
             ws = None
         i32 = dict(dtype=torch.int32, device=device)
-        ws = dict(max_tiles=max_tiles, rows=rows,
+        ws = dict(max_tiles=max_tiles, rows=rows, captured=False,
                   pair_row=torch.empty(rows, **i32), tile_expert=torch.full((max_tiles,), -1, **i32),
                   n_tiles=torch.zeros(1, **i32),
                   xs=torch.zeros(rows, hidden, dtype=BF, device=device),
@@ -383,4 +391,5 @@ def _prefill_workspace(device, max_tiles: int, bn: int, hidden: int, ffn: int, t
         else:      # bf16 activations
             ws["act"] = torch.zeros(rows, ffn, dtype=BF, device=device)
         _PREFILL_WS[key] = ws
+    ws["captured"] = ws["captured"] or _capturing(device)
     return ws

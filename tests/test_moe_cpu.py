@@ -69,3 +69,22 @@ def test_prompt_buffers_are_one_set_for_all_tile_widths(monkeypatch):
     assert len(moe._PREFILL_WS) == 1 and more["tile_expert"].numel() == 40 and more["xs"].shape[0] == more["pair_row"].numel() == 12 * 128
     wide = moe._prefill_workspace("cpu", 10, 192, 256, 256, 0)
     assert len(moe._PREFILL_WS) == 1 and wide["tile_expert"].numel() == 40 and all(wide[b].shape[0] == 1920 for b in ("xs", "h", "act", "y"))
+
+
+def test_prompt_buffers_of_a_captured_pass_are_kept(monkeypatch):
+    """A graph replays into the addresses it was captured with: its set outlives the growth that a longer prompt asks for."""
+    import gc
+    import weakref
+
+    from dgpp_b200.models import moe
+
+    monkeypatch.setattr(moe, "_PREFILL_WS", {})
+    monkeypatch.setattr(moe, "_PREFILL_WS_CAPTURED", [])
+    capturing = [True]
+    monkeypatch.setattr(moe, "_capturing", lambda device: capturing[0])
+    seen = weakref.ref(moe._prefill_workspace("cpu", 4, 32, 256, 256, 0)["y"])
+    capturing[0] = False
+    plain = weakref.ref(moe._prefill_workspace("cpu", 8, 32, 256, 256, 0)["y"])
+    moe._prefill_workspace("cpu", 16, 32, 256, 256, 0)
+    gc.collect()
+    assert seen() is not None and plain() is None
