@@ -55,8 +55,8 @@ def test_prefill_chunking_gives_the_same_tokens(setup):
         eng = _engine(model, chunk)
         outs[chunk] = eng.generate([prompt], max_tokens=8)[0]
         logits[chunk] = _last_logits(eng, prompt)
-    # prefill itself is the same exact kernel on different row groupings: first tokens and last-position logits agree
-    # to accumulation order of the attention tiles
+    # prefill itself is the same exact kernel on different row groupings: first tokens and last-position logits agree to the
+    # order of accumulation (K splits of the passes of up to 128 rows, tiles of the attention)
     for chunk in (64, 256):
         assert (logits[chunk] - logits[512]).abs().max().item() < 2e-2 * logits[512].abs().max().item()
         for i, (a, b) in enumerate(zip(outs[chunk], outs[512])):
