@@ -1,28 +1,33 @@
 // Activation producer + NVFP4 residual-term quantiser, one thread-block CLUSTER per row.
 //
 // A decode batch has only a handful of rows, so one CTA per row leaves the GPU idle; here the K columns of a row
-// are split over the CTAs of a cluster (up to 8), and the two row-wide reductions (sum of squares for RMSNorm,
-// max |x| for the activation scale) go through distributed shared memory: every CTA stores its partial into the
-// shared memory of every CTA of the cluster, the cluster synchronises, and every CTA folds its own copy of the
-// partials in ascending CTA order (so all CTAs compute bit-identical row statistics, and nobody reads a peer's
-// shared memory after the barrier).
+// are split over the CTAs of a cluster (up to 8).  A thread owns 8 columns (half a block of 16) from the load to the
+// packed codes, so a CTA has no barrier of its own; the two row-wide reductions (sum of squares for RMSNorm, max |x|
+// for the activation scale) are one exchange: every warp sends its pair of partials to every CTA of the cluster
+// (`st.async`, counted by the receiver's mbarrier), and every warp folds the CTA's copy in one fixed order, so
+// all CTAs compute bit-identical row statistics.  The cluster barrier that makes the mbarriers known to the peers, and
+// the loads of the norm weights, stand before the wait on the preceding grid.
+// What bounds it: one chain of latencies: loads, exchange, three terms one after the other.  A pass of 16 layers of 5120 / 17408 took
+// 1544 us at one row and 1741 at eight with a thread per block of 16, two barriers per reduction and cluster-wide barriers, 1440 and
+// 1624 so; 16 layers of 2048 at eight rows 1046, 968 so.  A quantiser then adds 4 to 8 us to its layer's chain (5 to 10 before).
 //
 // Modes, output layout and arithmetic are those of fused_act_quant_kernel in gemm_fp4.cu:
 //   0 plain rows, 1 swiglu([gate | up]), 2 rmsnorm(resid + delta) * w
 //   q rows [token tile][term][token], scale factors in tcgen05.cp atom order per token tile.
-#include <cooperative_groups.h>
 #include <string.h>
 
 #include "common/common.h"
 #include "common/dtypes.cuh"
 #include "common/ptx.cuh"
 #include "kernels/comm.cuh"
-
-namespace cg = cooperative_groups;
+#include "kernels/gemm_common.cuh"
 
 namespace dgpp {
 
-constexpr int kAqThreads = 128;
+constexpr int kAqMaxThreads = 512;
+constexpr int kAqMaxWarps = kAqMaxThreads / 32;
+constexpr int kAqMaxCluster = 8;
+constexpr int kAqSplitBlock = 4;      // attention splits whose partials are in flight at once
 constexpr int kAqAtom = 512;
 
 struct ClusterQuantArgs {
@@ -57,68 +62,86 @@ struct ClusterQuantArgs {
   int splits, hq, D;
 };
 
-__device__ __forceinline__ float warp_red(float v, bool is_max) {
+// Stores a pair of floats in a CTA of the cluster; the 8 bytes are counted by the mbarrier at `bar` there.
+__device__ __forceinline__ void st_async_f32x2(uint32_t addr, float x, float y, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(addr), "f"(x), "f"(y), "r"(bar)
+               : "memory");
+}
+
+// Eight columns of the folded decode attention row: split partials weighted by 2^(their max - the row's), ascending.
+__device__ __forceinline__ void fold_splits(const ClusterQuantArgs& a, int t, int col, float (&acc)[8], float& ll) {
+  const int h = col / a.D, d0 = col % a.D;
+  const size_t rh = static_cast<size_t>(t) * a.hq + h;
+  const float2* ml = reinterpret_cast<const float2*>(a.part_ml) + rh * a.splits;
+  const float* pa = a.part_acc + rh * a.splits * a.D + d0;
+  float mm = -INFINITY;
+#pragma unroll 8
+  for (int sp = 0; sp < a.splits; ++sp) mm = fmaxf(mm, ml[sp].x);
+  ll = 0.f;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float u = __shfl_xor_sync(0xffffffffu, v, o);
-    v = is_max ? fmaxf(v, u) : v + u;
+  for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+  for (int s0 = 0; s0 < a.splits; s0 += kAqSplitBlock) {
+    float2 m[kAqSplitBlock];
+    float4 v[kAqSplitBlock][2];
+#pragma unroll
+    for (int i = 0; i < kAqSplitBlock; ++i) {
+      if (s0 + i >= a.splits) break;
+      m[i] = ml[s0 + i];
+      const float4* src = reinterpret_cast<const float4*>(pa + static_cast<size_t>(s0 + i) * a.D);
+      v[i][0] = src[0];
+      v[i][1] = src[1];
+    }
+#pragma unroll
+    for (int i = 0; i < kAqSplitBlock; ++i) {
+      if (s0 + i >= a.splits) break;
+      const float cw = m[i].x == -INFINITY ? 0.f : __expf(m[i].x - mm);
+      ll += m[i].y * cw;
+      acc[0] += v[i][0].x * cw; acc[1] += v[i][0].y * cw; acc[2] += v[i][0].z * cw; acc[3] += v[i][0].w * cw;
+      acc[4] += v[i][1].x * cw; acc[5] += v[i][1].y * cw; acc[6] += v[i][1].z * cw; acc[7] += v[i][1].w * cw;
+    }
   }
-  return v;
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(kAqThreads) act_quant_cluster_kernel(ClusterQuantArgs a) {
+__global__ void __launch_bounds__(kAqMaxThreads) act_quant_cluster_kernel(ClusterQuantArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  bf16* seg = reinterpret_cast<bf16*>(smem_raw);  // this CTA's K / cl columns
-  __shared__ float wred[kAqThreads / 32];
-  // partials of every CTA of the cluster, PUSHED here by their owners before the cluster barrier: [0][i] sum of
-  // squares, [1][i] max |x| of CTA i's segment.  After the barrier a CTA reads only its own copy, so no CTA's shared
-  // memory is touched by a peer once the barrier has passed and no closing barrier is needed.
-  __shared__ float part[2][8];
-  cg::cluster_group cluster = cg::this_cluster();
-  pdl_wait();
-  const int c = blockIdx.x, t = blockIdx.y, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  if (a.group_list && (a.group_list[t / a.bn] < 0 || t % a.bn >= a.group_rows)) return;   // whole cluster leaves together
+  uint4* seg = reinterpret_cast<uint4*>(smem_raw);  // this CTA's K / cl columns; a thread reads back what it wrote
+  // (sum of squares, max |x|) of every warp of every CTA of the cluster
+  __shared__ __align__(16) float2 part[kAqMaxCluster * kAqMaxWarps];
+  __shared__ __align__(8) uint64_t arrived;
+  const int c = blockIdx.x, t = blockIdx.y, tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, wid = tid >> 5;
   const int cl = a.cl, K = a.K, kseg = K / cl, k0 = c * kseg, nvec = kseg / 8;
-  auto cta_reduce = [&](float v, bool is_max) {
-    v = warp_red(v, is_max);
-    if (lane == 0) wred[wid] = v;
-    __syncthreads();
-    float r = wred[0];
-    for (int i = 1; i < kAqThreads / 32; ++i) r = is_max ? fmaxf(r, wred[i]) : r + wred[i];
-    __syncthreads();
-    return r;
-  };
-  auto cluster_push = [&](int slot, float v) {
-    if (tid < cl) *cluster.map_shared_rank(&part[slot][c], tid) = v;
-  };
-  auto cluster_fold = [&](int slot, bool is_max) {
-    float r = 0.f;
-    for (int i = 0; i < cl; ++i) r = is_max ? fmaxf(r, part[slot][i]) : r + part[slot][i];
-    return r;
-  };
-  float amax = 0.f;
+  for (int i = tid; i < kAqMaxCluster * kAqMaxWarps; i += nthr) part[i] = make_float2(0.f, 0.f);
+  if (tid == 0) {
+    mbar_init(&arrived, 1);
+    mbar_expect_tx(&arrived, cl * (nthr / 32) * 8);
+    fence_mbar_init();
+  }
+  const uint4* wv = reinterpret_cast<const uint4*>(a.w + k0);
+  Pack16 w0;      // the norm weights of this thread's first columns
+  w0.u = make_uint4(0u, 0u, 0u, 0u);
+  if (MODE == 2 && tid < nvec) w0.u = wv[tid];
+  cluster_barrier();
+  pdl_wait();
+  if (a.group_list && (a.group_list[t / a.bn] < 0 || t % a.bn >= a.group_rows)) return;   // whole cluster leaves together
+  float ss = 0.f, amax = 0.f;
   uint32_t fold_epoch = 0;
   int fold_parity = 0;
   if (MODE == 2 && a.fold) {
     fold_epoch = *a.comm.epoch + 1;
     fold_parity = fold_epoch & 1;
     const int tile0 = k0 / 128, ntile = (k0 + kseg - 1) / 128 - tile0 + 1;
-    for (int i = tid; i < ntile * a.comm.world; i += kAqThreads) {
+    for (int i = tid; i < ntile * a.comm.world; i += nthr) {
       const int src = i / ntile, tl = tile0 + i % ntile;
-      if (!wait_flag(flag(a.comm, a.comm.rank, fold_parity, src, tl), fold_epoch)) {
-        if (atomicCAS(&a.status->code, 0, kTimeoutPeerFlag) == 0) a.status->detail = src;
-        atomicAdd(&a.status->count, 1);
-      }
+      if (!wait_flag(flag(a.comm, a.comm.rank, fold_parity, src, tl), fold_epoch)) report(a.status, kTimeoutPeerFlag, src);
     }
     __syncthreads();
   }
-  if (MODE == 2) {
-    const bf16* rr = a.in + static_cast<size_t>(t) * a.in_stride + k0;
-    float ss = 0.f, pm = 0.f;
-    for (int i = tid; i < nvec; i += kAqThreads) {
-      Pack16 x;
-      x.u = reinterpret_cast<const uint4*>(rr)[i];
+  for (int i = tid; i < nvec; i += nthr) {
+    Pack16 x;
+    if (MODE == 2) {
+      x.u = reinterpret_cast<const uint4*>(a.in + static_cast<size_t>(t) * a.in_stride + k0)[i];
+      uint4* sum_out = reinterpret_cast<uint4*>(a.resid_out + static_cast<size_t>(t) * K + k0) + i;
       if (a.fold) {
         float acc[8];
 #pragma unroll
@@ -132,112 +155,84 @@ __global__ void __launch_bounds__(kAqThreads) act_quant_cluster_kernel(ClusterQu
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) x.h[j] = f32_to_bf16(bf16_to_f32(x.h[j]) + bf16_to_f32(f32_to_bf16(acc[j])));
-        reinterpret_cast<uint4*>(a.resid_out + static_cast<size_t>(t) * K + k0)[i] = x.u;
+        *sum_out = x.u;
       } else if (a.delta) {
         Pack16 d;
         d.u = reinterpret_cast<const uint4*>(a.delta + static_cast<size_t>(t) * K + k0)[i];
 #pragma unroll
         for (int j = 0; j < 8; ++j) x.h[j] = f32_to_bf16(bf16_to_f32(x.h[j]) + bf16_to_f32(d.h[j]));
-        reinterpret_cast<uint4*>(a.resid_out + static_cast<size_t>(t) * K + k0)[i] = x.u;
+        *sum_out = x.u;
       }
-      Pack16 wv;
-      wv.u = reinterpret_cast<const uint4*>(a.w + k0)[i];
+      Pack16 w;
+      w.u = i == tid ? w0.u : wv[i];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float f = bf16_to_f32(x.h[j]);
         ss += f * f;
-        float gw = bf16_to_f32(wv.h[j]);
+        float gw = bf16_to_f32(w.h[j]);
         if (a.one_plus_w) gw += 1.f;
-        pm = fmaxf(pm, fabsf(f * gw));
+        amax = fmaxf(amax, fabsf(f * gw));
       }
-      reinterpret_cast<uint4*>(seg)[i] = x.u;
-    }
-    ss = cta_reduce(ss, false);
-    pm = cta_reduce(pm, true);
-    cluster_push(0, ss);
-    cluster_push(1, pm);
-    cluster.sync();
-    const float rstd = rsqrtf(cluster_fold(0, false) / static_cast<float>(K) + a.eps);
-    // Row scale from a bound instead of the exact maximum of the normalised row: |bf16(bf16(x rstd) w)| <=
-    // |x w| rstd (1 + 2^-8)^2, so max |x w| * rstd * 1.0079 covers every element (at most 0.8 % above the true
-    // maximum) and is known from this single pass: no second row-wide reduction.
-    amax = cluster_fold(1, true) * rstd * 1.0079f;
-    for (int i = tid; i < nvec; i += kAqThreads) {
-      Pack16 x, ww;
-      x.u = reinterpret_cast<const uint4*>(seg)[i];
-      ww.u = reinterpret_cast<const uint4*>(a.w + k0)[i];
+    } else {
+      if (MODE == 3) {
+        float acc[8], ll;
+        fold_splits(a, t, k0 + i * 8, acc, ll);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float nrm = bf16_to_f32(f32_to_bf16(bf16_to_f32(x.h[j]) * rstd));
-        float gw = bf16_to_f32(ww.h[j]);
-        if (a.one_plus_w) gw += 1.f;
-        x.h[j] = f32_to_bf16(nrm * gw);
-      }
-      reinterpret_cast<uint4*>(seg)[i] = x.u;
-      if (a.x_out) reinterpret_cast<uint4*>(a.x_out + static_cast<size_t>(t) * K + k0)[i] = x.u;
-    }
-  } else if (MODE == 3) {
-    for (int i = tid; i < nvec; i += kAqThreads) {
-      const int col = k0 + i * 8, h = col / a.D, d0 = col % a.D;
-      const size_t rh = static_cast<size_t>(t) * a.hq + h;
-      float mm = -INFINITY;
-      for (int sp = 0; sp < a.splits; ++sp) mm = fmaxf(mm, a.part_ml[(rh * a.splits + sp) * 2]);
-      float ll = 0.f, acc[8];
+        for (int j = 0; j < 8; ++j) x.h[j] = f32_to_bf16(ll > 0.f ? acc[j] / ll : 0.f);
+      } else {
+        const uint4* rr = reinterpret_cast<const uint4*>(a.in + static_cast<size_t>(t) * a.in_stride + k0);
+        x.u = rr[i];
+        if (MODE == 1) {
+          Pack16 u;
+          u.u = rr[K / 8 + i];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-      for (int sp = 0; sp < a.splits; ++sp) {
-        const float ms = a.part_ml[(rh * a.splits + sp) * 2];
-        const float cw = ms == -INFINITY ? 0.f : __expf(ms - mm);
-        ll += a.part_ml[(rh * a.splits + sp) * 2 + 1] * cw;
-        const float4* pa = reinterpret_cast<const float4*>(a.part_acc + (rh * a.splits + sp) * a.D + d0);
-        const float4 p0 = pa[0], p1 = pa[1];
-        acc[0] += p0.x * cw; acc[1] += p0.y * cw; acc[2] += p0.z * cw; acc[3] += p0.w * cw;
-        acc[4] += p1.x * cw; acc[5] += p1.y * cw; acc[6] += p1.z * cw; acc[7] += p1.w * cw;
-      }
-      Pack16 x;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        x.h[j] = f32_to_bf16(ll > 0.f ? acc[j] / ll : 0.f);
-        amax = fmaxf(amax, fabsf(bf16_to_f32(x.h[j])));
-      }
-      reinterpret_cast<uint4*>(seg)[i] = x.u;
-      if (a.x_out) reinterpret_cast<uint4*>(a.x_out + static_cast<size_t>(t) * K + k0)[i] = x.u;
-    }
-  } else {
-    const bf16* rr = a.in + static_cast<size_t>(t) * a.in_stride + k0;
-    for (int i = tid; i < nvec; i += kAqThreads) {
-      Pack16 x;
-      x.u = reinterpret_cast<const uint4*>(rr)[i];
-      if (MODE == 1) {
-        Pack16 u;
-        u.u = reinterpret_cast<const uint4*>(rr + K)[i];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          float gv = bf16_to_f32(x.h[j]), uv = bf16_to_f32(u.h[j]);
-          if (a.limit > 0.f) { gv = fminf(gv, a.limit); uv = fminf(fmaxf(uv, -a.limit), a.limit); }
-          float sl;
-          if (a.alpha > 0.f) {
-            sl = bf16_to_f32(f32_to_bf16(gv / (1.f + __expf(-a.alpha * gv))));
-            uv += 1.f;
-          } else {
-            sl = bf16_to_f32(f32_to_bf16(gv / (1.f + __expf(-gv))));
+          for (int j = 0; j < 8; ++j) {
+            float gv = bf16_to_f32(x.h[j]), uv = bf16_to_f32(u.h[j]);
+            if (a.limit > 0.f) { gv = fminf(gv, a.limit); uv = fminf(fmaxf(uv, -a.limit), a.limit); }
+            float sl;
+            if (a.alpha > 0.f) {
+              sl = bf16_to_f32(f32_to_bf16(gv / (1.f + __expf(-a.alpha * gv))));
+              uv += 1.f;
+            } else {
+              sl = bf16_to_f32(f32_to_bf16(gv / (1.f + __expf(-gv))));
+            }
+            x.h[j] = f32_to_bf16(sl * uv);
           }
-          x.h[j] = f32_to_bf16(sl * uv);
         }
       }
 #pragma unroll
       for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(bf16_to_f32(x.h[j])));
-      reinterpret_cast<uint4*>(seg)[i] = x.u;
       if (a.x_out) reinterpret_cast<uint4*>(a.x_out + static_cast<size_t>(t) * K + k0)[i] = x.u;
     }
+    seg[i] = x.u;
   }
-  if (MODE != 2) {
-    amax = cta_reduce(amax, true);
-    cluster_push(1, amax);
-    cluster.sync();
-    amax = cluster_fold(1, true);
-  } else {
-    __syncthreads();      // the normalised segment is complete in shared memory
+  // the row's statistics: this warp's partials to every CTA, then all of them from the own copy
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    if (MODE == 2) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  }
+  if (lane < cl)
+    st_async_f32x2(mapa_shared(smem_u32(&part[c * kAqMaxWarps + wid]), lane), ss, amax, mapa_shared(smem_u32(&arrived), lane));
+  if (!wait_bar(&arrived, 0) && lane == 0) report(a.status, kTimeoutConvert, 61);
+  {
+    const float4* pp = reinterpret_cast<const float4*>(part) + lane * 2;      // four pairs per lane
+    const float4 x = pp[0], y = pp[1];
+    ss = (x.x + x.z) + (y.x + y.z);
+    amax = fmaxf(fmaxf(x.y, x.w), fmaxf(y.y, y.w));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      if (MODE == 2) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    }
+  }
+  float rstd = 0.f;
+  if (MODE == 2) {
+    rstd = rsqrtf(ss / static_cast<float>(K) + a.eps);
+    // Row scale from a bound instead of the exact maximum of the normalised row: |bf16(bf16(x rstd) w)| <=
+    // |x w| rstd (1 + 2^-8)^2, so max |x w| * rstd * 1.0079 covers every element (at most 0.8 % above the true
+    // maximum) and is known from this single pass: no second row-wide reduction.
+    amax = amax * rstd * 1.0079f;
   }
   const float gs = amax > 0.f ? amax / (6.f * 256.f) : 1.f;
   if (c == 0 && tid == 0) a.g[t] = gs;
@@ -245,44 +240,59 @@ __global__ void __launch_bounds__(kAqThreads) act_quant_cluster_kernel(ClusterQu
   const int stages = K / 256;
   const int atoms = a.R * a.bn > 128 ? 2 : 1;
   const int tile = t / a.bn, m = t % a.bn;
-  for (int gl = tid; gl < kseg / 16; gl += kAqThreads) {
-    const int gi = k0 / 16 + gl;
-    Pack16 lo, hi;
-    lo.u = reinterpret_cast<const uint4*>(seg + gl * 16)[0];
-    hi.u = reinterpret_cast<const uint4*>(seg + gl * 16)[1];
-    float res[16];
+  for (int i0 = 0; i0 < nvec; i0 += nthr) {      // (whole warps: the two threads of a block exchange its maxima)
+    const int i = i0 + tid;
+    const bool on = i < nvec;
+    Pack16 x;
+    x.u = on ? seg[i] : make_uint4(0u, 0u, 0u, 0u);
+    if (MODE == 2 && on) {
+      Pack16 w;
+      w.u = i0 == 0 ? w0.u : wv[i];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      res[j] = bf16_to_f32(lo.h[j]) * inv_g;
-      res[8 + j] = bf16_to_f32(hi.h[j]) * inv_g;
+      for (int j = 0; j < 8; ++j) {
+        const float nrm = bf16_to_f32(f32_to_bf16(bf16_to_f32(x.h[j]) * rstd));
+        float gw = bf16_to_f32(w.h[j]);
+        if (a.one_plus_w) gw += 1.f;
+        x.h[j] = f32_to_bf16(nrm * gw);
+      }
+      if (a.x_out) reinterpret_cast<uint4*>(a.x_out + static_cast<size_t>(t) * K + k0)[i] = x.u;
     }
+    float res[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) res[j] = bf16_to_f32(x.h[j]) * inv_g;
+    const int gi = k0 / 16 + (i >> 1);
     const int st = gi >> 4, step = (gi >> 2) & 3, fi = gi & 3;
     for (int r = 0; r < a.R; ++r) {
-      float bm = 0.f;
-#pragma unroll
-      for (int j = 0; j < 16; ++j) bm = fmaxf(bm, fabsf(res[j]));
+      float bm = fmaxf(fmaxf(fmaxf(fabsf(res[0]), fabsf(res[1])), fmaxf(fabsf(res[2]), fabsf(res[3]))),
+                       fmaxf(fmaxf(fabsf(res[4]), fabsf(res[5])), fmaxf(fabsf(res[6]), fabsf(res[7]))));
+      bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
       const uint8_t sb = f32_to_e4m3(bm * (1.f / 6.f));
       const float s = e4m3_value_f32(bm * (1.f / 6.f));   // value of the code sb, without an fp8 decode of it
       const float inv_s = s > 0.f ? 1.f / s : 0.f;
-      float sc[16];
+      float sc[8];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) sc[j] = res[j] * inv_s;
-      const uint32_t w0 = f32x8_to_e2m1x8(sc), w1 = f32x8_to_e2m1x8(sc + 8);
-      e2m1x8_residual(w0, s, res);
-      e2m1x8_residual(w1, s, res + 8);
+      for (int j = 0; j < 8; ++j) sc[j] = res[j] * inv_s;
+      const uint32_t codes = f32x8_to_e2m1x8(sc);
+      e2m1x8_residual(codes, s, res);
+      if (!on) continue;
       const size_t ro = static_cast<size_t>(tile) * a.R * a.bn + static_cast<size_t>(r) * a.bn + m;
-      *reinterpret_cast<uint2*>(a.q + ro * (K / 2) + gi * 8) = make_uint2(w0, w1);
-      const int brow = r * a.bn + m, h = brow >> 7, mm = brow & 127;
-      const size_t atom_idx = ((static_cast<size_t>(tile) * stages + st) * 4 + step) * atoms + h;
-      a.sf[atom_idx * kAqAtom + (mm & 31) * 16 + (mm >> 5) * 4 + fi] = sb;
+      *reinterpret_cast<uint32_t*>(a.q + ro * (K / 2) + k0 / 2 + i * 4) = codes;
+      if ((i & 1) == 0) {
+        const int brow = r * a.bn + m, h = brow >> 7, mm = brow & 127;
+        const size_t atom_idx = ((static_cast<size_t>(tile) * stages + st) * 4 + step) * atoms + h;
+        a.sf[atom_idx * kAqAtom + (mm & 31) * 16 + (mm >> 5) * 4 + fi] = sb;
+      }
     }
   }
-  if (MODE == 2 && a.fold && tid == 0) {
-    __threadfence();
-    if (atomicAdd(a.comm.done_ctas, 1u) == gridDim.x * gridDim.y - 1) {
-      *a.comm.done_ctas = 0;
-      *a.comm.epoch = fold_epoch;
+  if (MODE == 2 && a.fold) {
+    __syncthreads();
+    if (tid == 0) {
       __threadfence();
+      if (atomicAdd(a.comm.done_ctas, 1u) == gridDim.x * gridDim.y - 1) {
+        *a.comm.done_ctas = 0;
+        *a.comm.epoch = fold_epoch;
+        __threadfence();
+      }
     }
   }
 }
@@ -292,7 +302,8 @@ static int launch_cluster(const ClusterQuantArgs& a, cudaStream_t st) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(a.cl, a.T, 1);
-  cfg.blockDim = dim3(kAqThreads, 1, 1);
+  const int vecs = a.K / a.cl / 8;      // one thread each, as far as a CTA goes
+  cfg.blockDim = dim3(vecs < kAqMaxThreads ? (vecs + 31) / 32 * 32 : kAqMaxThreads, 1, 1);
   cfg.dynamicSmemBytes = static_cast<size_t>(a.K / a.cl) * 2;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];

@@ -84,6 +84,33 @@ def test_fused_producers_match_reference(dev):
     assert ((xa.dequant() - ar.float()).abs().max() / ar.float().abs().max()).item() < 1e-2
 
 
+@pytest.mark.parametrize("rows,k,terms", [(1, 256, 3), (3, 768, 2), (16, 2304, 3), (5, 17408, 3), (2, 36864, 1)])
+def test_cluster_quantiser_matches_the_single_cta_one(dev, rows, k, terms):
+    """Rows split over a cluster: segments of less than a warp, of no whole number of warps, of more columns than threads hold at
+    once.  Plain and SwiGLU rows give the same codes, block scales and row scale as the one-CTA kernel (a maximum does not
+    depend on its order); the norm's sum of squares is added in another order, so its rows are compared as values."""
+    from dgpp_b200.ops import core as ops
+
+    torch.manual_seed(33)
+    bn = 16
+    x = torch.randn(rows, k, device=dev).to(BF)
+    gu = (2 * torch.randn(rows, 2 * k, device=dev)).to(BF)
+    d, w = torch.randn(rows, k, device=dev).to(BF), (1 + 0.1 * torch.randn(k, device=dev)).to(BF)
+    for m, (mode, inp, kw) in enumerate((("plain", x, {}), ("swiglu", gu, {}), ("rmsnorm", x, dict(delta=d, norm_w=w)))):
+        got, want = ops.QuantAct(bn, k, terms, bn, dev), ops.QuantAct(bn, k, terms, bn, dev)
+        ops.act_quant_nvfp4(inp.clone(), terms, out=got, mode=mode, **kw)
+        want.rows, x2 = rows, inp.clone()
+        ops.call("dgpp_act_quant_nvfp4", m, ops.ptr(x2), x2.stride(0), ops.ptr(kw.get("delta")), ops.ptr(kw.get("norm_w")), ops.ptr(x2), None,
+                 ops.ptr(want.q), ops.ptr(want.sf), ops.ptr(want.g), rows, bn, k, terms, bn, 1e-6, 0.0, 0.0, 0, ops.stream_ptr())
+        torch.cuda.synchronize()
+        ops.check_status()
+        if mode != "rmsnorm":
+            assert torch.equal(got.g, want.g) and torch.equal(got.q, want.q) and torch.equal(got.sf, want.sf), mode
+        else:      # one bf16 rounding of the normed value may fall the other way: 2^-8 of it, plus a step of the last term
+            a, b = got.dequant(), want.dequant()
+            assert ((a - b).norm() / b.norm()).item() < 2.0 ** -8 * (1 if terms > 1 else 8)
+
+
 def _filled_cache(dev, hq, hkv, ctx, page, slot, d=128):
     from dgpp_b200.engine.kv_cache import PagedKV
     from dgpp_b200.ops import core as ops, reference as ref
