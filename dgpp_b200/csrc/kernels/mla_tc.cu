@@ -5,14 +5,18 @@
 // (dc + dr) / 64 column blocks of [128, 64] bf16 with the 128-byte swizzle) and feeds both products:
 //
 //   MMA1   S^T[token, head]  = C_tile[128, dc + dr] . Q[head, dc + dr]^T          A = the tile read K-major
-//   softmax (thread = token): scores in log2 units, column maxima by shuffle + shared memory, p = 2^(s - m)
+//   softmax (thread = token and half of the heads): scores in log2 units, column maxima by shuffle + shared memory, p = 2^(s - m)
 //   MMA2   O^T[d, head]      = C_tile^T[d, 128 tokens] . P[head, 128 tokens]^T    A = the same tile read MN-major,
 //                                                                                  dc / 128 blocks of 128 latent dims
-//   accumulate (thread = latent dim of each block): o = (o + O^T) * 2^(m_old - m_new)
+//   accumulate (thread = latent dim of each block and half of the heads): o = (o + O^T) * 2^(m_old - m_new)
 //
 // The tile is single buffered (147 KB at dc + dr = 576): the PV product of tile i must retire before tile i + 1 lands.
 // S^T, P and O^T are double buffered, so the fold of tile i overlaps the load of tile i + 1.
-// Warps: 0 = TMA producer (walks the block table), 1 = MMA issuer / TMEM owner, 2..5 = softmax and accumulation.
+// Warps: 0 = TMA producer (walks the block table; the first tile is on its way while the queries are staged), 1 = MMA issuer / TMEM
+// owner, 2..9 = softmax and accumulation, two warps per TMEM lane quadrant.
+// What bounds it: one chain per tile at one CTA per SM: load, scores, maxima over the tokens, probabilities, values.
+// 8 rows x 32 heads over 4096 positions (18 splits, two tiles each): 36 us with four softmax warps of 32 heads per thread, shuffles for
+// every head's maximum and the first tile requested behind the queries, 25 so.
 // TERMS = 2 is the form for models whose scores and weights are 32-bit: queries (fp32 here) and probabilities enter the tensor
 // cores as two bf16 terms each (value + residual), side by side in the 32 columns, so a CTA takes 16 heads; outputs are fp32.
 // Every wait is bounded (status code + clean exit).  Split partials use the layout of mla.cu and its combine kernel.
@@ -29,7 +33,8 @@
 
 namespace dgpp {
 
-constexpr int kMtThreads = 192;
+constexpr int kMtThreads = 320;
+constexpr int kMtSoft = 256;   // softmax threads
 constexpr int kMtTile = 128;   // tokens per tile
 constexpr int kMtNQ = 32;      // head columns per CTA
 constexpr int kMtBlk = kMtTile * 128;   // 16 KB: one 64-element column block of the latent tile
@@ -51,6 +56,32 @@ struct MlaTcParams {
   float scale;
 };
 
+// N values per lane (N a power of two up to 32), reduced over the lanes: at distance o a lane keeps the half of its values that its bit
+// o names and adds the partner's share of them; lane i ends with value i * N / 32.
+template <bool MAX, int N>
+__device__ __forceinline__ float over_lanes(const float (&in)[N], int lane) {
+  float v[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = in[i];
+#pragma unroll
+  for (int step = 0; step < 5; ++step) {
+    const int o = 16 >> step, n = N >> (step + 1);
+    if (n > 0) {
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int i = 0; i < n; ++i) {
+        const float keep = up ? v[i + n] : v[i], give = up ? v[i] : v[i + n];
+        const float got = __shfl_xor_sync(0xffffffffu, give, o);
+        v[i] = MAX ? fmaxf(keep, got) : keep + got;
+      }
+    } else {
+      const float got = __shfl_xor_sync(0xffffffffu, v[0], o);
+      v[0] = MAX ? fmaxf(v[0], got) : v[0] + got;
+    }
+  }
+  return v[0];
+}
+
 // SPARSE: the tokens of a tile come from the row's selection list instead of consecutive positions; the four softmax
 // warps (idle while a tile loads: it is single buffered) gather them, thread = token: 72 16-byte chunks of the token's
 // latent row into the swizzled column blocks, then a proxy fence and one arrival per warp on the tile barrier.
@@ -58,6 +89,7 @@ template <int DC, int DR, bool SPARSE, int TERMS = 1>
 __global__ void __launch_bounds__(kMtThreads, 1)
 mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmC, MlaTcParams p) {
   constexpr int NH = kMtNQ / TERMS;      // heads per CTA
+  constexpr int HT = NH / 2;             // heads per softmax thread
   constexpr int D = DC + DR;
   constexpr int KB = D / 64;     // column blocks of the tile and of Q
   constexpr int MB = DC / 128;   // 128-dim output blocks
@@ -69,11 +101,11 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmC, MlaTcParams p) {
   unsigned char* sC = sp;  sp += kTileBytes;
   unsigned char* sQ = sp;  sp += KB * kQBlk;
   unsigned char* sP = sp;  sp += 2 * 2 * kQBlk;       // [buffer][64-token block][32 heads x 128 B]
-  float* red = reinterpret_cast<float*>(sp);   sp += 2 * 4 * kMtNQ * sizeof(float);   // [buffer][warp][head] tile maxima
+  float* red = reinterpret_cast<float*>(sp);   sp += 2 * 4 * kMtNQ * sizeof(float);   // [buffer][quadrant][head] tile maxima
   float* mrun = reinterpret_cast<float*>(sp);  sp += 2 * kMtNQ * sizeof(float);       // [buffer][head] running maxima
   float* corr = reinterpret_cast<float*>(sp);  sp += 2 * kMtNQ * sizeof(float);       // [buffer][head] 2^(m_old - m_new)
-  float* lred = reinterpret_cast<float*>(sp);  sp += 4 * kMtNQ * sizeof(float);       // [warp][head] probability mass
-  float* flags = reinterpret_cast<float*>(sp); sp += 2 * 4 * sizeof(float);           // [buffer][warp] 1 = this warp gave up
+  float* lred = reinterpret_cast<float*>(sp);  sp += 4 * kMtNQ * sizeof(float);       // [quadrant][head] probability mass
+  float* flags = reinterpret_cast<float*>(sp); sp += 2 * 8 * sizeof(float);           // [buffer][warp] 1 = this warp gave up
   uint64_t* c_full = reinterpret_cast<uint64_t*>(sp);
   uint64_t* c_empty = c_full + 1;
   uint64_t* s_full = c_empty + 1;   // [2]
@@ -107,8 +139,8 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmC, MlaTcParams p) {
   const int nheads = min(NH, p.heads - hg * NH);
 
   if (threadIdx.x == 0) {
-    mbar_init(c_full, SPARSE ? 4 : 1); mbar_init(c_empty, 1);
-    for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 4); mbar_init(&o_full[i], 1); }
+    mbar_init(c_full, SPARSE ? 8 : 1); mbar_init(c_empty, 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 8); mbar_init(&o_full[i], 1); }
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmC);
@@ -118,11 +150,25 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmC, MlaTcParams p) {
     tmem_relinquish();
   }
   pdl_wait();
+  const int ppt = kMtTile / p.page;
+  auto load_tile = [&](int i) {
+    mbar_expect_tx(c_full, kTileBytes);
+    const int page0 = (tile_begin + i) * kMtTile / p.page;
+    for (int pg = 0; pg < ppt; ++pg) {
+      const int pi = min(page0 + pg, p.max_blocks - 1);
+      const int r0 = bt[pi] * p.page;
+#pragma unroll
+      for (int kb = 0; kb < KB; ++kb)
+        tma_load_2d(sC + kb * kMtBlk + pg * p.page * 128, &tmC, kb * 64, r0, c_full);
+    }
+  };
+  if (!SPARSE && threadIdx.x == 0 && ntiles > 0) load_tile(0);      // (by the thread that made the barriers)
   // ---- the group's query rows as the B operand of MMA1: KB blocks of [32 heads, 64 elements], 128-byte swizzle
   if (warp >= 2) {
     const int t = threadIdx.x - 64;
     constexpr int kChunks = D / 8;   // 16-byte chunks per head
-    for (int i = t; i < NH * kChunks; i += 128) {
+#pragma unroll 3
+    for (int i = t; i < NH * kChunks; i += kMtSoft) {
       const int h = i / kChunks, c = i % kChunks;
       const size_t at = (static_cast<size_t>(row) * p.heads + hg * NH + h) * D + c * 8;
       Pack16 v, lo;
@@ -156,18 +202,9 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmC, MlaTcParams p) {
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (dense form)
     if (!SPARSE && elect_one()) {
-      const int ppt = kMtTile / p.page;
-      for (int i = 0; i < ntiles; ++i) {
+      for (int i = 1; i < ntiles; ++i) {
         if (!wait_bar(c_empty, (i & 1) ^ 1)) { report(p.status, kTimeoutStageEmpty, 51); *abort_flag = 1; break; }
-        mbar_expect_tx(c_full, kTileBytes);
-        const int page0 = (tile_begin + i) * kMtTile / p.page;
-        for (int pg = 0; pg < ppt; ++pg) {
-          const int pi = min(page0 + pg, p.max_blocks - 1);
-          const int r0 = bt[pi] * p.page;
-#pragma unroll
-          for (int kb = 0; kb < KB; ++kb)
-            tma_load_2d(sC + kb * kMtBlk + pg * p.page * 128, &tmC, kb * 64, r0, c_full);
-        }
+        load_tile(i);
         if (*abort_flag) break;
       }
     }
@@ -209,34 +246,45 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmC, MlaTcParams p) {
       }
     }
   } else {
-    // ------------------------------------------------------------------ softmax + accumulation (warps 2..5)
+    // ------------------------------------------------------------------ softmax + accumulation (warps 2..9)
     const int quad = warp & 3;
     const int idx = quad * 32 + lane;        // token lane for S^T, latent-dim lane for O^T
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    const int wslot = warp - 2;
+    const int wslot = warp - 2, half = wslot >> 2, h0 = half * HT;      // this thread's heads h0 .. h0 + HT - 1 of the CTA's
     const float sm = p.scale * 1.4426950408889634f;  // scores in log2 units
-    float l_thr[NH];
-    float o_acc[MB][NH];
+    float l_thr[HT];
+    float o_acc[MB][HT];
+    // this thread's columns of a pair of 16-column groups in tensor memory (TERMS = 2: the terms' sum)
+    auto columns = [&](uint32_t taddr, float (&v)[HT]) {
+      if constexpr (TERMS == 1) {
+        uint32_t raw[16];
+        tmem_ld_x16(taddr + half * 16, raw);
 #pragma unroll
-    for (int c = 0; c < NH; ++c) {
+        for (int c = 0; c < HT; ++c) v[c] = __uint_as_float(raw[c]);
+      } else {
+        uint32_t hi[8], lo[8];
+        tmem_ld_x8(taddr + half * 8, hi);
+        tmem_ld_x8(taddr + 16 + half * 8, lo);
+#pragma unroll
+        for (int c = 0; c < HT; ++c) v[c] = __uint_as_float(hi[c]) + __uint_as_float(lo[c]);
+      }
+    };
+#pragma unroll
+    for (int c = 0; c < HT; ++c) {
       l_thr[c] = 0.f;
 #pragma unroll
       for (int mb = 0; mb < MB; ++mb) o_acc[mb][c] = 0.f;
     }
-    auto fold = [&](int j) -> bool {   // o += O^T of tile j (both halves of the head columns)
+    auto fold = [&](int j) -> bool {   // o += O^T of tile j
       const int bp = j & 1;
       if (!wait_bar(&o_full[bp], (j >> 1) & 1)) return false;
       tc_fence_after();
 #pragma unroll
       for (int mb = 0; mb < MB; ++mb) {
+        float v[HT];
+        columns(tmem_o + (bp * MB + mb) * kMtNQ + lane_addr, v);
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          uint32_t oc[16];
-          tmem_ld_x16(tmem_o + (bp * MB + mb) * kMtNQ + half * 16 + lane_addr, oc);
-          tmem_ld_wait();
-#pragma unroll
-          for (int c = 0; c < 16; ++c) o_acc[mb][TERMS == 2 ? c : half * 16 + c] += __uint_as_float(oc[c]);
-        }
+        for (int c = 0; c < HT; ++c) o_acc[mb][c] += v[c];
       }
       return true;
     };
@@ -247,11 +295,11 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmC, MlaTcParams p) {
       const bool valid = t < len && t >= first;
       if (SPARSE) {
         if (wait_bar(c_empty, (i & 1) ^ 1)) {
-          // a warp gathers its 32 tokens one after the other: lanes take the 72 chunks of a token's row in turns, so the
+          // a warp gathers half of its quadrant's 32 tokens one after the other: lanes take the 72 chunks of a token's row in turns, so the
           // row is read with coalesced 512-byte requests; four tokens are in flight at a time
           const int my_tok = valid ? sel[t] : -1;
 #pragma unroll 1
-          for (int t4 = 0; t4 < 32; t4 += 4) {
+          for (int t4 = half * 16; t4 < half * 16 + 16; t4 += 4) {
             uint4 v[4][3];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
@@ -287,63 +335,60 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmC, MlaTcParams p) {
       bool okw = ok && wait_bar(&s_full[b], (i >> 1) & 1);
       if (!okw && ok) { report(p.status, kTimeoutAccum, 54); *abort_flag = 1; }
       tc_fence_after();
-      float s[NH];
+      float s[HT];
+      columns(tmem_s + b * kMtNQ + lane_addr, s);
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t raw[16];
-        tmem_ld_x16(tmem_s + b * kMtNQ + half * 16 + lane_addr, raw);
-        tmem_ld_wait();
+      for (int c = 0; c < HT; ++c) s[c] = valid ? s[c] * sm : -INFINITY;
+      const float mx = over_lanes<true>(s, lane);
+      if (lane % (32 / HT) == 0) red[(b * 4 + quad) * kMtNQ + h0 + lane / (32 / HT)] = mx;
+      if (lane == 0) flags[b * 8 + wslot] = (okw && !*abort_flag) ? 0.f : 1.f;
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      // a failed wait must not leave the other warps alone at the barriers: all eight read the verdicts and leave together
+      float gave_up = 0.f;
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
-          const float v = valid ? __uint_as_float(raw[c]) * sm : -INFINITY;
-          if constexpr (TERMS == 2) s[c] = half == 0 || !valid ? v : s[c] + v;
-          else s[half * 16 + c] = v;
-        }
-      }
-      float* rp = red + (b * 4 + wslot) * kMtNQ;
-#pragma unroll
-      for (int c = 0; c < NH; ++c) {
-        float mx = s[c];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (lane == 0) rp[c] = mx;
-      }
-      if (lane == 0) flags[b * 4 + wslot] = (okw && !*abort_flag) ? 0.f : 1.f;
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      // a failed wait must not leave the other warps alone at the barriers: all four read the verdicts and leave together
-      if (flags[b * 4] + flags[b * 4 + 1] + flags[b * 4 + 2] + flags[b * 4 + 3] != 0.f) { ok = false; break; }
-      const float* r0 = red + b * 4 * kMtNQ;
-      const float* m_prev = mrun + (b ^ 1) * kMtNQ;
+      for (int w = 0; w < 8; ++w) gave_up += flags[b * 8 + w];
+      if (gave_up != 0.f) { ok = false; break; }
+      const float* r0 = red + b * 4 * kMtNQ + h0;
+      const float* m_prev = mrun + (b ^ 1) * kMtNQ + h0;
       unsigned char* pbuf = sP + b * 2 * kQBlk + (idx >> 6) * kQBlk;
       const uint32_t pbyte = (idx & 63) * 2;
 #pragma unroll
-      for (int c = 0; c < NH; ++c) {
-        const float mt = fmaxf(fmaxf(r0[c], r0[kMtNQ + c]), fmaxf(r0[2 * kMtNQ + c], r0[3 * kMtNQ + c]));
-        const float mo = m_prev[c];
-        const float mn = fmaxf(mo, mt);
-        const float cr = (mo == -INFINITY) ? 0.f : exp2f(mo - mn);
-        const float pv = (valid && mn > -INFINITY) ? exp2f(s[c] - mn) : 0.f;
-        l_thr[c] = l_thr[c] * cr + pv;
-        if (idx == c) { mrun[b * kMtNQ + c] = mn; corr[b * kMtNQ + c] = cr; }
-        // P[head c][token idx]: row c of the 64-token block, 2 bytes at the token's column (128-byte swizzle)
-        const bf16 ph = f32_to_bf16(pv);
-        unsigned char* pd = pbuf + c * 128 + ((((pbyte >> 4) ^ (c & 7)) << 4) | (pbyte & 15));
-        *reinterpret_cast<bf16*>(pd) = ph;
-        if constexpr (TERMS == 2) *reinterpret_cast<bf16*>(pd + NH * 128) = f32_to_bf16(pv - bf16_to_f32(ph));
+      for (int c4 = 0; c4 < HT; c4 += 4) {
+        float4 m4[5];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) m4[w] = *reinterpret_cast<const float4*>(r0 + w * kMtNQ + c4);
+        m4[4] = *reinterpret_cast<const float4*>(m_prev + c4);
+        const float mo4[4] = {m4[4].x, m4[4].y, m4[4].z, m4[4].w};
+        const float mt4[4] = {fmaxf(fmaxf(m4[0].x, m4[1].x), fmaxf(m4[2].x, m4[3].x)), fmaxf(fmaxf(m4[0].y, m4[1].y), fmaxf(m4[2].y, m4[3].y)),
+                              fmaxf(fmaxf(m4[0].z, m4[1].z), fmaxf(m4[2].z, m4[3].z)), fmaxf(fmaxf(m4[0].w, m4[1].w), fmaxf(m4[2].w, m4[3].w))};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int c = c4 + j, h = h0 + c;
+          const float mo = mo4[j], mn = fmaxf(mo, mt4[j]);
+          const float cr = (mo == -INFINITY) ? 0.f : fast_exp2(mo - mn);
+          const float pv = (valid && mn > -INFINITY) ? fast_exp2(s[c] - mn) : 0.f;
+          l_thr[c] = l_thr[c] * cr + pv;
+          if (idx == c) { mrun[b * kMtNQ + h] = mn; corr[b * kMtNQ + h] = cr; }
+          // P[head h][token idx]: row h of the 64-token block, 2 bytes at the token's column (128-byte swizzle)
+          const bf16 ph = f32_to_bf16(pv);
+          unsigned char* pd = pbuf + h * 128 + ((((pbyte >> 4) ^ (h & 7)) << 4) | (pbyte & 15));
+          *reinterpret_cast<bf16*>(pd) = ph;
+          if constexpr (TERMS == 2) *reinterpret_cast<bf16*>(pd + NH * 128) = f32_to_bf16(pv - bf16_to_f32(ph));
+        }
       }
       fence_proxy_async_smem();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[b]);
-      asm volatile("bar.sync 1, 128;" ::: "memory");   // corr[b] / mrun[b] visible to all four warps
+      asm volatile("bar.sync 1, 256;" ::: "memory");   // corr[b] / mrun[b] visible to all eight warps
       // fold the previous tile's O^T (taken relative to the previous maxima), then rescale to this tile's maxima
       if (i > 0 && !fold(i - 1)) {
         report(p.status, kTimeoutAccum, 55);
         *abort_flag = 1;   // agreed on at the next tile's barrier
       }
-      const float* cb = corr + b * kMtNQ;
+      const float* cb = corr + b * kMtNQ + h0;
 #pragma unroll
-      for (int c = 0; c < NH; ++c) {
+      for (int c = 0; c < HT; ++c) {
         const float cr = cb[c];
 #pragma unroll
         for (int mb = 0; mb < MB; ++mb) o_acc[mb][c] *= cr;
@@ -356,21 +401,17 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmC, MlaTcParams p) {
       done = false;
     }
     // total probability mass per head: sum the per-thread partials
-#pragma unroll
-    for (int c = 0; c < NH; ++c) {
-      float l = l_thr[c];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-      if (lane == 0) lred[wslot * kMtNQ + c] = l;
-    }
-    asm volatile("bar.sync 1, 128;" ::: "memory");
+    const float lsum = over_lanes<false>(l_thr, lane);
+    if (lane % (32 / HT) == 0) lred[quad * kMtNQ + h0 + lane / (32 / HT)] = lsum;
+    asm volatile("bar.sync 1, 256;" ::: "memory");
     if (done) {
       const float* m_fin = mrun + ((ntiles > 0 ? (ntiles - 1) & 1 : 0)) * kMtNQ;
 #pragma unroll
-      for (int c = 0; c < NH; ++c) {
-        if (c < nheads) {
-          const float l = lred[c] + lred[kMtNQ + c] + lred[2 * kMtNQ + c] + lred[3 * kMtNQ + c];
-          const size_t rh = static_cast<size_t>(row) * p.heads + hg * NH + c;
+      for (int c = 0; c < HT; ++c) {
+        const int h = h0 + c;
+        if (h < nheads) {
+          const float l = lred[h] + lred[kMtNQ + h] + lred[2 * kMtNQ + h] + lred[3 * kMtNQ + h];
+          const size_t rh = static_cast<size_t>(row) * p.heads + hg * NH + h;
           if (p.splits == 1) {
             const float inv = l > 0.f ? 1.f / l : 0.f;
 #pragma unroll
@@ -385,7 +426,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmC, MlaTcParams p) {
             for (int mb = 0; mb < MB; ++mb) p.part_acc[pi * DC + mb * 128 + idx] = o_acc[mb][c];
             if (idx == 0) {
               // running max is kept in log2 units; the combine kernel works in natural-log units
-              p.part_ml[pi * 2] = ntiles > 0 ? m_fin[c] * 0.6931471805599453f : -INFINITY;
+              p.part_ml[pi * 2] = ntiles > 0 ? m_fin[h] * 0.6931471805599453f : -INFINITY;
               p.part_ml[pi * 2 + 1] = l;
             }
           }
@@ -458,7 +499,7 @@ __global__ void mla_tc_combine_kernel(const float* __restrict__ part_ml, const f
 
 template <int KB>
 constexpr size_t mla_tc_smem() {
-  return 1024 + KB * kMtBlk + KB * kMtNQ * 128 + 4 * kMtNQ * 128 + (2 * 4 + 2 + 2 + 4) * kMtNQ * 4 + 2 * 4 * 4 + 8 * 8 + 64;
+  return 1024 + KB * kMtBlk + KB * kMtNQ * 128 + 4 * kMtNQ * 128 + (2 * 4 + 2 + 2 + 4) * kMtNQ * 4 + 2 * 8 * 4 + 8 * 8 + 64;
 }
 
 }  // namespace dgpp
