@@ -16,8 +16,10 @@
 // tiles of a chunk stay in L2.
 //
 // What bounds it: at wide tiles the tensor pipe (2048 x 34816 x 5120: 474 us = 1540 TFLOP/s, 0.91 of the measured cuBLAS burst rate;
-// the single-CTA kernel 1216 us), at narrow ones the MMA thread's chain and the conversion (8 x 34816 x 5120: 49 us, 480
-// cycles per K = 64 block; 73 us).  2048 x 5120 x 17408: 564 -> 266 us, 173 x 5120 x 5120: 71 -> 27 us.
+// the single-CTA kernel 1216 us), at narrow ones the conversion (37 x 34816 x 5120: 40 us; a set's block takes some 1400 cycles, half
+// of them waits).  The weights have a producer of their own: behind the activations' ring, which ends 512 K ahead of the MMAs,
+// their loads were a round trip to HBM on every stage's way (converters waited 780 of 1900 cycles; 37 x 34816 x 5120 50 us, 256 experts'
+// gate-up and down products of 64 rows each 479 us, 392 so).  2048 x 5120 x 17408: 266 us, 173 x 5120 x 5120: 25 us.
 //
 // Handshakes (all waits bounded, expiry -> status code, everything unwinds, TMEM freed):
 //   own CTA:          raw_full / raw_empty (TMA -> converters), acc_full (MMA -> epilogue);
@@ -27,7 +29,7 @@
 //                     tile) have completed; the producers and the converters both wait for `done`.
 // (Arrivals on the other CTA's barriers release at CTA scope: what they order is tensor memory, by the tcgen05 fences; a
 // cluster-scope release took 1100 cycles per arrival, three times a block's MMAs.)
-// Warp roles (896 threads): warp 0 MMA issuer (first CTA) and TMEM owner, 1 TMA producer, 4..19 converters (four sets take turns
+// Warp roles (896 threads): warp 0 MMA issuer (first CTA) and TMEM owner, 1 TMA producer of the activations, 2 of the weights, 4..19 converters (four sets take turns
 // at the K = 64 blocks), 20..27 epilogue.
 // (reference counterpart: src/kernels/fp4w_gemm.cu, the W4A16 prefill GEMM.)
 #include <cuda_bf16.h>
@@ -46,7 +48,7 @@ constexpr int kPrBM = 128;          // weight rows per CTA
 constexpr int kPrBK = 64;
 constexpr int kPrMaxBN = 256;       // tokens per pair tile = MMA N, at most
 constexpr int kPrSets = 4;            // converter sets of four warps; set s takes block s of every 256 K
-constexpr int kPrMma = 0, kPrTma = 1, kPrConv = 4, kPrEpi = kPrConv + kPrSets * 4;   // first warp of each role
+constexpr int kPrMma = 0, kPrTma = 1, kPrRaw = 2, kPrConv = 4, kPrEpi = kPrConv + kPrSets * 4;   // first warp of each role
 constexpr int kPrEpiWarps = 8;        // two per lane quadrant, taking turns at 16 columns
 constexpr int kPrThreads = (kPrEpi + kPrEpiWarps) * 32;
 constexpr int kPrStages = 4, kPrSR = 4;   // stages of 128 K (activations and converted weights), raw stages of 256 K
@@ -162,7 +164,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA,   // packed weights
   cluster_barrier();      // the other CTA's barriers exist before anything arrives on them from here
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_wait();
+  // (weights do not depend on the grid before: their first stages are requested in front of the wait)
+  if (GROUPED || warp != kPrRaw) pdl_wait();
 
   // Unit u: k64 blocks [kb0, kb0 + nk), a multiple of four; first weight row (n0 in the tensor map, nc as a column of the output) and
   // first token of the tile.  False: nothing to do.
@@ -187,34 +190,47 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA,   // packed weights
     return true;
   };
 
-  if (warp == kPrTma) {
-    // ------------------------------------------------------------------ TMA producer (own weights, own token half)
+  if (warp == kPrRaw) {
+    // ------------------------------------------------------------------ TMA producer of the weights (own rows), up to 1024 K ahead
+    if (elect_one()) {
+      bool ok = true, waited = GROUPED;
+      int r = 0;
+      for (int u = first_unit; u < p.units && ok; u += unit_step) {
+        int n0, nc, m0, split, kb0, nk;
+        float alpha;
+        if (!unit_at(u, n0, nc, m0, split, kb0, nk, alpha)) continue;
+        for (int i = 0; i < nk; i += 4, ++r) {
+          const int sr = r % kPrSR, kb = kb0 + i;
+          if (!waited && r == kPrSR) { pdl_wait(); waited = true; }
+          if (!wait_bar(&raw_empty[sr], ((r / kPrSR) & 1) ^ 1)) { report(p.status, kTimeoutStageEmpty, 21); *abort_flag = 1; ok = false; break; }
+          if (*abort_flag) { ok = false; break; }
+          mbar_expect_tx(&raw_full[sr], kPrStageRaw + (WMODE == 1 ? kPrStageSf : 0));
+          tma_load_2d(sRaw + sr * kPrStageRaw, &tmA, kb * 32, n0, &raw_full[sr]);
+          if (GROUPED)
+            bulk_load_1d(sSf + sr * kPrStageSf, p.sf_tiled + (static_cast<size_t>(n0 / kPrBM) * (p.K / 256) + (kb >> 2)) * kPrStageSf, kPrStageSf, &raw_full[sr]);
+          else if (WMODE == 1) tma_load_2d(sSf + sr * kPrStageSf, &tmSf, kb * 4, n0, &raw_full[sr]);
+        }
+      }
+      if (!waited) pdl_wait();
+    }
+  } else if (warp == kPrTma) {
+    // ------------------------------------------------------------------ TMA producer of the activations (own token half)
     if (elect_one()) {
       const uint32_t stage_b = static_cast<uint32_t>(p.width / 2) * 128u;
-      int it = 0;
+      int stg = 0;
       bool ok = true;
       for (int u = first_unit; u < p.units && ok; u += unit_step) {
         int n0, nc, m0, split, kb0, nk;
         float alpha;
         if (!unit_at(u, n0, nc, m0, split, kb0, nk, alpha)) continue;
         const int mh = m0 + rank * (p.width / 2);
-        for (int i = 0; i < nk; ++i, ++it) {
-          const int kb = kb0 + i;
-          if ((it & 3) == 0) {
-            const int r = it >> 2, sr = r % kPrSR;
-            if (!wait_bar(&raw_empty[sr], ((r / kPrSR) & 1) ^ 1)) { report(p.status, kTimeoutStageEmpty, 21); *abort_flag = 1; ok = false; break; }
-            mbar_expect_tx(&raw_full[sr], kPrStageRaw + (WMODE == 1 ? kPrStageSf : 0));
-            tma_load_2d(sRaw + sr * kPrStageRaw, &tmA, kb * 32, n0, &raw_full[sr]);
-            if (GROUPED)
-              bulk_load_1d(sSf + sr * kPrStageSf, p.sf_tiled + (static_cast<size_t>(n0 / kPrBM) * (p.K / 256) + (kb >> 2)) * kPrStageSf, kPrStageSf, &raw_full[sr]);
-            else if (WMODE == 1) tma_load_2d(sSf + sr * kPrStageSf, &tmSf, kb * 4, n0, &raw_full[sr]);
-          }
-          const int stg = it >> 1, sl = stg % kPrStages;
-          if ((it & 1) == 0) {
-            if (!wait_bar(&done[sl], ((stg / kPrStages) & 1) ^ 1)) { report(p.status, kTimeoutStageEmpty, 22); *abort_flag = 1; ok = false; break; }
-            if (rank == 0) mbar_expect_tx(&full[sl], 4 * stage_b);
-          }
-          tma_load_2d_pair(sB + sl * kPrStageB + (it & 1) * kPrHalfB, &tmB, kb * kPrBK, mh, mapa_shared(smem_u32(&full[sl]), 0u));
+        for (int i = 0; i < nk; i += 2, ++stg) {
+          const int sl = stg % kPrStages, kb = kb0 + i;
+          if (!wait_bar(&done[sl], ((stg / kPrStages) & 1) ^ 1)) { report(p.status, kTimeoutStageEmpty, 22); *abort_flag = 1; ok = false; break; }
+          if (rank == 0) mbar_expect_tx(&full[sl], 4 * stage_b);
+          const uint32_t bar = mapa_shared(smem_u32(&full[sl]), 0u);
+          tma_load_2d_pair(sB + sl * kPrStageB, &tmB, kb * kPrBK, mh, bar);
+          tma_load_2d_pair(sB + sl * kPrStageB + kPrHalfB, &tmB, (kb + 1) * kPrBK, mh, bar);
         }
       }
     }
