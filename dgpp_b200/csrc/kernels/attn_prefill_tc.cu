@@ -1,24 +1,26 @@
-// Causal flash attention for prefill over the paged FP8 KV cache, on tcgen05 (kind::f8f6f4).
+// Causal flash attention for prefill over the paged FP8 KV cache, on tcgen05 (kind::f16).
 //
-// One CTA = one query head x 128 consecutive query positions of one request.  K / V tiles of 128 tokens come
-// from the cache pages by TMA exactly as stored (e4m3 bytes); nothing converts them:
+// Work comes in units of one query head x 128 consecutive query positions.  A CTA takes two units of one KV head (the units of a KV
+// head are numbered longest span first, heads fastest), or one where that already occupies the device.  K / V tiles of 128 tokens
+// come from the cache pages by TMA as stored (e4m3 bytes) and are expanded once per CTA to f16, scale included:
 //
-//   MMA1   S[q, t]  = (Q1 + Q2)[q, d] . K[t, d]^T          Q split into two e4m3 terms (A operand, K-major)
-//   softmax (two threads per query row, 64 tokens each): s = S * q_scale[q] * k_scale[t] * sm_scale, causal mask, running max / sum,
-//           P[q, t] = p * v_scale[t] * c_tile split into two e4m3 terms, written as the next A operand
-//   MMA2   O_tile[q, d] = (P1 + P2)[q, t] . V[t, d]        V is the B operand read MN-major (d contiguous)
-//   accumulate (two threads per query row, 64 fp32 registers each): o = o * corr + O_tile / c_tile
+//   K16[t, d] = f16(K[t, d] * k_scale[t] / 2^ck)      ck, cv: exponents of the tile's largest scales; the product is rounded once
+//   V16[t, d] = f16(V[t, d] * v_scale[t] / 2^cv)      (f16 splits the scale into two terms), to 11 bits
+//   MMA1   S[q, t]  = Q16[q, d] . K16[t, d]^T          Q16 = q / 2^e of its row, exact
+//   softmax (one thread per query row): s = S * sm, p = 2^(s + cv - m), causal mask, P as f16 over the scores' own columns
+//   MMA2   O[q, d] += P[q, t] . V16[t, d]              P is the A operand in tensor memory, V the B operand read MN-major
 //
-// S is double buffered in TMEM so MMA1 of tile i + 1 overlaps the softmax of tile i; the PV product of tile i
-// runs while the softmax threads exponentiate tile i + 1.  Both splits keep ~2^-8 relative operand error
-// (e4m3 value + e4m3 residual), K and V are exact.
-// Warps: 0 = TMA producer (pages + their scales), 1 = MMA issuer / TMEM owner, 2..9 = softmax: warps w and w + 4 share a TMEM lane
-// quadrant, the first has a row's tokens (and output columns) 0..63, the second 64..127; the halves of a row exchange
-// their maxima at the barrier that the tile's V scales need anyway, and their sums once at the end.
-// What bounds it: the softmax threads (some 25 instructions per score and 60 waits for TMEM loads per tile); one warp per
-// scheduler could not hide its own latencies.  Row tiles are dealt longest first.
-// One thread per row / two: a whole pass of 16 layers, 40 query and 8 KV heads at 8192 rows 119.0 / 110.9 ms, 2048 rows 22.98 / 21.85, 173 rows
-// 5.25 / 4.95 (the linears of the pass are in both figures).
+// O stays in tensor memory.  m is a row's reference, not its maximum: it moves only when a tile exceeds it by more than 2^8
+// (f16 and the fp32 sums have the range for that), so the accumulator is rescaled a few times per row instead of once per tile.
+// Whether it moves depends on the row alone: a row's bits do not depend on what else its pass, its CTA or its unit's partner does.
+//
+// Two units: the tensor core works for one while the other's threads exponentiate (S of unit u is rewritten right behind its PV
+// product).  One unit: two score buffers, S of tile i + 1 runs under the softmax of tile i.
+// Warps: 0..3 / 4..7 softmax of the units (TMEM lane quadrant = warp % 4), 8..11 expand K, 12..15 expand V (thread = token),
+// 16 TMA producer, 17 MMA issuer and TMEM owner.
+// What bounds it: MUFU and tensor pipe alike (a tile of two units: 2048 cycles each), then the handshakes between them.
+// 40 query and 8 KV heads, with two e4m3 terms of q and P, one unit per CTA and the accumulator in registers / so: 173 rows behind 3000
+// 97 / 65 us, 2048 rows 205 / 115, 2048 rows behind 6144 900 / 521.
 // (reference counterparts: src/kernels/full_attn.cu:442,679,983 tile / TMA / fp8-compute prefill kernels.)
 #include <cuda.h>
 #include <math.h>
@@ -31,10 +33,14 @@
 
 namespace dgpp {
 
-constexpr int kApThreads = 320;
-constexpr int kApHalf = 64;       // tokens and output columns of one softmax thread
 constexpr int kApTile = 128;
-constexpr int kApStages = 3;
+constexpr int kApConv = 8, kApTma = 16, kApMma = 17;     // first warp of each role behind the softmax warps
+constexpr int kApThreads = 18 * 32;
+constexpr int kApRing = 4, kApRaw = 2;                   // f16 tiles (K in the even slots, V in the odd ones), tiles as stored
+constexpr int kApRawBytes = kApTile * 128;               // 16 KB
+constexpr int kApBlk = kApTile * 128;                    // 16 KB: 64 columns of an f16 tile
+constexpr int kApF16Bytes = 2 * kApBlk;
+constexpr float kApSlack = 8.f;                          // a row's reference may lag its maximum by this power of two
 
 struct AttnPrefillParams {
   const bf16* q;            // [T, q_stride]: head h at column h * 128 (already rotated)
@@ -45,351 +51,405 @@ struct AttnPrefillParams {
   bf16* out;                // [T, hq * 128]
   DeviceStatus* status;
   int T, pos0, hq, hkv, page, max_blocks, window;
+  int units, per_cta;       // units of a KV head, units of a CTA (1 or 2)
   float scale;
 };
 
-__device__ __forceinline__ uint32_t sw128_off(uint32_t row, uint32_t byte_in_row) {
-  return row * 128u + ((((byte_in_row >> 4) ^ (row & 7u)) << 4) | (byte_in_row & 15u));
+constexpr size_t attn_prefill_smem_bytes() {
+  return 1024 + 2 * kApF16Bytes + kApRing * kApF16Bytes + kApRaw * (kApRawBytes + kApTile * 4) + 2 * 4 * 4 +
+         (2 * kApRing + 2 * kApRaw + 6) * 8 + 16;
 }
 
-// Row maximum of raw score * k_scale over the 64 tokens from `cb` of a tile (scores read from TMEM).
-template <bool kMask>
-__device__ __forceinline__ float tile_row_max(uint32_t taddr, const float* ks, int cb, int t0, int my_pos, int my_first) {
-  float mt = -INFINITY;
-#pragma unroll 2
-  for (int c0 = cb; c0 < cb + kApHalf; c0 += 16) {
-    uint32_t raw[16];
-    tmem_ld_x16(taddr + c0, raw);
-    tmem_ld_wait();
-#pragma unroll
-    for (int q4 = 0; q4 < 4; ++q4) {
-      const float4 k4 = *reinterpret_cast<const float4*>(ks + c0 + q4 * 4);
-      const float kk[4] = {k4.x, k4.y, k4.z, k4.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float sv = __uint_as_float(raw[q4 * 4 + j]) * kk[j];
-        if (kMask) {
-          const int t = t0 + c0 + q4 * 4 + j;
-          mt = fmaxf(mt, (t <= my_pos && t >= my_first) ? sv : -INFINITY);
-        } else {
-          mt = fmaxf(mt, sv);
-        }
-      }
-    }
-  }
-  return mt;
+__device__ __forceinline__ float exp2_of(int e) { return __uint_as_float(static_cast<uint32_t>(e + 127) << 23); }   // -126 <= e <= 127
+
+// (lo, hi) of a pair of packed fp32 values: one instruction for two lanes of arithmetic.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z, w;\n\t"
+      "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+      "fma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;\n\t}\n"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, w;\n\t"
+      "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "add.rn.f32x2 w, x, y;\n\tmov.b64 {%0, %1}, w;\n\t}\n"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
 }
 
-// Probabilities of 64 tokens: p = 2^(raw * k_scale * sm - m); P = p * v_scale * c_tile as two e4m3 terms written
-// to row r of the swizzled A operand (term 2 one tile further).  Returns the row sum of p.
+// 32 scores of a row from tensor memory, tokens t0 .. t0 + 31; those the row does not see become -inf.
 template <bool kMask>
-__device__ __forceinline__ float tile_probs(uint32_t taddr, const float* ks, const float* vs, unsigned char* sP, int r,
-                                            float sm, float neg_m, float c_tile, int cb, int t0, int my_pos, int my_first) {
-  float lsum = 0.f;
-#pragma unroll 2
-  for (int c0 = cb; c0 < cb + kApHalf; c0 += 16) {
-    uint32_t raw[16];
-    tmem_ld_x16(taddr + c0, raw);
-    tmem_ld_wait();
-    Pack16 a, bq;
+__device__ __forceinline__ void scores_x32(uint32_t taddr, int t0, int my_pos, int my_first, uint32_t (&s)[32]) {
+  tmem_ld_x32(taddr, s);
+  if (kMask) {
 #pragma unroll
-    for (int q4 = 0; q4 < 4; ++q4) {
-      const float4 k4 = *reinterpret_cast<const float4*>(ks + c0 + q4 * 4);
-      const float4 v4 = *reinterpret_cast<const float4*>(vs + c0 + q4 * 4);
-      const float kk[4] = {k4.x, k4.y, k4.z, k4.w};
-      const float vv[4] = {v4.x, v4.y, v4.z, v4.w};
-      float pw[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float e = fmaf(__uint_as_float(raw[q4 * 4 + j]) * kk[j], sm, neg_m);
-        if (kMask) {
-          const int t = t0 + c0 + q4 * 4 + j;
-          e = (t <= my_pos && t >= my_first) ? e : -INFINITY;
-        }
-        const float pv = fast_exp2(e);
-        lsum += pv;
-        pw[j] = pv * (vv[j] * c_tile);
-      }
-      f32x2_to_e4m3x2_two_term(pw[0], pw[1], a.s[q4 * 2], bq.s[q4 * 2]);
-      f32x2_to_e4m3x2_two_term(pw[2], pw[3], a.s[q4 * 2 + 1], bq.s[q4 * 2 + 1]);
-    }
-    *reinterpret_cast<uint4*>(sP + sw128_off(r, c0)) = a.u;
-    *reinterpret_cast<uint4*>(sP + kApTile * 128 + sw128_off(r, c0)) = bq.u;
+    for (int j = 0; j < 32; ++j)
+      if (t0 + j > my_pos || t0 + j < my_first) s[j] = 0xff800000u;
   }
-  return lsum;
+}
+__device__ __forceinline__ float max_x32(const uint32_t (&s)[32], float m) {
+  float m4[4] = {m, -INFINITY, -INFINITY, -INFINITY};      // (four chains)
+#pragma unroll
+  for (int j = 0; j < 32; j += 8)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) m4[c] = fmaxf(fmaxf(m4[c], __uint_as_float(s[j + c])), __uint_as_float(s[j + 4 + c]));
+  return fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+}
+// Probabilities 2^(s * sm + off) of 32 scores as 16 words of the A operand at `paddr`; their sum is added to `sum`.
+__device__ __forceinline__ void probs_x32(const uint32_t (&s)[32], float sm, float off, uint32_t paddr, float2 (&sum)[2]) {
+  uint32_t o[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    float2 e = fma2(make_float2(__uint_as_float(s[2 * j]), __uint_as_float(s[2 * j + 1])), make_float2(sm, sm), make_float2(off, off));
+    e.x = fast_exp2(e.x);
+    e.y = fast_exp2(e.y);
+    sum[j & 1] = add2(sum[j & 1], e);
+    const __half2 h = __floats2half2_rn(e.x, e.y);
+    o[j] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  tmem_st_x16_async(paddr, o);
+}
+
+// Scores of one tile -> probabilities.  Tokens 64..127 stay in registers between the two passes; the P operand takes over their
+// columns (64 words at column 64), tokens 0..63 are read again.  `ref` is the row's reference m, `lsum` its probability mass in
+// units of 2^m; `rescale(corr)` multiplies the accumulator (called by all lanes of a warp or by none).
+template <bool kMask, class Rescale>
+__device__ __forceinline__ void softmax_tile(uint32_t ts, int t0, int my_pos, int my_first, float sm, int cv, float& ref, float& lsum,
+                                             Rescale rescale) {
+  uint32_t a[32], b[32], c[32];
+  scores_x32<kMask>(ts, t0, my_pos, my_first, a);
+  float mt = max_x32(a, -INFINITY);
+  scores_x32<kMask>(ts + 32, t0 + 32, my_pos, my_first, a);
+  mt = max_x32(a, mt);
+  scores_x32<kMask>(ts + 64, t0 + 64, my_pos, my_first, b);
+  mt = max_x32(b, mt);
+  scores_x32<kMask>(ts + 96, t0 + 96, my_pos, my_first, c);
+  mt = max_x32(c, mt);
+  const float top = fmaf(mt, sm, static_cast<float>(cv));   // sm > 0
+  const bool move = top > ref + kApSlack;      // (the first tile with a visible token: ref = -inf)
+  if (__any_sync(0xffffffffu, move)) {
+    const float next = move ? top : ref;
+    const float corr = (move && ref != -INFINITY) ? fast_exp2(ref - next) : 1.f;
+    ref = next;
+    lsum *= corr;
+    rescale(corr);
+  }
+  const float off = ref == -INFINITY ? 0.f : static_cast<float>(cv) - ref;
+  float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+  probs_x32(b, sm, off, ts + 96, sum);
+  probs_x32(c, sm, off, ts + 112, sum);
+  scores_x32<kMask>(ts, t0, my_pos, my_first, a);
+  probs_x32(a, sm, off, ts + 64, sum);
+  scores_x32<kMask>(ts + 32, t0 + 32, my_pos, my_first, a);
+  probs_x32(a, sm, off, ts + 80, sum);
+  lsum = fmaf((sum[0].x + sum[0].y) + (sum[1].x + sum[1].y), exp2_of(-cv), lsum);
+  tmem_st_wait();
 }
 
 __global__ void __launch_bounds__(kApThreads, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                        AttnPrefillParams p) {
   constexpr int D = 128;
-  constexpr int kTileBytes = kApTile * D;  // 16 KB
   extern __shared__ __align__(1024) unsigned char smem_dyn[];
   unsigned char* sp = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
-  unsigned char* sQ = sp;  sp += 2 * kTileBytes;             // Q1, Q2
-  unsigned char* sP = sp;  sp += 2 * kTileBytes;             // P1, P2
-  unsigned char* sK = sp;  sp += kApStages * kTileBytes;
-  unsigned char* sV = sp;  sp += kApStages * kTileBytes;
-  float* sKs = reinterpret_cast<float*>(sp);  sp += kApStages * kApTile * sizeof(float);
-  float* sVs = reinterpret_cast<float*>(sp);  sp += kApStages * kApTile * sizeof(float);
-  float* red = reinterpret_cast<float*>(sp);  sp += 2 * 16 * sizeof(float);           // [parity][4 maxima of V scales, 8 verdicts]
-  float* mx = reinterpret_cast<float*>(sp);   sp += 2 * 2 * kApTile * sizeof(float);  // [parity][half][row] maxima (last: row sums)
-  uint64_t* kv_full = reinterpret_cast<uint64_t*>(sp);
-  uint64_t* kv_empty = kv_full + kApStages;
-  uint64_t* s_full = kv_empty + kApStages;   // [2]
-  uint64_t* p_full = s_full + 2;             // [1]
-  uint64_t* o_full = p_full + 1;             // [1]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 1);
+  unsigned char* sQ = sp;    sp += 2 * kApF16Bytes;
+  unsigned char* sRing = sp; sp += kApRing * kApF16Bytes;
+  unsigned char* sRaw = sp;  sp += kApRaw * kApRawBytes;
+  float* sScale = reinterpret_cast<float*>(sp);  sp += kApRaw * kApTile * sizeof(float);
+  int* sExp = reinterpret_cast<int*>(sp);        sp += 2 * 4 * sizeof(int);     // [K, V][tile & 3] exponents of the tile's scales
+  uint64_t* raw_full = reinterpret_cast<uint64_t*>(sp);
+  uint64_t* raw_empty = raw_full + kApRaw;
+  uint64_t* ring_full = raw_empty + kApRaw;
+  uint64_t* ring_empty = ring_full + kApRing;
+  uint64_t* s_full = ring_empty + kApRing;   // [2] per score buffer
+  uint64_t* p_full = s_full + 2;             // [2] per score buffer
+  uint64_t* o_full = p_full + 2;             // [2] per unit
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int head = blockIdx.x, kvh = head / (p.hq / p.hkv);
-  const int row0 = static_cast<int>(gridDim.y - 1 - blockIdx.y) * kApTile;   // first chunk row of this CTA, the longest spans first
-  const int rows = min(kApTile, p.T - row0);
-  const int last_pos = p.pos0 + row0 + rows - 1;
-  const int first_pos = p.pos0 + row0;
-  const int first_tok = (p.window > 0 && first_pos + 1 > p.window) ? first_pos + 1 - p.window : 0;
+  const int group = p.hq / p.hkv, kvh = blockIdx.x % p.hkv;
+  const int unit0 = static_cast<int>(blockIdx.x) / p.hkv * p.per_cta;
+  const bool dual = p.per_cta == 2;
+  const int row_tiles = p.units / group;
+  // unit u of this KV head: query head, first row; tiles are counted from the first that any of the CTA's rows sees
+  auto unit_row = [&](int u) { return (row_tiles - 1 - u / group) * kApTile; };
+  const int low_row = unit_row(min(unit0 + p.per_cta - 1, p.units - 1));
+  const int low_pos = p.pos0 + low_row;
+  const int first_tok = (p.window > 0 && low_pos + 1 > p.window) ? low_pos + 1 - p.window : 0;
   const int base = first_tok & ~(kApTile - 1);
-  const int ntiles = (last_pos + 1 - base + kApTile - 1) / kApTile;
+  auto unit_last = [&](int u) { return p.pos0 + min(unit_row(u) + kApTile, p.T) - 1; };
+  auto unit_tiles = [&](int u) { return u < p.units ? (unit_last(u) + kApTile - base) / kApTile : 0; };
+  const int n0 = unit_tiles(unit0), n1 = dual ? unit_tiles(unit0 + 1) : 0;       // n0 >= n1, n0 >= 1
+  const int last_pos = unit_last(unit0);
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kApStages; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1); }
-    mbar_init(&s_full[0], 1); mbar_init(&s_full[1], 1);
-    mbar_init(p_full, 8);
-    mbar_init(o_full, 1);
+    for (int i = 0; i < kApRaw; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 4); }
+    for (int i = 0; i < kApRing; ++i) { mbar_init(&ring_full[i], 4); mbar_init(&ring_empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 4); mbar_init(&o_full[i], 1); }
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
   }
-  if (warp == 1) {
+  if (warp == kApMma) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
   pdl_wait();
-  // ---- quantise this CTA's query rows into two e4m3 terms (two threads per row, 64 columns each)
+  // ---- the units' query rows as f16 (thread = row): scaled by a power of two to a largest magnitude of 128..256
+  const int sub = warp >> 2;
   float q_scale = 1.f;
-  if (warp >= 2) {
-    const int r = (warp & 3) * 32 + lane, half = (warp - 2) >> 2;   // the TMEM lane quadrant this warp may read: warp % 4
-    float v[kApHalf];
+  if (warp < kApConv && (sub == 0 || n1 > 0)) {
+    const int r = (warp & 3) * 32 + lane, row = unit_row(unit0 + sub) + r;
+    const int head = kvh * group + (unit0 + sub) % group;
+    const uint4* src = reinterpret_cast<const uint4*>(p.q + static_cast<size_t>(row) * p.q_stride + head * D);
+    const bool live = row < p.T;
     float amax = 0.f;
-    if (r < rows) {
-      const uint4* src = reinterpret_cast<const uint4*>(p.q + static_cast<size_t>(row0 + r) * p.q_stride + head * D);
 #pragma unroll
-      for (int c = 0; c < kApHalf / 8; ++c) {
-        Pack16 x, y;
-        x.u = src[half * (kApHalf / 8) + c];
-        y.u = src[(half ^ 1) * (kApHalf / 8) + c];
+    for (int c = 0; c < D / 8; ++c) {
+      Pack16 x;
+      x.u = live ? src[c] : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          v[c * 8 + j] = bf16_to_f32(x.h[j]);
-          amax = fmaxf(amax, fmaxf(fabsf(v[c * 8 + j]), fabsf(bf16_to_f32(y.h[j]))));
-        }
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < kApHalf; ++j) v[j] = 0.f;
+      for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(bf16_to_f32(x.h[j])));
     }
-    q_scale = amax > 0.f ? amax / 448.f : 1.f;
-    const float inv = 1.f / q_scale;
+    const int e = max(static_cast<int>((__float_as_uint(amax) >> 23) & 255u), 8);      // biased exponent of the largest
+    const float mul = __uint_as_float(static_cast<uint32_t>(261 - e) << 23);
+    q_scale = __uint_as_float(static_cast<uint32_t>(e - 7) << 23);
 #pragma unroll
-    for (int c = 0; c < kApHalf / 16; ++c) {
-      Pack16 a, b;
+    for (int c = 0; c < D / 8; ++c) {
+      Pack16 x, y;
+      x.u = live ? src[c] : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        f32x2_to_e4m3x2_two_term(v[c * 16 + 2 * j] * inv, v[c * 16 + 2 * j + 1] * inv, a.s[j], b.s[j]);
-      *reinterpret_cast<uint4*>(sQ + sw128_off(r, half * kApHalf + c * 16)) = a.u;
-      *reinterpret_cast<uint4*>(sQ + kTileBytes + sw128_off(r, half * kApHalf + c * 16)) = b.u;
+      for (int j = 0; j < 4; ++j) {
+        const __half2 h = __floats2half2_rn(bf16_to_f32(x.h[2 * j]) * mul, bf16_to_f32(x.h[2 * j + 1]) * mul);
+        y.w[j] = *reinterpret_cast<const uint32_t*>(&h);
+      }
+      *reinterpret_cast<uint4*>(sQ + sub * kApF16Bytes + (c >> 3) * kApBlk + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = y.u;
     }
     fence_proxy_async_smem();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_s = tmem_base;          // 2 x 128 columns
-  const uint32_t tmem_o = tmem_base + 256;    // 128 columns
+  const uint32_t tmem_base = *tmem_slot;      // score buffers at columns 0 and 128, accumulators at 256 and 384
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
+  if (warp == kApTma) {
+    // ------------------------------------------------------------------ TMA producer: K0, V0, K1, V1, ...
     if (elect_one()) {
-      const int ppt = kApTile / p.page;
-      for (int i = 0; i < ntiles; ++i) {
-        const int s = i % kApStages;
-        if (!wait_bar(&kv_empty[s], ((i / kApStages) & 1) ^ 1)) { report(p.status, kTimeoutStageEmpty, 31); *abort_flag = 1; break; }
-        mbar_expect_tx(&kv_full[s], 2 * kTileBytes + 2 * kApTile * sizeof(float));
+      const int ppt = kApTile / p.page, last_page = min(last_pos / p.page, p.max_blocks - 1);
+      bool ok = true;
+      for (int i = 0; i < n0 && ok; ++i) {
         const int page0 = (base + i * kApTile) / p.page;
-        for (int pg = 0; pg < ppt; ++pg) {
-          const int pi = min(page0 + pg, p.max_blocks - 1);
-          const int blk = p.block_table[pi];
-          const int r0 = (blk * p.hkv + kvh) * p.page;
-          tma_load_2d(sK + s * kTileBytes + pg * p.page * D, &tmK, 0, r0, &kv_full[s]);
-          tma_load_2d(sV + s * kTileBytes + pg * p.page * D, &tmV, 0, r0, &kv_full[s]);
-          bulk_load_1d(sKs + s * kApTile + pg * p.page, p.k_scale + r0, p.page * sizeof(float), &kv_full[s]);
-          bulk_load_1d(sVs + s * kApTile + pg * p.page, p.v_scale + r0, p.page * sizeof(float), &kv_full[s]);
+        for (int v = 0; v < 2; ++v) {      // item 2 i + v, raw slot v
+          if (!wait_bar(&raw_empty[v], (i & 1) ^ 1)) { report(p.status, kTimeoutStageEmpty, 31); *abort_flag = 1; ok = false; break; }
+          mbar_expect_tx(&raw_full[v], kApRawBytes + kApTile * sizeof(float));
+          for (int pg = 0; pg < ppt; ++pg) {
+            const int r0 = (p.block_table[min(page0 + pg, last_page)] * p.hkv + kvh) * p.page;
+            tma_load_2d(sRaw + v * kApRawBytes + pg * p.page * D, v ? &tmV : &tmK, 0, r0, &raw_full[v]);
+            bulk_load_1d(sScale + v * kApTile + pg * p.page, (v ? p.v_scale : p.k_scale) + r0, p.page * sizeof(float), &raw_full[v]);
+          }
         }
         if (*abort_flag) break;
       }
     }
-  } else if (warp == 1) {
+  } else if (warp == kApMma) {
     // ------------------------------------------------------------------ MMA issuer
     if (elect_one()) {
-      constexpr uint32_t idesc1 = umma_idesc_f8(128, 128, 0u, 0u);                 // Q (K-major) x K (K-major)
-      constexpr uint32_t idesc2 = umma_idesc_f8(128, 128, 0u, 0u) | (1u << 16);    // P (K-major) x V (MN-major B)
-      const uint32_t q_addr = smem_u32(sQ), p_addr = smem_u32(sP);
-      auto mma2 = [&](int j) {
-        const int s = j % kApStages;
-        const uint32_t v_addr = smem_u32(sV + s * kTileBytes);
-#pragma unroll
-        for (int term = 0; term < 2; ++term)
-#pragma unroll
-          for (int k = 0; k < 4; ++k)  // 32 tokens per step: P advances 32 bytes, V advances 32 token rows
-            umma_f8f6f4(tmem_o, umma_desc_sw128(p_addr + term * kTileBytes + k * 32), umma_desc_sw128(v_addr + k * 4096),
-                        idesc2, (term > 0 || k > 0) ? 1u : 0u);
-        umma_commit(o_full);
-        umma_commit(&kv_empty[s]);
-      };
+      constexpr uint32_t idesc1 = umma_idesc_f16(128, 128, 0u, 0u);                 // Q (K-major) x K (K-major)
+      constexpr uint32_t idesc2 = umma_idesc_f16(128, 128, 0u, 0u) | (1u << 16);    // P (tensor memory) x V (MN-major B)
+      const uint32_t q_addr = smem_u32(sQ), ring = smem_u32(sRing);
       bool ok = true;
-      for (int i = 0; i < ntiles && ok; ++i) {
-        const int s = i % kApStages, b = i & 1;
-        if (!wait_bar(&kv_full[s], (i / kApStages) & 1)) { report(p.status, kTimeoutTmaFull, 32); *abort_flag = 1; ok = false; break; }
+      auto wait = [&](uint64_t* bar, uint32_t parity, int code, int detail) {
+        if (!ok) return;
+        if (!wait_bar(bar, parity) || *abort_flag) { report(p.status, code, detail); *abort_flag = 1; ok = false; }
         tc_fence_after();
-        const uint32_t k_addr = smem_u32(sK + s * kTileBytes);
+      };
+      // item j of the ring: slot j % 4, phase j / 4; tile i's K is item 2 i, its V item 2 i + 1
+      auto wait_item = [&](int j) { wait(&ring_full[j & 3], (j >> 2) & 1, kTimeoutTmaFull, 32); };
+      auto scores = [&](int u, int buf, int i) {
+        const uint32_t k_addr = ring + ((2 * i) & 3) * kApF16Bytes, a_addr = q_addr + u * kApF16Bytes;
 #pragma unroll
-        for (int term = 0; term < 2; ++term)
+        for (int k = 0; k < 8; ++k)
+          umma_f16(tmem_base + buf * 128, umma_desc_sw128(a_addr + (k >> 2) * kApBlk + (k & 3) * 32),
+                   umma_desc_sw128(k_addr + (k >> 2) * kApBlk + (k & 3) * 32), idesc1, k > 0 ? 1u : 0u);
+        umma_commit(&s_full[buf]);
+      };
+      auto values = [&](int u, int buf, int i) {
+        const uint32_t v_addr = ring + ((2 * i + 1) & 3) * kApF16Bytes;
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_f8f6f4(tmem_s + b * 128, umma_desc_sw128(q_addr + term * kTileBytes + k * 32), umma_desc_sw128(k_addr + k * 32),
-                        idesc1, (term > 0 || k > 0) ? 1u : 0u);
-        umma_commit(&s_full[b]);
-        if (i > 0) {
-          if (!wait_bar(p_full, (i - 1) & 1)) { report(p.status, kTimeoutConvert, 33); *abort_flag = 1; ok = false; break; }
-          tc_fence_after();
-          mma2(i - 1);
-        }
-        if (*abort_flag) ok = false;
+        for (int k = 0; k < 8; ++k)      // 16 tokens per step: 8 columns of P, two 8-row groups of V
+          umma_f16_ts(tmem_base + 256 + u * 128, tmem_base + buf * 128 + 64 + k * 8, umma_desc_sw128_mn(v_addr + k * 2048, kApBlk), idesc2,
+                      (i > 0 || k > 0) ? 1u : 0u);
+        umma_commit(&o_full[u]);
+      };
+      wait_item(0);
+      if (ok) {
+        scores(0, 0, 0);
+        if (n1 > 0) scores(1, 1, 0);
+        umma_commit(&ring_empty[0]);
       }
-      if (ok && ntiles > 0) {
-        if (wait_bar(p_full, (ntiles - 1) & 1)) {
-          tc_fence_after();
-          mma2(ntiles - 1);
+      for (int i = 0; i < n0 && ok; ++i) {
+        if (dual) {
+          wait(&p_full[0], i & 1, kTimeoutConvert, 33);
+          wait_item(2 * i + 1);
+          if (ok) values(0, 0, i);
+          if (i + 1 < n0) {
+            wait_item(2 * i + 2);
+            if (ok) scores(0, 0, i + 1);
+          }
+          if (i < n1) {
+            wait(&p_full[1], i & 1, kTimeoutConvert, 34);
+            if (ok) values(1, 1, i);
+          }
+          if (ok) umma_commit(&ring_empty[(2 * i + 1) & 3]);
+          if (i + 1 < n1 && ok) scores(1, 1, i + 1);
+          if (i + 1 < n0 && ok) umma_commit(&ring_empty[(2 * i + 2) & 3]);
         } else {
-          report(p.status, kTimeoutConvert, 34);
-          *abort_flag = 1;
+          if (i + 1 < n0) {
+            wait_item(2 * i + 2);
+            if (ok) {
+              scores(0, (i + 1) & 1, i + 1);
+              umma_commit(&ring_empty[(2 * i + 2) & 3]);
+            }
+          }
+          wait(&p_full[i & 1], (i >> 1) & 1, kTimeoutConvert, 33);
+          wait_item(2 * i + 1);
+          if (ok) {
+            values(0, i & 1, i);
+            umma_commit(&ring_empty[(2 * i + 1) & 3]);
+          }
         }
       }
     }
-  } else {
-    // ------------------------------------------------------------------ softmax + accumulation (two threads per query row)
-    const int quad = warp & 3, half = (warp - 2) >> 2, cb = half * kApHalf;
-    const int r = quad * 32 + lane;
-    const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    const int my_pos = p.pos0 + row0 + r;
+  } else if (warp >= kApConv) {
+    // ------------------------------------------------------------------ expansion to f16: four warps for K, four for V, thread = token
+    const int v = (warp - kApConv) >> 2, t = (warp & 3) * 32 + lane;
+    bool ok = true;
+    for (int i = 0; i < n0; ++i) {
+      const int j = 2 * i + v, slot = j & 3;
+      bool okw = wait_bar(&raw_full[v], i & 1);
+      if (!okw) report(p.status, kTimeoutTmaFull, 35);
+      // exponent of the tile's largest scale, seen tokens only (others hold whatever the page held and become zeros)
+      const int t0 = base + i * kApTile;
+      const float4 s4 = *reinterpret_cast<const float4*>(sScale + v * kApTile + lane * 4);
+      float mx = t0 + lane * 4 <= last_pos ? s4.x : 0.f;
+      mx = fmaxf(mx, t0 + lane * 4 + 1 <= last_pos ? s4.y : 0.f);
+      mx = fmaxf(mx, t0 + lane * 4 + 2 <= last_pos ? s4.z : 0.f);
+      mx = fmaxf(mx, t0 + lane * 4 + 3 <= last_pos ? s4.w : 0.f);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      const int ex = max(min(static_cast<int>(__float_as_uint(mx) >> 23), 227), 27) - 127;      // (2^-100 .. 2^100)
+      const bool live = t0 + t <= last_pos;
+      const float sc = live ? sScale[v * kApTile + t] * exp2_of(-ex) : 0.f;
+      const __half2 hi = __float2half2_rn(sc);
+      const __half2 lo = __float2half2_rn(sc - __low2float(hi));
+      if (okw && !wait_bar(&ring_empty[slot], ((j >> 2) & 1) ^ 1)) { report(p.status, kTimeoutStageEmpty, 36); okw = false; }
+      if (!okw) *abort_flag = 1;
+      ok = __all_sync(0xffffffffu, okw && !*abort_flag);
+      if (!ok) break;
+      const unsigned char* raw = sRaw + v * kApRawBytes + t * 128;
+      unsigned char* dst = sRing + slot * kApF16Bytes + t * 128;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        Pack16 x, y[2];
+        x.u = *reinterpret_cast<const uint4*>(raw + ((c ^ (t & 7)) << 4));
+        if (!live) x.u = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const __half2 h = e4m3x2_to_h2(x.s[k]);
+          const __half2 r = __hfma2(h, hi, __hmul2(h, lo));
+          y[k >> 2].w[k & 3] = *reinterpret_cast<const uint32_t*>(&r);
+        }
+        unsigned char* blk = dst + (c >> 2) * kApBlk;
+        *reinterpret_cast<uint4*>(blk + (((c * 2) & 7) ^ (t & 7)) * 16) = y[0].u;
+        *reinterpret_cast<uint4*>(blk + (((c * 2 + 1) & 7) ^ (t & 7)) * 16) = y[1].u;
+      }
+      if (warp == kApConv + 4 * v && lane == 0) sExp[v * 4 + (i & 3)] = ex;
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) { mbar_arrive(&raw_empty[v]); mbar_arrive(&ring_full[slot]); }
+    }
+  } else if (sub == 0 || n1 > 0) {
+    // ------------------------------------------------------------------ softmax (thread = query row of unit `sub`)
+    const int r = (warp & 3) * 32 + lane, n = sub == 0 ? n0 : n1;
+    const uint32_t lanes = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    const uint32_t acc = lanes + 256 + sub * 128;
+    const int row = unit_row(unit0 + sub) + r;
+    const int my_pos = p.pos0 + row;
     const int my_first = (p.window > 0 && my_pos + 1 > p.window) ? my_pos + 1 - p.window : 0;
     const float sm = p.scale * 1.4426950408889634f * q_scale;
-    float m_run = -INFINITY, l_run = 0.f, inv_c_prev = 0.f;
-    float o[kApHalf];
-#pragma unroll
-    for (int j = 0; j < kApHalf; ++j) o[j] = 0.f;
+    float ref = -INFINITY, lsum = 0.f;
     bool ok = true;
-    for (int i = 0; i < ntiles; ++i) {
-      const int s = i % kApStages, b = i & 1;
-      const bool okw = ok && wait_bar(&s_full[b], (i >> 1) & 1);
-      if (!okw && ok) { report(p.status, kTimeoutAccum, 35); *abort_flag = 1; }
+    for (int i = 0; i < n; ++i) {
+      const int buf = dual ? sub : (i & 1), phase = dual ? (i & 1) : ((i >> 1) & 1), jv = 2 * i + 1;
+      // (V's exponent is wanted here; its tile is expanded long before this product needs it)
+      bool okw = wait_bar(&ring_full[jv & 3], (jv >> 2) & 1) && wait_bar(&s_full[buf], phase);
+      if (!okw) { report(p.status, kTimeoutAccum, 37); *abort_flag = 1; }
+      ok = __all_sync(0xffffffffu, okw && !*abort_flag);
+      if (!ok) break;
       tc_fence_after();
-      const float* ks = sKs + s * kApTile;
-      const float* vs = sVs + s * kApTile;
       const int t0 = base + i * kApTile;
-      // pass 1: maximum of this thread's scaled, masked scores (the scores are re-read from TMEM in pass 2 instead of being
-      // kept in registers next to the output accumulators)
+      const int ck = sExp[i & 3], cv = sExp[4 + (i & 3)];
+      const uint32_t ts = lanes + buf * 128;
+      // the accumulator of the tiles before, times the rows' corrections: all of their products must have landed
+      auto rescale = [&](float corr) {
+        if (i == 0) return;
+        // (two units: S of this tile was issued behind that product, its barrier is complete)
+        if (!__all_sync(0xffffffffu, wait_bar(&o_full[sub], (i - 1) & 1))) { report(p.status, kTimeoutAccum, 38); *abort_flag = 1; return; }
+        tc_fence_after();
+#pragma unroll 1
+        for (int c = 0; c < D; c += 16) {
+          uint32_t o[16];
+          tmem_ld_x16(acc + c, o);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * corr);
+          tmem_st_x16_async(acc + c, o);
+        }
+      };
       // warp-uniform choice: tcgen05.ld is .sync.aligned, every lane of the warp must take the same path
       const bool full = __all_sync(0xffffffffu, (t0 + kApTile - 1 <= my_pos) && (t0 >= my_first)) != 0;
-      mx[b * 2 * kApTile + half * kApTile + r] =
-          full ? tile_row_max<false>(tmem_s + b * 128 + lane_addr, ks, cb, t0, my_pos, my_first)
-               : tile_row_max<true>(tmem_s + b * 128 + lane_addr, ks, cb, t0, my_pos, my_first);
-      // tile-wide max of the V scales (fixes the range of the e4m3 P operand)
-      {
-        float vm = (half == 0 && t0 + r <= last_pos) ? vs[r] : 0.f;
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, off));
-        if (lane == 0) {
-          if (half == 0) red[b * 16 + quad] = vm;
-          red[b * 16 + 4 + half * 4 + quad] = (okw && !*abort_flag) ? 0.f : 1.f;
-        }
-      }
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      const float* rr = red + b * 16;
-      if (rr[4] + rr[5] + rr[6] + rr[7] + rr[8] + rr[9] + rr[10] + rr[11] != 0.f) { ok = false; break; }
-      const float vmax = fmaxf(fmaxf(rr[0], rr[1]), fmaxf(rr[2], rr[3]));
-      const float c_tile = vmax > 0.f ? 256.f / vmax : 0.f;
-      const float mt = fmaxf(mx[b * 2 * kApTile + r], mx[b * 2 * kApTile + kApTile + r]);
-      const float mn = fmaxf(m_run, mt * sm);   // sm > 0: scaling commutes with the maximum
-      const float corr = (m_run == -INFINITY) ? 0.f : fast_exp2(m_run - mn);
-      m_run = mn;
-      // the previous tile's PV product must be folded in before P is overwritten
-      if (i > 0) {
-        if (__all_sync(0xffffffffu, wait_bar(o_full, (i - 1) & 1))) {
-          tc_fence_after();
-#pragma unroll
-          for (int c0 = 0; c0 < kApHalf; c0 += 16) {
-            uint32_t raw[16];
-            tmem_ld_x16(tmem_o + lane_addr + cb + c0, raw);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) o[c0 + j] += __uint_as_float(raw[j]) * inv_c_prev;
-          }
-        } else {
-          report(p.status, kTimeoutAccum, 36);
-          *abort_flag = 1;
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < kApHalf; ++j) o[j] *= corr;
-      // pass 2: probabilities -> two e4m3 terms of P (row r of the A operand)
-      const float neg_m = (mn == -INFINITY) ? 0.f : -mn;
-      const float lsum = full ? tile_probs<false>(tmem_s + b * 128 + lane_addr, ks, vs, sP, r, sm, neg_m, c_tile, cb, t0, my_pos, my_first)
-                              : tile_probs<true>(tmem_s + b * 128 + lane_addr, ks, vs, sP, r, sm, neg_m, c_tile, cb, t0, my_pos, my_first);
-      l_run = l_run * corr + lsum;
-      inv_c_prev = c_tile > 0.f ? 1.f / c_tile : 0.f;
-      fence_proxy_async_smem();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
-    }
-    if (ok && !*abort_flag && ntiles > 0) {
-      if (__all_sync(0xffffffffu, wait_bar(o_full, (ntiles - 1) & 1))) {
-        tc_fence_after();
-#pragma unroll
-        for (int c0 = 0; c0 < kApHalf; c0 += 16) {
-          uint32_t raw[16];
-          tmem_ld_x16(tmem_o + lane_addr + cb + c0, raw);
-#pragma unroll
-          for (int j = 0; j < 16; ++j) o[c0 + j] += __uint_as_float(raw[j]) * inv_c_prev;
-        }
-      } else {
-        report(p.status, kTimeoutAccum, 37);
+      if (full) softmax_tile<false>(ts, t0, my_pos, my_first, sm * exp2_of(ck), cv, ref, lsum, rescale);
+      else softmax_tile<true>(ts, t0, my_pos, my_first, sm * exp2_of(ck), cv, ref, lsum, rescale);
+      // one unit: S of this tile says nothing of the product before it, whose phase must be behind us before the last one is waited for
+      if (!dual && i > 0 && i == n - 1 && !__all_sync(0xffffffffu, wait_bar(&o_full[sub], (i - 1) & 1))) {
+        report(p.status, kTimeoutAccum, 38);
         *abort_flag = 1;
       }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_full[buf]);
     }
-    // a row's probability mass: the two threads' sums, in the same order for both (the maxima of both parities are behind a barrier)
-    asm volatile("bar.sync 1, 256;" ::: "memory");
-    mx[half * kApTile + r] = l_run;
-    asm volatile("bar.sync 1, 256;" ::: "memory");
-    if (r < rows) {
-      const float l = mx[r] + mx[kApTile + r];
-      const float inv_l = l > 0.f ? 1.f / l : 0.f;
-      uint4* dst = reinterpret_cast<uint4*>(p.out + (static_cast<size_t>(row0 + r) * p.hq + head) * D + cb);
+    if (ok && !__all_sync(0xffffffffu, wait_bar(&o_full[sub], (n - 1) & 1))) { report(p.status, kTimeoutAccum, 39); *abort_flag = 1; ok = false; }
+    if (ok) {
+      tc_fence_after();
+      const int head = kvh * group + (unit0 + sub) % group;
+      const float inv_l = lsum > 0.f ? 1.f / lsum : 0.f;
+      uint4* dst = reinterpret_cast<uint4*>(p.out + (static_cast<size_t>(row) * p.hq + head) * D);
+#pragma unroll 1
+      for (int c = 0; c < D; c += 32) {
+        uint32_t o[32];
+        tmem_ld_x32(acc + c, o);
+        if (row < p.T) {
 #pragma unroll
-      for (int c = 0; c < kApHalf / 8; ++c) {
-        Pack16 x;
+          for (int k = 0; k < 4; ++k) {
+            Pack16 x;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) x.h[j] = f32_to_bf16(o[c * 8 + j] * inv_l);
-        dst[c] = x.u;
+            for (int j = 0; j < 8; ++j) x.h[j] = f32_to_bf16(__uint_as_float(o[k * 8 + j]) * inv_l);
+            dst[c / 8 + k] = x.u;
+          }
+        }
       }
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem_base, 512);
+  if (warp == kApMma) tmem_dealloc(tmem_base, 512);
 }
 
 }  // namespace dgpp
@@ -422,16 +482,22 @@ DGPP_API int dgpp_attn_prefill_tc(const void* q, int64_t q_stride, const void* k
     return -1;
   if (make_tmap_2d(&tV, v_cache, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, 128, total_rows, 128, 128, page, CU_TENSOR_MAP_SWIZZLE_128B))
     return -1;
-  constexpr size_t smem = 1024 + (4 + 2 * kApStages) * kApTile * 128 + 2 * kApStages * kApTile * 4 + 2 * 16 * 4 + 4 * kApTile * 4 +
-                          (2 * kApStages + 4) * 8 + 64;
+  constexpr size_t smem = attn_prefill_smem_bytes();
+  static_assert(smem <= 227 * 1024, "shared memory budget exceeded");
   static bool attr = false;
+  static int sms = 0;
   if (!attr) {
+    int dev = 0;
+    DGPP_CUDA_OK(cudaGetDevice(&dev));
+    DGPP_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     DGPP_CUDA_OK(cudaFuncSetAttribute(attn_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(smem)));
     attr = true;
   }
-  dim3 grid(hq, dgpp_ceil_div(T, kApTile));
-  attn_prefill_tc_kernel<<<grid, kApThreads, smem, st>>>(tK, tV, p);
+  // Two units per CTA share an expanded tile and fill each other's waits; where units are fewer than SMs, one each is the shorter span.
+  p.units = hq / hkv * dgpp_ceil_div(T, kApTile);
+  p.per_cta = static_cast<int64_t>(p.units) * hkv <= sms ? 1 : 2;
+  attn_prefill_tc_kernel<<<hkv * dgpp_ceil_div(p.units, p.per_cta), kApThreads, smem, st>>>(tK, tV, p);
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -213,6 +213,51 @@ def test_attn_prefill_tc(dev, hq, hkv, ctx, page, pos0, T):
     assert (out.float() - base.float()).abs().max().item() < 0.03
 
 
+@pytest.mark.parametrize("hq,hkv,ctx,page,pos0,T,window", [(4, 1, 1, 64, 0, 1, 0), (5, 1, 200, 64, 73, 127, 0), (4, 4, 300, 128, 172, 128, 0),
+                                                          (10, 2, 1500, 16, 1371, 129, 0), (40, 8, 1000, 64, 300, 513, 0),
+                                                          (48, 16, 700, 64, 0, 500, 200), (8, 2, 900, 32, 640, 260, 130)])
+def test_attn_prefill_tc_error(dev, hq, hkv, ctx, page, pos0, T, window):
+    """Edges of the row and token tiles, one unit per CTA and two (an odd number of units among them), windows, block scales that
+    differ by 2^16 inside a tile, and whatever bytes the unwritten rest of a page holds.  Q is exact, K, V and P are rounded
+    once to 11 bits and the output to 8: 2^-9 relative error of an output element, twice that allowed for the sums."""
+    from dgpp_b200.ops import core as ops
+
+    torch.manual_seed(6)
+    kv, qkv, pos, req = _filled_cache(dev, hq, hkv, ctx, page, slot=1)
+    cache, scale = kv.layers[0], 1.0 / math.sqrt(128)
+    tok = torch.arange(ctx, device=dev)
+    blk, off = kv.block_table[1].long()[tok // page], tok % page
+    written = torch.zeros(cache.k.shape[0], page, dtype=torch.bool, device=dev)
+    written[blk, off] = True
+    k0, v0 = cache.k_scale[blk, :, off].clone(), cache.v_scale[blk, :, off].clone()
+    cache.k.view(torch.uint8).masked_fill_(~written[:, None, :, None], 0x7F)          # e4m3 NaN
+    cache.v.view(torch.uint8).masked_fill_(~written[:, None, :, None], 0x7F)
+    cache.k_scale.masked_fill_(~written[:, None, :], float("nan"))
+    cache.v_scale.masked_fill_(~written[:, None, :], float("nan"))
+    spread = torch.exp2(-torch.randint(0, 17, (ctx, 1), device=dev).float())
+    cache.k_scale[blk, :, off] = k0 * spread.flip(0)
+    cache.v_scale[blk, :, off] = v0 * spread
+    q = qkv[pos0:pos0 + T]
+    out = ops.attn_prefill_tc(q, q.stride(0), cache, kv.block_table[1], pos0, hq, hkv, 128, scale, window=window)
+    torch.cuda.synchronize()
+    ops.check_status()
+    K = (cache.k[blk, :, off].view(torch.float8_e4m3fn).double() * cache.k_scale[blk, :, off].double().unsqueeze(-1)).permute(1, 2, 0)
+    V = (cache.v[blk, :, off].view(torch.float8_e4m3fn).double() * cache.v_scale[blk, :, off].double().unsqueeze(-1)).transpose(0, 1)
+    Q = q[:, :hq * 128].double().view(T, hkv, hq // hkv, 128).permute(1, 2, 0, 3)
+    S = torch.einsum("ghtd,gdc->ghtc", Q, K) * scale
+    mine = torch.arange(pos0, pos0 + T, device=dev)
+    seen = tok[None, :] <= mine[:, None]
+    if window:
+        seen &= tok[None, :] > mine[:, None] - window
+    want = torch.einsum("ghtc,gcd->ghtd", S.masked_fill(~seen, float("-inf")).softmax(-1), V).permute(2, 0, 1, 3).reshape(T, hq * 128)
+    err = (out.double() - want).view(T, hq, 128).norm(dim=-1) / want.view(T, hq, 128).norm(dim=-1)
+    assert err.max().item() < 2.0 ** -8, err.max().item()
+    # a row's bits do not depend on the chunk it came in
+    if T > 129:
+        part = ops.attn_prefill_tc(q[-129:], q.stride(0), cache, kv.block_table[1], pos0 + T - 129, hq, hkv, 128, scale, window=window)
+        assert torch.equal(part, out[-129:])
+
+
 @pytest.mark.parametrize("hq,hkv,ctx,page,splits", [(16, 2, 333, 64, 1), (16, 2, 1500, 64, 5), (8, 2, 700, 16, 2),
                                                     (4, 4, 130, 128, 3), (16, 2, 300, 64, 16)])
 def test_attn_decode_tc_head_dim_256(dev, hq, hkv, ctx, page, splits):
