@@ -25,6 +25,7 @@
 namespace dgpp {
 
 constexpr int kAqMaxThreads = 512;
+constexpr int kAqNormThreads = 128;   // of the norm's rows: who adds which squares is part of the per-layer kernel's contract
 constexpr int kAqMaxWarps = kAqMaxThreads / 32;
 constexpr int kAqMaxCluster = 8;
 constexpr int kAqSplitBlock = 4;      // attention splits whose partials are in flight at once
@@ -216,14 +217,18 @@ __global__ void __launch_bounds__(kAqMaxThreads) act_quant_cluster_kernel(Cluste
     st_async_f32x2(mapa_shared(smem_u32(&part[c * kAqMaxWarps + wid]), lane), ss, amax, mapa_shared(smem_u32(&arrived), lane));
   if (!wait_bar(&arrived, 0) && lane == 0) report(a.status, kTimeoutConvert, 61);
   {
-    const float4* pp = reinterpret_cast<const float4*>(part) + lane * 2;      // four pairs per lane
+    const float4* pp = reinterpret_cast<const float4*>(part) + lane * 2;      // four pairs per lane, in order of CTA and warp
     const float4 x = pp[0], y = pp[1];
-    ss = (x.x + x.z) + (y.x + y.z);
     amax = fmaxf(fmaxf(x.y, x.w), fmaxf(y.y, y.w));
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      if (MODE == 2) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    if (MODE == 2) {
+      // the norm's rows have at most four warps per CTA: lane 4 c holds those of CTA c; warps, then CTAs in ascending order (the sum
+      // that the per-layer kernel forms)
+      const float r = x.x + x.z + y.x + y.z;
+      ss = 0.f;
+#pragma unroll
+      for (int i = 0; i < kAqMaxCluster; ++i) ss += __shfl_sync(0xffffffffu, r, i * (kAqMaxWarps / 4));
     }
   }
   float rstd = 0.f;
@@ -302,8 +307,8 @@ static int launch_cluster(const ClusterQuantArgs& a, cudaStream_t st) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(a.cl, a.T, 1);
-  const int vecs = a.K / a.cl / 8;      // one thread each, as far as a CTA goes
-  cfg.blockDim = dim3(vecs < kAqMaxThreads ? (vecs + 31) / 32 * 32 : kAqMaxThreads, 1, 1);
+  const int vecs = a.K / a.cl / 8, most = MODE == 2 ? kAqNormThreads : kAqMaxThreads;      // one thread each, as far as a CTA goes
+  cfg.blockDim = dim3(vecs < most ? (vecs + 31) / 32 * 32 : most, 1, 1);
   cfg.dynamicSmemBytes = static_cast<size_t>(a.K / a.cl) * 2;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
