@@ -16,10 +16,12 @@
 // tiles of a chunk stay in L2.
 //
 // What bounds it: at wide tiles the tensor pipe (2048 x 34816 x 5120: 474 us = 1540 TFLOP/s, 0.91 of the measured cuBLAS burst rate;
-// the single-CTA kernel 1216 us), at narrow ones the conversion (37 x 34816 x 5120: 40 us; a set's block takes some 1400 cycles, half
-// of them waits).  The weights have a producer of their own: behind the activations' ring, which ends 512 K ahead of the MMAs,
-// their loads were a round trip to HBM on every stage's way (converters waited 780 of 1900 cycles; 37 x 34816 x 5120 50 us, 256 experts'
-// gate-up and down products of 64 rows each 479 us, 392 so).  2048 x 5120 x 17408: 266 us, 173 x 5120 x 5120: 25 us.
+// the single-CTA kernel 1216 us), at narrow ones the conversion: 345 cycles per K = 64 block up to 128 tokens, 208 of them the integer
+// pipe's.  A set of converter warps has a stage of the ring to itself and converts its two blocks behind one wait for raw weights and one
+// for the stage's columns (a block at a time, four sets to a raw stage: 480 cycles, half of them waits; 37 x 34816 x 5120 40 us, 36 so).
+// The weights have a producer of their own: behind the activations' ring, which ends 512 K ahead of the MMAs,
+// their loads were a round trip to HBM on every stage's way (converters waited 780 of 1900 cycles; 37 x 34816 x 5120 50 us).
+// 2048 x 5120 x 17408: 266 us, 173 x 5120 x 5120: 20 us.
 //
 // Handshakes (all waits bounded, expiry -> status code, everything unwinds, TMEM freed):
 //   own CTA:          raw_full / raw_empty (TMA -> converters), acc_full (MMA -> epilogue);
@@ -29,8 +31,8 @@
 //                     tile) have completed; the producers and the converters both wait for `done`.
 // (Arrivals on the other CTA's barriers release at CTA scope: what they order is tensor memory, by the tcgen05 fences; a
 // cluster-scope release took 1100 cycles per arrival, three times a block's MMAs.)
-// Warp roles (896 threads): warp 0 MMA issuer (first CTA) and TMEM owner, 1 TMA producer of the activations, 2 of the weights, 4..19 converters (four sets take turns
-// at the K = 64 blocks), 20..27 epilogue.
+// Warp roles (896 threads): warp 0 MMA issuer (first CTA) and TMEM owner, 1 TMA producer of the activations, 2 of the weights, 4..19 converters (four sets, one
+// per stage of the ring), 20..27 epilogue.
 // (reference counterpart: src/kernels/fp4w_gemm.cu, the W4A16 prefill GEMM.)
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -47,7 +49,7 @@ namespace dgpp {
 constexpr int kPrBM = 128;          // weight rows per CTA
 constexpr int kPrBK = 64;
 constexpr int kPrMaxBN = 256;       // tokens per pair tile = MMA N, at most
-constexpr int kPrSets = 4;            // converter sets of four warps; set s takes block s of every 256 K
+constexpr int kPrSets = 4;            // converter sets of four warps; set s has stage s of the ring, two K = 64 blocks at a time
 constexpr int kPrMma = 0, kPrTma = 1, kPrRaw = 2, kPrConv = 4, kPrEpi = kPrConv + kPrSets * 4;   // first warp of each role
 constexpr int kPrEpiWarps = 8;        // two per lane quadrant, taking turns at 16 columns
 constexpr int kPrThreads = (kPrEpi + kPrEpiWarps) * 32;
@@ -143,8 +145,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA,   // packed weights
   const int num_kb = p.K / kPrBK;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kPrStages; ++i) { mbar_init(&full[i], 1 + 2 * 2 * 4); mbar_init(&done[i], 1); }
-    for (int i = 0; i < kPrSR; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], kPrSets * 4); }
+    for (int i = 0; i < kPrStages; ++i) { mbar_init(&full[i], 1 + 2 * 4); mbar_init(&done[i], 1); }
+    for (int i = 0; i < kPrSR; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 2 * 4); }
     mbar_init(acc_full, 1);
     mbar_init(acc_empty, 2 * kPrEpiWarps);
     *abort_flag = 0;
@@ -270,53 +272,70 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA,   // packed weights
     const int set = (warp - kPrConv) >> 2, q = warp & 3, row = q * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     const float k112 = 5.192296858534828e33f;
-    int it = set;              // this set's next k64 block, counted over all units
+    int stg = 0;               // stages (128 K) of the units so far
     bool ok = true;
     for (int u = first_unit; u < p.units && ok; u += unit_step) {
       int n0, nc, m0, split, kb0, nk;
       float alpha;
       if (!unit_at(u, n0, nc, m0, split, kb0, nk, alpha)) continue;
-      // MXFP4: two scale bytes per block by plain loads, one block of this set ahead
+      const int nstg = nk / 2;
+      const int first = (set - stg) & (kPrStages - 1);      // this set's first stage of the unit
+      // MXFP4: four scale bytes per stage by plain loads, one stage of this set ahead
       const uint8_t* sf_row = nullptr;
       uint32_t e8 = 0;
       if (WMODE == 3) {
         sf_row = p.sf_plain + static_cast<size_t>(min(n0 + row, p.N - 1)) * (p.K / 32) + kb0 * 2;
-        e8 = *reinterpret_cast<const uint16_t*>(sf_row + set * 2);
+        if (first < nstg) e8 = *reinterpret_cast<const uint32_t*>(sf_row + first * 4);
       }
-      for (int i = set; i < nk; i += kPrSets, it += kPrSets) {
-        const int r = it >> 2, sr = r % kPrSR, stg = it >> 1, sl = stg % kPrStages;
+      for (int i = first; i < nstg; i += kPrStages) {
+        const int at = stg + i, r = at >> 1, sr = r % kPrSR, half = at & 1;      // (units begin with a raw stage: both counts are even there)
         bool okw = wait_bar(&raw_full[sr], (r / kPrSR) & 1);
         const unsigned char* raw = sRaw + sr * kPrStageRaw + row * 128;
-        Pack16 w0, w1;
-        w0.u = *reinterpret_cast<const uint4*>(raw + (((set * 2) ^ (row & 7)) << 4));
-        w1.u = *reinterpret_cast<const uint4*>(raw + (((set * 2 + 1) ^ (row & 7)) << 4));
-        bf162 s[4];
+        Pack16 w[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) w[c].u = *reinterpret_cast<const uint4*>(raw + (((half * 4 + c) ^ (row & 7)) << 4));
+        uint32_t four[2] = {0u, 0u};
         if (WMODE == 1) {
-          const uint32_t four = *reinterpret_cast<const uint32_t*>(
-              sSf + sr * kPrStageSf + (GROUPED ? set * 512 + lane * 16 + q * 4 : row * 16 + set * 4));
-          const float2 lo = __half22float2(e4m3x2_to_h2(static_cast<uint16_t>(four & 0xFFFFu)));
-          const float2 hi = __half22float2(e4m3x2_to_h2(static_cast<uint16_t>(four >> 16)));
-          s[0] = __float2bfloat162_rn(lo.x * k112); s[1] = __float2bfloat162_rn(lo.y * k112);
-          s[2] = __float2bfloat162_rn(hi.x * k112); s[3] = __float2bfloat162_rn(hi.y * k112);
-        } else {
-          s[0] = s[1] = __float2bfloat162_rn(e8m0_to_f32(static_cast<uint8_t>(e8 & 255u)) * k112);
-          s[2] = s[3] = __float2bfloat162_rn(e8m0_to_f32(static_cast<uint8_t>(e8 >> 8)) * k112);
-          if (i + kPrSets < nk) e8 = *reinterpret_cast<const uint16_t*>(sf_row + (i + kPrSets) * 2);
+#pragma unroll
+          for (int b = 0; b < 2; ++b)
+            four[b] = *reinterpret_cast<const uint32_t*>(
+                sSf + sr * kPrStageSf + (GROUPED ? (half * 2 + b) * 512 + lane * 16 + q * 4 : row * 16 + (half * 2 + b) * 4));
         }
-        uint32_t o[32];
-        expand_e2m1x64(w0, w1, s, o);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&raw_empty[sr]);   // this warp is done with the raw stage
-        if (okw) okw = wait_bar(&done[sl], ((stg / kPrStages) & 1) ^ 1);   // the stage's columns are free
-        if (!okw) { report(p.status, kTimeoutTmaFull, 26); *abort_flag = 1; }
-        ok = __all_sync(0xffffffffu, okw && !*abort_flag);
+        const uint32_t e8_now = e8;
+        if (WMODE == 3 && i + kPrStages < nstg) e8 = *reinterpret_cast<const uint32_t*>(sf_row + (i + kPrStages) * 4);
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          bf162 s[4];
+          if (WMODE == 1) {
+            const float2 lo = __half22float2(e4m3x2_to_h2(static_cast<uint16_t>(four[b] & 0xFFFFu)));
+            const float2 hi = __half22float2(e4m3x2_to_h2(static_cast<uint16_t>(four[b] >> 16)));
+            s[0] = __float2bfloat162_rn(lo.x * k112); s[1] = __float2bfloat162_rn(lo.y * k112);
+            s[2] = __float2bfloat162_rn(hi.x * k112); s[3] = __float2bfloat162_rn(hi.y * k112);
+          } else {
+            const uint32_t e = e8_now >> (16 * b);
+            s[0] = s[1] = __float2bfloat162_rn(e8m0_to_f32(static_cast<uint8_t>(e & 255u)) * k112);
+            s[2] = s[3] = __float2bfloat162_rn(e8m0_to_f32(static_cast<uint8_t>((e >> 8) & 255u)) * k112);
+          }
+          uint32_t o[32];
+          expand_e2m1x64(w[2 * b], w[2 * b + 1], s, o);
+          if (b == 0) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&raw_empty[sr]);   // this warp is done with its half of the raw stage
+            if (okw) okw = wait_bar(&done[set], ((at / kPrStages) & 1) ^ 1);   // the stage's columns are free
+            if (!okw) { report(p.status, kTimeoutTmaFull, 26); *abort_flag = 1; }
+            ok = __all_sync(0xffffffffu, okw && !*abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+          }
+          tmem_st_x32_async(tmem_base + kPrColA + set * 64 + b * 32 + lane_addr, o);
+        }
         if (!ok) break;
-        tc_fence_after();
-        tmem_st_x32(tmem_base + kPrColA + sl * 64 + (it & 1) * 32 + lane_addr, o);
+        tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive_pair(mapa_shared(smem_u32(&full[sl]), 0u));
+        if (lane == 0) mbar_arrive_pair(mapa_shared(smem_u32(&full[set]), 0u));
       }
+      stg += nstg;
     }
   } else if (warp >= kPrEpi) {
     // ------------------------------------------------------------------ epilogue: own 128 rows x bn tokens
@@ -476,7 +495,7 @@ static int pair_slots(int* slots) {
   if (!cached) {
     auto kern = gemm_tc_pair_kernel<WMODE, GROUPED>;
     constexpr size_t smem = pair_smem_bytes();
-    static_assert(kPrSets == 4, "a set's blocks are the same quarter of every raw stage");
+    static_assert(kPrSets == kPrStages && (kPrStages & (kPrStages - 1)) == 0, "a set has one stage of the ring");
     static_assert(smem <= 227 * 1024, "shared memory budget exceeded");
     DGPP_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     cudaLaunchConfig_t cfg = {};
