@@ -497,7 +497,7 @@ DGPP_API int dgpp_attn_prefill_tc(const void* q, int64_t q_stride, const void* k
   // Two units per CTA share an expanded tile and fill each other's waits; where units are fewer than SMs, one each is the shorter span.
   p.units = hq / hkv * dgpp_ceil_div(T, kApTile);
   p.per_cta = static_cast<int64_t>(p.units) * hkv <= sms ? 1 : 2;
-  attn_prefill_tc_kernel<<<hkv * dgpp_ceil_div(p.units, p.per_cta), kApThreads, smem, st>>>(tK, tV, p);
+  DGPP_CUDA_OK(launch_early(attn_prefill_tc_kernel, hkv * dgpp_ceil_div(p.units, p.per_cta), kApThreads, smem, st, tK, tV, p));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }

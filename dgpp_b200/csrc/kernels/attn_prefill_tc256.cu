@@ -456,7 +456,7 @@ DGPP_API int dgpp_attn_prefill_tc256(const void* q, int64_t q_stride, const void
     attr = true;
   }
   dim3 grid(dgpp_ceil_div(T, kA2Tile), hq);
-  attn_prefill_tc256_kernel<<<grid, kA2Threads, smem, st>>>(tK, tV, p);
+  DGPP_CUDA_OK(launch_early(attn_prefill_tc256_kernel, grid, kA2Threads, smem, st, tK, tV, p));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -299,9 +299,9 @@ DGPP_API int dgpp_embed_gather(const void* ids, const void* table, void* out, in
                                cudaStream_t st) {
   DGPP_REQUIRE(hidden % 8 == 0, "embed_gather: hidden %d must be a multiple of 8", hidden);
   if (rows == 0) return 0;
-  embed_gather_kernel<<<rows, kRowThreads, 0, st>>>(static_cast<const int32_t*>(ids),
+  DGPP_CUDA_OK(launch_early(embed_gather_kernel, rows, kRowThreads, 0, st, static_cast<const int32_t*>(ids),
                                                    static_cast<const bf16*>(table), static_cast<bf16*>(out), hidden,
-                                                   vocab);
+                                                   vocab));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -319,18 +319,18 @@ DGPP_API int dgpp_rmsnorm(const void* resid, const void* delta, const void* w, v
       cudaFuncSetAttribute(rmsnorm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
       attr_set = true;
     }
-    rmsnorm_kernel<true><<<rows, kRowThreads, smem, st>>>(
+    DGPP_CUDA_OK(launch_early(rmsnorm_kernel<true>, rows, kRowThreads, smem, st, 
         static_cast<const bf16*>(resid), static_cast<const bf16*>(delta), static_cast<const bf16*>(w),
-        static_cast<bf16*>(resid_out), static_cast<bf16*>(out), hidden, eps, one_plus_w);
+        static_cast<bf16*>(resid_out), static_cast<bf16*>(out), hidden, eps, one_plus_w));
   } else {
     static bool attr_set2 = false;
     if (!attr_set2) {
       cudaFuncSetAttribute(rmsnorm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
       attr_set2 = true;
     }
-    rmsnorm_kernel<false><<<rows, kRowThreads, smem, st>>>(static_cast<const bf16*>(resid), nullptr,
+    DGPP_CUDA_OK(launch_early(rmsnorm_kernel<false>, rows, kRowThreads, smem, st, static_cast<const bf16*>(resid), nullptr,
                                                           static_cast<const bf16*>(w), nullptr,
-                                                          static_cast<bf16*>(out), hidden, eps, one_plus_w);
+                                                          static_cast<bf16*>(out), hidden, eps, one_plus_w));
   }
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
@@ -347,8 +347,8 @@ DGPP_API int dgpp_swiglu(const void* gate_up, void* out, int rows, int inter, fl
   if (rows == 0) return 0;
   const dim3 block = swiglu_block(inter);
   dim3 grid(dgpp_ceil_div(inter / 8, block.x), dgpp_ceil_div(rows, block.y));
-  swiglu_kernel<<<grid, block, 0, st>>>(static_cast<const bf16*>(gate_up), static_cast<bf16*>(out), inter,
-                                        limit, alpha, nullptr, rows);
+  DGPP_CUDA_OK(launch_early(swiglu_kernel, grid, block, 0, st, static_cast<const bf16*>(gate_up), static_cast<bf16*>(out), inter,
+                                        limit, alpha, nullptr, rows));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -361,8 +361,8 @@ DGPP_API int dgpp_swiglu_tiles(const void* gate_up, void* out, const void* tiles
   if (n_tiles <= 0) return 0;
   const dim3 block = swiglu_block(inter);
   dim3 grid(dgpp_ceil_div(inter / 8, block.x), dgpp_ceil_div(bn, block.y), n_tiles);
-  swiglu_kernel<<<grid, block, 0, st>>>(static_cast<const bf16*>(gate_up), static_cast<bf16*>(out), inter, limit, alpha,
-                                        static_cast<const int32_t*>(tiles), bn);
+  DGPP_CUDA_OK(launch_early(swiglu_kernel, grid, block, 0, st, static_cast<const bf16*>(gate_up), static_cast<bf16*>(out), inter, limit, alpha,
+                                        static_cast<const int32_t*>(tiles), bn));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -393,7 +393,7 @@ DGPP_API int dgpp_copy_bytes(const void* src, void* dst, int64_t bytes, cudaStre
   if (bytes == 0) return 0;
   const int64_t nvec = bytes / 16;
   int blocks = static_cast<int>(nvec / 256 < 1 ? 1 : (nvec / 256 > 1184 ? 1184 : nvec / 256));
-  copy_rows_kernel<<<blocks, 256, 0, st>>>(static_cast<const uint4*>(src), static_cast<uint4*>(dst), nvec);
+  DGPP_CUDA_OK(launch_early(copy_rows_kernel, blocks, 256, 0, st, static_cast<const uint4*>(src), static_cast<uint4*>(dst), nvec));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -402,8 +402,8 @@ DGPP_API int dgpp_add_bf16(const void* a, const void* b, void* y, int64_t n, cud
   DGPP_REQUIRE(n % 8 == 0, "add: n must be a multiple of 8");
   if (n == 0) return 0;
   const int64_t n8 = n / 8;
-  add_kernel<<<static_cast<int>(dgpp_ceil_div64(n8, 256)), 256, 0, st>>>(
-      static_cast<const bf16*>(a), static_cast<const bf16*>(b), static_cast<bf16*>(y), n8);
+  DGPP_CUDA_OK(launch_early(add_kernel, static_cast<int>(dgpp_ceil_div64(n8, 256)), 256, 0, st, 
+      static_cast<const bf16*>(a), static_cast<const bf16*>(b), static_cast<bf16*>(y), n8));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -373,20 +373,20 @@ static int gdn_recurrent_launch(const void* q, int64_t q_stride, const void* k, 
   a.seg = seg; a.snap = static_cast<float*>(snap);
   a.gate_k = static_cast<const bf16*>(gate_k); a.gate_stride = gate_stride; a.lower_bound = lower_bound;
   dim3 pgrid(T, hk + 1 + (gate_k ? hv : 0));
-  if (dk == 64) gdn_prep_kernel<64><<<pgrid, 64, 0, st>>>(a);
-  else if (dk == 128) gdn_prep_kernel<128><<<pgrid, 128, 0, st>>>(a);
-  else gdn_prep_kernel<256><<<pgrid, 256, 0, st>>>(a);
+  if (dk == 64) DGPP_CUDA_OK(launch_early(gdn_prep_kernel<64>, pgrid, 64, 0, st, a));
+  else if (dk == 128) DGPP_CUDA_OK(launch_early(gdn_prep_kernel<128>, pgrid, 128, 0, st, a));
+  else DGPP_CUDA_OK(launch_early(gdn_prep_kernel<256>, pgrid, 256, 0, st, a));
   DGPP_CUDA_OK(cudaGetLastError());
   dim3 grid(dv / kGdnCols, hv, seg > 0 ? T / seg : (sequential ? 1 : T));
   if (gate_k) {
-    if (dk == 64) gdn_recurrent_kernel<64, true><<<grid, kGdnThreads, 0, st>>>(a);
-    else gdn_recurrent_kernel<128, true><<<grid, kGdnThreads, 0, st>>>(a);
+    if (dk == 64) DGPP_CUDA_OK(launch_early(gdn_recurrent_kernel<64, true>, grid, kGdnThreads, 0, st, a));
+    else DGPP_CUDA_OK(launch_early(gdn_recurrent_kernel<128, true>, grid, kGdnThreads, 0, st, a));
     DGPP_CUDA_OK(cudaGetLastError());
     return 0;
   }
-  if (dk == 64) gdn_recurrent_kernel<64><<<grid, kGdnThreads, 0, st>>>(a);
-  else if (dk == 128) gdn_recurrent_kernel<128><<<grid, kGdnThreads, 0, st>>>(a);
-  else gdn_recurrent_kernel<256><<<grid, kGdnThreads, 0, st>>>(a);
+  if (dk == 64) DGPP_CUDA_OK(launch_early(gdn_recurrent_kernel<64>, grid, kGdnThreads, 0, st, a));
+  else if (dk == 128) DGPP_CUDA_OK(launch_early(gdn_recurrent_kernel<128>, grid, kGdnThreads, 0, st, a));
+  else DGPP_CUDA_OK(launch_early(gdn_recurrent_kernel<256>, grid, kGdnThreads, 0, st, a));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -442,9 +442,9 @@ DGPP_API int dgpp_gdn_prep(const void* q, int64_t q_stride, const void* k, int64
   a.prep = static_cast<float*>(prep);
   a.T = T; a.hk = hk; a.hv = hv; a.dk = dk;
   dim3 pgrid(T, hk + 1);
-  if (dk == 64) gdn_prep_kernel<64><<<pgrid, 64, 0, st>>>(a);
-  else if (dk == 128) gdn_prep_kernel<128><<<pgrid, 128, 0, st>>>(a);
-  else gdn_prep_kernel<256><<<pgrid, 256, 0, st>>>(a);
+  if (dk == 64) DGPP_CUDA_OK(launch_early(gdn_prep_kernel<64>, pgrid, 64, 0, st, a));
+  else if (dk == 128) DGPP_CUDA_OK(launch_early(gdn_prep_kernel<128>, pgrid, 128, 0, st, a));
+  else DGPP_CUDA_OK(launch_early(gdn_prep_kernel<256>, pgrid, 256, 0, st, a));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -466,18 +466,18 @@ static int gdn_conv_launch(const void* x, int64_t x_stride, const void* w, const
   a.T = T; a.C = C; a.W = W; a.sequential = sequential;
   a.seg = seg; a.snap = static_cast<float*>(snap);
   if (!sequential && seg == 0 && !snap) {       // batched decode rows: one kernel
-    gdn_conv_decode_kernel<<<dim3(dgpp_ceil_div(C, 256), T), 256, 0, st>>>(a);
+    DGPP_CUDA_OK(launch_early(gdn_conv_decode_kernel, dim3(dgpp_ceil_div(C, 256), T), 256, 0, st, a));
     DGPP_CUDA_OK(cudaGetLastError());
     return 0;
   }
   const bool pairs = C % 2 == 0 && x_stride % 2 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 3) == 0;
   if (sequential && seg == 0 && W == 4 && pairs && static_cast<int64_t>(T) * C >= kConvRunInputs)
-    gdn_conv_run_kernel<<<dim3(dgpp_ceil_div(C, 512), dgpp_ceil_div(T, kConvRun)), 256, 0, st>>>(a);
+    DGPP_CUDA_OK(launch_early(gdn_conv_run_kernel, dim3(dgpp_ceil_div(C, 512), dgpp_ceil_div(T, kConvRun)), 256, 0, st, a));
   else
-    gdn_conv_kernel<<<dim3(dgpp_ceil_div(C, 256), T), 256, 0, st>>>(a);
+    DGPP_CUDA_OK(launch_early(gdn_conv_kernel, dim3(dgpp_ceil_div(C, 256), T), 256, 0, st, a));
   DGPP_CUDA_OK(cudaGetLastError());
   if (W > 1) {
-    gdn_conv_state_kernel<<<dim3(dgpp_ceil_div(C, 256), seg > 0 ? T / seg : (sequential ? 1 : T)), 256, 0, st>>>(a);
+    DGPP_CUDA_OK(launch_early(gdn_conv_state_kernel, dim3(dgpp_ceil_div(C, 256), seg > 0 ? T / seg : (sequential ? 1 : T)), 256, 0, st, a));
     DGPP_CUDA_OK(cudaGetLastError());
   }
   return 0;
@@ -499,9 +499,9 @@ DGPP_API int dgpp_gated_rmsnorm(const void* o, const void* z, int64_t z_stride, 
                                 int heads, int d, float eps, cudaStream_t st) {
   if (rows == 0) return 0;
   const int warps = rows * heads;
-  gated_rmsnorm_kernel<<<dgpp_ceil_div(warps * 32, 256), 256, 0, st>>>(
+  DGPP_CUDA_OK(launch_early(gated_rmsnorm_kernel, dgpp_ceil_div(warps * 32, 256), 256, 0, st, 
       static_cast<const bf16*>(o), static_cast<const bf16*>(z), z_stride, static_cast<const bf16*>(w),
-      static_cast<bf16*>(out), rows, heads, d, eps);
+      static_cast<bf16*>(out), rows, heads, d, eps));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }

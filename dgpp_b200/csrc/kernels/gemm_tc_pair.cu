@@ -73,6 +73,7 @@ struct PairParams {
   int T, N, K, ldc;
   int bn, m_tiles, units, splits, kb_per_split;
   int width;                 // columns of a tile's MMAs: bn, rounded up to a multiple of 32
+  int preload;               // weights may be read before the preceding grid has finished
   int vec;                   // rows of `out` (and `resid`) can be accessed as 16-byte vectors
   // Grouped form (experts): the matrices are stacked along N ([experts * N, K], N a multiple of 256); token tile t holds rows
   // t * bn .. of x and `out` and belongs to matrix groups[t] (negative: nothing to do).  The block scales come in the
@@ -166,8 +167,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA,   // packed weights
   cluster_barrier();      // the other CTA's barriers exist before anything arrives on them from here
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // (weights do not depend on the grid before: their first stages are requested in front of the wait)
-  if (GROUPED || warp != kPrRaw) pdl_wait();
+  // (in a captured pass no kernel writes weights: their first stages are requested in front of the wait)
+  const bool preload = !GROUPED && p.preload;
+  if (!preload || warp != kPrRaw) pdl_wait();
 
   // Unit u: k64 blocks [kb0, kb0 + nk), a multiple of four; first weight row (n0 in the tensor map, nc as a column of the output) and
   // first token of the tile.  False: nothing to do.
@@ -195,7 +197,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA,   // packed weights
   if (warp == kPrRaw) {
     // ------------------------------------------------------------------ TMA producer of the weights (own rows), up to 1024 K ahead
     if (elect_one()) {
-      bool ok = true, waited = GROUPED;
+      bool ok = true, waited = !preload;
       int r = 0;
       for (int u = first_unit; u < p.units && ok; u += unit_step) {
         int n0, nc, m0, split, kb0, nk;
@@ -554,9 +556,10 @@ static void pair_shape(int T, int N, int K, int slots, int max_splits, int* bn_o
 }
 
 template <int WMODE, bool GROUPED>
-static int launch_pair(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tSf, const PairParams& p, int slots, cudaStream_t st) {
+static int launch_pair(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tSf, PairParams& p, int slots, cudaStream_t st) {
+  p.preload = stream_captures(st);
   const int pairs = p.units < slots ? p.units : slots;
-  gemm_tc_pair_kernel<WMODE, GROUPED><<<2 * pairs, kPrThreads, pair_smem_bytes(), st>>>(tA, tB, tSf, p);
+  DGPP_CUDA_OK(launch_early(gemm_tc_pair_kernel<WMODE, GROUPED>, 2 * pairs, kPrThreads, pair_smem_bytes(), st, tA, tB, tSf, p));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }

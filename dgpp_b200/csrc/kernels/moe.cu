@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(128) moe_combine_push_kernel(const bf16* __res
 
 static int launch_select(const RouterArgs& a, cudaStream_t st) {
   auto kern = a.E <= 32 ? moe_router_select_kernel<1> : a.E <= 128 ? moe_router_select_kernel<4> : moe_router_select_kernel<kMoeMaxExperts / 32>;
-  kern<<<a.T, kRouterThreads, 0, st>>>(a);
+  DGPP_CUDA_OK(launch_early(kern, a.T, kRouterThreads, 0, st, a));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -413,8 +413,8 @@ DGPP_API int dgpp_moe_route(const void* x, int64_t x_stride, const void* gate, c
   const dim3 grid(dgpp_ceil_div(E, kRouterThreads / 32), dgpp_ceil_div(T, kRouterRowsPerCta));
   const dim3 tiles(dgpp_ceil_div(E, kRouterTileE * kRouterThreads / 32), grid.y);
   // (two CTAs per SM take the tiles: below one for each, the finer split is the faster one)
-  if (tiles.x * tiles.y >= 296) moe_router_logits_tile_kernel<<<tiles, kRouterThreads, 0, st>>>(a);
-  else moe_router_logits_kernel<<<grid, kRouterThreads, 0, st>>>(a);
+  if (tiles.x * tiles.y >= 296) DGPP_CUDA_OK(launch_early(moe_router_logits_tile_kernel, tiles, kRouterThreads, 0, st, a));
+  else DGPP_CUDA_OK(launch_early(moe_router_logits_kernel, grid, kRouterThreads, 0, st, a));
   DGPP_CUDA_OK(cudaGetLastError());
   return launch_select(a, st);
 }
@@ -440,9 +440,9 @@ DGPP_API int dgpp_moe_select(const void* logits, int64_t logits_stride, const vo
 DGPP_API int dgpp_moe_active(const void* ids, int T, int k, int E, int slots, void* list, void* slot_of, void* n_active,
                              int e_begin, int e_end, cudaStream_t st) {
   DGPP_REQUIRE(E >= 1 && E <= kMoeMaxExperts && slots >= 1, "moe_active: bad sizes");
-  moe_active_kernel<<<1, 512, 0, st>>>(static_cast<const int32_t*>(ids), T, k, E, slots, static_cast<int32_t*>(list),
+  DGPP_CUDA_OK(launch_early(moe_active_kernel, 1, 512, 0, st, static_cast<const int32_t*>(ids), T, k, E, slots, static_cast<int32_t*>(list),
                                        static_cast<int32_t*>(slot_of), static_cast<int32_t*>(n_active), e_begin,
-                                       e_end > 0 ? e_end : E);
+                                       e_end > 0 ? e_end : E));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -452,10 +452,10 @@ DGPP_API int dgpp_moe_combine(const void* y, const void* shared, const void* ids
   DGPP_REQUIRE(H % 8 == 0, "moe_combine: hidden %d must be a multiple of 8", H);
   if (T == 0) return 0;
   dim3 grid(dgpp_ceil_div(H / 8, 256), T);
-  moe_combine_kernel<<<grid, 256, 0, st>>>(static_cast<const bf16*>(y), static_cast<const bf16*>(shared),
+  DGPP_CUDA_OK(launch_early(moe_combine_kernel, grid, 256, 0, st, static_cast<const bf16*>(y), static_cast<const bf16*>(shared),
                                            static_cast<const int32_t*>(ids), static_cast<const float*>(w),
                                            static_cast<const int32_t*>(slot_of), static_cast<bf16*>(out), T, H, k,
-                                           rows_per_slot);
+                                           rows_per_slot));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }

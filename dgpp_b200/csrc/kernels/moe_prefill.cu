@@ -185,7 +185,7 @@ DGPP_API int dgpp_moe_segment_sort(const void* ids, void* pair_row, void* tile_e
     DGPP_CUDA_OK(cudaFuncSetAttribute(moe_segment_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
     attr = true;
   }
-  moe_segment_sort_kernel<<<1, kSortThreads, smem, st>>>(a);
+  DGPP_CUDA_OK(launch_early(moe_segment_sort_kernel, 1, kSortThreads, smem, st, a));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -194,8 +194,8 @@ DGPP_API int dgpp_moe_gather_rows(const void* x, int64_t x_stride, const void* p
                                   cudaStream_t st) {
   DGPP_REQUIRE(H % 8 == 0 && x_stride % 8 == 0, "moe_gather_rows: hidden %d / stride must be multiples of 8", H);
   if (T == 0) return 0;
-  moe_gather_rows_kernel<<<T * k, 128, 0, st>>>(static_cast<const bf16*>(x), x_stride, static_cast<const int32_t*>(pair_row),
-                                                static_cast<bf16*>(xs), H, k);
+  DGPP_CUDA_OK(launch_early(moe_gather_rows_kernel, T * k, 128, 0, st, static_cast<const bf16*>(x), x_stride, static_cast<const int32_t*>(pair_row),
+                                                static_cast<bf16*>(xs), H, k));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -205,9 +205,9 @@ DGPP_API int dgpp_moe_combine_rows(const void* y, const void* shared, const void
   DGPP_REQUIRE(H % 8 == 0, "moe_combine_rows: hidden %d must be a multiple of 8", H);
   if (T == 0) return 0;
   dim3 grid(dgpp_ceil_div(H / 8, 256), T);
-  moe_combine_rows_kernel<<<grid, 256, 0, st>>>(static_cast<const bf16*>(y), static_cast<const bf16*>(shared),
+  DGPP_CUDA_OK(launch_early(moe_combine_rows_kernel, grid, 256, 0, st, static_cast<const bf16*>(y), static_cast<const bf16*>(shared),
                                                 static_cast<const int32_t*>(pair_row), static_cast<const float*>(w),
-                                                static_cast<bf16*>(out), H, k);
+                                                static_cast<bf16*>(out), H, k));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }

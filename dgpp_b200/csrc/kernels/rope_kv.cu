@@ -161,9 +161,9 @@ DGPP_API int dgpp_rope_kv_write(void* qkv, const void* positions, const void* ro
   p.mscale = mscale; p.eps = eps; p.kv_fp8 = kv_fp8; p.norm_one_plus_w = norm_one_plus_w;
   const int warps = rows * (hq + 2 * hkv);
   const int blocks = dgpp_ceil_div(warps, 4);
-  if (d == 64) rope_kv_kernel<64><<<blocks, 128, 0, st>>>(p);
-  else if (d == 128) rope_kv_kernel<128><<<blocks, 128, 0, st>>>(p);
-  else rope_kv_kernel<256><<<blocks, 128, 0, st>>>(p);
+  if (d == 64) DGPP_CUDA_OK(launch_early(rope_kv_kernel<64>, blocks, 128, 0, st, p));
+  else if (d == 128) DGPP_CUDA_OK(launch_early(rope_kv_kernel<128>, blocks, 128, 0, st, p));
+  else DGPP_CUDA_OK(launch_early(rope_kv_kernel<256>, blocks, 128, 0, st, p));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }
