@@ -640,6 +640,169 @@ struct Fp4Cfg {
   static constexpr size_t smem() { return 1024 + S * stage_bytes() + (2 * S + 1) * 8 + 64; }
 };
 
+// Grouped linears (experts) without split K, persistent: the CTAs of one resident wave walk (slot, weight tile) units.  A unit is short
+// (two stages of K in a down product of 512), so what a launch with one CTA per unit spent its time on was starting CTAs: barriers, tensor
+// memory, a round trip to HBM, an epilogue, 4 waves of them.  Here the producer runs ahead into the next unit, and the accumulators are
+// double buffered: the epilogue of a unit runs under the products of the next.  81 slots x 2048 x 512 and 81 slots x
+// 1024 x 2048, 8 rows: 22.7 and 19 us, 8.9 each on average so (floor 7.3 each).  Operands, their order and the epilogue's arithmetic are those of the kernel above: the same bits.
+template <int BN, int S>
+__global__ void __launch_bounds__(kF4Threads, BN <= 96 ? 2 : 1)
+gemm_fp4_units_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Fp4Params p, int units) {
+  constexpr int kStageB = BN * 128;
+  constexpr int kAtomsB = BN > 128 ? 2 : 1;
+  constexpr int kSfaBytes = 4 * kF4Atom, kSfbBytes = 4 * kAtomsB * kF4Atom;
+  constexpr uint32_t kStageTx = kF4StageA + kSfaBytes + kStageB + kSfbBytes;
+  extern __shared__ __align__(1024) unsigned char smem_dyn[];
+  unsigned char* sp = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
+  unsigned char* sA = sp;    sp += S * kF4StageA;
+  unsigned char* sB = sp;    sp += S * kStageB;
+  unsigned char* sSfa = sp;  sp += S * kSfaBytes;
+  unsigned char* sSfb = sp;  sp += S * kSfbBytes;
+  uint64_t* full = reinterpret_cast<uint64_t*>(sp);
+  uint64_t* empty = full + S;
+  uint64_t* acc_full = empty + S;      // [2]
+  uint64_t* acc_empty = acc_full + 2;  // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int bn_tok = BN / p.R, nst = p.K / kF4StageK;
+  constexpr uint32_t kAccs = BN <= 128 ? 2 : 1;      // (256 columns and their scale factors leave no room for a second)
+  constexpr uint32_t kColD = BN < 32 ? 32 : BN;
+  constexpr uint32_t kColSfa = 16, kColSfb = 16 * kAtomsB;
+  constexpr uint32_t kNeed = kAccs * kColD + 2 * kColSfa + 2 * kColSfb;
+  constexpr uint32_t kTmemCols = kNeed <= 64 ? 64 : (kNeed <= 128 ? 128 : (kNeed <= 256 ? 256 : 512));
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < S; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 4); }
+    *abort_flag = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_sfa = tmem_base + kAccs * kColD, tmem_sfb = tmem_sfa + 2 * kColSfa;
+  pdl_wait();
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ producer: weights, activations, scales
+    if (elect_one()) {
+      int it = 0;
+      bool ok = true;
+      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+        const int grp = u / p.group_tiles, e = p.group_list[grp];
+        if (e < 0) continue;
+        const int tile = e * p.group_tiles + u % p.group_tiles, b_grp = p.group_b ? grp : 0;
+        for (int i = 0; i < nst; ++i, ++it) {
+          const int s = it % S;
+          if (!wait_bar(&empty[s], ((it / S) & 1) ^ 1) || *abort_flag) { report(p.status, kTimeoutStageEmpty, 13); *abort_flag = 1; ok = false; break; }
+          mbar_expect_tx(&full[s], kStageTx);
+          tma_load_2d(sA + s * kF4StageA, &tmA, i * 128, tile * kF4BM, &full[s]);
+          bulk_load_1d(sSfa + s * kSfaBytes, p.sfa + (static_cast<size_t>(tile) * nst + i) * kSfaBytes, kSfaBytes, &full[s]);
+          tma_load_2d(sB + s * kStageB, &tmB, i * 128, b_grp * BN, &full[s]);
+          bulk_load_1d(sSfb + s * kSfbBytes, p.sfb + (static_cast<size_t>(b_grp) * nst + i) * kSfbBytes, kSfbBytes, &full[s]);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (elect_one()) {
+      constexpr uint32_t idesc = umma_idesc_fp4bs(kF4BM, BN, 0u);
+      int it = 0, n = 0;
+      bool ok = true;
+      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+        if (p.group_list[u / p.group_tiles] < 0) continue;
+        const uint32_t a = n % kAccs, d = tmem_base + a * kColD;
+        if (!wait_bar(&acc_empty[a], ((n / kAccs) & 1) ^ 1)) { report(p.status, kTimeoutAccum, 14); *abort_flag = 1; break; }
+        for (int i = 0; i < nst; ++i, ++it) {
+          const int s = it % S;
+          if (!wait_bar(&full[s], (it / S) & 1) || *abort_flag) { report(p.status, kTimeoutTmaFull, 16); *abort_flag = 1; ok = false; break; }
+          tc_fence_after();
+          const uint32_t t_sfa = tmem_sfa + (it & 1) * kColSfa, t_sfb = tmem_sfb + (it & 1) * kColSfb;
+          for (int j = 0; j < 4; ++j)
+            tmem_cp_32x128b_warpx4(t_sfa + 4 * j, umma_desc_nosw(smem_u32(sSfa + s * kSfaBytes + j * kF4Atom), 0, 128));
+          for (int j = 0; j < 4 * kAtomsB; ++j)
+            tmem_cp_32x128b_warpx4(t_sfb + 4 * j, umma_desc_nosw(smem_u32(sSfb + s * kSfbBytes + j * kF4Atom), 0, 128));
+          const uint32_t a_addr = smem_u32(sA + s * kF4StageA), b_addr = smem_u32(sB + s * kStageB);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            umma_nvfp4(d, umma_desc_sw128(a_addr + j * 32), umma_desc_sw128(b_addr + j * 32), idesc, t_sfa + 4 * j, t_sfb + 4 * kAtomsB * j,
+                       (i > 0 || j > 0) ? 1u : 0u);
+          umma_commit(&empty[s]);
+        }
+        umma_commit(&acc_full[a]);
+        ++n;
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ epilogue (warps 2..5: 128 weight rows x the slot's tokens)
+    const int q = warp & 3;
+    const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
+    int n = 0;
+    for (int u = blockIdx.x; u < units; u += gridDim.x) {
+      const int grp = u / p.group_tiles, e = p.group_list[grp];
+      if (e < 0) continue;
+      const int a = n % kAccs;
+      const float alpha = p.group_alpha ? p.group_alpha[e] : p.alpha;
+      const float* gvec = p.g + (p.group_b ? grp * p.T_pad : 0);
+      bool ok = wait_bar(&acc_full[a], (n / kAccs) & 1);
+      if (!ok) { report(p.status, kTimeoutAccum, 15); *abort_flag = 1; }
+      ok = __all_sync(0xffffffffu, ok && !*abort_flag);
+      if (!ok) break;
+      tc_fence_after();
+      bf16* out = p.out + static_cast<size_t>(grp) * p.group_out_stride + (u % p.group_tiles) * kF4BM + q * 32 + lane;
+#pragma unroll 1
+      for (int c0 = 0; c0 < p.T; c0 += 16) {
+        float v[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = 0.f;
+        for (int r = 0; r < p.R; ++r) {  // add the residual-term column groups
+          uint32_t rr[16];
+          tmem_ld_x16(tmem_base + a * kColD + lane_addr + r * bn_tok + c0, rr);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(rr[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (c0 + j < p.T) out[static_cast<size_t>(c0 + j) * p.ldc] = f32_to_bf16(v[j] * alpha * gvec[c0 + j]);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[a]);
+      ++n;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
+}
+
+template <int BN>
+static int launch_fp4_units(const CUtensorMap& tA, const CUtensorMap& tB, const Fp4Params& p, cudaStream_t st) {
+  using C = Fp4Cfg<BN>;
+  auto kern = gemm_fp4_units_kernel<BN, C::S>;
+  static int slots = 0;      // CTAs of one resident wave
+  constexpr size_t smem = C::smem() + 3 * 8;
+  static_assert(smem <= 227 * 1024, "shared memory budget exceeded");
+  if (!slots) {
+    int dev = 0, sms = 0;
+    DGPP_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    DGPP_CUDA_OK(cudaGetDevice(&dev));
+    DGPP_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    slots = sms * (BN <= 96 ? 2 : 1);
+  }
+  const int units = p.grid_x;
+  DGPP_CUDA_OK(launch_early(kern, units < slots ? units : slots, kF4Threads, smem, st, tA, tB, p, units));
+  return 0;
+}
+
 template <int BN>
 static int launch_fp4(const CUtensorMap& tA, const CUtensorMap& tB, const Fp4Params& p, int splits, cudaStream_t st) {
   using C = Fp4Cfg<BN>;
@@ -865,6 +1028,18 @@ DGPP_API int dgpp_gemm_fp4_grouped(int bn, const void* xq, const void* xsf, cons
   const uint64_t b_rows = static_cast<uint64_t>(R) * bn * (group_b ? slots : 1);
   if (make_tmap_2d(&tB, xq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K / 2, b_rows, K / 2, 128, bnn, CU_TENSOR_MAP_SWIZZLE_128B))
     return -1;
+  if (splits == 1) {
+    switch (bnn) {
+      case 16: return launch_fp4_units<16>(tA, tB, p, st);
+      case 32: return launch_fp4_units<32>(tA, tB, p, st);
+      case 48: return launch_fp4_units<48>(tA, tB, p, st);
+      case 64: return launch_fp4_units<64>(tA, tB, p, st);
+      case 96: return launch_fp4_units<96>(tA, tB, p, st);
+      case 128: return launch_fp4_units<128>(tA, tB, p, st);
+      case 192: return launch_fp4_units<192>(tA, tB, p, st);
+      case 256: return launch_fp4_units<256>(tA, tB, p, st);
+    }
+  }
   switch (bnn) {
     case 16: return launch_fp4<16>(tA, tB, p, splits, st);
     case 32: return launch_fp4<32>(tA, tB, p, splits, st);
