@@ -73,11 +73,11 @@ __device__ __forceinline__ void st_async_f32x2(uint32_t addr, float x, float y, 
 __device__ __forceinline__ void fold_splits(const ClusterQuantArgs& a, int t, int col, float (&acc)[8], float& ll) {
   const int h = col / a.D, d0 = col % a.D;
   const size_t rh = static_cast<size_t>(t) * a.hq + h;
-  const float2* ml = reinterpret_cast<const float2*>(a.part_ml) + rh * a.splits;
+  const float* ml = a.part_ml + rh * a.splits * 2;
   const float* pa = a.part_acc + rh * a.splits * a.D + d0;
   float mm = -INFINITY;
 #pragma unroll 8
-  for (int sp = 0; sp < a.splits; ++sp) mm = fmaxf(mm, ml[sp].x);
+  for (int sp = 0; sp < a.splits; ++sp) mm = fmaxf(mm, ml[sp * 2]);
   ll = 0.f;
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc[j] = 0.f;
@@ -87,7 +87,7 @@ __device__ __forceinline__ void fold_splits(const ClusterQuantArgs& a, int t, in
 #pragma unroll
     for (int i = 0; i < kAqSplitBlock; ++i) {
       if (s0 + i >= a.splits) break;
-      m[i] = ml[s0 + i];
+      m[i] = make_float2(ml[(s0 + i) * 2], ml[(s0 + i) * 2 + 1]);
       const float4* src = reinterpret_cast<const float4*>(pa + static_cast<size_t>(s0 + i) * a.D);
       v[i][0] = src[0];
       v[i][1] = src[1];

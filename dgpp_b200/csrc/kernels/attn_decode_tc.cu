@@ -129,20 +129,62 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     tmem_relinquish();
   }
   pdl_wait();
-  // ---- quantise q of this kv head's G query heads into two e4m3 terms (B operand of MMA1)
-  float q_scale[G];
+  float qv[NH][G];      // requested in front of everything that depends on a table
   if (warp >= 2) {
     const int d = threadIdx.x - 64;  // 0..127
 #pragma unroll
-    for (int h = 0; h < G; ++h) {
-      float a = 0.f;
+    for (int h = 0; h < G; ++h)
 #pragma unroll
-      for (int hf = 0; hf < NH; ++hf)
-        a = fmaxf(a, fabsf(bf16_to_f32(p.q[static_cast<size_t>(row) * p.q_stride + (kvh * G + h) * D + hf * 128 + d])));
+      for (int hf = 0; hf < NH; ++hf) qv[hf][h] = bf16_to_f32(p.q[static_cast<size_t>(row) * p.q_stride + (kvh * G + h) * D + hf * 128 + d]);
+  }
+  // The first tiles are on their way and their token scales requested while q is staged: warp 0 looks up all of their pages at once (at
+  // most 3 x 8), its first lane, which made the barriers, issues.  (Looked up one by one behind the staging: 17.4 us at 8 rows of 40 / 8 heads
+  // over 2048, 14.8 so; 8 rows of 16 / 2 heads of 256: 14.1, 11.4 so.)
+  const int ppt = kAdTile / p.page;  // pages per tile
+  auto page_block = [&](int tile, int pg) {
+    const int page0 = (base + (tile_begin + tile) * kAdTile) / p.page;
+    return bt[min(sl == nullptr ? page0 + pg : cache_pos((page0 + pg) * p.page) / p.page, p.max_blocks - 1)];
+  };
+  auto load_page = [&](int s, int pg, int blk) {
+    const int r0 = (blk * p.hkv + kvh) * p.page;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
-      if (lane == 0) redl[(warp - 2) * 8 + h] = a;
+    for (int hf = 0; hf < NH; ++hf) {
+      tma_load_2d(sK + s * kStage + hf * kHalf + pg * p.page * 128, &tmK, hf * 128, r0, &kv_full[s]);
+      tma_load_2d(sV + s * kStage + hf * kHalf + pg * p.page * 128, &tmV, hf * 128, r0, &kv_full[s]);
     }
+  };
+  if (warp == 0) {
+    const int pages = min(ntiles, kAdStages) * ppt;
+    const int mine = lane < pages ? page_block(lane / ppt, lane % ppt) : 0;
+    for (int i = 0; i < pages; ++i) {
+      const int blk = __shfl_sync(0xffffffffu, mine, i);
+      if (lane == 0) {
+        if (i % ppt == 0) mbar_expect_tx(&kv_full[i / ppt], 2 * kStage);
+        load_page(i / ppt, i % ppt, blk);
+      }
+    }
+    __syncwarp();
+  }
+  auto load_scales = [&](int i, float& ks, float& vs, bool& valid) {
+    const int t = base + (tile_begin + i) * kAdTile + (warp & 3) * 32 + lane;      // token of this lane of TMEM
+    valid = t >= first && t < len;
+    const int tc = cache_pos(max(0, min(t, len - 1)));
+    const int pi = min(tc / p.page, p.max_blocks - 1);
+    const size_t tok = (static_cast<size_t>(bt[pi]) * p.hkv + kvh) * p.page + tc % p.page;
+    ks = p.k_scale[tok];
+    vs = valid ? p.v_scale[tok] : 0.f;
+  };
+  float ks_n = 0.f, vs_n = 0.f;
+  bool valid_n = false;
+  if (warp >= 2 && ntiles > 0) load_scales(0, ks_n, vs_n, valid_n);
+  // ---- quantise q of this kv head's G query heads into two e4m3 terms (B operand of MMA1)
+  float q_scale[G];
+  if (warp >= 2) {
+    float a[8];
+#pragma unroll
+    for (int h = 0; h < 8; ++h) a[h] = h < G ? (NH == 2 ? fmaxf(fabsf(qv[0][h < G ? h : 0]), fabsf(qv[NH - 1][h < G ? h : 0])) : fabsf(qv[0][h < G ? h : 0])) : 0.f;
+    const float m = over_lanes<true>(a, lane);
+    if ((lane & 3) == 0) redl[(warp - 2) * 8 + (lane >> 2)] = m;
   }
   __syncthreads();
   if (warp >= 2) {
@@ -159,7 +201,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       for (int hf = 0; hf < NH; ++hf) {
         uint8_t b1 = 0, b2 = 0;
         if (h < G) {
-          const float v = bf16_to_f32(p.q[static_cast<size_t>(row) * p.q_stride + (kvh * G + h) * D + hf * 128 + d]) / sc;
+          const float v = qv[hf][h < G ? h : 0] / sc;
           b1 = f32_to_e4m3(v);
           b2 = f32_to_e4m3((v - e4m3_value_f32(v)) * 16.f);   // residual against the VALUE of b1 (no fp8 decode of b1)
         }
@@ -179,22 +221,11 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (elect_one()) {
-      const int ppt = kAdTile / p.page;  // pages per tile
-      for (int i = 0; i < ntiles; ++i) {
+      for (int i = kAdStages; i < ntiles; ++i) {
         const int s = i % kAdStages;
         if (!wait_bar(&kv_empty[s], ((i / kAdStages) & 1) ^ 1)) { report(p.status, kTimeoutStageEmpty, 21); *abort_flag = 1; break; }
         mbar_expect_tx(&kv_full[s], 2 * kStage);
-        const int page0 = (base + (tile_begin + i) * kAdTile) / p.page;
-        for (int pg = 0; pg < ppt; ++pg) {
-          const int pi = min(sl == nullptr ? page0 + pg : cache_pos((page0 + pg) * p.page) / p.page, p.max_blocks - 1);
-          const int blk = bt[pi];
-          const int r0 = (blk * p.hkv + kvh) * p.page;
-#pragma unroll
-          for (int hf = 0; hf < NH; ++hf) {
-            tma_load_2d(sK + s * kStage + hf * kHalf + pg * p.page * 128, &tmK, hf * 128, r0, &kv_full[s]);
-            tma_load_2d(sV + s * kStage + hf * kHalf + pg * p.page * 128, &tmV, hf * 128, r0, &kv_full[s]);
-          }
-        }
+        for (int pg = 0; pg < ppt; ++pg) load_page(s, pg, page_block(i, pg));
         if (*abort_flag) break;
       }
     }
@@ -263,19 +294,6 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     }
     float inv_c_prev = 0.f;
     bool ok = true;
-    // token scales of the first tile
-    auto load_scales = [&](int i, float& ks, float& vs, bool& valid) {
-      const int t = base + (tile_begin + i) * kAdTile + idx;
-      valid = t >= first && t < len;
-      const int tc = cache_pos(max(0, min(t, len - 1)));
-      const int pi = min(tc / p.page, p.max_blocks - 1);
-      const size_t tok = (static_cast<size_t>(bt[pi]) * p.hkv + kvh) * p.page + tc % p.page;
-      ks = p.k_scale[tok];
-      vs = valid ? p.v_scale[tok] : 0.f;
-    };
-    float ks_n = 0.f, vs_n = 0.f;
-    bool valid_n = false;
-    if (ntiles > 0) load_scales(0, ks_n, vs_n, valid_n);
     for (int i = 0; i < ntiles; ++i) {
       const int b = i & 1;
       const float ks = ks_n, vs = vs_n;
@@ -300,24 +318,28 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       for (int h = 0; h < G; ++h) {
         const float raw = (__uint_as_float(c[h]) + __uint_as_float(c[8 + h]) * 0.0625f) * q_scale[h] * ks * sm;
         s[h] = valid ? raw : -INFINITY;
-        float mx = s[h];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (lane == 0) rp[h] = mx;
       }
+      // maxima of the scores (rp[0 .. G)) and of the V scales (rp[8]) over the warp's tokens
       {
-        float vm = vs;
+        float a[8];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, o));
-        if (lane == 0) {
-          rp[G] = vm;
-          rp[11] = (okw && !*abort_flag) ? 0.f : 1.f;
+        for (int h = 0; h < 8; ++h) a[h] = h < G ? s[h < G ? h : 0] : vs;
+        const float m = over_lanes<true>(a, lane);
+        if ((lane & 3) == 0) rp[lane >> 2] = m;
+        float vm = vs;
+        if (G == 8) {
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, o));
+        } else {
+          vm = m;
         }
+        if (lane == 31) rp[8] = vm;      // (lane 31 holds the last of the eight)
+        if (lane == 0) rp[11] = (okw && !*abort_flag) ? 0.f : 1.f;
       }
       asm volatile("bar.sync 1, 128;" ::: "memory");
       const float* r0 = red + (b * 4) * 12;
       if (r0[11] + r0[12 + 11] + r0[24 + 11] + r0[36 + 11] != 0.f) { ok = false; break; }
-      const float vmax = fmaxf(fmaxf(r0[G], r0[12 + G]), fmaxf(r0[24 + G], r0[36 + G]));
+      const float vmax = fmaxf(fmaxf(r0[8], r0[12 + 8]), fmaxf(r0[24 + 8], r0[36 + 8]));
       const float c_tile = vmax > 0.f ? 256.f / vmax : 0.f;
       float corr[G];
       uint8_t pb1[8], pb2[8];
@@ -327,8 +349,8 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       for (int h = 0; h < G; ++h) {
         const float mt = fmaxf(fmaxf(r0[h], r0[12 + h]), fmaxf(r0[24 + h], r0[36 + h]));
         const float mn = fmaxf(m_run[h], mt);
-        corr[h] = (m_run[h] == -INFINITY) ? 0.f : exp2f(m_run[h] - mn);
-        const float pv = (valid && mn > -INFINITY) ? exp2f(s[h] - mn) : 0.f;
+        corr[h] = (m_run[h] == -INFINITY) ? 0.f : fast_exp2(m_run[h] - mn);
+        const float pv = (valid && mn > -INFINITY) ? fast_exp2(s[h] - mn) : 0.f;
         l_thr[h] = l_thr[h] * corr[h] + pv;
         m_run[h] = mn;
         const float pw = pv * vs * c_tile;
@@ -390,12 +412,12 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     }
     // total probability mass per head: sum the per-thread partials
     asm volatile("bar.sync 1, 128;" ::: "memory");
+    {
+      float l[8];
 #pragma unroll
-    for (int h = 0; h < G; ++h) {
-      float l = l_thr[h];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-      if (lane == 0) redl[wslot * 8 + h] = l;
+      for (int h = 0; h < 8; ++h) l[h] = h < G ? l_thr[h < G ? h : 0] : 0.f;
+      const float sum = over_lanes<false>(l, lane);
+      if ((lane & 3) == 0) redl[wslot * 8 + (lane >> 2)] = sum;
     }
     asm volatile("bar.sync 1, 128;" ::: "memory");
 #pragma unroll
@@ -425,18 +447,34 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
 
 __global__ void attn_tc_combine_kernel(const float* __restrict__ part_ml, const float* __restrict__ part_acc,
                                        bf16* __restrict__ out, int splits) {
+  // (eight splits' values are in flight at once)
+  constexpr int kBatch = 8;
   pdl_wait();
   const size_t rh = blockIdx.x;
   const int d = threadIdx.x;
   const int D = blockDim.x;
+  const float* ml = part_ml + rh * splits * 2;
+  const float* pa = part_acc + rh * splits * D + d;
   float mm = -INFINITY;
-  for (int s = 0; s < splits; ++s) mm = fmaxf(mm, part_ml[(rh * splits + s) * 2]);
+#pragma unroll 8
+  for (int s = 0; s < splits; ++s) mm = fmaxf(mm, ml[s * 2]);
   float ll = 0.f, a = 0.f;
-  for (int s = 0; s < splits; ++s) {
-    const float ms = part_ml[(rh * splits + s) * 2];
-    const float c = ms == -INFINITY ? 0.f : __expf(ms - mm);
-    ll += part_ml[(rh * splits + s) * 2 + 1] * c;
-    a += part_acc[(rh * splits + s) * D + d] * c;
+  for (int s0 = 0; s0 < splits; s0 += kBatch) {
+    float ms[kBatch], ls[kBatch], v[kBatch];
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      const bool has = s0 + i < splits;
+      ms[i] = has ? ml[(s0 + i) * 2] : -INFINITY;
+      ls[i] = has ? ml[(s0 + i) * 2 + 1] : 0.f;
+      v[i] = has ? pa[static_cast<size_t>(s0 + i) * D] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      if (s0 + i >= splits) break;
+      const float c = ms[i] == -INFINITY ? 0.f : __expf(ms[i] - mm);
+      ll += ls[i] * c;
+      a += v[i] * c;
+    }
   }
   out[rh * D + d] = f32_to_bf16(ll > 0.f ? a / ll : 0.f);
 }

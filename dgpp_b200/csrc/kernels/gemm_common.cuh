@@ -28,6 +28,32 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity) {
   }
 }
 
+// N values per lane (N a power of two up to 32), reduced over the lanes: at distance o a lane keeps the half of its values that its bit
+// o names and adds the partner's share of them; lane i ends with value i * N / 32.
+template <bool MAX, int N>
+__device__ __forceinline__ float over_lanes(const float (&in)[N], int lane) {
+  float v[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = in[i];
+#pragma unroll
+  for (int step = 0; step < 5; ++step) {
+    const int o = 16 >> step, n = N >> (step + 1);
+    if (n > 0) {
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int i = 0; i < n; ++i) {
+        const float keep = up ? v[i + n] : v[i], give = up ? v[i] : v[i + n];
+        const float got = __shfl_xor_sync(0xffffffffu, give, o);
+        v[i] = MAX ? fmaxf(keep, got) : keep + got;
+      }
+    } else {
+      const float got = __shfl_xor_sync(0xffffffffu, v[0], o);
+      v[0] = MAX ? fmaxf(v[0], got) : v[0] + got;
+    }
+  }
+  return v[0];
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);

@@ -56,32 +56,6 @@ struct MlaTcParams {
   float scale;
 };
 
-// N values per lane (N a power of two up to 32), reduced over the lanes: at distance o a lane keeps the half of its values that its bit
-// o names and adds the partner's share of them; lane i ends with value i * N / 32.
-template <bool MAX, int N>
-__device__ __forceinline__ float over_lanes(const float (&in)[N], int lane) {
-  float v[N];
-#pragma unroll
-  for (int i = 0; i < N; ++i) v[i] = in[i];
-#pragma unroll
-  for (int step = 0; step < 5; ++step) {
-    const int o = 16 >> step, n = N >> (step + 1);
-    if (n > 0) {
-      const bool up = (lane & o) != 0;
-#pragma unroll
-      for (int i = 0; i < n; ++i) {
-        const float keep = up ? v[i + n] : v[i], give = up ? v[i] : v[i + n];
-        const float got = __shfl_xor_sync(0xffffffffu, give, o);
-        v[i] = MAX ? fmaxf(keep, got) : keep + got;
-      }
-    } else {
-      const float got = __shfl_xor_sync(0xffffffffu, v[0], o);
-      v[0] = MAX ? fmaxf(v[0], got) : v[0] + got;
-    }
-  }
-  return v[0];
-}
-
 // SPARSE: the tokens of a tile come from the row's selection list instead of consecutive positions; the four softmax
 // warps (idle while a tile loads: it is single buffered) gather them, thread = token: 72 16-byte chunks of the token's
 // latent row into the swizzled column blocks, then a proxy fence and one arrival per warp on the tile barrier.
@@ -154,12 +128,16 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmC, MlaTcParams p) {
   auto load_tile = [&](int i) {
     mbar_expect_tx(c_full, kTileBytes);
     const int page0 = (tile_begin + i) * kMtTile / p.page;
-    for (int pg = 0; pg < ppt; ++pg) {
-      const int pi = min(page0 + pg, p.max_blocks - 1);
-      const int r0 = bt[pi] * p.page;
+    int blk[kMtTile / 16];      // all looked up before the first is used
+#pragma unroll
+    for (int pg = 0; pg < kMtTile / 16; ++pg)
+      if (pg < ppt) blk[pg] = bt[min(page0 + pg, p.max_blocks - 1)];
+#pragma unroll
+    for (int pg = 0; pg < kMtTile / 16; ++pg) {
+      if (pg >= ppt) break;
 #pragma unroll
       for (int kb = 0; kb < KB; ++kb)
-        tma_load_2d(sC + kb * kMtBlk + pg * p.page * 128, &tmC, kb * 64, r0, c_full);
+        tma_load_2d(sC + kb * kMtBlk + pg * p.page * 128, &tmC, kb * 64, blk[pg] * p.page, c_full);
     }
   };
   if (!SPARSE && threadIdx.x == 0 && ntiles > 0) load_tile(0);      // (by the thread that made the barriers)
