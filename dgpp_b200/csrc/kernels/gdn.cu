@@ -56,34 +56,39 @@ struct GdnArgs {
 };
 
 // Token-parallel part: unit-norm q (scaled by dk^-1/2) and k per key head, decay and write strength per value head.
-// grid (T, hk + 1): blocks y < hk normalise one key head (dk threads), block y == hk does the per-head scalars.
+// grid (T, ceil(hk / 4) + 1, more for KDA), 128 threads: a warp of the first blocks normalises one key head, dk / 32 neighbouring channels per
+// lane; the next block does the per-head scalars.  Memory bound (2048 tokens x 16 heads of 128: 37 us with a block and 16-bit
+// loads per head, 12 so).
+constexpr int kPrepThreads = 128, kPrepHeads = kPrepThreads / 32;
 template <int DK>
-__global__ void __launch_bounds__(DK) gdn_prep_kernel(GdnArgs a) {
-  __shared__ float red[2][DK / 32];
+__global__ void __launch_bounds__(kPrepThreads) gdn_prep_kernel(GdnArgs a) {
   pdl_wait();
   const int t = blockIdx.x, tid = threadIdx.x;
+  const unsigned scalars = static_cast<unsigned>((a.hk + kPrepHeads - 1) / kPrepHeads);      // the block of the per-head scalars
   float* qn = a.prep;
   float* kn = qn + static_cast<size_t>(a.T) * a.hk * DK;
   float* dec = kn + static_cast<size_t>(a.T) * a.hk * DK;
   float* bet = dec + static_cast<size_t>(a.T) * a.hv;
-  if (static_cast<int>(blockIdx.y) > a.hk) {
-    // KDA: per-channel decay of value head (blockIdx.y - hk - 1), one thread per key channel
-    const int h = static_cast<int>(blockIdx.y) - a.hk - 1;
+  if (blockIdx.y > scalars) {
+    // KDA: per-channel decay of value head (blockIdx.y - scalars - 1)
+    const int h = static_cast<int>(blockIdx.y - scalars) - 1;
     float* deck = bet + static_cast<size_t>(a.T) * a.hv;
-    const float x = bf16_to_f32(a.gate_k[static_cast<size_t>(t) * a.gate_stride + h * DK + tid]) + a.dt_bias[h * DK + tid];
-    const float g = a.lower_bound / (1.f + expf(-expf(a.A_log[h]) * x));
-    deck[(static_cast<size_t>(t) * a.hv + h) * DK + tid] = expf(g);
+    for (int c = tid; c < DK; c += kPrepThreads) {
+      const float x = bf16_to_f32(a.gate_k[static_cast<size_t>(t) * a.gate_stride + h * DK + c]) + a.dt_bias[h * DK + c];
+      const float g = a.lower_bound / (1.f + expf(-expf(a.A_log[h]) * x));
+      deck[(static_cast<size_t>(t) * a.hv + h) * DK + c] = expf(g);
+    }
     return;
   }
-  if (blockIdx.y == static_cast<unsigned>(a.hk) && a.gate_k) {
-    for (int h = tid; h < a.hv; h += DK) {
+  if (blockIdx.y == scalars && a.gate_k) {
+    for (int h = tid; h < a.hv; h += kPrepThreads) {
       dec[static_cast<size_t>(t) * a.hv + h] = 1.f;
       bet[static_cast<size_t>(t) * a.hv + h] = 1.f / (1.f + expf(-bf16_to_f32(a.beta[static_cast<size_t>(t) * a.ab_stride + h])));
     }
     return;
   }
-  if (blockIdx.y == static_cast<unsigned>(a.hk)) {
-    for (int h = tid; h < a.hv; h += DK) {
+  if (blockIdx.y == scalars) {
+    for (int h = tid; h < a.hv; h += kPrepThreads) {
       const float al = bf16_to_f32(a.alpha[static_cast<size_t>(t) * a.ab_stride + h]) + a.dt_bias[h];
       const float softplus = al > 20.f ? al : log1pf(expf(al));
       dec[static_cast<size_t>(t) * a.hv + h] = expf(-expf(a.A_log[h]) * softplus);
@@ -91,34 +96,57 @@ __global__ void __launch_bounds__(DK) gdn_prep_kernel(GdnArgs a) {
     }
     return;
   }
-  const int h = blockIdx.y;
-  const float qv = bf16_to_f32(a.q[static_cast<size_t>(t) * a.q_stride + h * DK + tid]);
-  const float kv = bf16_to_f32(a.k[static_cast<size_t>(t) * a.k_stride + h * DK + tid]);
-  float q2 = qv * qv, k2 = kv * kv;
+  const int h = static_cast<int>(blockIdx.y) * kPrepHeads + (tid >> 5), lane = tid & 31;
+  if (h >= a.hk) return;
+  constexpr int PER = DK / 32;
+  const bf16* qp = a.q + static_cast<size_t>(t) * a.q_stride + h * DK + lane * PER;
+  const bf16* kp = a.k + static_cast<size_t>(t) * a.k_stride + h * DK + lane * PER;
+  float qv[PER], kv[PER];
+  float q2 = 0.f, k2 = 0.f;
+  // (pairs where rows and strides allow; a lane's channels begin at an even one)
+  if (((reinterpret_cast<uintptr_t>(qp) | reinterpret_cast<uintptr_t>(kp)) & 3) == 0) {
+#pragma unroll
+    for (int j = 0; j < PER; j += 2) {
+      const float2 x = __bfloat1622float2(*reinterpret_cast<const bf162*>(qp + j)), y = __bfloat1622float2(*reinterpret_cast<const bf162*>(kp + j));
+      qv[j] = x.x; qv[j + 1] = x.y; kv[j] = y.x; kv[j + 1] = y.y;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < PER; ++j) { qv[j] = bf16_to_f32(qp[j]); kv[j] = bf16_to_f32(kp[j]); }
+  }
+#pragma unroll
+  for (int j = 0; j < PER; ++j) { q2 += qv[j] * qv[j]; k2 += kv[j] * kv[j]; }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     q2 += __shfl_xor_sync(0xffffffffu, q2, o);
     k2 += __shfl_xor_sync(0xffffffffu, k2, o);
   }
-  if ((tid & 31) == 0) { red[0][tid >> 5] = q2; red[1][tid >> 5] = k2; }
-  __syncthreads();
-  float qs = 0.f, ks = 0.f;
+  const float qf = rsqrtf(q2 + 1e-6f), qd = rsqrtf(static_cast<float>(DK)), kf = rsqrtf(k2 + 1e-6f);
+  const size_t o = (static_cast<size_t>(t) * a.hk + h) * DK + lane * PER;
+  const bool pairs = (reinterpret_cast<uintptr_t>(qn) & 7) == 0;
 #pragma unroll
-  for (int w = 0; w < DK / 32; ++w) { qs += red[0][w]; ks += red[1][w]; }
-  const size_t o = (static_cast<size_t>(t) * a.hk + h) * DK + tid;
-  qn[o] = qv * rsqrtf(qs + 1e-6f) * rsqrtf(static_cast<float>(DK));
-  kn[o] = kv * rsqrtf(ks + 1e-6f);
+  for (int j = 0; j < PER; j += 2) {
+    const float2 x = make_float2(qv[j] * qf * qd, qv[j + 1] * qf * qd), y = make_float2(kv[j] * kf, kv[j + 1] * kf);
+    if (pairs) {
+      *reinterpret_cast<float2*>(qn + o + j) = x;
+      *reinterpret_cast<float2*>(kn + o + j) = y;
+    } else {
+      qn[o + j] = x.x; qn[o + j + 1] = x.y;
+      kn[o + j] = y.x; kn[o + j + 1] = y.y;
+    }
+  }
 }
 
 // Sequential part.  Thread (column j, part p) keeps state rows p, p + 8, p + 16, ... of column j in registers; the
 // normalised keys / queries of kGdnChunk tokens are staged in shared memory (one block-wide sync pair per chunk).
+// The state is requested in front of the wait on the preceding grid: that is always the preparation's, which writes neither states
+// nor slots and lets this grid start only after all work before it.
 template <int DK, bool KDA = false>
 __global__ void __launch_bounds__(kGdnThreads) gdn_recurrent_kernel(GdnArgs a) {
   constexpr int PER = DK / kGdnParts;          // state rows per thread
   __shared__ float ks[kGdnChunk][DK], qs[kGdnChunk][DK];
   __shared__ float dks[KDA ? kGdnChunk : 1][KDA ? DK : 1];     // KDA: per-channel decays of the staged tokens
   __shared__ float vs[kGdnChunk][kGdnCols], ds[kGdnChunk], bs[kGdnChunk];
-  pdl_wait();
   const int tid = threadIdx.x;
   const int col = tid / kGdnParts, part = tid % kGdnParts;
   const int h = blockIdx.y, j = blockIdx.x * kGdnCols + col;
@@ -135,6 +163,7 @@ __global__ void __launch_bounds__(kGdnThreads) gdn_recurrent_kernel(GdnArgs a) {
   float s[PER];
 #pragma unroll
   for (int i = 0; i < PER; ++i) s[i] = sp[static_cast<size_t>(part + kGdnParts * i) * a.dv];
+  pdl_wait();
   for (int t0 = first; t0 < last; t0 += kGdnChunk) {
     const int n = min(kGdnChunk, last - t0);
     __syncthreads();                            // the previous chunk's readers are done
@@ -311,13 +340,21 @@ __global__ void __launch_bounds__(256) gdn_conv_decode_kernel(ConvArgs a) {
   if (c >= a.C) return;
   const int t = blockIdx.y;
   float* st = a.state + static_cast<size_t>(a.row_slot[t]) * (a.W - 1) * a.C + c;
-  float v[4];
-  for (int i = 0; i < a.W - 1; ++i) v[i] = st[static_cast<size_t>(i) * a.C];
-  v[a.W - 1] = bf16_to_f32(a.x[static_cast<size_t>(t) * a.x_stride + c]);
+  const float x = bf16_to_f32(a.x[static_cast<size_t>(t) * a.x_stride + c]);
+  float v[4], w[4];      // (W <= 4; all of a thread's loads in flight together)
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v[i] = i < a.W - 1 ? st[static_cast<size_t>(i) * a.C] : x;
+    w[i] = i < a.W ? bf16_to_f32(a.w[c * a.W + i]) : 0.f;
+  }
   float acc = a.bias ? bf16_to_f32(a.bias[c]) : 0.f;
-  for (int i = 0; i < a.W; ++i) acc = fmaf(bf16_to_f32(a.w[c * a.W + i]), v[i], acc);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (i < a.W) acc = fmaf(w[i], v[i], acc);
   a.out[static_cast<size_t>(t) * a.C + c] = f32_to_bf16(acc / (1.f + expf(-acc)));
-  for (int i = 0; i < a.W - 1; ++i) st[static_cast<size_t>(i) * a.C] = v[i + 1];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    if (i < a.W - 1) st[static_cast<size_t>(i) * a.C] = v[i + 1];
 }
 
 // out[t, h, :] = rmsnorm(o[t, h, :]) * w * silu(z[t, h, :]); one warp per (row, head).
@@ -372,10 +409,10 @@ static int gdn_recurrent_launch(const void* q, int64_t q_stride, const void* k, 
   a.T = T; a.hk = hk; a.hv = hv; a.dk = dk; a.dv = dv; a.sequential = sequential;
   a.seg = seg; a.snap = static_cast<float*>(snap);
   a.gate_k = static_cast<const bf16*>(gate_k); a.gate_stride = gate_stride; a.lower_bound = lower_bound;
-  dim3 pgrid(T, hk + 1 + (gate_k ? hv : 0));
-  if (dk == 64) DGPP_CUDA_OK(launch_early(gdn_prep_kernel<64>, pgrid, 64, 0, st, a));
-  else if (dk == 128) DGPP_CUDA_OK(launch_early(gdn_prep_kernel<128>, pgrid, 128, 0, st, a));
-  else DGPP_CUDA_OK(launch_early(gdn_prep_kernel<256>, pgrid, 256, 0, st, a));
+  dim3 pgrid(T, dgpp_ceil_div(hk, kPrepHeads) + 1 + (gate_k ? hv : 0));
+  if (dk == 64) DGPP_CUDA_OK(launch_early(gdn_prep_kernel<64>, pgrid, kPrepThreads, 0, st, a));
+  else if (dk == 128) DGPP_CUDA_OK(launch_early(gdn_prep_kernel<128>, pgrid, kPrepThreads, 0, st, a));
+  else DGPP_CUDA_OK(launch_early(gdn_prep_kernel<256>, pgrid, kPrepThreads, 0, st, a));
   DGPP_CUDA_OK(cudaGetLastError());
   dim3 grid(dv / kGdnCols, hv, seg > 0 ? T / seg : (sequential ? 1 : T));
   if (gate_k) {
@@ -441,10 +478,10 @@ DGPP_API int dgpp_gdn_prep(const void* q, int64_t q_stride, const void* k, int64
   a.A_log = static_cast<const float*>(A_log); a.dt_bias = static_cast<const float*>(dt_bias);
   a.prep = static_cast<float*>(prep);
   a.T = T; a.hk = hk; a.hv = hv; a.dk = dk;
-  dim3 pgrid(T, hk + 1);
-  if (dk == 64) DGPP_CUDA_OK(launch_early(gdn_prep_kernel<64>, pgrid, 64, 0, st, a));
-  else if (dk == 128) DGPP_CUDA_OK(launch_early(gdn_prep_kernel<128>, pgrid, 128, 0, st, a));
-  else DGPP_CUDA_OK(launch_early(gdn_prep_kernel<256>, pgrid, 256, 0, st, a));
+  dim3 pgrid(T, dgpp_ceil_div(hk, kPrepHeads) + 1);
+  if (dk == 64) DGPP_CUDA_OK(launch_early(gdn_prep_kernel<64>, pgrid, kPrepThreads, 0, st, a));
+  else if (dk == 128) DGPP_CUDA_OK(launch_early(gdn_prep_kernel<128>, pgrid, kPrepThreads, 0, st, a));
+  else DGPP_CUDA_OK(launch_early(gdn_prep_kernel<256>, pgrid, kPrepThreads, 0, st, a));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }
