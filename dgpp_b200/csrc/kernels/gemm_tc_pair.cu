@@ -520,11 +520,11 @@ static int pair_slots(int* slots) {
 
 // Token tile and K splits of one product.  The product takes as many units one after the other as one pair gets: wide tiles reuse a
 // converted weight more often, narrower ones (or splits, where there are fewer tiles than pairs) fill the last round.  A K = 64
-// block counts as 400 + 1.2 bn cycles, a tile's drain as 15 bn + 500 (the accumulator is not double-buffered: its other half
-// holds the converted weights), s splits as 1000 and 400 s for every 32 tokens of a tile (their fold is s round trips to L2).
-// These are fitted to whole products, 21 shapes of 512 x 512 to 34816 x 5120 at 1 to 2048 rows with every tile and split count
-// (alone, a block takes 480 cycles up to 160 tokens, 530 at 192 and 655 at 256; with that the choice is the worse one): what they
-// choose is within 1.1 % of the best above 128 rows, and 1.2 % on average, 19 % at most (128 x 2560 x 8192) up to 128 rows.
+// block counts as 345 cycles (the conversion) or 80 + 1.95 bn (the MMAs), whichever is more, a tile's drain and the next one's fill as
+// 15 bn + 1500 (the accumulator is not double-buffered: its other half holds the converted weights), s splits as 1000 and 400 s for every
+// 32 tokens of a tile (their fold is s round trips to L2).  Fitted to six shapes of 4096 x 2048 to 34816 x 5120 at 129 to 2048 rows with every
+// tile: what they choose is within 0.2 % of the best on average, 4 % at most (34816 x 5120 at 953 rows: 276 us at 256 tokens, which 400 + 1.2 bn
+// chose, 230 at 192).
 // Up to 128 rows the splits are those of 128 rows, above there are none: on either side of that line a row's bits do not depend
 // on how many others share its pass, and prompt products touch no workspace, so that products on several streams share
 // nothing.  (A long K over few tiles pays for that: 173 x 5120 x 17408 79 us, 47 in three splits.)
@@ -541,7 +541,8 @@ static void pair_search(int T, int N, int K, int slots, int fewest, int most, in
       const int per = dgpp_ceil_div(raws, s);
       if (dgpp_ceil_div(raws, per) != s) continue;
       const int rounds = dgpp_ceil_div(tiles * s, slots);
-      const double unit = per * 4 * (400 + 1.2 * bn) + 15.0 * bn + 500;
+      const double block = 80 + 1.95 * bn;
+      const double unit = per * 4 * (block < 345 ? 345 : block) + 15.0 * bn + 1500;
       const double cost = rounds * unit + (s > 1 ? 1000 + 400.0 * s * dgpp_ceil_div(bn < T ? bn : T, 32) : 0.0);
       if (best == 0 || cost < best) { best = cost; *bn_out = bn; *splits_out = s; }
     }
