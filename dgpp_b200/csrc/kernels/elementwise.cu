@@ -52,7 +52,9 @@ embed_gather_kernel(const int32_t* __restrict__ ids, const bf16* __restrict__ ta
 
 // out = rmsnorm(resid (+ delta)); when delta != nullptr the sum is also written back to resid_out.
 // gemma_style: weight is applied as (1 + w).
-template <bool kAdd>
+// VPT: vectors of a row per thread, held in registers with their weights between the two passes (0: rows of more than 4 x 256 vectors, through
+// shared memory).  A single row is a chain of latencies, and the weights' round trip now runs beside the sum of squares.
+template <bool kAdd, int VPT>
 __global__ void __launch_bounds__(kRowThreads)
 rmsnorm_kernel(const bf16* __restrict__ resid, const bf16* __restrict__ delta, const bf16* __restrict__ w,
                bf16* __restrict__ resid_out, bf16* __restrict__ out, int hidden, float eps, int one_plus_w) {
@@ -63,12 +65,8 @@ rmsnorm_kernel(const bf16* __restrict__ resid, const bf16* __restrict__ delta, c
   const size_t base = static_cast<size_t>(blockIdx.x) * hidden;
   const int nvec = hidden / 8;
   float ss = 0.f;
-  for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
-    Pack16 a;
-    a.u = reinterpret_cast<const uint4*>(resid + base)[i];
+  auto add_squares = [&](int i, Pack16& a, const Pack16& d) {
     if (kAdd) {
-      Pack16 d;
-      d.u = reinterpret_cast<const uint4*>(delta + base)[i];
 #pragma unroll
       for (int j = 0; j < 8; ++j) a.h[j] = f32_to_bf16(bf16_to_f32(a.h[j]) + bf16_to_f32(d.h[j]));
       reinterpret_cast<uint4*>(resid_out + base)[i] = a.u;
@@ -78,14 +76,9 @@ rmsnorm_kernel(const bf16* __restrict__ resid, const bf16* __restrict__ delta, c
       float f = bf16_to_f32(a.h[j]);
       ss += f * f;
     }
-    reinterpret_cast<uint4*>(row_s)[i] = a.u;
-  }
-  const float total = block_sum(ss, scratch);
-  const float rstd = rsqrtf(total / static_cast<float>(hidden) + eps);
-  for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
-    Pack16 a, ww, o;
-    a.u = reinterpret_cast<const uint4*>(row_s)[i];
-    ww.u = reinterpret_cast<const uint4*>(w)[i];
+  };
+  auto scale = [&](int i, const Pack16& a, const Pack16& ww, float rstd) {
+    Pack16 o;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       float n = bf16_to_f32(f32_to_bf16(bf16_to_f32(a.h[j]) * rstd));
@@ -94,7 +87,67 @@ rmsnorm_kernel(const bf16* __restrict__ resid, const bf16* __restrict__ delta, c
       o.h[j] = f32_to_bf16(n * g);
     }
     reinterpret_cast<uint4*>(out + base)[i] = o.u;
+  };
+  if constexpr (VPT > 0) {
+    Pack16 a[VPT], d[VPT], ww[VPT];
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const int i = threadIdx.x + k * kRowThreads;
+      if (i >= nvec) break;
+      a[k].u = reinterpret_cast<const uint4*>(resid + base)[i];
+      if (kAdd) d[k].u = reinterpret_cast<const uint4*>(delta + base)[i];
+    }
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const int i = threadIdx.x + k * kRowThreads;
+      if (i < nvec) ww[k].u = reinterpret_cast<const uint4*>(w)[i];
+    }
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const int i = threadIdx.x + k * kRowThreads;
+      if (i < nvec) add_squares(i, a[k], d[k]);
+    }
+    const float rstd = rsqrtf(block_sum(ss, scratch) / static_cast<float>(hidden) + eps);
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const int i = threadIdx.x + k * kRowThreads;
+      if (i < nvec) scale(i, a[k], ww[k], rstd);
+    }
+  } else {
+    for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
+      Pack16 a, d;
+      a.u = reinterpret_cast<const uint4*>(resid + base)[i];
+      if (kAdd) d.u = reinterpret_cast<const uint4*>(delta + base)[i];
+      add_squares(i, a, d);
+      reinterpret_cast<uint4*>(row_s)[i] = a.u;
+    }
+    const float rstd = rsqrtf(block_sum(ss, scratch) / static_cast<float>(hidden) + eps);
+    for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
+      Pack16 a, ww;
+      a.u = reinterpret_cast<const uint4*>(row_s)[i];
+      ww.u = reinterpret_cast<const uint4*>(w)[i];
+      scale(i, a, ww, rstd);
+    }
   }
+}
+
+template <bool kAdd>
+static int launch_rmsnorm(const bf16* resid, const bf16* delta, const bf16* w, bf16* resid_out, bf16* out, int rows, int hidden, float eps,
+                          int one_plus_w, cudaStream_t st) {
+  const int vpt = dgpp_ceil_div(hidden / 8, kRowThreads);
+  auto kern = vpt <= 1 ? rmsnorm_kernel<kAdd, 1> : vpt == 2 ? rmsnorm_kernel<kAdd, 2> : vpt == 3 ? rmsnorm_kernel<kAdd, 3>
+                                                          : vpt == 4 ? rmsnorm_kernel<kAdd, 4> : rmsnorm_kernel<kAdd, 0>;
+  size_t smem = 0;
+  if (vpt > 4) {
+    smem = static_cast<size_t>(hidden) * 2;
+    static bool attr = false;
+    if (!attr) {
+      DGPP_CUDA_OK(cudaFuncSetAttribute(rmsnorm_kernel<kAdd, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+      attr = true;
+    }
+  }
+  DGPP_CUDA_OK(launch_early(kern, rows, kRowThreads, smem, st, resid, delta, w, resid_out, out, hidden, eps, one_plus_w));
+  return 0;
 }
 
 // gate_up: [rows, 2*inter] (gate then up); out: [rows, inter].  limit > 0 clamps gate above and up both sides.
@@ -311,29 +364,10 @@ DGPP_API int dgpp_rmsnorm(const void* resid, const void* delta, const void* w, v
   DGPP_REQUIRE(hidden % 8 == 0, "rmsnorm: hidden %d must be a multiple of 8", hidden);
   DGPP_REQUIRE(hidden * 2 <= 96 * 1024, "rmsnorm: hidden %d too large for the row buffer", hidden);
   if (rows == 0) return 0;
-  const size_t smem = static_cast<size_t>(hidden) * 2;
-  if (delta) {
-    static bool attr_set = false;
-    if (!attr_set) {
-      cudaFuncSetAttribute(rmsnorm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-      cudaFuncSetAttribute(rmsnorm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-      attr_set = true;
-    }
-    DGPP_CUDA_OK(launch_early(rmsnorm_kernel<true>, rows, kRowThreads, smem, st, 
-        static_cast<const bf16*>(resid), static_cast<const bf16*>(delta), static_cast<const bf16*>(w),
-        static_cast<bf16*>(resid_out), static_cast<bf16*>(out), hidden, eps, one_plus_w));
-  } else {
-    static bool attr_set2 = false;
-    if (!attr_set2) {
-      cudaFuncSetAttribute(rmsnorm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-      attr_set2 = true;
-    }
-    DGPP_CUDA_OK(launch_early(rmsnorm_kernel<false>, rows, kRowThreads, smem, st, static_cast<const bf16*>(resid), nullptr,
-                                                          static_cast<const bf16*>(w), nullptr,
-                                                          static_cast<bf16*>(out), hidden, eps, one_plus_w));
-  }
-  DGPP_CUDA_OK(cudaGetLastError());
-  return 0;
+  const bf16 *x = static_cast<const bf16*>(resid), *ww = static_cast<const bf16*>(w);
+  bf16* y = static_cast<bf16*>(out);
+  if (delta) return launch_rmsnorm<true>(x, static_cast<const bf16*>(delta), ww, static_cast<bf16*>(resid_out), y, rows, hidden, eps, one_plus_w, st);
+  return launch_rmsnorm<false>(x, nullptr, ww, nullptr, y, rows, hidden, eps, one_plus_w, st);
 }
 
 static dim3 swiglu_block(int inter) {
