@@ -479,3 +479,51 @@ def test_swiglu_of_several_rows_per_block(dev, inter, rows, bn):
     keep = torch.ones(rows, dtype=torch.bool, device=dev)
     keep[bn:2 * bn] = False
     assert torch.equal(out[keep], ops.swiglu(gu)[keep]) and (out[~keep] == 7.0).all()
+
+
+@pytest.mark.parametrize("d,hq,hkv,rot,norm", [(128, 10, 2, 128, True), (256, 5, 1, 64, True), (64, 33, 4, 64, False)])
+def test_rope_of_many_heads_per_warp(dev, d, hq, hkv, rot, norm):
+    """A pass with so many rows that a warp takes several heads (a remainder of a group of four, and of the heads' share,
+    among them) writes what passes of a few rows, a warp per head, write: rotated rows, cache bytes and scales."""
+    from dgpp_b200.engine.kv_cache import PagedKV
+    from dgpp_b200.ops import core as ops, reference as ref
+
+    torch.manual_seed(d + hq)
+    heads, page = hq + 2 * hkv, 64
+    rows = 32 * 200 * 7 // heads
+    inv_freq, _ = ref.rope_inv_freq(rot, 1e4, dev)
+    qkv = torch.randn(rows, heads * d, device=dev).to(torch.bfloat16)
+    w = (1 + 0.1 * torch.randn(2, d, device=dev)).to(torch.bfloat16) if norm else (None, None)
+    pos = torch.randperm(rows, device=dev).to(torch.int32)
+    req = torch.zeros(rows, device=dev, dtype=torch.int32)
+    got = []
+    for step in (rows, 3):
+        kv = PagedKV(1, hkv, d, rows // page + 4, 2, rows // page + 2, page, True, dev)
+        assert kv.reserve(0, rows)
+        x = qkv.clone()
+        for i in range(0, rows if step == rows else 301, step):
+            ops.rope_kv_write(x[i:i + step], pos[i:i + step], req[i:i + step], kv.block_table, inv_freq, kv.layers[0], hq, hkv, d, rot_dim=rot,
+                              q_norm_w=w[0], k_norm_w=w[1])
+        got.append((x, kv.layers[0], kv.block_table[0].long()))
+    at = pos[:303].long()
+    (x, c, bt), (y, e, bt2) = got
+    assert torch.equal(x[:303], y[:303])
+    for name in ("k", "v", "k_scale", "v_scale"):
+        a, b = getattr(c, name), getattr(e, name)
+        assert torch.equal(a[bt[at // page], :, at % page], b[bt2[at // page], :, at % page]), name
+
+
+@pytest.mark.parametrize("hidden", [8, 2048, 2056, 4104, 6144, 8192, 8200])
+def test_rmsnorm_of_every_register_count(dev, hidden):
+    """Rows of one to four vectors per thread with remainders, and one vector more (through shared memory)."""
+    from dgpp_b200.ops import core as ops, reference as ref
+
+    torch.manual_seed(hidden)
+    x, d = (torch.randn(3, hidden, device=dev).to(torch.bfloat16) for _ in range(2))
+    w = (1 + 0.1 * torch.randn(hidden, device=dev)).to(torch.bfloat16)
+    r = x.clone()
+    want, res = ref.rmsnorm(x, w, 1e-6, d)
+    got = ops.rmsnorm(r, w, 1e-6, delta=d)
+    assert torch.equal(r, res)
+    _close(got, want, 2 ** -6, 1e-3)          # two bf16 roundings, either of which may fall the other way
+    _close(ops.rmsnorm(x, w, 1e-6), ref.rmsnorm(x, w, 1e-6)[0], 2 ** -6, 1e-3)
