@@ -2,7 +2,7 @@
 // ordered combine around the grouped expert GEMMs: on bf16 rows in tiles of 32 to 192 (gemm_tc_pair.cu), or with 4-bit activations
 // in tiles of 64 (gemm_fp4.cu, grouped mode with one token tile per slot).
 //
-//   moe_segment_sort_kernel   one CTA.  Histogram of the pairs per local expert, tiles per expert = ceil(n_e / bn),
+//   moe_segment_sort_kernel   one cluster.  Histogram of the pairs per local expert, tiles per expert = ceil(n_e / bn),
 //                             exclusive scan -> first tile of every expert; then a STABLE rank of every pair inside its
 //                             expert (pairs keep their (token, k) order), so row = tile * bn + rank % bn is a pure function
 //                             of the routing result.  Outputs pair_row [T * k] (-1: expert lives on another rank),
@@ -22,6 +22,10 @@ namespace dgpp {
 constexpr int kSortThreads = 1024;
 constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kSortMaxExperts = 512;
+// CTAs of the sort (one cluster).  A warp ranks 32 pairs at a time, and the matching of their experts is slow: on one SM, 16384 pairs were
+// 23 us; loading a warp's ids ahead changed nothing.  Eight SMs: 11 us.  Below a few pairs per warp one CTA does.
+constexpr int kSortCtas = 8;
+constexpr int kSortSplitPairs = 2048;
 
 struct SortArgs {
   const int32_t* ids;      // [T, k] global expert ids
@@ -32,16 +36,17 @@ struct SortArgs {
 };
 
 __global__ void __launch_bounds__(kSortThreads) moe_segment_sort_kernel(SortArgs a) {
-  // per-warp histograms (later: per-warp running offsets), the experts' totals / first tiles
+  // per-warp histograms (later: per-warp running offsets), the experts' totals in this CTA / first tiles
   extern __shared__ int ssm[];
   int* hist = ssm;                                  // [warps][E]
   int* first_tile = hist + kSortWarps * a.E;        // [E]
   int* total = first_tile + a.E;                    // [E]
   pdl_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = blockIdx.x, ctas = gridDim.x;    // one cluster
   const int P = a.T * a.k;
-  const int seg = (P + kSortWarps - 1) / kSortWarps;           // pairs per warp, contiguous and in order
-  const int p0 = warp * seg, p1 = min(P, p0 + seg);
+  const int seg = (P + ctas * kSortWarps - 1) / (ctas * kSortWarps);      // pairs per warp, contiguous and in order
+  const int p0 = min(P, (rank * kSortWarps + warp) * seg), p1 = min(P, p0 + seg);
   for (int i = tid; i < kSortWarps * a.E; i += kSortThreads) hist[i] = 0;
   __syncthreads();
   // pass 1: histogram of this warp's segment (shared-memory atomics: counts are order-independent)
@@ -53,6 +58,7 @@ __global__ void __launch_bounds__(kSortThreads) moe_segment_sort_kernel(SortArgs
   // per expert: exclusive scan over the warps (a warp's pairs come before the next warp's) and the total
   for (int e = tid; e < a.E; e += kSortThreads) {
     int run = 0;
+#pragma unroll 8
     for (int w = 0; w < kSortWarps; ++w) {
       const int c = hist[w * a.E + e];
       hist[w * a.E + e] = run;
@@ -60,12 +66,25 @@ __global__ void __launch_bounds__(kSortThreads) moe_segment_sort_kernel(SortArgs
     }
     total[e] = run;
   }
-  __syncthreads();
-  // tiles per expert and their first tile (thread = expert, a scan over the block: one thread's walk over 512 experts was most of
-  // this kernel, 55 us at 2048 rows of 8 picks, 23 so)
+  cluster_barrier();
+  // over the CTAs of the cluster (thread = expert): pairs in the CTAs before this one, pairs in all of them
+  int ahead = 0, count = 0;
+  if (tid < a.E) {
+    const uint32_t mine = smem_u32(total + tid);
+#pragma unroll
+    for (int c = 0; c < kSortCtas; ++c) {
+      if (c >= ctas) break;
+      int v;
+      asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(mapa_shared(mine, c)) : "memory");
+      ahead += c < rank ? v : 0;
+      count += v;
+    }
+  }
+  // tiles per expert and their first tile (a scan over the block: one thread's walk over 512 experts was most of this kernel, 55 us at
+  // 2048 rows of 8 picks on one CTA, 23 so)
   {
     __shared__ int warp_sum[kSortWarps];
-    const int nt = tid < a.E ? (total[tid] + a.bn - 1) / a.bn : 0;
+    const int nt = tid < a.E ? (count + a.bn - 1) / a.bn : 0;
     int incl = nt;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -81,10 +100,14 @@ __global__ void __launch_bounds__(kSortThreads) moe_segment_sort_kernel(SortArgs
     }
     const int t = before + incl - nt;
     if (tid < a.E) first_tile[tid] = t;
-    for (int i = 0; i < nt && t + i < a.max_tiles; ++i) a.tile_expert[t + i] = tid;
-    for (int i = all + tid; i < a.max_tiles; i += kSortThreads) a.tile_expert[i] = -1;
-    if (tid == 0) *a.n_tiles = min(all, a.max_tiles);
+    if (rank == 0) {
+      for (int i = 0; i < nt && t + i < a.max_tiles; ++i) a.tile_expert[t + i] = tid;
+      for (int i = all + tid; i < a.max_tiles; i += kSortThreads) a.tile_expert[i] = -1;
+      if (tid == 0) *a.n_tiles = min(all, a.max_tiles);
+    }
   }
+  cluster_barrier();      // every CTA has read the others' totals: their places take what comes before this CTA
+  if (tid < a.E) total[tid] = ahead;
   __syncthreads();
   // pass 2: stable rank.  A warp walks its segment 32 pairs at a time; lanes with the same expert form a group whose
   // members are ranked by lane order, the group's lowest lane advances the warp's running offset of that expert.
@@ -107,7 +130,7 @@ __global__ void __launch_bounds__(kSortThreads) moe_segment_sort_kernel(SortArgs
     if (p < p1) {
       int row = -1;
       if (e >= 0) {
-        const int r = start + rank_in_group;
+        const int r = total[e] + start + rank_in_group;
         const int tile = first_tile[e] + r / a.bn;
         row = tile < a.max_tiles ? tile * a.bn + r % a.bn : -1;
       }
@@ -130,7 +153,10 @@ __global__ void __launch_bounds__(128) moe_gather_rows_kernel(const bf16* __rest
   for (int i = threadIdx.x; i < H / 8; i += blockDim.x) dst[i] = src[i];
 }
 
-// grid (ceil(H / 8 / 256), T)
+// grid (ceil(H / 8 / 256), T).  Memory bound; four of a token's rows are in flight per thread (2048 tokens of 8 rows of 4096: 34 us with one, 30
+// so).
+constexpr int kCombineRowsBatch = 4;
+
 __global__ void __launch_bounds__(256) moe_combine_rows_kernel(const bf16* __restrict__ y, const bf16* __restrict__ shared,
                                                                const int32_t* __restrict__ pair_row, const float* __restrict__ w,
                                                                bf16* __restrict__ out, int H, int k) {
@@ -138,23 +164,33 @@ __global__ void __launch_bounds__(256) moe_combine_rows_kernel(const bf16* __res
   const int t = blockIdx.y;
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v * 8 >= H) return;
+  Pack16 sh;
+  if (shared) sh.u = *reinterpret_cast<const uint4*>(shared + static_cast<size_t>(t) * H + v * 8);
   float acc[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-  for (int i = 0; i < k; ++i) {
-    const int row = pair_row[t * k + i];
-    if (row < 0) continue;
-    const float wi = w[t * k + i];
-    Pack16 p;
-    p.u = *reinterpret_cast<const uint4*>(y + static_cast<size_t>(row) * H + v * 8);
+  for (int i0 = 0; i0 < k; i0 += kCombineRowsBatch) {
+    int row[kCombineRowsBatch];
+    float wi[kCombineRowsBatch];
+    Pack16 p[kCombineRowsBatch];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] = fmaf(wi, bf16_to_f32(p.h[j]), acc[j]);
+    for (int i = 0; i < kCombineRowsBatch; ++i) {
+      row[i] = i0 + i < k ? pair_row[t * k + i0 + i] : -1;
+      wi[i] = i0 + i < k ? w[t * k + i0 + i] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < kCombineRowsBatch; ++i)
+      if (row[i] >= 0) p[i].u = *reinterpret_cast<const uint4*>(y + static_cast<size_t>(row[i]) * H + v * 8);
+#pragma unroll
+    for (int i = 0; i < kCombineRowsBatch; ++i) {
+      if (row[i] < 0) continue;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[j] = fmaf(wi[i], bf16_to_f32(p[i].h[j]), acc[j]);
+    }
   }
   if (shared) {
-    Pack16 p;
-    p.u = *reinterpret_cast<const uint4*>(shared + static_cast<size_t>(t) * H + v * 8);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] += bf16_to_f32(p.h[j]);
+    for (int j = 0; j < 8; ++j) acc[j] += bf16_to_f32(sh.h[j]);
   }
   Pack16 o;
 #pragma unroll
@@ -185,7 +221,20 @@ DGPP_API int dgpp_moe_segment_sort(const void* ids, void* pair_row, void* tile_e
     DGPP_CUDA_OK(cudaFuncSetAttribute(moe_segment_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
     attr = true;
   }
-  DGPP_CUDA_OK(launch_early(moe_segment_sort_kernel, 1, kSortThreads, smem, st, a));
+  cudaLaunchConfig_t cfg = {};
+  const int ctas = T * k >= kSortSplitPairs ? kSortCtas : 1;
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(kSortThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = static_cast<unsigned>(ctas); at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = stream_captures(st) ? 1 : 2;
+  DGPP_CUDA_OK(cudaLaunchKernelEx(&cfg, moe_segment_sort_kernel, a));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -186,6 +186,12 @@ def test_segment_sort_is_a_stable_counting_sort_into_tiles(dev, T, k, E, e0, e1)
         assert rows[p] == (want_rows[p] if e0 <= x < e1 else -1)
 
 
+@pytest.mark.parametrize("T,k,E,e0,e1", [(255, 8, 40, 0, 40), (2048, 8, 40, 0, 40), (2049, 8, 40, 8, 33), (4097, 9, 512, 0, 512)])
+def test_segment_sort_over_a_cluster(dev, T, k, E, e0, e1):
+    """The last pair count that one CTA sorts, and clusters whose warps have whole and partial segments."""
+    test_segment_sort_is_a_stable_counting_sort_into_tiles(dev, T, k, E, e0, e1)
+
+
 @pytest.mark.parametrize("rows,shared,terms,tol", [(100, 512, 3, 2e-2), (700, 0, 3, 2e-2), (700, 512, 1, 1.2e-1),
                                                    (300, 0, 2, 2e-2)])
 def test_moe_prefill_path_matches_the_expert_loop(dev, rows, shared, terms, tol):
