@@ -329,7 +329,7 @@ class MoEBlock:
         xs, h, act, y = ws["xs"][:rows], ws["h"][:rows], ws["act"][:rows], ws["y"][:rows]
         ops.moe_gather_rows(xn, pair_row, xs, c.top_k)
         ops.gemm_tc_pair_grouped(xs, w.gu_q, w.gu_sf, w.gu_alpha, h, 2 * c.moe_ffn, c.hidden, self.stack_experts, tiles, bn)
-        ops.swiglu_tiles(h, act, tiles, bn, c.swiglu_limit, c.swiglu_alpha)
+        ops.swiglu_rows(h, act, pair_row, c.swiglu_limit, c.swiglu_alpha)
         ops.gemm_tc_pair_grouped(act, w.down_q, w.down_sf, w.down_alpha, y, c.hidden, c.moe_ffn, self.stack_experts, tiles, bn)
         sh = None
         if w.shared_gu is not None:

@@ -83,6 +83,16 @@ def swiglu_tiles(gate_up: torch.Tensor, out: torch.Tensor, tiles: torch.Tensor, 
     return out
 
 
+_lib.declare("dgpp_swiglu_rows", [P, P, P, I, I, F, F, P])
+
+
+def swiglu_rows(gate_up: torch.Tensor, out: torch.Tensor, rows_of: torch.Tensor, limit: float = 0.0, alpha: float = 0.0) -> torch.Tensor:
+    """`swiglu` of the rows that `rows_of` (int32, any order, negative entries: none) lists; the others are left alone."""
+    _chk(gate_up, torch.bfloat16, "gate_up")
+    call("dgpp_swiglu_rows", ptr(gate_up), ptr(out), ptr(rows_of), rows_of.numel(), out.shape[-1], float(limit), float(alpha), stream_ptr())
+    return out
+
+
 def argmax(logits: torch.Tensor, id_base: int = 0, out_id: Optional[torch.Tensor] = None,
            out_val: Optional[torch.Tensor] = None):
     rows, vocab = logits.shape

@@ -527,3 +527,19 @@ def test_rmsnorm_of_every_register_count(dev, hidden):
     assert torch.equal(r, res)
     _close(got, want, 2 ** -6, 1e-3)          # two bf16 roundings, either of which may fall the other way
     _close(ops.rmsnorm(x, w, 1e-6), ref.rmsnorm(x, w, 1e-6)[0], 2 ** -6, 1e-3)
+
+
+@pytest.mark.parametrize("inter,rows", [(8, 9), (1536, 40), (2056, 5)])
+def test_swiglu_of_listed_rows(dev, inter, rows):
+    """Rows in any order; entries below zero and rows that are not listed are left alone."""
+    from dgpp_b200.ops import core as ops
+
+    torch.manual_seed(inter + 1)
+    gu = torch.randn(rows, 2 * inter, device=dev).to(torch.bfloat16)
+    listed = torch.randperm(rows, device=dev)[:rows // 2].to(torch.int32)
+    of = torch.full((2 * listed.numel() + 1,), -1, dtype=torch.int32, device=dev)
+    of[1::2] = listed
+    out = ops.swiglu_rows(gu, torch.full((rows, inter), 7.0, device=dev, dtype=torch.bfloat16), of)
+    keep = torch.zeros(rows, dtype=torch.bool, device=dev)
+    keep[listed.long()] = True
+    assert torch.equal(out[keep], ops.swiglu(gu)[keep]) and (out[~keep] == 7.0).all()
