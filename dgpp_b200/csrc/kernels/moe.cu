@@ -83,62 +83,86 @@ __global__ void __launch_bounds__(kRouterThreads) moe_router_logits_kernel(Route
   }
 }
 
-// The same products at prompt sizes: a warp owns four experts and eight tokens, so a lane converts its share of 12 rows for 32
-// products and not of 9 for 8 (that kernel is bound by the conversions and the loads), and the 32 sums are exchanged as they are added,
-// 31 shuffles and not 160.  Every dot product is the same lane-strided chain and the same tree: the same bits.  grid (ceil(E / 32),
-// ceil(T / 8)).  2048 rows x 256 experts x 4096: 299 us there, 160 here.
-constexpr int kRouterTileE = 4;
-
-__global__ void __launch_bounds__(kRouterThreads, 2) moe_router_logits_tile_kernel(RouterArgs a) {
+// The same products at prompt sizes: a warp owns RE experts and eight tokens, so a lane converts its share of RE + 8 rows for 8 RE
+// products and not of 9 for 8 (that kernel is bound by the conversions and the loads), and the sums are exchanged as they are added,
+// 31 shuffles for 32 and not 160.  Every dot product is the same lane-strided chain and the same tree: the same bits.  grid (ceil(E / (8 RE)),
+// ceil(T / 8)).  2048 rows x 256 experts x 4096: 299 us there, 160 with four experts per warp, 146 with eight, which ask for the next
+// step's rows before this step's products (one CTA per SM).
+template <int RE>
+__global__ void __launch_bounds__(kRouterThreads, RE == 4 ? 2 : 1) moe_router_logits_tile_kernel(RouterArgs a) {
   pdl_wait();
-  constexpr int RT = kRouterRowsPerCta, RE = kRouterTileE;
+  constexpr int RT = kRouterRowsPerCta, NB = RE == 4 ? 1 : 2;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int e0 = (blockIdx.x * (kRouterThreads / 32) + wid) * RE, t0 = blockIdx.y * RT;
   if (e0 >= a.E) return;
-  const bf16 *gp[RE], *xp[RT];           // (rows past the end repeat the last one)
+  // (rows past the end repeat the last one)
+  auto gate_row = [&](int e) { return a.gate + static_cast<size_t>(min(e0 + e, a.E - 1)) * a.H; };
+  auto x_row = [&](int r) { return a.x + static_cast<size_t>(min(t0 + r, a.T - 1)) * a.x_stride; };
+  float acc[RE / 4][RT * 4];
 #pragma unroll
-  for (int e = 0; e < RE; ++e) gp[e] = a.gate + static_cast<size_t>(min(e0 + e, a.E - 1)) * a.H;
+  for (int h = 0; h < RE / 4; ++h)
 #pragma unroll
-  for (int r = 0; r < RT; ++r) xp[r] = a.x + static_cast<size_t>(min(t0 + r, a.T - 1)) * a.x_stride;
-  float acc[RT * RE];
+    for (int i = 0; i < RT * 4; ++i) acc[h][i] = 0.f;
+  uint4 g[NB][RE], x[NB][RT];
+  auto request = [&](int b, int i) {
 #pragma unroll
-  for (int i = 0; i < RT * RE; ++i) acc[i] = 0.f;
-  for (int i = lane * 8; i < a.H; i += 32 * 8) {
-    uint4 g[RE], x[RT];
+    for (int e = 0; e < RE; ++e) g[b][e] = *reinterpret_cast<const uint4*>(gate_row(e) + i);
 #pragma unroll
-    for (int e = 0; e < RE; ++e) g[e] = *reinterpret_cast<const uint4*>(gp[e] + i);
-#pragma unroll
-    for (int r = 0; r < RT; ++r) x[r] = *reinterpret_cast<const uint4*>(xp[r] + i);
+    for (int r = 0; r < RT; ++r) x[b][r] = *reinterpret_cast<const uint4*>(x_row(r) + i);
+  };
+  auto products = [&](int b) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       float glo[RE], ghi[RE];
 #pragma unroll
       for (int e = 0; e < RE; ++e) {
-        const uint32_t w = q == 0 ? g[e].x : q == 1 ? g[e].y : q == 2 ? g[e].z : g[e].w;
+        const uint32_t w = q == 0 ? g[b][e].x : q == 1 ? g[b][e].y : q == 2 ? g[b][e].z : g[b][e].w;
         glo[e] = __uint_as_float(w << 16);
         ghi[e] = __uint_as_float(w & 0xffff0000u);
       }
 #pragma unroll
       for (int r = 0; r < RT; ++r) {
-        const uint32_t w = q == 0 ? x[r].x : q == 1 ? x[r].y : q == 2 ? x[r].z : x[r].w;
+        const uint32_t w = q == 0 ? x[b][r].x : q == 1 ? x[b][r].y : q == 2 ? x[b][r].z : x[b][r].w;
         const float lo = __uint_as_float(w << 16), hi = __uint_as_float(w & 0xffff0000u);
 #pragma unroll
-        for (int e = 0; e < RE; ++e) acc[r * RE + e] = fmaf(hi, ghi[e], fmaf(lo, glo[e], acc[r * RE + e]));
+        for (int e = 0; e < RE; ++e) {
+          float& c = acc[e / 4][r * 4 + e % 4];
+          c = fmaf(hi, ghi[e], fmaf(lo, glo[e], c));
+        }
       }
     }
-  }
-  // 32 sums over 32 lanes: at distance o a lane keeps the half of its sums that its bit o names and adds the partner's share of them
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const bool up = (lane & o) != 0;
-#pragma unroll
-    for (int i = 0; i < o; ++i) {
-      const float keep = up ? acc[i + o] : acc[i], give = up ? acc[i] : acc[i + o];
-      acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+  };
+  constexpr int kStep = 32 * 8;
+  if (NB == 1) {
+    for (int i = lane * 8; i < a.H; i += kStep) {
+      request(0, i);
+      products(0);
+    }
+  } else {
+    int i = lane * 8;
+    if (i < a.H) request(0, i);
+    for (; i < a.H; i += 2 * kStep) {
+      if (i + kStep < a.H) request(NB - 1, i + kStep);
+      products(0);
+      if (i + 2 * kStep < a.H) request(0, i + 2 * kStep);
+      if (i + kStep < a.H) products(NB - 1);
     }
   }
-  const int t = t0 + lane / RE, e = e0 + lane % RE;
-  if (t < a.T && e < a.E) a.logits_out[t * a.logits_stride + e] = acc[0];
+#pragma unroll
+  for (int h = 0; h < RE / 4; ++h) {
+    // 32 sums over 32 lanes: at distance o a lane keeps the half of its sums that its bit o names and adds the partner's share of them
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int i = 0; i < o; ++i) {
+        const float keep = up ? acc[h][i + o] : acc[h][i], give = up ? acc[h][i] : acc[h][i + o];
+        acc[h][i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+    }
+    const int t = t0 + lane / 4, e = e0 + 4 * h + lane % 4;
+    if (t < a.T && e < a.E) a.logits_out[t * a.logits_stride + e] = acc[h][0];
+  }
 }
 
 // Selection: one CTA per token over its row of logits.  PER: expert values that a lane of the picking warp holds, E <= 32 PER (2048
@@ -299,32 +323,50 @@ __global__ void __launch_bounds__(512) moe_active_kernel(const int32_t* ids, int
 }
 
 // y: [slots, rows_per_slot, H] bf16; shared (optional): [T, H] bf16; out: [T, H] bf16.
-__global__ void __launch_bounds__(256) moe_combine_kernel(const bf16* __restrict__ y, const bf16* __restrict__ shared,
+// Latency bound at decode sizes: lane i of every warp looks up choice i's slot, and eight of the chosen rows are in flight at a time (one
+// id, slot and row after the other: 6.4 us at 8 rows of 10 choices, 3.5 so).
+constexpr int kCombineThreads = 128, kCombineBatch = 8;
+
+__global__ void __launch_bounds__(kCombineThreads) moe_combine_kernel(const bf16* __restrict__ y, const bf16* __restrict__ shared,
                                                           const int32_t* __restrict__ ids, const float* __restrict__ w,
                                                           const int32_t* __restrict__ slot_of, bf16* __restrict__ out,
                                                           int T, int H, int k, int rows_per_slot) {
   pdl_wait();
-  const int t = blockIdx.y;
+  const int t = blockIdx.y, lane = threadIdx.x & 31;
   const int v = blockIdx.x * blockDim.x + threadIdx.x;   // 8-wide vector index
-  if (v * 8 >= H) return;
+  const bool live = v * 8 < H;
+  Pack16 sh;
+  if (shared && live) sh.u = *reinterpret_cast<const uint4*>(shared + static_cast<size_t>(t) * H + v * 8);
   float acc[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-  for (int i = 0; i < k; ++i) {
-    const int e = ids[t * k + i];
-    const int s = slot_of[e];
-    if (s < 0) continue;
-    const float wi = w[t * k + i];
-    Pack16 p;
-    p.u = *reinterpret_cast<const uint4*>(y + (static_cast<size_t>(s) * rows_per_slot + t) * H + v * 8);
+  int slot = -1;
+  float weight = 0.f;
+  for (int i0 = 0; i0 < k; i0 += kCombineBatch) {
+    if ((i0 & 31) == 0) {
+      const bool has = i0 + lane < k;
+      slot = has ? slot_of[ids[t * k + i0 + lane]] : -1;
+      weight = has ? w[t * k + i0 + lane] : 0.f;
+    }
+    Pack16 p[kCombineBatch];
+    int s[kCombineBatch];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] = fmaf(wi, bf16_to_f32(p.h[j]), acc[j]);
+    for (int i = 0; i < kCombineBatch; ++i) {
+      s[i] = __shfl_sync(0xffffffffu, slot, (i0 + i) & 31);
+      if (live && s[i] >= 0) p[i].u = *reinterpret_cast<const uint4*>(y + (static_cast<size_t>(s[i]) * rows_per_slot + t) * H + v * 8);
+    }
+#pragma unroll
+    for (int i = 0; i < kCombineBatch; ++i) {
+      const float wi = __shfl_sync(0xffffffffu, weight, (i0 + i) & 31);
+      if (s[i] < 0) continue;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[j] = fmaf(wi, bf16_to_f32(p[i].h[j]), acc[j]);
+    }
   }
+  if (!live) return;
   if (shared) {
-    Pack16 p;
-    p.u = *reinterpret_cast<const uint4*>(shared + static_cast<size_t>(t) * H + v * 8);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] += bf16_to_f32(p.h[j]);
+    for (int j = 0; j < 8; ++j) acc[j] += bf16_to_f32(sh.h[j]);
   }
   Pack16 o;
 #pragma unroll
@@ -411,9 +453,11 @@ DGPP_API int dgpp_moe_route(const void* x, int64_t x_stride, const void* gate, c
   a.softmax = softmax; a.norm_topk = norm_topk; a.scaling = scaling;
   DGPP_REQUIRE(logits_out != nullptr, "moe_route: a [T, E] fp32 logits buffer is required");
   const dim3 grid(dgpp_ceil_div(E, kRouterThreads / 32), dgpp_ceil_div(T, kRouterRowsPerCta));
-  const dim3 tiles(dgpp_ceil_div(E, kRouterTileE * kRouterThreads / 32), grid.y);
-  // (two CTAs per SM take the tiles: below one for each, the finer split is the faster one)
-  if (tiles.x * tiles.y >= 296) DGPP_CUDA_OK(launch_early(moe_router_logits_tile_kernel, tiles, kRouterThreads, 0, st, a));
+  auto tiles = [&](int experts) { return dim3(dgpp_ceil_div(E, experts * kRouterThreads / 32), grid.y); };
+  // (a CTA per SM takes the tiles of eight experts per warp, two those of four: below two and one waves of them the finer split is faster)
+  const dim3 t8 = tiles(8), t4 = tiles(4);
+  if (t8.x * t8.y >= 296) DGPP_CUDA_OK(launch_early(moe_router_logits_tile_kernel<8>, t8, kRouterThreads, 0, st, a));
+  else if (t4.x * t4.y >= 296) DGPP_CUDA_OK(launch_early(moe_router_logits_tile_kernel<4>, t4, kRouterThreads, 0, st, a));
   else DGPP_CUDA_OK(launch_early(moe_router_logits_kernel, grid, kRouterThreads, 0, st, a));
   DGPP_CUDA_OK(cudaGetLastError());
   return launch_select(a, st);
@@ -451,8 +495,8 @@ DGPP_API int dgpp_moe_combine(const void* y, const void* shared, const void* ids
                               void* out, int T, int H, int k, int rows_per_slot, cudaStream_t st) {
   DGPP_REQUIRE(H % 8 == 0, "moe_combine: hidden %d must be a multiple of 8", H);
   if (T == 0) return 0;
-  dim3 grid(dgpp_ceil_div(H / 8, 256), T);
-  DGPP_CUDA_OK(launch_early(moe_combine_kernel, grid, 256, 0, st, static_cast<const bf16*>(y), static_cast<const bf16*>(shared),
+  dim3 grid(dgpp_ceil_div(H / 8, kCombineThreads), T);
+  DGPP_CUDA_OK(launch_early(moe_combine_kernel, grid, kCombineThreads, 0, st, static_cast<const bf16*>(y), static_cast<const bf16*>(shared),
                                            static_cast<const int32_t*>(ids), static_cast<const float*>(w),
                                            static_cast<const int32_t*>(slot_of), static_cast<bf16*>(out), T, H, k,
                                            rows_per_slot));
