@@ -139,7 +139,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   }
   // The first tiles are on their way and their token scales requested while q is staged: warp 0 looks up all of their pages at once (at
   // most 3 x 8), its first lane, which made the barriers, issues.  (Looked up one by one behind the staging: 17.4 us at 8 rows of 40 / 8 heads
-  // over 2048, 14.8 so; 8 rows of 16 / 2 heads of 256: 14.1, 11.4 so.)
+  // over 2048, 16.4 so; 8 rows of 16 / 2 heads of 256: 14.1, 12.6 so; a row over 64 positions 7.7, 7.2 so.)
   const int ppt = kAdTile / p.page;  // pages per tile
   auto page_block = [&](int tile, int pg) {
     const int page0 = (base + (tile_begin + tile) * kAdTile) / p.page;

@@ -70,6 +70,12 @@ def test_router_logits_do_not_depend_on_the_batch(dev, rows, experts, hidden):
     assert torch.equal(all_, few)
 
 
+@pytest.mark.parametrize("rows,experts,hidden", [(603, 512, 2048), (2369, 37, 264), (2400, 70, 8)])
+def test_router_logits_of_eight_experts_per_warp(dev, rows, experts, hidden):
+    """The widest tiles, with remainders of tokens, experts and steps (an odd number of them, and less than one)."""
+    test_router_logits_do_not_depend_on_the_batch(dev, rows, experts, hidden)
+
+
 @pytest.mark.parametrize("rows,shared", [(1, 0), (8, 512), (16, 0)])
 def test_moe_block_matches_reference(dev, rows, shared):
     from dgpp_b200.models.moe import MoEBlock, MoEConfig, MoEWeights, moe_reference
