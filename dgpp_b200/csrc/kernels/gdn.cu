@@ -183,6 +183,9 @@ __global__ void __launch_bounds__(kGdnThreads) gdn_recurrent_kernel(GdnArgs a) {
       bs[tid] = bet[static_cast<size_t>(t0 + tid) * a.hv + h];
     }
     __syncthreads();
+    // (Unrolled by hand: with the state's loads in front of the wait the compiler leaves the loop rolled.  2048 tokens x 16 heads of 128,
+    // preparation included: 903 us rolled, 774 so; 48 tokens x 32 heads 27.3 / 24.8.)
+#pragma unroll 4
     for (int tt = 0; tt < n; ++tt) {
       const float decay = ds[tt];
       float m = 0.f;
