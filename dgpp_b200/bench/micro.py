@@ -283,7 +283,7 @@ def bench_attn_prefill(args, dev):
     ms = run([fn] * 2, args)
     ops.check_status()
     report(args, "attn_prefill_tc", ms, flops=4.0 * ctx * ctx / 2 * d * hq, bytes_=2.0 * ctx * hkv * d + 4.0 * ctx * hq * d,
-           ctx=ctx, hq=hq, hkv=hkv, head_dim=d, note="causal, bf16-equivalent FLOPs (two-term fp8 operands issue 4x the MMAs)")
+           ctx=ctx, hq=hq, hkv=hkv, head_dim=d, note="causal, FLOPs of one product each" + (" (two-term fp8 operands issue 4x the MMAs)" if d == 256 else " (f16 operands)"))
 
 
 def bench_act_quant(args, dev):

@@ -1,7 +1,7 @@
 // Causal flash attention for prefill at head_dim 256 over the paged FP8 KV cache, on tcgen05 (kind::f8f6f4).
 //
-// Same arithmetic as the head_dim-128 kernel (attn_prefill_tc.cu): one CTA = one query head x 128 consecutive query
-// positions; Q and P are carried as two e4m3 terms, K / V go from the cache pages to the tensor core untouched.  A
+// One CTA = one query head x 128 consecutive query positions; Q and P are carried as two e4m3 terms, K / V go from the cache
+// pages to the tensor core untouched (the head_dim-128 kernel expands them to f16 instead: at 256 its tiles would not fit).  A
 // 256-wide head is two 128-byte halves everywhere (tiles are [rows, 128 B] with the 128-byte swizzle, half 0 then half 1):
 //
 //   MMA1   S[q, t]        = sum over halves, terms of Q[q, half] . K[t, half]^T       16 MMAs of 128 x 128 x 32
