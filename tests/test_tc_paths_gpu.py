@@ -111,6 +111,27 @@ def test_cluster_quantiser_matches_the_single_cta_one(dev, rows, k, terms):
             assert ((a - b).norm() / b.norm()).item() < 2.0 ** -8 * (1 if terms > 1 else 8)
 
 
+@pytest.mark.parametrize("rows,k,terms,bn", [(65, 256, 3, 16), (130, 5120, 3, 64), (129, 2304, 1, 128), (66, 24320, 2, 16)])
+def test_bulk_quantiser_matches_the_cluster_one(dev, rows, k, terms, bn):
+    """One CTA per row above 64 rows: fewer blocks of 16 than threads, a remainder of them, the widest row; the same bits as the
+    cluster form (the row statistic is a maximum), the copy of the rows included."""
+    from dgpp_b200.ops import core as ops
+
+    torch.manual_seed(34)
+    pad = (rows + bn - 1) // bn * bn
+    for m, (mode, cols) in enumerate((("plain", k), ("swiglu", 2 * k))):
+        inp = (2 * torch.randn(rows, cols, device=dev)).to(BF)
+        inp[1].zero_()
+        got, want = ops.QuantAct(pad, k, terms, bn, dev), ops.QuantAct(pad, k, terms, bn, dev)
+        x1, x2 = (torch.empty(rows, k, device=dev, dtype=BF) for _ in range(2))
+        ops.act_quant_nvfp4(inp, terms, out=got, mode=mode, x_out=x1)
+        ops.call("dgpp_act_quant_nvfp4_cluster", m, ops.ptr(inp), inp.stride(0), None, None, None, ops.ptr(x2), ops.ptr(want.q), ops.ptr(want.sf),
+                 ops.ptr(want.g), rows, pad, k, terms, bn, 8, 1e-6, 0.0, 0.0, 0, None, None, 0, ops.stream_ptr())
+        torch.cuda.synchronize()
+        ops.check_status()
+        assert torch.equal(got.g, want.g) and torch.equal(got.q, want.q) and torch.equal(got.sf, want.sf) and torch.equal(x1, x2), mode
+
+
 def _filled_cache(dev, hq, hkv, ctx, page, slot, d=128):
     from dgpp_b200.engine.kv_cache import PagedKV
     from dgpp_b200.ops import core as ops, reference as ref
