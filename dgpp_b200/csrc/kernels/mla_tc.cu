@@ -96,7 +96,9 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmC, MlaTcParams p) {
   const int first = p.window > 0 ? max(0, len - p.window) : 0;
   const int32_t* sel = nullptr;
   if (SPARSE) {
-    // listed tokens at or before the row's own position (lists are ascending, so they form a prefix of the list)
+    // listed tokens at or before the row's own position (lists are ascending, so they form a prefix of the list); the list is the
+    // preceding kernel's output
+    pdl_wait_only();
     sel = p.sel + static_cast<size_t>(row) * p.sel_stride;
     int n = 0;
     for (int i0 = 0; i0 < p.sel_stride; i0 += kMtThreads) {
