@@ -383,6 +383,8 @@ __device__ __forceinline__ void l2_prefetch_bulk(const void* p, uint32_t bytes) 
 // pdl_wait(): block until the preceding grid has completed and its memory is visible, THEN allow the next grid
 // in the stream / graph to start launching.  Triggering only after the wait keeps the overlap to one kernel deep:
 // a grid's prologue can run under its immediate predecessor only, never under an older, still running grid.
+// A CTA that allocates tensor memory has a barrier between the allocation and this: CTAs of the next grid on the same SM could
+// take the columns first otherwise and then wait for this grid, which waits for them.
 __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -96,7 +96,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   int sel_n = 0;
   if (p.sel != nullptr) {
     // the list is the previous kernel's output: nothing of it may be read before that kernel has finished
-    pdl_wait();
+    pdl_wait_only();
     sl = p.sel + (static_cast<size_t>(row) * p.hkv + kvh) * p.sel_k;
     for (int j = 0; j < p.sel_k; ++j) sel_n += sl[j] >= 0 ? 1 : 0;
     len = sel_n > 0 ? (sel_n - 1) * p.sel_block + pos_row % p.sel_block + 1 : 0;   // every listed block is full but the last
@@ -128,6 +128,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
   }
+  __syncthreads();      // the columns are this CTA's before the next grid is let in
   pdl_wait();
   float qv[NH][G];      // requested in front of everything that depends on a table
   if (warp >= 2) {

@@ -201,6 +201,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  __syncthreads();      // the columns are this CTA's before the next grid is let in
   pdl_wait();
   // ---- the units' query rows as f16 (thread = row): scaled by a power of two to a largest magnitude of 128..256
   const int sub = warp >> 2;

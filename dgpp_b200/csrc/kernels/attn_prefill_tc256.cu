@@ -167,6 +167,7 @@ attn_prefill_tc256_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  __syncthreads();      // the columns are this CTA's before the next grid is let in
   pdl_wait();
   // ---- quantise the query rows into two e4m3 terms: thread (set, row) converts half `set` of its row; the row scale is
   //      the maximum over both halves (exchanged through shared memory)

@@ -71,6 +71,7 @@ dsa_index_tc_kernel(const __grid_constant__ CUtensorMap tmK, IndexTcParams p) {
     tmem_alloc(tmem_slot, 128);
     tmem_relinquish();
   }
+  __syncthreads();      // the columns are this CTA's before the next grid is let in
   pdl_wait();
   if (warp >= 2) {
     // query heads as the B operand: two column blocks of [64 heads, 64 elements]; heads beyond hi are zero
@@ -209,6 +210,7 @@ dsa_index_tc_fp8_kernel(const __grid_constant__ CUtensorMap tmK, IndexTcFp8Param
     tmem_alloc(tmem_slot, 256);
     tmem_relinquish();
   }
+  __syncthreads();      // the columns are this CTA's before the next grid is let in
   pdl_wait();
   if (warp >= 2) {
     // two threads per head: amax over the head, then the two e4m3 terms of the thread's 64 elements

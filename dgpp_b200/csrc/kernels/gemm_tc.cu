@@ -142,7 +142,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA,   // bf16 weights, or pa
   const int m0 = my * BN;
   int a_row = n0, b_row = m0;                        // first weight row and first activation row of this CTA
   if (!kQuant && p.groups != nullptr) {
-    pdl_wait();
+    pdl_wait_only();
     const int e = p.groups[my];
     if (e < 0) return;
     a_row = e * p.N + n0;

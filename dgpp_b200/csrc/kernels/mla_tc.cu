@@ -125,6 +125,7 @@ mla_decode_tc_kernel(const __grid_constant__ CUtensorMap tmC, MlaTcParams p) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  __syncthreads();      // the columns are this CTA's before the next grid is let in
   pdl_wait();
   const int ppt = kMtTile / p.page;
   auto load_tile = [&](int i) {

@@ -154,6 +154,7 @@ window_attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     tmem_alloc(tmem_slot, tmem_cols);
     tmem_relinquish();
   }
+  __syncthreads();      // the columns are this CTA's before the next grid is let in
   pdl_wait();
   // the run this tile lies in (tiles are dealt run by run)
   int tile = blockIdx.x, row0 = 0, ntok = 0, flat0 = 0;

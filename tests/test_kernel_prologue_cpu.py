@@ -21,6 +21,22 @@ def kernels():
 
 
 KERNELS = dict(kernels())
+ALLOCATING = {name: body for name, body in KERNELS.items() if re.search(r"\btmem_alloc(_pair)?\(", body)}
+
+
+def test_allocating_kernels_are_found():
+    assert len(ALLOCATING) >= 13 and "attn_prefill_tc_kernel" in ALLOCATING and "gemm_tc_pair_kernel" in ALLOCATING
+
+
+@pytest.mark.parametrize("name", sorted(ALLOCATING))
+def test_dependents_are_let_in_behind_the_allocation(name):
+    """The release of the next grid (`pdl_wait` carries it) stands behind the allocation, a barrier of the block between them."""
+    body = ALLOCATING[name]
+    alloc = re.search(r"\btmem_alloc(_pair)?\(", body).start()
+    release = re.search(r"\b(pdl_wait|pdl_launch_dependents)\(\)", body)
+    assert release is not None and release.start() > alloc
+    between = body[alloc:release.start()]
+    assert "__syncthreads()" in between or "cluster_barrier()" in between
 
 
 @pytest.mark.parametrize("name", ["attn_decode_tc_kernel", "mla_decode_tc_kernel"])
