@@ -2,17 +2,20 @@
 //
 // Work comes in units of one query head x 128 consecutive query positions.  A CTA takes two units of one KV head (the units of a KV
 // head are numbered longest span first, heads fastest), or one where that already occupies the device.  K / V tiles of 128 tokens
-// come from the cache pages by TMA as stored (e4m3 bytes) and are expanded once per CTA to f16, scale included:
+// come from the cache pages by TMA as stored (e4m3 bytes) and are expanded once per CTA to f16:
 //
-//   K16[t, d] = f16(K[t, d] * k_scale[t] / 2^ck)      ck, cv: exponents of the tile's largest scales; the product is rounded once
-//   V16[t, d] = f16(V[t, d] * v_scale[t] / 2^cv)      (f16 splits the scale into two terms), to 11 bits
-//   MMA1   S[q, t]  = Q16[q, d] . K16[t, d]^T          Q16 = q / 2^e of its row, exact
-//   softmax (one thread per query row): s = S * sm, p = 2^(s + cv - m), causal mask, P as f16 over the scores' own columns
+//   K16[t, d] = f16(K[t, d] * k_scale[t]) / 2^ck       ck, cv: exponents of the largest scales up to this tile; the products are
+//   V16[t, d] = f16(V[t, d] * v_scale[t]) / 2^cv       rounded once to 11 bits (the scale's mantissa in two f16 terms)
+//   MMA1   S[q, t]  = Q16[q, d] . K16[t, d]^T          Q16 = q / 2^e of its row, exact down to 2^-22 of the row's largest
+//   softmax (one thread per query row): s = S * sm * 2^ck, p = 2^(s - m), causal mask, P as f16 over the scores' own columns
 //   MMA2   O[q, d] += P[q, t] . V16[t, d]              P is the A operand in tensor memory, V the B operand read MN-major
 //
-// O stays in tensor memory.  m is a row's reference, not its maximum: it moves only when a tile exceeds it by more than 2^8
-// (f16 and the fp32 sums have the range for that), so the accumulator is rescaled a few times per row instead of once per tile.
-// Whether it moves depends on the row alone: a row's bits do not depend on what else its pass, its CTA or its unit's partner does.
+// O stays in tensor memory, in units of 2^cv.  m is a row's reference, not its maximum: it moves only when a tile exceeds it by more
+// than 2^8 (f16 and the fp32 sums have the range for that; the lazily moved maximum is a published method of flash attention on this
+// chip), so the accumulator is rescaled a few times per row, and when cv grows, instead of once per tile.  Whether m moves depends
+// on the row alone, and ck, cv are powers of two; what ties a row's bits to tokens it does not see is f16's range alone: elements of
+// K and V below 2^-14 of the largest scale's power of two are held to 2^-25 of it.  Tokens whose row is zero (their scale is a
+// placeholder) do not count for the exponents.
 //
 // Two units: the tensor core works for one while the other's threads exponentiate (S of unit u is rewritten right behind its PV
 // product).  One unit: two score buffers, S of tile i + 1 runs under the softmax of tile i.
@@ -20,7 +23,7 @@
 // 16 TMA producer, 17 MMA issuer and TMEM owner.
 // What bounds it: MUFU and tensor pipe alike (a tile of two units: 2048 cycles each), then the handshakes between them.
 // 40 query and 8 KV heads, with two e4m3 terms of q and P, one unit per CTA and the accumulator in registers / so: 173 rows behind 3000
-// 97 / 65 us, 2048 rows 205 / 115, 2048 rows behind 6144 900 / 521.
+// 92 / 64 us, 2048 rows 172 / 113, 2048 rows behind 6144 944 / 550 (the scales' mantissas, powers of two and zero rows are 5 % of that).
 // (reference counterparts: src/kernels/full_attn.cu:442,679,983 tile / TMA / fp8-compute prefill kernels.)
 #include <cuda.h>
 #include <math.h>
@@ -56,7 +59,7 @@ struct AttnPrefillParams {
 };
 
 constexpr size_t attn_prefill_smem_bytes() {
-  return 1024 + 2 * kApF16Bytes + kApRing * kApF16Bytes + kApRaw * (kApRawBytes + kApTile * 4) + 2 * 4 * 4 +
+  return 1024 + 2 * kApF16Bytes + kApRing * kApF16Bytes + kApRaw * (kApRawBytes + kApTile * 4) + 24 * 4 +
          (2 * kApRing + 2 * kApRaw + 6) * 8 + 16;
 }
 
@@ -81,7 +84,6 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
       : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return d;
 }
-
 // 32 scores of a row from tensor memory, tokens t0 .. t0 + 31; those the row does not see become -inf.
 template <bool kMask>
 __device__ __forceinline__ void scores_x32(uint32_t taddr, int t0, int my_pos, int my_first, uint32_t (&s)[32]) {
@@ -117,10 +119,10 @@ __device__ __forceinline__ void probs_x32(const uint32_t (&s)[32], float sm, flo
 
 // Scores of one tile -> probabilities.  Tokens 64..127 stay in registers between the two passes; the P operand takes over their
 // columns (64 words at column 64), tokens 0..63 are read again.  `ref` is the row's reference m, `lsum` its probability mass in
-// units of 2^m; `rescale(corr)` multiplies the accumulator (called by all lanes of a warp or by none).
+// units of 2^m; `rescale(corr)` multiplies the accumulator (called by all lanes of a warp or by none; `regrow`: in any case).
 template <bool kMask, class Rescale>
-__device__ __forceinline__ void softmax_tile(uint32_t ts, int t0, int my_pos, int my_first, float sm, int cv, float& ref, float& lsum,
-                                             Rescale rescale) {
+__device__ __forceinline__ void softmax_tile(uint32_t ts, int t0, int my_pos, int my_first, float sm, bool regrow, float& ref,
+                                             float& lsum, Rescale rescale) {
   uint32_t a[32], b[32], c[32];
   scores_x32<kMask>(ts, t0, my_pos, my_first, a);
   float mt = max_x32(a, -INFINITY);
@@ -130,16 +132,16 @@ __device__ __forceinline__ void softmax_tile(uint32_t ts, int t0, int my_pos, in
   mt = max_x32(b, mt);
   scores_x32<kMask>(ts + 96, t0 + 96, my_pos, my_first, c);
   mt = max_x32(c, mt);
-  const float top = fmaf(mt, sm, static_cast<float>(cv));   // sm > 0
+  const float top = mt * sm;                   // sm > 0
   const bool move = top > ref + kApSlack;      // (the first tile with a visible token: ref = -inf)
-  if (__any_sync(0xffffffffu, move)) {
+  if (__any_sync(0xffffffffu, move) || regrow) {
     const float next = move ? top : ref;
     const float corr = (move && ref != -INFINITY) ? fast_exp2(ref - next) : 1.f;
     ref = next;
     lsum *= corr;
     rescale(corr);
   }
-  const float off = ref == -INFINITY ? 0.f : static_cast<float>(cv) - ref;
+  const float off = ref == -INFINITY ? 0.f : -ref;
   float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
   probs_x32(b, sm, off, ts + 96, sum);
   probs_x32(c, sm, off, ts + 112, sum);
@@ -147,7 +149,7 @@ __device__ __forceinline__ void softmax_tile(uint32_t ts, int t0, int my_pos, in
   probs_x32(a, sm, off, ts + 64, sum);
   scores_x32<kMask>(ts + 32, t0 + 32, my_pos, my_first, a);
   probs_x32(a, sm, off, ts + 80, sum);
-  lsum = fmaf((sum[0].x + sum[0].y) + (sum[1].x + sum[1].y), exp2_of(-cv), lsum);
+  lsum += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
   tmem_st_wait();
 }
 
@@ -161,7 +163,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
   unsigned char* sRing = sp; sp += kApRing * kApF16Bytes;
   unsigned char* sRaw = sp;  sp += kApRaw * kApRawBytes;
   float* sScale = reinterpret_cast<float*>(sp);  sp += kApRaw * kApTile * sizeof(float);
-  int* sExp = reinterpret_cast<int*>(sp);        sp += 2 * 4 * sizeof(int);     // [K, V][tile & 3] exponents of the tile's scales
+  int* sExp = reinterpret_cast<int*>(sp);        sp += 2 * 4 * sizeof(int);        // [K, V][tile & 3] exponents ck, cv
+  int* sMax = reinterpret_cast<int*>(sp);        sp += 2 * 2 * 4 * sizeof(int);    // [K, V][tile & 1][warp] largest exponent of a warp's scales
   uint64_t* raw_full = reinterpret_cast<uint64_t*>(sp);
   uint64_t* raw_empty = raw_full + kApRaw;
   uint64_t* ring_full = raw_empty + kApRaw;
@@ -332,46 +335,65 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     // ------------------------------------------------------------------ expansion to f16: four warps for K, four for V, thread = token
     const int v = (warp - kApConv) >> 2, t = (warp & 3) * 32 + lane;
     bool ok = true;
+    int unit = -100;      // exponent of the largest scale so far, at least this
+    constexpr int kGaveUp = 1 << 20;
     for (int i = 0; i < n0; ++i) {
       const int j = 2 * i + v, slot = j & 3;
       bool okw = wait_bar(&raw_full[v], i & 1);
       if (!okw) report(p.status, kTimeoutTmaFull, 35);
-      // exponent of the tile's largest scale, seen tokens only (others hold whatever the page held and become zeros)
-      const int t0 = base + i * kApTile;
-      const float4 s4 = *reinterpret_cast<const float4*>(sScale + v * kApTile + lane * 4);
-      float mx = t0 + lane * 4 <= last_pos ? s4.x : 0.f;
-      mx = fmaxf(mx, t0 + lane * 4 + 1 <= last_pos ? s4.y : 0.f);
-      mx = fmaxf(mx, t0 + lane * 4 + 2 <= last_pos ? s4.z : 0.f);
-      mx = fmaxf(mx, t0 + lane * 4 + 3 <= last_pos ? s4.w : 0.f);
+      Pack16 x[8];
+      const unsigned char* raw = sRaw + v * kApRawBytes + t * 128;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      const int ex = max(min(static_cast<int>(__float_as_uint(mx) >> 23), 227), 27) - 127;      // (2^-100 .. 2^100)
-      const bool live = t0 + t <= last_pos;
-      const float sc = live ? sScale[v * kApTile + t] * exp2_of(-ex) : 0.f;
-      const __half2 hi = __float2half2_rn(sc);
-      const __half2 lo = __float2half2_rn(sc - __low2float(hi));
+      for (int c = 0; c < 8; ++c) x[c].u = *reinterpret_cast<const uint4*>(raw + ((c ^ (t & 7)) << 4));
+      // tokens that no row of this CTA sees hold whatever the page held and become zeros
+      const int tok = base + i * kApTile + t;
+      uint32_t any = 0;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) any |= x[c].w[0] | x[c].w[1] | x[c].w[2] | x[c].w[3];
+      const bool live = tok >= first_tok && tok <= last_pos && (any & 0x7f7f7f7fu) != 0;
+      const float sc = live ? sScale[v * kApTile + t] : 0.f;
+      const int e = static_cast<int>((__float_as_uint(sc) >> 23) & 255u) - 127;
+      // a failed wait must not leave the other warps alone at the barrier: all four read the verdicts and leave together
+      const int top = __reduce_max_sync(0xffffffffu, !okw || *abort_flag ? kGaveUp : (live ? e : -127));
+      int* tops = sMax + (v * 2 + (i & 1)) * 4;
+      if (lane == 0) tops[warp & 3] = top;
+      if (v) asm volatile("bar.sync 2, 128;" ::: "memory");
+      else asm volatile("bar.sync 1, 128;" ::: "memory");
+      const int4 m4 = *reinterpret_cast<const int4*>(tops);
+      const int most = max(max(m4.x, m4.y), max(m4.z, m4.w));
+      if (most == kGaveUp) { *abort_flag = 1; break; }
+      unit = max(unit, min(most, 127));
+      // mantissa (in two terms) and power of two of the scale; f16 has no power of two below 2^-24, what is below that loses bits anyway
+      const float m = e == 128 ? sc : __uint_as_float((__float_as_uint(sc) & 0x007fffffu) | 0x3f800000u);
+      const int d = e - unit, b = min(d + 24, 0);
+      const float mb = m * exp2_of(max(b, -126));
+      const __half2 hi = __float2half2_rn(mb);
+      const __half2 lo = __float2half2_rn(mb - __low2float(hi));
+      const __half2 pow = __float2half2_rn(exp2_of(min(max(d - b, -24), 0)));
       if (okw && !wait_bar(&ring_empty[slot], ((j >> 2) & 1) ^ 1)) { report(p.status, kTimeoutStageEmpty, 36); okw = false; }
       if (!okw) *abort_flag = 1;
       ok = __all_sync(0xffffffffu, okw && !*abort_flag);
-      if (!ok) break;
-      const unsigned char* raw = sRaw + v * kApRawBytes + t * 128;
+      if (!ok) continue;      // (to the verdict of the next tile)
+      if (!__all_sync(0xffffffffu, live)) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          if (!live) x[c].u = make_uint4(0u, 0u, 0u, 0u);
+      }
       unsigned char* dst = sRing + slot * kApF16Bytes + t * 128;
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
-        Pack16 x, y[2];
-        x.u = *reinterpret_cast<const uint4*>(raw + ((c ^ (t & 7)) << 4));
-        if (!live) x.u = make_uint4(0u, 0u, 0u, 0u);
+        Pack16 y[2];
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          const __half2 h = e4m3x2_to_h2(x.s[k]);
-          const __half2 r = __hfma2(h, hi, __hmul2(h, lo));
+          const __half2 h = e4m3x2_to_h2(x[c].s[k]);
+          const __half2 r = __hmul2(__hfma2(h, hi, __hmul2(h, lo)), pow);
           y[k >> 2].w[k & 3] = *reinterpret_cast<const uint32_t*>(&r);
         }
         unsigned char* blk = dst + (c >> 2) * kApBlk;
         *reinterpret_cast<uint4*>(blk + (((c * 2) & 7) ^ (t & 7)) * 16) = y[0].u;
         *reinterpret_cast<uint4*>(blk + (((c * 2 + 1) & 7) ^ (t & 7)) * 16) = y[1].u;
       }
-      if (warp == kApConv + 4 * v && lane == 0) sExp[v * 4 + (i & 3)] = ex;
+      if (warp == kApConv + 4 * v && lane == 0) sExp[v * 4 + (i & 3)] = unit;
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) { mbar_arrive(&raw_empty[v]); mbar_arrive(&ring_full[slot]); }
@@ -386,6 +408,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     const int my_first = (p.window > 0 && my_pos + 1 > p.window) ? my_pos + 1 - p.window : 0;
     const float sm = p.scale * 1.4426950408889634f * q_scale;
     float ref = -INFINITY, lsum = 0.f;
+    int cv = 0;
     bool ok = true;
     for (int i = 0; i < n; ++i) {
       const int buf = dual ? sub : (i & 1), phase = dual ? (i & 1) : ((i >> 1) & 1), jv = 2 * i + 1;
@@ -396,11 +419,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
       if (!ok) break;
       tc_fence_after();
       const int t0 = base + i * kApTile;
-      const int ck = sExp[i & 3], cv = sExp[4 + (i & 3)];
+      const int cv_before = cv;
+      cv = sExp[4 + (i & 3)];
+      const bool regrow = i > 0 && cv != cv_before;
+      const float sm_t = sm * exp2_of(sExp[i & 3]);
       const uint32_t ts = lanes + buf * 128;
-      // the accumulator of the tiles before, times the rows' corrections: all of their products must have landed
+      // the accumulator of the tiles before, times the rows' corrections and in its new unit: all of their products must have landed
       auto rescale = [&](float corr) {
         if (i == 0) return;
+        corr *= exp2_of(max(cv_before - cv, -126));
         // (two units: S of this tile was issued behind that product, its barrier is complete)
         if (!__all_sync(0xffffffffu, wait_bar(&o_full[sub], (i - 1) & 1))) { report(p.status, kTimeoutAccum, 38); *abort_flag = 1; return; }
         tc_fence_after();
@@ -415,8 +442,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
       };
       // warp-uniform choice: tcgen05.ld is .sync.aligned, every lane of the warp must take the same path
       const bool full = __all_sync(0xffffffffu, (t0 + kApTile - 1 <= my_pos) && (t0 >= my_first)) != 0;
-      if (full) softmax_tile<false>(ts, t0, my_pos, my_first, sm * exp2_of(ck), cv, ref, lsum, rescale);
-      else softmax_tile<true>(ts, t0, my_pos, my_first, sm * exp2_of(ck), cv, ref, lsum, rescale);
+      if (full) softmax_tile<false>(ts, t0, my_pos, my_first, sm_t, regrow, ref, lsum, rescale);
+      else softmax_tile<true>(ts, t0, my_pos, my_first, sm_t, regrow, ref, lsum, rescale);
       // one unit: S of this tile says nothing of the product before it, whose phase must be behind us before the last one is waited for
       if (!dual && i > 0 && i == n - 1 && !__all_sync(0xffffffffu, wait_bar(&o_full[sub], (i - 1) & 1))) {
         report(p.status, kTimeoutAccum, 38);
@@ -430,7 +457,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     if (ok) {
       tc_fence_after();
       const int head = kvh * group + (unit0 + sub) % group;
-      const float inv_l = lsum > 0.f ? 1.f / lsum : 0.f;
+      const float inv_l = lsum > 0.f ? 1.f / lsum : 0.f, unit = exp2_of(cv);
       uint4* dst = reinterpret_cast<uint4*>(p.out + (static_cast<size_t>(row) * p.hq + head) * D);
 #pragma unroll 1
       for (int c = 0; c < D; c += 32) {
@@ -441,7 +468,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
           for (int k = 0; k < 4; ++k) {
             Pack16 x;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) x.h[j] = f32_to_bf16(__uint_as_float(o[k * 8 + j]) * inv_l);
+            for (int j = 0; j < 8; ++j) x.h[j] = f32_to_bf16(__uint_as_float(o[k * 8 + j]) * inv_l * unit);
             dst[c / 8 + k] = x.u;
           }
         }
