@@ -30,6 +30,7 @@ constexpr int kAqMaxWarps = kAqMaxThreads / 32;
 constexpr int kAqMaxCluster = 8;
 constexpr int kAqSplitBlock = 4;      // attention splits whose partials are in flight at once
 constexpr int kAqAtom = 512;
+constexpr int kAqMaxSegment = 48 * 1024;      // bytes of a row in one CTA
 
 struct ClusterQuantArgs {
   const bf16* in;
@@ -380,6 +381,14 @@ __global__ void __launch_bounds__(kAqBulkThreads) act_quant_bulk_kernel(ClusterQ
   }
 }
 
+// A row segment of up to 48 KB is admitted; with the kernels' own static shared memory that is more than a launch gets unasked.
+template <class Kernel>
+static int allow_segment(Kernel kern, size_t bytes) {
+  constexpr size_t kUnasked = 46 * 1024;
+  if (bytes > kUnasked) DGPP_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kAqMaxSegment));
+  return 0;
+}
+
 template <int MODE>
 static int launch_cluster(const ClusterQuantArgs& a, cudaStream_t st) {
   cudaLaunchConfig_t cfg;
@@ -396,6 +405,7 @@ static int launch_cluster(const ClusterQuantArgs& a, cudaStream_t st) {
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  if (allow_segment(act_quant_cluster_kernel<MODE>, cfg.dynamicSmemBytes)) return -1;
   DGPP_CUDA_OK(cudaLaunchKernelEx(&cfg, act_quant_cluster_kernel<MODE>, a));
   return 0;
 }
@@ -415,7 +425,7 @@ DGPP_API int dgpp_act_quant_nvfp4_cluster(int mode, const void* in, int64_t in_s
   DGPP_REQUIRE((K / cl) % 16 == 0 && K % cl == 0, "act_quant: K %d does not split over %d CTAs", K, cl);
   DGPP_REQUIRE(R >= 1 && R <= 4 && R * bn <= 256, "act_quant: bad terms %d / tile %d", R, bn);
   DGPP_REQUIRE(T_pad % bn == 0 && T_pad >= T, "act_quant: T_pad %d must be a multiple of bn %d and >= T", T_pad, bn);
-  DGPP_REQUIRE(static_cast<size_t>(K / cl) * 2 <= 48 * 1024, "act_quant: segment too large");
+  DGPP_REQUIRE(static_cast<size_t>(K / cl) * 2 <= kAqMaxSegment, "act_quant: segment too large");
   if (T == 0) return 0;
   ClusterQuantArgs a;
   a.in = static_cast<const bf16*>(in);
@@ -445,8 +455,9 @@ DGPP_API int dgpp_act_quant_nvfp4_cluster(int mode, const void* in, int64_t in_s
   }
   if (cl == 1 && (mode == 0 || mode == 1)) {
     const size_t smem = static_cast<size_t>(K) * 2;
-    if (mode == 0) act_quant_bulk_kernel<0><<<T, kAqBulkThreads, smem, st>>>(a);
-    else act_quant_bulk_kernel<1><<<T, kAqBulkThreads, smem, st>>>(a);
+    auto kern = mode == 0 ? act_quant_bulk_kernel<0> : act_quant_bulk_kernel<1>;
+    if (allow_segment(kern, smem)) return -1;
+    kern<<<T, kAqBulkThreads, smem, st>>>(a);
     DGPP_CUDA_OK(cudaGetLastError());
     return 0;
   }
@@ -470,7 +481,7 @@ DGPP_API int dgpp_attn_combine_quant(const void* part_ml, const void* part_acc, 
   DGPP_REQUIRE((K / cl) % 16 == 0 && K % cl == 0, "attn_combine_quant: K %d does not split over %d CTAs", K, cl);
   DGPP_REQUIRE(R >= 1 && R <= 4 && R * bn <= 256, "attn_combine_quant: bad terms %d / tile %d", R, bn);
   DGPP_REQUIRE(T_pad % bn == 0 && T_pad >= T, "attn_combine_quant: T_pad %d must be a multiple of bn %d and >= T", T_pad, bn);
-  DGPP_REQUIRE(static_cast<size_t>(K / cl) * 2 <= 48 * 1024, "attn_combine_quant: segment too large");
+  DGPP_REQUIRE(static_cast<size_t>(K / cl) * 2 <= kAqMaxSegment, "attn_combine_quant: segment too large");
   if (T == 0) return 0;
   ClusterQuantArgs a;
   memset(&a, 0, sizeof(a));

@@ -113,7 +113,7 @@ def test_cluster_quantiser_matches_the_single_cta_one(dev, rows, k, terms):
 
 @pytest.mark.parametrize("rows,k,terms,bn", [(65, 256, 3, 16), (130, 5120, 3, 64), (129, 2304, 1, 128), (66, 24320, 2, 16)])
 def test_bulk_quantiser_matches_the_cluster_one(dev, rows, k, terms, bn):
-    """One CTA per row above 64 rows: fewer blocks of 16 than threads, a remainder of them, the widest row; the same bits as the
+    """One CTA per row above 64 rows: fewer blocks of 16 than threads, a remainder of them, a wide row; the same bits as the
     cluster form (the row statistic is a maximum), the copy of the rows included."""
     from dgpp_b200.ops import core as ops
 
@@ -130,6 +130,48 @@ def test_bulk_quantiser_matches_the_cluster_one(dev, rows, k, terms, bn):
         torch.cuda.synchronize()
         ops.check_status()
         assert torch.equal(got.g, want.g) and torch.equal(got.q, want.q) and torch.equal(got.sf, want.sf) and torch.equal(x1, x2), mode
+
+
+@pytest.mark.parametrize("rows,k,mode", [(65, 24576, "plain"), (65, 24576, "swiglu"), (65, 24832, "plain"), (66, 48640, "swiglu"),
+                                         (65, 49152, "plain"), (2, 49152, "rmsnorm"), (1, 196608, "plain")])
+def test_quantiser_of_the_widest_rows(dev, rows, k, mode):
+    """Row segments up to the 48 KB that a CTA takes, and one past it (two CTAs): every width that the entry point's own
+    bound admits is launched.  Three terms keep a value to 2^-3 of a 4-bit step each: well below 1e-2 of a row's largest."""
+    from dgpp_b200.ops import core as ops, reference as ref
+
+    torch.manual_seed(35)
+    x = torch.randn(rows, 2 * k if mode == "swiglu" else k, device=dev).to(BF)
+    w = (1 + 0.1 * torch.randn(k, device=dev)).to(BF) if mode == "rmsnorm" else None
+    got = ops.act_quant_nvfp4(x, 3, mode=mode, norm_w=w)
+    torch.cuda.synchronize()
+    ops.check_status()
+    want = x if mode == "plain" else ops.swiglu(x) if mode == "swiglu" else ref.rmsnorm(x, w, 1e-6)[0]
+    err = (got.dequant() - want.float()).abs().amax(1) / want.float().abs().amax(1)
+    assert err.max().item() < 1e-2
+
+
+@pytest.mark.parametrize("m,k", [(0, 24576), (1, 24576), (2, 24320), (2, 24576)])
+def test_quantiser_of_one_whole_row_per_cta(dev, m, k):
+    """One CTA per row up to 48 KB of it, all modes; plain and SwiGLU rows bit for bit as in a cluster of eight."""
+    from dgpp_b200.ops import core as ops
+
+    torch.manual_seed(36)
+    x = torch.randn(3, 2 * k if m == 1 else k, device=dev).to(BF)
+    w = (1 + 0.1 * torch.randn(k, device=dev)).to(BF)
+    got = []
+    for cl in (1, 8):
+        a = ops.QuantAct(16, k, 3, 16, dev)
+        a.rows = 3
+        ops.call("dgpp_act_quant_nvfp4_cluster", m, ops.ptr(x), x.stride(0), None, ops.ptr(w), None, None, ops.ptr(a.q), ops.ptr(a.sf), ops.ptr(a.g),
+                 3, 16, k, 3, 16, cl, 1e-6, 0.0, 0.0, 0, None, None, 0, ops.stream_ptr())
+        got.append(a)
+    torch.cuda.synchronize()
+    ops.check_status()
+    a, b = got
+    if m != 2:
+        assert torch.equal(a.g, b.g) and torch.equal(a.q, b.q) and torch.equal(a.sf, b.sf)
+    else:      # the sum of squares in another order: one bf16 rounding of the normed value may fall the other way
+        assert ((a.dequant() - b.dequant()).norm() / b.dequant().norm()).item() < 2.0 ** -8
 
 
 def _filled_cache(dev, hq, hkv, ctx, page, slot, d=128):
