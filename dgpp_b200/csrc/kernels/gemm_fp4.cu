@@ -96,6 +96,25 @@ __device__ __forceinline__ void push_flags(const Fp4Params& p, int parity, uint3
   if (warp == 2 && lane < p.comm.world) st_release_sys(flag(p.comm, lane, parity, p.comm.rank, blockIdx.x), epoch);
 }
 
+// Debug time stamp `slot` of CTA (0, 0, 0).
+__device__ __forceinline__ void trace_stamp(const Fp4Params& p, int slot) {
+  if (p.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t) :: "memory");
+    p.trace[slot] = t;
+  }
+}
+// This CTA's share of the L2 prefetch that the caller asked for; all lanes of one warp.
+__device__ __forceinline__ void request_prefetch(const Fp4Params& p, int lane) {
+  constexpr int64_t kChunk = 16384;
+  const int64_t ctas = static_cast<int64_t>(gridDim.x) * gridDim.y * gridDim.z;
+  const int64_t cta = (static_cast<int64_t>(blockIdx.z) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  for (int64_t off = (cta * 32 + lane) * kChunk; off < p.pf_bytes; off += ctas * 32 * kChunk) {
+    const uint32_t n = static_cast<uint32_t>(min(kChunk, p.pf_bytes - off)) & ~15u;
+    if (n) l2_prefetch_bulk(p.pf_ptr + off, n);
+  }
+}
+
 // BN = MMA N = (token tile) x (residual terms): with R > 1 the terms of one token tile are stacked along N
 // (rows r * bn_tok + m of the B operand) so a K=64 step is ONE tcgen05.mma whatever R is; the epilogue adds the
 // R column groups.  Stacking needs the whole batch in one token tile (decode); R = 1 tiles freely.
@@ -123,14 +142,7 @@ gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmA,   // packed weights as 
   int* last_flag = const_cast<int*>(abort_flag) + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool tracing = p.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
-  auto stamp = [&](int slot) {
-    if (tracing) {
-      unsigned long long t;
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t) :: "memory");
-      p.trace[slot] = t;
-    }
-  };
+  auto stamp = [&](int slot) { trace_stamp(p, slot); };
   if (threadIdx.x == 0) stamp(0);
   const int bn_tok = BN / p.R;             // tokens per tile
   const int m0 = blockIdx.y * bn_tok;
@@ -231,15 +243,7 @@ gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmA,   // packed weights as 
       }
     }
     __syncwarp();
-    if (p.pf_bytes > 0) {
-      constexpr int64_t kChunk = 16384;
-      const int64_t ctas = static_cast<int64_t>(gridDim.x) * gridDim.y * gridDim.z;
-      const int64_t cta = (static_cast<int64_t>(blockIdx.z) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-      for (int64_t off = (cta * 32 + lane) * kChunk; off < p.pf_bytes; off += ctas * 32 * kChunk) {
-        const uint32_t n = static_cast<uint32_t>(min(kChunk, p.pf_bytes - off)) & ~15u;
-        if (n) l2_prefetch_bulk(p.pf_ptr + off, n);
-      }
-    }
+    request_prefetch(p, lane);
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (elect_one()) {
@@ -666,6 +670,7 @@ gemm_fp4_units_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) trace_stamp(p, 0);
   const int bn_tok = BN / p.R, nst = p.K / kF4StageK;
   constexpr uint32_t kAccs = BN <= 128 ? 2 : 1;      // (256 columns and their scale factors leave no room for a second)
   constexpr uint32_t kColD = BN < 32 ? 32 : BN;
@@ -689,7 +694,9 @@ gemm_fp4_units_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_sfa = tmem_base + kAccs * kColD, tmem_sfb = tmem_sfa + 2 * kColSfa;
+  if (threadIdx.x == 0) trace_stamp(p, 1);
   pdl_wait();
+  if (threadIdx.x == 0) trace_stamp(p, 2);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer: weights, activations, scales
@@ -711,6 +718,8 @@ gemm_fp4_units_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         }
       }
     }
+    __syncwarp();
+    request_prefetch(p, lane);
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (elect_one()) {
@@ -724,6 +733,7 @@ gemm_fp4_units_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         for (int i = 0; i < nst; ++i, ++it) {
           const int s = it % S;
           if (!wait_bar(&full[s], (it / S) & 1) || *abort_flag) { report(p.status, kTimeoutTmaFull, 16); *abort_flag = 1; ok = false; break; }
+          if (it == 0) trace_stamp(p, 3);
           tc_fence_after();
           const uint32_t t_sfa = tmem_sfa + (it & 1) * kColSfa, t_sfb = tmem_sfb + (it & 1) * kColSfb;
           for (int j = 0; j < 4; ++j)
@@ -740,6 +750,7 @@ gemm_fp4_units_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         umma_commit(&acc_full[a]);
         ++n;
       }
+      trace_stamp(p, 4);
     }
   } else {
     // ------------------------------------------------------------------ epilogue (warps 2..5: 128 weight rows x the slot's tokens)
@@ -756,6 +767,7 @@ gemm_fp4_units_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       if (!ok) { report(p.status, kTimeoutAccum, 15); *abort_flag = 1; }
       ok = __all_sync(0xffffffffu, ok && !*abort_flag);
       if (!ok) break;
+      if (warp == 2 && lane == 0) trace_stamp(p, 5);      // (the last one stays)
       tc_fence_after();
       bf16* out = p.out + static_cast<size_t>(grp) * p.group_out_stride + (u % p.group_tiles) * kF4BM + q * 32 + lane;
 #pragma unroll 1
@@ -781,6 +793,7 @@ gemm_fp4_units_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   }
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0) trace_stamp(p, 6);
   if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
 }
 
@@ -887,9 +900,9 @@ DGPP_API int dgpp_act_quant_nvfp4(int mode, const void* in, int64_t in_stride, c
 // One-shot hint for the NEXT dgpp_gemm_fp4 / dgpp_gemm_fp4_grouped call of this thread: the bytes its CTAs ask L2
 // to fetch once their own loads are issued (normally the packed weights of the projection that runs next).
 static unsigned long long* g_trace = nullptr;
-// Debug aid: while a device buffer of 8 uint64 is set, CTA (0,0,0) of every dgpp_gemm_fp4 launch stores %globaltimer
-// (ns) at: 0 entry, 1 prologue done, 2 preceding grid complete, 3 first stage landed, 4 last MMA issued,
-// 5 accumulator complete, 6 epilogue done.  Pass null to switch it off.
+// Debug aid: while a device buffer of 8 uint64 is set, CTA (0,0,0) of every dgpp_gemm_fp4 / dgpp_gemm_fp4_grouped launch stores
+// %globaltimer (ns) at: 0 entry, 1 prologue done, 2 preceding grid complete, 3 first stage landed, 4 last MMA issued,
+// 5 accumulator complete (its last one), 6 epilogue done.  Pass null to switch it off.
 DGPP_API int dgpp_gemm_fp4_set_trace(void* dev_u64x8) {
   g_trace = static_cast<unsigned long long*>(dev_u64x8);
   return 0;

@@ -512,6 +512,50 @@ def test_pair_gemm_grouped_equals_the_plain_form_per_matrix(bn):
         assert torch.equal(out[rows], want), (t, e)
 
 
+@pytest.mark.parametrize("bn,terms,slots", [(16, 1, 5), (16, 2, 5), (16, 3, 300), (64, 1, 5), (32, 3, 170), (128, 1, 5), (64, 3, 160), (256, 1, 80)])
+@pytest.mark.parametrize("own_rows", [False, True])
+def test_grouped_block_scaled_linear_equals_the_plain_one_per_matrix(bn, terms, slots, own_rows):
+    """Every tile width, one unit per CTA and several (both accumulators, or the one that 256 columns leave room for), unused
+    slots between, shared rows and the slots' own: the bits of the plain product with the slot's matrix.  The debug stamps
+    are written by the grouped form as well."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from dgpp_b200.ops import core as ops
+    from dgpp_b200.quant.formats import random_quant_linear
+
+    dev = torch.device("cuda:0")
+    torch.manual_seed(bn + terms)
+    n, k, experts, rows = 256, 768, 3, bn - 3
+    ws = [random_quant_linear(n, k, "nvfp4", dev) for _ in range(experts)]
+    q, sf = torch.cat([w.payload for w in ws]), torch.cat([w.tiled_scales().reshape(-1) for w in ws])
+    alphas = torch.tensor([w.alpha for w in ws], device=dev)
+    groups = [-1 if i % 4 == 1 else (i * 7 // 3) % experts for i in range(slots)]
+    tiles = slots if own_rows else 1
+    xa = ops.QuantAct(tiles * bn, k, terms, bn, dev)
+    ops.act_quant_nvfp4(torch.randn(tiles * bn, k, device=dev).to(BF), terms, out=xa)
+    out = torch.full((slots, bn, n), 7.0, device=dev, dtype=BF)
+    stamps = torch.zeros(8, dtype=torch.int64, device=dev)
+    ops.call("dgpp_gemm_fp4_set_trace", ops.ptr(stamps))
+    try:
+        ops.gemm_fp4_grouped(xa, q, sf, alphas, out, rows, n, k, experts, torch.tensor(groups, dtype=torch.int32, device=dev), own_rows)
+    finally:
+        ops.call("dgpp_gemm_fp4_set_trace", None)
+    torch.cuda.synchronize()
+    ops.check_status()
+    for s, e in enumerate(groups):
+        if e < 0:
+            assert (out[s] == 7.0).all()
+            continue
+        one = ops.QuantAct(bn, k, terms, bn, dev)
+        t = s if own_rows else 0
+        one.q, one.sf, one.g = (v.reshape(tiles, -1)[t].reshape(shape) for v, shape in ((xa.q, one.q.shape), (xa.sf, one.sf.shape), (xa.g, one.g.shape)))
+        one.rows = rows
+        assert torch.equal(out[s, :rows], ops.gemm_fp4(one, ws[e], splits=1)), (s, e)
+        assert (out[s, rows:] == 7.0).all()
+    st = stamps.tolist()[:7]
+    assert 0 < st[0] <= st[1] <= st[2] <= st[3] <= min(st[4], st[5]) and max(st[4], st[5]) <= st[6], st
+
+
 @pytest.mark.parametrize("rows,n,k,splits", [(8, 40960, 512, 2), (128, 10240, 2048, 8)])
 def test_pair_gemm_split_counters_are_at_rest_after_several_units_per_pair(rows, n, k, splits):
     """More (tile, split) units than pairs, so that every pair counts itself in at several tiles: all counters end at zero, and a second
