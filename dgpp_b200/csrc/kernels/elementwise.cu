@@ -153,18 +153,18 @@ static int launch_rmsnorm(const bf16* resid, const bf16* delta, const bf16* w, b
 // gate_up: [rows, 2*inter] (gate then up); out: [rows, inter].  limit > 0 clamps gate above and up both sides.
 // alpha > 0 selects the scaled-sigmoid form  gate * sigmoid(alpha * gate) * (up + 1)  (alpha = 0: silu(gate) * up).
 // tiles (optional, one entry per bn rows): rows of tiles with a negative entry are skipped.  rows_of (optional): the bn rows to work
-// on, negative entries skipped (16384 of 33000 tile rows, 1536 columns each: 81 us over whole tiles, 33 so).
+// on, entries outside 0 .. rows - 1 skipped (16384 of 33000 tile rows, 1536 columns each: 81 us over whole tiles, 33 so).
 // Memory bound.  A block has as many rows as 256 threads hold, none of them idle over narrow rows (33000 tile rows of 1536 columns and
 // 2048 shared ones: 93 us with one row per 256-thread block, 87 so).  grid (columns, rows of a
 // tile, tiles); listed rows: (columns, rows, further rows).
 __global__ void __launch_bounds__(kRowThreads)
 swiglu_kernel(const bf16* __restrict__ gate_up, bf16* __restrict__ out, int inter, float limit, float alpha,
-              const int32_t* __restrict__ tiles, int bn, const int32_t* __restrict__ rows_of) {
+              const int32_t* __restrict__ tiles, int bn, const int32_t* __restrict__ rows_of, int rows) {
   pdl_wait();
   const int in_tile = (rows_of != nullptr ? blockIdx.z * gridDim.y + blockIdx.y : blockIdx.y) * blockDim.y + threadIdx.y;
   if (in_tile >= bn || (tiles != nullptr && tiles[blockIdx.z] < 0)) return;
   const int listed = rows_of != nullptr ? rows_of[in_tile] : in_tile;
-  if (listed < 0) return;
+  if (listed < 0 || (rows_of != nullptr && listed >= rows)) return;
   const size_t row = rows_of != nullptr ? listed : in_tile + static_cast<size_t>(blockIdx.z) * bn;
   const bf16* g = gate_up + row * 2 * inter;
   const bf16* u = g + inter;
@@ -386,13 +386,13 @@ DGPP_API int dgpp_swiglu(const void* gate_up, void* out, int rows, int inter, fl
   const dim3 block = swiglu_block(inter);
   dim3 grid(dgpp_ceil_div(inter / 8, block.x), dgpp_ceil_div(rows, block.y));
   DGPP_CUDA_OK(launch_early(swiglu_kernel, grid, block, 0, st, static_cast<const bf16*>(gate_up), static_cast<bf16*>(out), inter,
-                                        limit, alpha, nullptr, rows, nullptr));
+                                        limit, alpha, nullptr, rows, nullptr, 0));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }
 
-// The same over the n rows that `rows_of` lists (negative entries: none).
-DGPP_API int dgpp_swiglu_rows(const void* gate_up, void* out, const void* rows_of, int n, int inter, float limit, float alpha,
+// The same over the n rows that `rows_of` lists, of `rows` there are (other entries: none).
+DGPP_API int dgpp_swiglu_rows(const void* gate_up, void* out, const void* rows_of, int n, int rows, int inter, float limit, float alpha,
                               cudaStream_t st) {
   DGPP_REQUIRE(inter % 8 == 0, "swiglu: inter %d must be a multiple of 8", inter);
   DGPP_REQUIRE(rows_of != nullptr, "swiglu: row list required");
@@ -401,7 +401,7 @@ DGPP_API int dgpp_swiglu_rows(const void* gate_up, void* out, const void* rows_o
   const int row_blocks = dgpp_ceil_div(n, block.y), deep = dgpp_ceil_div(row_blocks, 65535);
   dim3 grid(dgpp_ceil_div(inter / 8, block.x), dgpp_ceil_div(row_blocks, deep), deep);
   DGPP_CUDA_OK(launch_early(swiglu_kernel, grid, block, 0, st, static_cast<const bf16*>(gate_up), static_cast<bf16*>(out), inter, limit, alpha,
-                            nullptr, n, static_cast<const int32_t*>(rows_of)));
+                            nullptr, n, static_cast<const int32_t*>(rows_of), rows));
   return 0;
 }
 
@@ -414,7 +414,7 @@ DGPP_API int dgpp_swiglu_tiles(const void* gate_up, void* out, const void* tiles
   const dim3 block = swiglu_block(inter);
   dim3 grid(dgpp_ceil_div(inter / 8, block.x), dgpp_ceil_div(bn, block.y), n_tiles);
   DGPP_CUDA_OK(launch_early(swiglu_kernel, grid, block, 0, st, static_cast<const bf16*>(gate_up), static_cast<bf16*>(out), inter, limit, alpha,
-                                        static_cast<const int32_t*>(tiles), bn, nullptr));
+                                        static_cast<const int32_t*>(tiles), bn, nullptr, 0));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
 }

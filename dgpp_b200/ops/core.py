@@ -83,13 +83,17 @@ def swiglu_tiles(gate_up: torch.Tensor, out: torch.Tensor, tiles: torch.Tensor, 
     return out
 
 
-_lib.declare("dgpp_swiglu_rows", [P, P, P, I, I, F, F, P])
+_lib.declare("dgpp_swiglu_rows", [P, P, P, I, I, I, F, F, P])
 
 
 def swiglu_rows(gate_up: torch.Tensor, out: torch.Tensor, rows_of: torch.Tensor, limit: float = 0.0, alpha: float = 0.0) -> torch.Tensor:
-    """`swiglu` of the rows that `rows_of` (int32, any order, negative entries: none) lists; the others are left alone."""
+    """`swiglu` of the rows that `rows_of` (int32, any order; entries that name no row: none) lists; the others are left alone."""
     _chk(gate_up, torch.bfloat16, "gate_up")
-    call("dgpp_swiglu_rows", ptr(gate_up), ptr(out), ptr(rows_of), rows_of.numel(), out.shape[-1], float(limit), float(alpha), stream_ptr())
+    _chk(out, torch.bfloat16, "out")
+    _chk(rows_of, torch.int32, "rows_of")
+    rows, inter = out.shape
+    assert gate_up.shape == (rows, 2 * inter) and gate_up.is_contiguous() and out.is_contiguous() and rows_of.is_contiguous()
+    call("dgpp_swiglu_rows", ptr(gate_up), ptr(out), ptr(rows_of), rows_of.numel(), rows, inter, float(limit), float(alpha), stream_ptr())
     return out
 
 

@@ -543,3 +543,18 @@ def test_swiglu_of_listed_rows(dev, inter, rows):
     keep = torch.zeros(rows, dtype=torch.bool, device=dev)
     keep[listed.long()] = True
     assert torch.equal(out[keep], ops.swiglu(gu)[keep]) and (out[~keep] == 7.0).all()
+
+
+def test_swiglu_of_listed_rows_checks_its_arguments(dev):
+    """Types and shapes are refused on the host; an entry past the rows names none."""
+    from dgpp_b200.ops import core as ops
+
+    gu, out = torch.randn(6, 32, device=dev).to(torch.bfloat16), torch.full((6, 16), 7.0, device=dev, dtype=torch.bfloat16)
+    of = torch.tensor([6, 2, 1 << 30, -5], dtype=torch.int32, device=dev)
+    for bad in ((gu.float(), out, of), (gu, out.float(), of), (gu, out, of.long()), (gu, out[:5], of), (gu, out[:, :8], of)):
+        with pytest.raises((AssertionError, TypeError)):
+            ops.swiglu_rows(*bad)
+    ops.swiglu_rows(gu, out, of)
+    keep = torch.zeros(6, dtype=torch.bool, device=dev)
+    keep[2] = True
+    assert torch.equal(out[keep], ops.swiglu(gu)[keep]) and (out[~keep] == 7.0).all()
