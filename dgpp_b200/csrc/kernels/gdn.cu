@@ -418,17 +418,20 @@ static int gdn_recurrent_launch(const void* q, int64_t q_stride, const void* k, 
   else DGPP_CUDA_OK(launch_early(gdn_prep_kernel<256>, pgrid, kPrepThreads, 0, st, a));
   DGPP_CUDA_OK(cudaGetLastError());
   dim3 grid(dv / kGdnCols, hv, seg > 0 ? T / seg : (sequential ? 1 : T));
-  if (gate_k) {
-    if (dk == 64) DGPP_CUDA_OK(launch_early(gdn_recurrent_kernel<64, true>, grid, kGdnThreads, 0, st, a));
-    else DGPP_CUDA_OK(launch_early(gdn_recurrent_kernel<128, true>, grid, kGdnThreads, 0, st, a));
-    DGPP_CUDA_OK(cudaGetLastError());
+  // One long run is few blocks for a long time: placed early, beside the preparation's last ones, they share SMs that others leave empty (T
+  // tokens x heads x width, us early / plain: 173 x 32 x 128 92 / 72, 512 x 16 x 256 450 / 343, 48 x 16 x 128 21.6 / 24.7).
+  constexpr int kEarlyTokens = 32;
+  auto launch = [&](void (*kern)(GdnArgs)) -> int {
+    if (sequential && seg <= 0 && T > kEarlyTokens) {
+      kern<<<grid, kGdnThreads, 0, st>>>(a);
+      DGPP_CUDA_OK(cudaGetLastError());
+    } else {
+      DGPP_CUDA_OK(launch_early(kern, grid, kGdnThreads, 0, st, a));
+    }
     return 0;
-  }
-  if (dk == 64) DGPP_CUDA_OK(launch_early(gdn_recurrent_kernel<64>, grid, kGdnThreads, 0, st, a));
-  else if (dk == 128) DGPP_CUDA_OK(launch_early(gdn_recurrent_kernel<128>, grid, kGdnThreads, 0, st, a));
-  else DGPP_CUDA_OK(launch_early(gdn_recurrent_kernel<256>, grid, kGdnThreads, 0, st, a));
-  DGPP_CUDA_OK(cudaGetLastError());
-  return 0;
+  };
+  if (gate_k) return dk == 64 ? launch(gdn_recurrent_kernel<64, true>) : launch(gdn_recurrent_kernel<128, true>);
+  return dk == 64 ? launch(gdn_recurrent_kernel<64>) : dk == 128 ? launch(gdn_recurrent_kernel<128>) : launch(gdn_recurrent_kernel<256>);
 }
 
 DGPP_API int dgpp_gdn_recurrent(const void* q, int64_t q_stride, const void* k, int64_t k_stride, const void* v,
