@@ -457,9 +457,11 @@ DGPP_API int dgpp_moe_route(const void* x, int64_t x_stride, const void* gate, c
   DGPP_REQUIRE(logits_out != nullptr, "moe_route: a [T, E] fp32 logits buffer is required");
   const dim3 grid(dgpp_ceil_div(E, kRouterThreads / 32), dgpp_ceil_div(T, kRouterRowsPerCta));
   auto tiles = [&](int experts) { return dim3(dgpp_ceil_div(E, experts * kRouterThreads / 32), grid.y); };
-  // (a CTA per SM takes the tiles of eight experts per warp, two those of four: below two and one waves of them the finer split is faster)
+  // A CTA per SM takes the tiles of eight experts per warp, two those of four.  The wide ones want seven waves (1024 CTAs) whose warps have experts
+  // (us, four / eight per warp, hidden 4096: 256 experts x 8192 rows 621 / 586, x 1024 79 / 82; 128 x 2400 93 / 97; 96 x 8192, a quarter
+  // of the warps idle, 229 / 239; 8 x 8192, all but one idle, 53 / 92), the narrow ones a wave.
   const dim3 t8 = tiles(8), t4 = tiles(4);
-  if (t8.x * t8.y >= 296) DGPP_CUDA_OK(launch_early(moe_router_logits_tile_kernel<8>, t8, kRouterThreads, 0, st, a));
+  if (t8.x * t8.y >= 1024 && 5 * E >= 4 * 64 * static_cast<int>(t8.x)) DGPP_CUDA_OK(launch_early(moe_router_logits_tile_kernel<8>, t8, kRouterThreads, 0, st, a));
   else if (t4.x * t4.y >= 296) DGPP_CUDA_OK(launch_early(moe_router_logits_tile_kernel<4>, t4, kRouterThreads, 0, st, a));
   else DGPP_CUDA_OK(launch_early(moe_router_logits_kernel, grid, kRouterThreads, 0, st, a));
   DGPP_CUDA_OK(cudaGetLastError());

@@ -70,7 +70,8 @@ def test_router_logits_do_not_depend_on_the_batch(dev, rows, experts, hidden):
     assert torch.equal(all_, few)
 
 
-@pytest.mark.parametrize("rows,experts,hidden", [(603, 512, 2048), (2369, 37, 264), (2400, 70, 8)])
+@pytest.mark.parametrize("rows,experts,hidden", [(603, 512, 2048), (2369, 37, 264), (2400, 70, 8), (1021, 505, 264), (8190, 59, 8),
+                                                 (8200, 61, 2048)])
 def test_router_logits_of_eight_experts_per_warp(dev, rows, experts, hidden):
     """The widest tiles, with remainders of tokens, experts and steps (an odd number of them, and less than one)."""
     test_router_logits_do_not_depend_on_the_batch(dev, rows, experts, hidden)
