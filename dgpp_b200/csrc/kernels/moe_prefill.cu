@@ -35,6 +35,8 @@ struct SortArgs {
   int T, k, E, e_begin, e_end, bn, max_tiles;
 };
 
+// CLUSTER: kSortCtas CTAs of one cluster; otherwise one CTA alone.
+template <bool CLUSTER>
 __global__ void __launch_bounds__(kSortThreads) moe_segment_sort_kernel(SortArgs a) {
   // per-warp histograms (later: per-warp running offsets), the experts' totals in this CTA / first tiles
   extern __shared__ int ssm[];
@@ -43,7 +45,7 @@ __global__ void __launch_bounds__(kSortThreads) moe_segment_sort_kernel(SortArgs
   int* total = first_tile + a.E;                    // [E]
   pdl_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int rank = blockIdx.x, ctas = gridDim.x;    // one cluster
+  const int rank = CLUSTER ? blockIdx.x : 0, ctas = CLUSTER ? kSortCtas : 1;
   const int P = a.T * a.k;
   const int seg = (P + ctas * kSortWarps - 1) / (ctas * kSortWarps);      // pairs per warp, contiguous and in order
   const int p0 = min(P, (rank * kSortWarps + warp) * seg), p1 = min(P, p0 + seg);
@@ -66,14 +68,15 @@ __global__ void __launch_bounds__(kSortThreads) moe_segment_sort_kernel(SortArgs
     }
     total[e] = run;
   }
-  cluster_barrier();
+  if (CLUSTER) cluster_barrier();
+  else __syncthreads();
   // over the CTAs of the cluster (thread = expert): pairs in the CTAs before this one, pairs in all of them
   int ahead = 0, count = 0;
-  if (tid < a.E) {
+  if (!CLUSTER && tid < a.E) count = total[tid];
+  if (CLUSTER && tid < a.E) {
     const uint32_t mine = smem_u32(total + tid);
 #pragma unroll
     for (int c = 0; c < kSortCtas; ++c) {
-      if (c >= ctas) break;
       int v;
       asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(mapa_shared(mine, c)) : "memory");
       ahead += c < rank ? v : 0;
@@ -106,8 +109,10 @@ __global__ void __launch_bounds__(kSortThreads) moe_segment_sort_kernel(SortArgs
       if (tid == 0) *a.n_tiles = min(all, a.max_tiles);
     }
   }
-  cluster_barrier();      // every CTA has read the others' totals: their places take what comes before this CTA
-  if (tid < a.E) total[tid] = ahead;
+  if (CLUSTER) {
+    cluster_barrier();      // every CTA has read the others' totals: their places take what comes before this CTA
+    if (tid < a.E) total[tid] = ahead;
+  }
   __syncthreads();
   // pass 2: stable rank.  A warp walks its segment 32 pairs at a time; lanes with the same expert form a group whose
   // members are ranked by lane order, the group's lowest lane advances the warp's running offset of that expert.
@@ -130,7 +135,7 @@ __global__ void __launch_bounds__(kSortThreads) moe_segment_sort_kernel(SortArgs
     if (p < p1) {
       int row = -1;
       if (e >= 0) {
-        const int r = total[e] + start + rank_in_group;
+        const int r = (CLUSTER ? total[e] : 0) + start + rank_in_group;
         const int tile = first_tile[e] + r / a.bn;
         row = tile < a.max_tiles ? tile * a.bn + r % a.bn : -1;
       }
@@ -218,24 +223,27 @@ DGPP_API int dgpp_moe_segment_sort(const void* ids, void* pair_row, void* tile_e
   const size_t smem = (static_cast<size_t>(kSortWarps) * E + 2 * E) * sizeof(int);
   static bool attr = false;
   if (!attr) {
-    DGPP_CUDA_OK(cudaFuncSetAttribute(moe_segment_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+    DGPP_CUDA_OK(cudaFuncSetAttribute(moe_segment_sort_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+    DGPP_CUDA_OK(cudaFuncSetAttribute(moe_segment_sort_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
     attr = true;
   }
+  if (T * k < kSortSplitPairs) {
+    DGPP_CUDA_OK(launch_early(moe_segment_sort_kernel<false>, 1, kSortThreads, smem, st, a));
+    return 0;
+  }
   cudaLaunchConfig_t cfg = {};
-  const int ctas = T * k >= kSortSplitPairs ? kSortCtas : 1;
-  cfg.gridDim = dim3(ctas);
+  cfg.gridDim = dim3(kSortCtas);
   cfg.blockDim = dim3(kSortThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = static_cast<unsigned>(ctas); at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  at[0].val.clusterDim.x = kSortCtas; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = stream_captures(st) ? 1 : 2;
-  DGPP_CUDA_OK(cudaLaunchKernelEx(&cfg, moe_segment_sort_kernel, a));
-  DGPP_CUDA_OK(cudaGetLastError());
+  DGPP_CUDA_OK(cudaLaunchKernelEx(&cfg, moe_segment_sort_kernel<true>, a));
   return 0;
 }
 
