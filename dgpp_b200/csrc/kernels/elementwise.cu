@@ -157,15 +157,20 @@ static int launch_rmsnorm(const bf16* resid, const bf16* delta, const bf16* w, b
 // Memory bound.  A block has as many rows as 256 threads hold, none of them idle over narrow rows (33000 tile rows of 1536 columns and
 // 2048 shared ones: 93 us with one row per 256-thread block, 87 so).  grid (columns, rows of a
 // tile, tiles); listed rows: (columns, rows, further rows).
+// LISTED: rows_of instead of rows or tiles.
+template <bool LISTED>
 __global__ void __launch_bounds__(kRowThreads)
 swiglu_kernel(const bf16* __restrict__ gate_up, bf16* __restrict__ out, int inter, float limit, float alpha,
               const int32_t* __restrict__ tiles, int bn, const int32_t* __restrict__ rows_of, int rows) {
   pdl_wait();
-  const int in_tile = (rows_of != nullptr ? blockIdx.z * gridDim.y + blockIdx.y : blockIdx.y) * blockDim.y + threadIdx.y;
-  if (in_tile >= bn || (tiles != nullptr && tiles[blockIdx.z] < 0)) return;
-  const int listed = rows_of != nullptr ? rows_of[in_tile] : in_tile;
-  if (listed < 0 || (rows_of != nullptr && listed >= rows)) return;
-  const size_t row = rows_of != nullptr ? listed : in_tile + static_cast<size_t>(blockIdx.z) * bn;
+  const int in_tile = (LISTED ? blockIdx.z * gridDim.y + blockIdx.y : blockIdx.y) * blockDim.y + threadIdx.y;
+  if (in_tile >= bn || (!LISTED && tiles != nullptr && tiles[blockIdx.z] < 0)) return;
+  size_t row = in_tile + static_cast<size_t>(blockIdx.z) * bn;
+  if (LISTED) {
+    const int listed = rows_of[in_tile];
+    if (listed < 0 || listed >= rows) return;
+    row = listed;
+  }
   const bf16* g = gate_up + row * 2 * inter;
   const bf16* u = g + inter;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -385,7 +390,7 @@ DGPP_API int dgpp_swiglu(const void* gate_up, void* out, int rows, int inter, fl
   if (rows == 0) return 0;
   const dim3 block = swiglu_block(inter);
   dim3 grid(dgpp_ceil_div(inter / 8, block.x), dgpp_ceil_div(rows, block.y));
-  DGPP_CUDA_OK(launch_early(swiglu_kernel, grid, block, 0, st, static_cast<const bf16*>(gate_up), static_cast<bf16*>(out), inter,
+  DGPP_CUDA_OK(launch_early(swiglu_kernel<false>, grid, block, 0, st, static_cast<const bf16*>(gate_up), static_cast<bf16*>(out), inter,
                                         limit, alpha, nullptr, rows, nullptr, 0));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
@@ -400,7 +405,7 @@ DGPP_API int dgpp_swiglu_rows(const void* gate_up, void* out, const void* rows_o
   const dim3 block = swiglu_block(inter);
   const int row_blocks = dgpp_ceil_div(n, block.y), deep = dgpp_ceil_div(row_blocks, 65535);
   dim3 grid(dgpp_ceil_div(inter / 8, block.x), dgpp_ceil_div(row_blocks, deep), deep);
-  DGPP_CUDA_OK(launch_early(swiglu_kernel, grid, block, 0, st, static_cast<const bf16*>(gate_up), static_cast<bf16*>(out), inter, limit, alpha,
+  DGPP_CUDA_OK(launch_early(swiglu_kernel<true>, grid, block, 0, st, static_cast<const bf16*>(gate_up), static_cast<bf16*>(out), inter, limit, alpha,
                             nullptr, n, static_cast<const int32_t*>(rows_of), rows));
   return 0;
 }
@@ -413,7 +418,7 @@ DGPP_API int dgpp_swiglu_tiles(const void* gate_up, void* out, const void* tiles
   if (n_tiles <= 0) return 0;
   const dim3 block = swiglu_block(inter);
   dim3 grid(dgpp_ceil_div(inter / 8, block.x), dgpp_ceil_div(bn, block.y), n_tiles);
-  DGPP_CUDA_OK(launch_early(swiglu_kernel, grid, block, 0, st, static_cast<const bf16*>(gate_up), static_cast<bf16*>(out), inter, limit, alpha,
+  DGPP_CUDA_OK(launch_early(swiglu_kernel<false>, grid, block, 0, st, static_cast<const bf16*>(gate_up), static_cast<bf16*>(out), inter, limit, alpha,
                                         static_cast<const int32_t*>(tiles), bn, nullptr, 0));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
