@@ -7,7 +7,7 @@
 //     FP8 e4m3 with one fp32 scale per (token, kv head) = amax / 448, or plain bf16.
 // A warp has one or more neighbouring heads of a row: their angles are the same, so sines and cosines (full range reduction, most of
 // a head's instructions) are taken once, and the heads' loads are in flight together.  head_dim is 64, 128 or 256.
-// 2048 rows x 56 heads of 128: 35 us with a warp per head, 25 so.
+// 2048 rows x 56 heads of 128: 30.5 us with a warp per head, 19.5 so.
 // (operator family: src/kernels/qsa.cu:104-252 norm_rope / kv_append(_fp8) of the reference)
 #include "common/common.h"
 #include "common/dtypes.cuh"
@@ -42,36 +42,44 @@ __global__ void __launch_bounds__(128) rope_kv_kernel(RopeKvParams p) {
   const int lane = threadIdx.x & 31;
   const int heads = p.hq + 2 * p.hkv, per_warp = U == 1 ? 1 : p.heads_per_warp, per_row = (heads + per_warp - 1) / per_warp;
   if (warp >= p.rows * per_row) return;
-  const int row = warp / per_row, h_begin = warp % per_row * per_warp, h_end = min(heads, h_begin + per_warp);
+  const int row = warp / per_row, h_begin = warp % per_row * per_warp;
+  const int h_end = U == 1 ? h_begin + 1 : min(heads, h_begin + per_warp);
   bf16* src = p.qkv + static_cast<size_t>(row) * heads * D;
-  const int pos = p.positions[row];
-  const int half = p.rot_dim / 2;
-  float sn[PER], cs[PER];      // whole rotary: of elements j < PER / 2 (j + PER / 2 is the partner); partial: of every element
-  if (h_begin < p.hq + p.hkv) {
-    if (p.rot_dim == D) {
-#pragma unroll
-      for (int j = 0; j < PER / 2; ++j) sincosf(static_cast<float>(pos) * p.inv_freq[lane + 32 * j], &sn[j], &cs[j]);
-    } else {
-#pragma unroll
-      for (int j = 0; j < PER; ++j) {
-        const int a = lane + 32 * j;
-        if (a < p.rot_dim) sincosf(static_cast<float>(pos) * p.inv_freq[a < half ? a : a - half], &sn[j], &cs[j]);
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      sn[j] *= p.mscale;
-      cs[j] *= p.mscale;
-    }
-  }
-  for (int h0 = h_begin; h0 < h_end; h0 += U) {
-    bf16 in[U][PER];
+  bf16 in[U][PER];
+  auto request = [&](int h0) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (h0 + u >= h_end) break;
 #pragma unroll
       for (int j = 0; j < PER; ++j) in[u][j] = src[(h0 + u) * D + lane + 32 * j];
     }
+  };
+  if (U == 1) request(h_begin);      // on its way while the angles are taken (four heads' registers cost more than that gives)
+  const int pos = p.positions[row];
+  const int half = p.rot_dim / 2;
+  float sn[PER], cs[PER];      // whole rotary: of elements j < PER / 2 (j + PER / 2 is the partner); partial: of every element
+  if (h_begin < p.hq + p.hkv) {
+    if (p.rot_dim == D) {
+#pragma unroll
+      for (int j = 0; j < PER / 2; ++j) {
+        sincosf(static_cast<float>(pos) * p.inv_freq[lane + 32 * j], &sn[j], &cs[j]);
+        sn[j] *= p.mscale;
+        cs[j] *= p.mscale;
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < PER; ++j) {
+        const int a = lane + 32 * j;
+        if (a < p.rot_dim) {
+          sincosf(static_cast<float>(pos) * p.inv_freq[a < half ? a : a - half], &sn[j], &cs[j]);
+          sn[j] *= p.mscale;
+          cs[j] *= p.mscale;
+        }
+      }
+    }
+  }
+  for (int h0 = h_begin; h0 < h_end; h0 += U) {
+    if (U > 1) request(h0);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int head = h0 + u;
@@ -183,7 +191,10 @@ DGPP_API int dgpp_rope_kv_write(void* qkv, const void* positions, const void* ro
   p.v_scale = static_cast<float*>(v_scale);
   p.rows = rows; p.hq = hq; p.hkv = hkv; p.d = d; p.rot_dim = rot_dim; p.page = page; p.max_blocks = max_blocks;
   p.mscale = mscale; p.eps = eps; p.kv_fp8 = kv_fp8; p.norm_one_plus_w = norm_one_plus_w;
-  // several heads per warp only where that leaves warps enough (32 per SM) to hide what a head waits for
+  // Several heads per warp only where that leaves warps enough to hide what a head waits for: `share` heads for each of the 32 warps
+  // that an SM holds.  Heads of 64 columns are nearly all sines and gain first, those of 256 have loads enough in flight at eight.
+  // (us with 1 / 4 / 8 / 16 heads per warp: 56 heads of 128, 384 rows 6.6 / 6.8 / 7.6 / 9.0, 768 rows 11.9 / 10.0 / 11.1 / 10.1, 2048 rows 30.5 /
+  // 21.1 / 20.9 / 19.5; 20 of 256, 1024 rows 8.5 / 8.8 / 7.0 / 8.0; 10 of 64, 1500 rows 4.7 / 3.8 / 3.9 / 5.1.)
   static int sms = 0;
   if (!sms) {
     int dev = 0;
@@ -192,7 +203,8 @@ DGPP_API int dgpp_rope_kv_write(void* qkv, const void* positions, const void* ro
   }
   const int heads = hq + 2 * hkv;
   const int64_t share = static_cast<int64_t>(rows) * heads / (32 * sms);
-  p.heads_per_warp = static_cast<int>(share < 1 ? 1 : (share > 16 ? 16 : share));
+  if (d == 256) p.heads_per_warp = share < 4 ? 1 : 8;
+  else p.heads_per_warp = share < (d == 64 ? 3 : 6) ? 1 : share < (d == 64 ? 8 : 12) ? 4 : share < 16 ? 8 : 16;
   const int blocks = dgpp_ceil_div(rows * dgpp_ceil_div(heads, p.heads_per_warp), 4);
   const bool one = p.heads_per_warp == 1;
   auto kern = d == 64 ? (one ? rope_kv_kernel<64, 1> : rope_kv_kernel<64, 4>)
