@@ -158,10 +158,9 @@ __global__ void __launch_bounds__(128) moe_gather_rows_kernel(const bf16* __rest
   for (int i = threadIdx.x; i < H / 8; i += blockDim.x) dst[i] = src[i];
 }
 
-// grid (ceil(H / 8 / 256), T).  Memory bound; four of a token's rows are in flight per thread (2048 tokens of 8 rows of 4096: 34 us with one, 30
-// so).
-constexpr int kCombineRowsBatch = 4;
-
+// grid (ceil(H / 8 / 256), T).  Memory bound; B of a token's rows are in flight per thread, four where there are three or more (2048 tokens of
+// 8 rows of 4096: 31.8 us with one, 27.7 so), otherwise as many as there are (2 rows of 4096: 8.1 us with two, 9.2 with four; one: 6.8 / 8.0).
+template <int B>
 __global__ void __launch_bounds__(256) moe_combine_rows_kernel(const bf16* __restrict__ y, const bf16* __restrict__ shared,
                                                                const int32_t* __restrict__ pair_row, const float* __restrict__ w,
                                                                bf16* __restrict__ out, int H, int k) {
@@ -174,20 +173,20 @@ __global__ void __launch_bounds__(256) moe_combine_rows_kernel(const bf16* __res
   float acc[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-  for (int i0 = 0; i0 < k; i0 += kCombineRowsBatch) {
-    int row[kCombineRowsBatch];
-    float wi[kCombineRowsBatch];
-    Pack16 p[kCombineRowsBatch];
+  for (int i0 = 0; i0 < k; i0 += B) {
+    int row[B];
+    float wi[B];
+    Pack16 p[B];
 #pragma unroll
-    for (int i = 0; i < kCombineRowsBatch; ++i) {
+    for (int i = 0; i < B; ++i) {
       row[i] = i0 + i < k ? pair_row[t * k + i0 + i] : -1;
       wi[i] = i0 + i < k ? w[t * k + i0 + i] : 0.f;
     }
 #pragma unroll
-    for (int i = 0; i < kCombineRowsBatch; ++i)
+    for (int i = 0; i < B; ++i)
       if (row[i] >= 0) p[i].u = *reinterpret_cast<const uint4*>(y + static_cast<size_t>(row[i]) * H + v * 8);
 #pragma unroll
-    for (int i = 0; i < kCombineRowsBatch; ++i) {
+    for (int i = 0; i < B; ++i) {
       if (row[i] < 0) continue;
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[j] = fmaf(wi[i], bf16_to_f32(p[i].h[j]), acc[j]);
@@ -262,7 +261,8 @@ DGPP_API int dgpp_moe_combine_rows(const void* y, const void* shared, const void
   DGPP_REQUIRE(H % 8 == 0, "moe_combine_rows: hidden %d must be a multiple of 8", H);
   if (T == 0) return 0;
   dim3 grid(dgpp_ceil_div(H / 8, 256), T);
-  DGPP_CUDA_OK(launch_early(moe_combine_rows_kernel, grid, 256, 0, st, static_cast<const bf16*>(y), static_cast<const bf16*>(shared),
+  auto kern = k >= 3 ? moe_combine_rows_kernel<4> : k == 2 ? moe_combine_rows_kernel<2> : moe_combine_rows_kernel<1>;
+  DGPP_CUDA_OK(launch_early(kern, grid, 256, 0, st, static_cast<const bf16*>(y), static_cast<const bf16*>(shared),
                                                 static_cast<const int32_t*>(pair_row), static_cast<const float*>(w),
                                                 static_cast<bf16*>(out), H, k));
   DGPP_CUDA_OK(cudaGetLastError());
