@@ -87,6 +87,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
+  constexpr int kHeads2 = G <= 1 ? 1 : G <= 2 ? 2 : G <= 4 ? 4 : 8;      // heads' values reduced together
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kvh = blockIdx.x, split = blockIdx.y, row = blockIdx.z;
   const int req = p.row_req[row];
@@ -138,8 +139,9 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
 #pragma unroll
       for (int hf = 0; hf < NH; ++hf) qv[hf][h] = bf16_to_f32(p.q[static_cast<size_t>(row) * p.q_stride + (kvh * G + h) * D + hf * 128 + d]);
   }
-  // The first tiles are on their way and their token scales requested while q is staged: warp 0 looks up all of their pages at once (at
-  // most 3 x 8), its first lane, which made the barriers, issues.  (Looked up one by one behind the staging: 17.4 us at 8 rows of 40 / 8 heads
+  // The first tile is on its way and its token scales requested while q is staged: warp 0 looks up its pages at once (at most 8),
+  // its first lane, which made the barriers, issues; the other stages' tiles follow behind the staging, which waits for warp 0 (requested
+  // in front of it as well: 11.3 us at a row of 32 / 32 heads over 2048 in four splits, 10.3 so).  (Looked up one by one behind the staging: 17.4 us at 8 rows of 40 / 8 heads
   // over 2048, 16.4 so; 8 rows of 16 / 2 heads of 256: 14.1, 12.6 so; a row over 64 positions 7.7, 7.2 so.)
   const int ppt = kAdTile / p.page;  // pages per tile
   auto page_block = [&](int tile, int pg) {
@@ -154,15 +156,12 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       tma_load_2d(sV + s * kStage + hf * kHalf + pg * p.page * 128, &tmV, hf * 128, r0, &kv_full[s]);
     }
   };
-  if (warp == 0) {
-    const int pages = min(ntiles, kAdStages) * ppt;
-    const int mine = lane < pages ? page_block(lane / ppt, lane % ppt) : 0;
-    for (int i = 0; i < pages; ++i) {
+  if (warp == 0 && ntiles > 0) {
+    const int mine = lane < ppt ? page_block(0, lane) : 0;
+    if (lane == 0) mbar_expect_tx(&kv_full[0], 2 * kStage);
+    for (int i = 0; i < ppt; ++i) {
       const int blk = __shfl_sync(0xffffffffu, mine, i);
-      if (lane == 0) {
-        if (i % ppt == 0) mbar_expect_tx(&kv_full[i / ppt], 2 * kStage);
-        load_page(i / ppt, i % ppt, blk);
-      }
+      if (lane == 0) load_page(0, i, blk);
     }
     __syncwarp();
   }
@@ -181,11 +180,11 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   // ---- quantise q of this kv head's G query heads into two e4m3 terms (B operand of MMA1)
   float q_scale[G];
   if (warp >= 2) {
-    float a[8];
+    float a[kHeads2];
 #pragma unroll
-    for (int h = 0; h < 8; ++h) a[h] = h < G ? (NH == 2 ? fmaxf(fabsf(qv[0][h < G ? h : 0]), fabsf(qv[NH - 1][h < G ? h : 0])) : fabsf(qv[0][h < G ? h : 0])) : 0.f;
+    for (int h = 0; h < kHeads2; ++h) a[h] = h < G ? (NH == 2 ? fmaxf(fabsf(qv[0][h < G ? h : 0]), fabsf(qv[NH - 1][h < G ? h : 0])) : fabsf(qv[0][h < G ? h : 0])) : 0.f;
     const float m = over_lanes<true>(a, lane);
-    if ((lane & 3) == 0) redl[(warp - 2) * 8 + (lane >> 2)] = m;
+    if (lane % (32 / kHeads2) == 0) redl[(warp - 2) * 8 + lane / (32 / kHeads2)] = m;
   }
   __syncthreads();
   if (warp >= 2) {
@@ -222,7 +221,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (elect_one()) {
-      for (int i = kAdStages; i < ntiles; ++i) {
+      for (int i = 1; i < ntiles; ++i) {
         const int s = i % kAdStages;
         if (!wait_bar(&kv_empty[s], ((i / kAdStages) & 1) ^ 1)) { report(p.status, kTimeoutStageEmpty, 21); *abort_flag = 1; break; }
         mbar_expect_tx(&kv_full[s], 2 * kStage);
@@ -322,17 +321,29 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       }
       // maxima of the scores (rp[0 .. G)) and of the V scales (rp[8]) over the warp's tokens
       {
-        float a[8];
-#pragma unroll
-        for (int h = 0; h < 8; ++h) a[h] = h < G ? s[h < G ? h : 0] : vs;
-        const float m = over_lanes<true>(a, lane);
-        if ((lane & 3) == 0) rp[lane >> 2] = m;
         float vm = vs;
-        if (G == 8) {
+        if (G <= 2 || G == 8) {
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, o));
+        }
+        if constexpr (G <= 2) {      // (few chains: latency counts, not the number of shuffles)
+          float a[G];
+#pragma unroll
+          for (int h = 0; h < G; ++h) a[h] = s[h];
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int h = 0; h < G; ++h) a[h] = fmaxf(a[h], __shfl_xor_sync(0xffffffffu, a[h], o));
+#pragma unroll
+          for (int h = 0; h < G; ++h)
+            if (lane == h) rp[h] = a[h];
         } else {
-          vm = m;
+          float a[8];
+#pragma unroll
+          for (int h = 0; h < 8; ++h) a[h] = h < G ? s[h < G ? h : 0] : vs;
+          const float m = over_lanes<true>(a, lane);
+          if ((lane & 3) == 0) rp[lane >> 2] = m;
+          if (G < 8) vm = m;
         }
         if (lane == 31) rp[8] = vm;      // (lane 31 holds the last of the eight)
         if (lane == 0) rp[11] = (okw && !*abort_flag) ? 0.f : 1.f;
@@ -414,11 +425,11 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     // total probability mass per head: sum the per-thread partials
     asm volatile("bar.sync 1, 128;" ::: "memory");
     {
-      float l[8];
+      float l[kHeads2];
 #pragma unroll
-      for (int h = 0; h < 8; ++h) l[h] = h < G ? l_thr[h < G ? h : 0] : 0.f;
+      for (int h = 0; h < kHeads2; ++h) l[h] = h < G ? l_thr[h < G ? h : 0] : 0.f;
       const float sum = over_lanes<false>(l, lane);
-      if ((lane & 3) == 0) redl[wslot * 8 + (lane >> 2)] = sum;
+      if (lane % (32 / kHeads2) == 0) redl[wslot * 8 + lane / (32 / kHeads2)] = sum;
     }
     asm volatile("bar.sync 1, 128;" ::: "memory");
 #pragma unroll
