@@ -26,6 +26,7 @@ namespace dgpp {
 
 constexpr int kAqMaxThreads = 512;
 constexpr int kAqNormThreads = 128;   // of the norm's rows: who adds which squares is part of the per-layer kernel's contract
+constexpr int kAqNormWarps = kAqNormThreads / 32;
 constexpr int kAqMaxWarps = kAqMaxThreads / 32;
 constexpr int kAqMaxCluster = 8;
 constexpr int kAqSplitBlock = 4;      // attention splits whose partials are in flight at once
@@ -121,6 +122,27 @@ __device__ __forceinline__ void swiglu8(const ClusterQuantArgs& a, Pack16& x, co
   }
 }
 
+// Eight columns of a row to be normed: their squares, and the largest |x w|.
+__device__ __forceinline__ void norm_statistics(const ClusterQuantArgs& a, const Pack16& x, const Pack16& w, float& ss, float& amax) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float f = bf16_to_f32(x.h[j]);
+    ss += f * f;
+    float gw = bf16_to_f32(w.h[j]);
+    if (a.one_plus_w) gw += 1.f;
+    amax = fmaxf(amax, fabsf(f * gw));
+  }
+}
+__device__ __forceinline__ void norm_scale(const ClusterQuantArgs& a, Pack16& x, const Pack16& w, float rstd) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float nrm = bf16_to_f32(f32_to_bf16(bf16_to_f32(x.h[j]) * rstd));
+    float gw = bf16_to_f32(w.h[j]);
+    if (a.one_plus_w) gw += 1.f;
+    x.h[j] = f32_to_bf16(nrm * gw);
+  }
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(kAqMaxThreads) act_quant_cluster_kernel(ClusterQuantArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -184,14 +206,7 @@ __global__ void __launch_bounds__(kAqMaxThreads) act_quant_cluster_kernel(Cluste
       }
       Pack16 w;
       w.u = i == tid ? w0.u : wv[i];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float f = bf16_to_f32(x.h[j]);
-        ss += f * f;
-        float gw = bf16_to_f32(w.h[j]);
-        if (a.one_plus_w) gw += 1.f;
-        amax = fmaxf(amax, fabsf(f * gw));
-      }
+      norm_statistics(a, x, w, ss, amax);
     } else {
       if (MODE == 3) {
         float acc[8], ll;
@@ -259,13 +274,7 @@ __global__ void __launch_bounds__(kAqMaxThreads) act_quant_cluster_kernel(Cluste
     if (MODE == 2 && on) {
       Pack16 w;
       w.u = i0 == 0 ? w0.u : wv[i];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float nrm = bf16_to_f32(f32_to_bf16(bf16_to_f32(x.h[j]) * rstd));
-        float gw = bf16_to_f32(w.h[j]);
-        if (a.one_plus_w) gw += 1.f;
-        x.h[j] = f32_to_bf16(nrm * gw);
-      }
+      norm_scale(a, x, w, rstd);
       if (a.x_out) reinterpret_cast<uint4*>(a.x_out + static_cast<size_t>(t) * K + k0)[i] = x.u;
     }
     float res[8];
@@ -308,15 +317,20 @@ __global__ void __launch_bounds__(kAqMaxThreads) act_quant_cluster_kernel(Cluste
   }
 }
 
-// Bulk rows (rows fill the SMs by themselves): one CTA of 128 threads per row, a thread per block of 16.  Plain rows and swiglu only:
-// their row statistic is a maximum, so the results are the cluster form's bit for bit.  Bound by issue slots rather than latency
-// there: no exchange, no mbarrier, no shuffles per term and 8-byte stores of codes.  2048 x 5120, three terms, plain / swiglu:
-// cluster form of one CTA 41.0 / 49.2 us, so 16.3 / 25.1; 128 rows 5.7 / 6.7 and 4.6 / 7.0.
+// Bulk rows (rows fill the SMs by themselves): one CTA of 128 threads per row, a thread per block of 16.  The results are the cluster
+// form's bit for bit: a maximum does not depend on its order, and the norm's squares are added as the warps of a cluster of `cl` CTAs
+// would add them, whose places this CTA's warps take in turns.  Bound by issue slots rather than latency there: no exchange, no
+// mbarrier, no shuffles per term and 8-byte stores of codes.  2048 x 5120, three terms, plain / swiglu: cluster form of one CTA 41.0 /
+// 49.2 us, so 16.3 / 25.1; 128 rows 5.7 / 6.7 and 4.6 / 7.0.  2048 normed rows of 5120 against
+// eight CTAs each: 75.6 us, 28.7 so.
 constexpr int kAqBulkThreads = 128;
+// Normed rows beyond this many (us, this form / a cluster of eight: 2048 columns 128 rows 3.9 / 4.7; 5120 columns 128 rows 7.7 / 6.8, 173
+// rows 8.6 / 10.0; 17408 columns 173 rows 20.7 / 17.9, 256 rows 20.9 / 23.0).
+static int bulk_norm_rows(int K) { return K <= 2048 ? 64 : K <= 6144 ? 160 : 255; }
 
 template <int MODE>
 __global__ void __launch_bounds__(kAqBulkThreads) act_quant_bulk_kernel(ClusterQuantArgs a) {
-  static_assert(MODE == 0 || MODE == 1, "rows whose statistic is a maximum");
+  static_assert(MODE >= 0 && MODE <= 2, "plain, swiglu or normed rows");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint4* row = reinterpret_cast<uint4*>(smem_raw);
   __shared__ float wmax[kAqBulkThreads / 32];
@@ -324,8 +338,44 @@ __global__ void __launch_bounds__(kAqBulkThreads) act_quant_bulk_kernel(ClusterQ
   const int t = blockIdx.x, tid = threadIdx.x, K = a.K;
   if (a.group_list && (a.group_list[t / a.bn] < 0 || t % a.bn >= a.group_rows)) return;
   const uint4* rr = reinterpret_cast<const uint4*>(a.in + static_cast<size_t>(t) * a.in_stride);
-  float amax = 0.f;
-  for (int i = tid; i < K / 8; i += kAqBulkThreads) {
+  const uint4* wv = reinterpret_cast<const uint4*>(a.w);
+  float amax = 0.f, rstd = 0.f;
+  if (MODE == 2) {
+    __shared__ __align__(16) float squares[kAqMaxCluster * kAqNormWarps];
+    const int lane = tid & 31, nvec = K / a.cl / 8, warps = nvec < kAqNormThreads ? (nvec + 31) / 32 : kAqNormWarps;
+    for (int vw = tid >> 5; vw < a.cl * warps; vw += kAqBulkThreads / 32) {      // warp vw % warps of CTA vw / warps
+      const int c = vw / warps;
+      float ss = 0.f;
+      for (int i = (vw - c * warps) * 32 + lane; i < nvec; i += warps * 32) {
+        const int at = c * nvec + i;
+        Pack16 x, w;
+        x.u = rr[at];
+        w.u = wv[at];
+        if (a.delta) {
+          Pack16 d;
+          d.u = reinterpret_cast<const uint4*>(a.delta + static_cast<size_t>(t) * K)[at];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) x.h[j] = f32_to_bf16(bf16_to_f32(x.h[j]) + bf16_to_f32(d.h[j]));
+          reinterpret_cast<uint4*>(a.resid_out + static_cast<size_t>(t) * K)[at] = x.u;
+        }
+        norm_statistics(a, x, w, ss, amax);
+        row[at] = x.u;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      if (lane == 0) squares[c * kAqNormWarps + (vw - c * warps)] = ss;
+    }
+    if (tid < kAqMaxCluster * kAqNormWarps && (tid / kAqNormWarps >= a.cl || tid % kAqNormWarps >= warps)) squares[tid] = 0.f;
+    __syncthreads();
+    float ss = 0.f;
+#pragma unroll
+    for (int c = 0; c < kAqMaxCluster; ++c) {
+      const float4 s4 = reinterpret_cast<const float4*>(squares)[c];
+      ss += s4.x + s4.y + s4.z + s4.w;
+    }
+    rstd = rsqrtf(ss / static_cast<float>(K) + a.eps);
+  }
+  for (int i = tid; MODE != 2 && i < K / 8; i += kAqBulkThreads) {
     Pack16 x;
     x.u = rr[i];
     if (MODE == 1) {
@@ -344,6 +394,7 @@ __global__ void __launch_bounds__(kAqBulkThreads) act_quant_bulk_kernel(ClusterQ
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < kAqBulkThreads / 32; ++i) amax = fmaxf(amax, wmax[i]);
+  if (MODE == 2) amax = amax * rstd * 1.0079f;      // (a bound, as in the cluster form)
   const float gs = amax > 0.f ? amax / (6.f * 256.f) : 1.f;
   if (tid == 0) a.g[t] = gs;
   const float inv_g = 1.f / gs;
@@ -352,6 +403,18 @@ __global__ void __launch_bounds__(kAqBulkThreads) act_quant_bulk_kernel(ClusterQ
     Pack16 lo, hi;
     lo.u = row[gi * 2];
     hi.u = row[gi * 2 + 1];
+    if (MODE == 2) {
+      Pack16 w[2];
+      w[0].u = wv[gi * 2];
+      w[1].u = wv[gi * 2 + 1];
+      norm_scale(a, lo, w[0], rstd);
+      norm_scale(a, hi, w[1], rstd);
+      if (a.x_out) {
+        uint4* xo = reinterpret_cast<uint4*>(a.x_out + static_cast<size_t>(t) * K);
+        xo[gi * 2] = lo.u;
+        xo[gi * 2 + 1] = hi.u;
+      }
+    }
     float res[16];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -453,9 +516,9 @@ DGPP_API int dgpp_act_quant_nvfp4_cluster(int mode, const void* in, int64_t in_s
     a.fold = 1;
     a.comm = c->st;
   }
-  if (cl == 1 && (mode == 0 || mode == 1)) {
-    const size_t smem = static_cast<size_t>(K) * 2;
-    auto kern = mode == 0 ? act_quant_bulk_kernel<0> : act_quant_bulk_kernel<1>;
+  const size_t smem = static_cast<size_t>(K) * 2;
+  if ((cl == 1 && (mode == 0 || mode == 1)) || (mode == 2 && !a.fold && T > bulk_norm_rows(K) && smem <= kAqMaxSegment)) {
+    auto kern = mode == 0 ? act_quant_bulk_kernel<0> : mode == 1 ? act_quant_bulk_kernel<1> : act_quant_bulk_kernel<2>;
     if (allow_segment(kern, smem)) return -1;
     kern<<<T, kAqBulkThreads, smem, st>>>(a);
     DGPP_CUDA_OK(cudaGetLastError());
