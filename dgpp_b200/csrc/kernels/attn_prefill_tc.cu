@@ -23,7 +23,7 @@
 // 16 TMA producer, 17 MMA issuer and TMEM owner.
 // What bounds it: MUFU and tensor pipe alike (a tile of two units: 2048 cycles each), then the handshakes between them.
 // 40 query and 8 KV heads, with two e4m3 terms of q and P, one unit per CTA and the accumulator in registers / so: 173 rows behind 3000
-// 92 / 64 us, 2048 rows 172 / 113, 2048 rows behind 6144 944 / 550 (the scales' mantissas, powers of two and zero rows are 5 % of that).
+// 92 / 64 us, 2048 rows 172 / 112, 2048 rows behind 6144 944 / 547 (the scales' mantissas, powers of two and zero rows are 5 % of that).
 // (reference counterparts: src/kernels/full_attn.cu:442,679,983 tile / TMA / fp8-compute prefill kernels.)
 #include <cuda.h>
 #include <math.h>
@@ -204,7 +204,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
-  __syncthreads();      // the columns are this CTA's before the next grid is let in
+  tc_fence_before();
+  __syncthreads();      // the barriers are there, and the columns this CTA's before the next grid is let in
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;      // score buffers at columns 0 and 128, accumulators at 256 and 384
   pdl_wait();
   // ---- the units' query rows as f16 (thread = row): scaled by a power of two to a largest magnitude of 128..256
   const int sub = warp >> 2;
@@ -215,33 +218,30 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     const uint4* src = reinterpret_cast<const uint4*>(p.q + static_cast<size_t>(row) * p.q_stride + head * D);
     const bool live = row < p.T;
     float amax = 0.f;
+    Pack16 x[D / 8];
 #pragma unroll
-    for (int c = 0; c < D / 8; ++c) {
-      Pack16 x;
-      x.u = live ? src[c] : make_uint4(0u, 0u, 0u, 0u);
+    for (int c = 0; c < D / 8; ++c) x[c].u = live ? src[c] : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(bf16_to_f32(x.h[j])));
-    }
+    for (int c = 0; c < D / 8; ++c)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(bf16_to_f32(x[c].h[j])));
     const int e = max(static_cast<int>((__float_as_uint(amax) >> 23) & 255u), 8);      // biased exponent of the largest
     const float mul = __uint_as_float(static_cast<uint32_t>(261 - e) << 23);
     q_scale = __uint_as_float(static_cast<uint32_t>(e - 7) << 23);
 #pragma unroll
     for (int c = 0; c < D / 8; ++c) {
-      Pack16 x, y;
-      x.u = live ? src[c] : make_uint4(0u, 0u, 0u, 0u);
+      Pack16 y;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const __half2 h = __floats2half2_rn(bf16_to_f32(x.h[2 * j]) * mul, bf16_to_f32(x.h[2 * j + 1]) * mul);
+        const __half2 h = __floats2half2_rn(bf16_to_f32(x[c].h[2 * j]) * mul, bf16_to_f32(x[c].h[2 * j + 1]) * mul);
         y.w[j] = *reinterpret_cast<const uint32_t*>(&h);
       }
       *reinterpret_cast<uint4*>(sQ + sub * kApF16Bytes + (c >> 3) * kApBlk + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = y.u;
     }
     fence_proxy_async_smem();
   }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;      // score buffers at columns 0 and 128, accumulators at 256 and 384
+  // (K and V are on their way and being expanded meanwhile: only the softmax warps and the MMA issuer meet here)
+  if (warp < kApConv || warp == kApMma) asm volatile("bar.sync 3, 288;" ::: "memory");
 
   if (warp == kApTma) {
     // ------------------------------------------------------------------ TMA producer: K0, V0, K1, V1, ...
@@ -480,6 +480,28 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
   if (warp == kApMma) tmem_dealloc(tmem_base, 512);
 }
 
+// Two units per CTA share an expanded tile and fill each other's waits: 3.4 us per tile against 2.3 for one alone, behind 8 us for a
+// CTA's first and last steps.  One each is the shorter span where units are fewer than SMs, and up to twice as many where the second
+// wave's, the short ones, fit behind the first one's last: unit sms + i follows unit sms - 1 - i.  (us, one / two per CTA: 40 heads
+// over 512 rows 28.3 / 31.1, behind 5000 more 191 / 151; 32 heads over 768 rows 33.6 / 38.4; 64 over 512 35.0 / 31.2; 8 over 4096 83 / 114.)
+static int units_per_cta(const AttnPrefillParams& p, int sms) {
+  const int64_t all = static_cast<int64_t>(p.units) * p.hkv;
+  if (all <= sms) return 1;
+  if (all > 2 * sms) return 2;
+  const int row_tiles = dgpp_ceil_div(p.T, kApTile);
+  auto tiles = [&](int u) {      // of the u-th longest unit
+    const int row = (row_tiles - 1 - u / p.hq) * kApTile, low = p.pos0 + row;
+    const int first = p.window > 0 && low + 1 > p.window ? low + 1 - p.window : 0;
+    return (p.pos0 + (row + kApTile < p.T ? row + kApTile : p.T) - 1) / kApTile - first / kApTile + 1;
+  };
+  double one = 8 + 2.3 * tiles(0);
+  for (int i = 0; i < all - sms; ++i) {
+    const double two_waves = 16 + 2.3 * (tiles(sms - 1 - i) + tiles(sms + i));
+    if (two_waves > one) one = two_waves;
+  }
+  return one <= 8.5 + 3.4 * tiles(0) ? 1 : 2;
+}
+
 }  // namespace dgpp
 
 using namespace dgpp;
@@ -522,9 +544,8 @@ DGPP_API int dgpp_attn_prefill_tc(const void* q, int64_t q_stride, const void* k
                                       static_cast<int>(smem)));
     attr = true;
   }
-  // Two units per CTA share an expanded tile and fill each other's waits; where units are fewer than SMs, one each is the shorter span.
   p.units = hq / hkv * dgpp_ceil_div(T, kApTile);
-  p.per_cta = static_cast<int64_t>(p.units) * hkv <= sms ? 1 : 2;
+  p.per_cta = units_per_cta(p, sms);
   DGPP_CUDA_OK(launch_early(attn_prefill_tc_kernel, hkv * dgpp_ceil_div(p.units, p.per_cta), kApThreads, smem, st, tK, tV, p));
   DGPP_CUDA_OK(cudaGetLastError());
   return 0;
