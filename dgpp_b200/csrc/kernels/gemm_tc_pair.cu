@@ -525,7 +525,9 @@ static int pair_slots(int* slots) {
 // 32 tokens of a tile (their fold is s round trips to L2).  Fitted to six shapes of 4096 x 2048 to 34816 x 5120 at 129 to 2048 rows with every
 // tile: what they choose is within 0.2 % of the best on average, 4 % at most (34816 x 5120 at 953 rows: 276 us at 256 tokens, which 400 + 1.2 bn
 // chose, 230 at 192).
-// Up to 128 rows the splits are those of 128 rows, above there are none: on either side of that line a row's bits do not depend
+// Up to 128 rows the splits are those of 128 rows (seven shapes of 512 x 512 to 34816 x 5120 at 8, 37, 64 and 128 rows against every tile
+// and split count: within 4 % of the best, but for 2560 x 8192 at 8 rows, 15.8 us, 14.7 in six splits instead of three, and
+// 4096 x 2048 at 128, 12.8, 11.5 without splits), above there are none: on either side of that line a row's bits do not depend
 // on how many others share its pass, and prompt products touch no workspace, so that products on several streams share
 // nothing.  (A long K over few tiles pays for that: 173 x 5120 x 17408 79 us, 47 in three splits.)
 constexpr int kPrSplitRows = 128;
