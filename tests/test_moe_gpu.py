@@ -224,3 +224,22 @@ def test_moe_prefill_path_matches_the_expert_loop(dev, rows, shared, terms, tol)
     ids, wts = ops.moe_route(x[:9], w.gate, w.bias, cfg.top_k, cfg.n_group, cfg.topk_group, False, True, 1.5)
     want = moe_reference(x[:9], w, ids=ids.long(), wts=wts)
     assert (got[:9].float() - want.float()).abs().max().item() <= tol * want.float().abs().max().item() + 2e-3
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 6, 9])
+def test_combine_of_rows_for_every_count_in_flight(dev, k):
+    """One, two and four rows in flight with remainders, missing pairs among them: a 32-bit sum in the choices' order, once
+    rounded to bf16."""
+    from dgpp_b200.ops import core as ops
+
+    torch.manual_seed(k)
+    T, H = 37, 264
+    y, sh = torch.randn(200, H, device=dev).to(BF), torch.randn(T, H, device=dev).to(BF)
+    rows = torch.randperm(200, device=dev)[:T * k % 190].repeat(k * T)[:T * k].to(torch.int32)
+    rows[::5] = -1
+    w = torch.rand(T, k, device=dev)
+    out = ops.moe_combine_rows(y, sh, rows, w, torch.empty(T, H, dtype=BF, device=dev))
+    torch.cuda.synchronize()
+    picked = y[rows.clamp_min(0).long()].double() * (rows >= 0).unsqueeze(1)
+    want = (picked.view(T, k, H) * w.double().unsqueeze(-1)).sum(1) + sh.double()
+    assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()

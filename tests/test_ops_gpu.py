@@ -558,3 +558,27 @@ def test_swiglu_of_listed_rows_checks_its_arguments(dev):
     keep = torch.zeros(6, dtype=torch.bool, device=dev)
     keep[2] = True
     assert torch.equal(out[keep], ops.swiglu(gu)[keep]) and (out[~keep] == 7.0).all()
+
+
+@pytest.mark.parametrize("rows,d,hq,hkv", [(1410, 128, 41, 7), (1500, 64, 37, 7), (1100, 256, 19, 1)])
+def test_rope_of_sixteen_heads_per_warp(dev, rows, d, hq, hkv):
+    """The largest share of heads per warp, with remainders: the rows that passes of a few rows write."""
+    from dgpp_b200.engine.kv_cache import PagedKV
+    from dgpp_b200.ops import core as ops, reference as ref
+
+    torch.manual_seed(d)
+    inv_freq, _ = ref.rope_inv_freq(d, 1e4, dev)
+    x = torch.randn(rows, (hq + 2 * hkv) * d, device=dev).to(torch.bfloat16)
+    y = x.clone()
+    pos, req = torch.arange(rows, device=dev, dtype=torch.int32), torch.zeros(rows, device=dev, dtype=torch.int32)
+    kv = [PagedKV(1, hkv, d, rows // 64 + 4, 2, rows // 64 + 2, 64, True, dev) for _ in range(2)]
+    for c in kv:
+        assert c.reserve(0, rows)
+    ops.rope_kv_write(x, pos, req, kv[0].block_table, inv_freq, kv[0].layers[0], hq, hkv, d)
+    for i in range(0, rows, 30):
+        ops.rope_kv_write(y[i:i + 30], pos[i:i + 30], req[i:i + 30], kv[1].block_table, inv_freq, kv[1].layers[0], hq, hkv, d)
+    at = pos.long()
+    assert torch.equal(x, y)
+    for name in ("k", "v", "k_scale", "v_scale"):
+        a, b = (getattr(c.layers[0], name)[c.block_table[0].long()[at // 64], :, at % 64] for c in kv)
+        assert torch.equal(a, b), name

@@ -174,6 +174,32 @@ def test_quantiser_of_one_whole_row_per_cta(dev, m, k):
         assert ((a.dequant() - b.dequant()).norm() / b.dequant().norm()).item() < 2.0 ** -8
 
 
+@pytest.mark.parametrize("k,one_plus,with_delta", [(256, 0, True), (2048, 1, False), (5120, 0, True), (5888, 1, True), (8192, 0, True), (17408, 0, False)])
+def test_bulk_quantiser_of_normed_rows_matches_the_cluster_one(dev, k, one_plus, with_delta):
+    """Above the line one CTA per row, in passes of 64 rows a cluster each: the same codes, scales, normed rows and sums, bit for
+    bit (segments of less than a warp, of no whole number of warps, and of several columns per thread)."""
+    from dgpp_b200.ops import core as ops
+
+    torch.manual_seed(37)
+    rows, terms, bn = 272, 2, 16
+    x, d = torch.randn(rows, k, device=dev).to(BF), torch.randn(rows, k, device=dev).to(BF)
+    x[5].zero_()
+    w = (0.1 * torch.randn(k, device=dev) + 1 - one_plus).to(BF)
+    args = dict(mode="rmsnorm", norm_w=w, one_plus_w=bool(one_plus))
+    got, xs, xn = ops.QuantAct(rows, k, terms, bn, dev), x.clone(), torch.empty_like(x)
+    ops.act_quant_nvfp4(xs, terms, out=got, x_out=xn, delta=d if with_delta else None, **args)
+    for r in range(0, rows, 64):
+        part = x[r:r + 64].clone()
+        want, n = ops.QuantAct(part.shape[0], k, terms, bn, dev), torch.empty_like(part)
+        ops.act_quant_nvfp4(part, terms, out=want, x_out=n, delta=d[r:r + 64] if with_delta else None, **args)
+        torch.cuda.synchronize()
+        ops.check_status()
+        at = slice(r, r + part.shape[0])
+        assert torch.equal(got.g[at], want.g) and torch.equal(xn[at], n) and torch.equal(xs[at], part)
+        assert torch.equal(got.q.view(rows, -1)[at], want.q.view(part.shape[0], -1))
+        assert torch.equal(got.sf.view(rows, -1)[at], want.sf.view(part.shape[0], -1))
+
+
 def _filled_cache(dev, hq, hkv, ctx, page, slot, d=128):
     from dgpp_b200.engine.kv_cache import PagedKV
     from dgpp_b200.ops import core as ops, reference as ref
