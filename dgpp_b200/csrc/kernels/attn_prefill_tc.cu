@@ -23,7 +23,7 @@
 // 16 TMA producer, 17 MMA issuer and TMEM owner.
 // What bounds it: MUFU and tensor pipe alike (a tile of two units: 2048 cycles each), then the handshakes between them.
 // 40 query and 8 KV heads, with two e4m3 terms of q and P, one unit per CTA and the accumulator in registers / so: 173 rows behind 3000
-// 92 / 64 us, 2048 rows 172 / 112, 2048 rows behind 6144 944 / 547 (the scales' mantissas, powers of two and zero rows are 5 % of that).
+// 92 / 61 us, 2048 rows 172 / 106, 2048 rows behind 6144 944 / 547 (the scales' mantissas, powers of two and zero rows are 5 % of that).
 // (reference counterparts: src/kernels/full_attn.cu:442,679,983 tile / TMA / fp8-compute prefill kernels.)
 #include <cuda.h>
 #include <math.h>
